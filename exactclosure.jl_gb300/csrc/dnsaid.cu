@@ -21,6 +21,7 @@
 #include "fields.cuh"
 #include "filter.cuh"
 #include "internal.cuh"
+#include "sepfilter.cuh"
 
 struct exc_dnsaid {
   int n = 0, m = 0, c = 0;
@@ -46,6 +47,8 @@ struct exc_dnsaid {
   double* pl = nullptr;    // LES pressure M (paper mode)
   double* dsig = nullptr;  // closure divergence 3M (paper mode)
   double* rc9 = nullptr;   // surface-filtered flux 9M (surface mode)
+  double* uf = nullptr;    // fine-filtered velocity at the classic closure's sample points 18M
+  exc::SepWork sep;        // scratch of the filters
   double t = 0;
   int steps = 0;
   bool started = false;
@@ -99,6 +102,24 @@ __global__ void sub_sym_kernel(long long M, double* __restrict__ r9, const doubl
     for (int k = 0; k < 9; ++k) r9[k * M + i] -= s6[map[k] * M + i];
 }
 
+// sigma2 of `step_ΔHπ_classic!` (src/N.jl:1143-1145) at the LES points from
+// the fine-filtered velocities uf (order of classic_targets): 2 values for
+// each diagonal component (s11, s22, s33), 4 for the others (s12, s23, s31).
+__global__ void classic_stress_kernel(long long M, const double* __restrict__ uf, double inv_h, double visc,
+                                      double* __restrict__ s6) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < M; i += (long long)gridDim.x * blockDim.x) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const double* f = uf + (k < 3 ? 2 * k : 6 + 4 * (k - 3)) * M + i;
+      const double uir = f[0], uil = f[M];
+      const double ujr = k < 3 ? uir : f[2 * M], ujl = k < 3 ? uil : f[3 * M];
+      const double etaj_ui = (uir + uil) / 2, etai_uj = (ujr + ujl) / 2;
+      const double dj_ui = (uir - uil) * inv_h, di_uj = (ujr - ujl) * inv_h;
+      s6[k * M + i] = etaj_ui * etai_uj - visc * (dj_ui + di_uj);
+    }
+  }
+}
+
 int gridsz(long long cnt) {
   long long b = (cnt + 255) / 256;
   return (int)(b < 152LL * 16 ? b : 152LL * 16);
@@ -136,10 +157,85 @@ int propose_dt(exc_dnsaid* d, double cfl, double* dt) {
   return EXC_OK;
 }
 
+int run_filters(exc_dnsaid* d, const SepTaps& taps, const std::vector<SepTarget>& targets) {
+  return sep_filter(&d->sep, d->n, d->c, 1.0 / (d->l / d->n), d->visc, taps, targets, d->u, d->p, d->st);
+}
+
+// Targets of the filtered velocity at the LES faces: volume filter, or face
+// average with `face`.
+void velocity_targets(exc_dnsaid* d, bool face, double* out, SepTaps& taps, std::vector<SepTarget>& v) {
+  const long long M = (long long)d->m * d->m * d->m;
+  for (int i = 0; i < 3; ++i) {
+    SepTarget t{SEP_U + i, -1, {}, out + i * M};
+    for (int a = 0; a < 3; ++a) t.t[a] = taps.add(d->c, a == i, face && a == i, fd(d), nfd(d));
+    v.push_back(t);
+  }
+}
+
+// The components of r = sigma(u) + p I (sigma alone without `with_p`) with
+// the boxes and point samples of the flux filters.
+enum FluxFilter {
+  FLUX_FACE,     // rDHi (src/N.jl:1038-1073): point along the derivative axis j
+  FLUX_VOLUME,   // sigmaDH (src/N.jl:1088-1115): boxes only, 6 components
+  FLUX_SURFACE,  // surfacefilter!(., true) (src/NavierStokes.jl:368): point along i, the axis of the velocity
+  FLUX_LINE      // linefilter! off the diagonal (src/NavierStokes.jl:386-394), FLUX_SURFACE on it
+};
+void flux_targets(exc_dnsaid* d, FluxFilter kind, bool with_p, double* out, SepTaps& taps, std::vector<SepTarget>& v) {
+  const long long M = (long long)d->m * d->m * d->m;
+  const int sym[3][3] = {{0, 3, 5}, {3, 1, 4}, {5, 4, 2}};
+  const int six[6][2] = {{0, 0}, {1, 1}, {2, 2}, {0, 1}, {1, 2}, {2, 0}};
+  const int count = kind == FLUX_VOLUME ? 6 : 9;
+  for (int k = 0; k < count; ++k) {
+    // 9 components in the order s11, s21, s31, s12, ... (src/N.jl:181)
+    const int i = kind == FLUX_VOLUME ? six[k][0] : k % 3, j = kind == FLUX_VOLUME ? six[k][1] : k / 3;
+    SepTarget t{SEP_SIGMA + sym[i][j], i == j && with_p ? (int)SEP_P : -1, {}, out + k * M};
+    for (int a = 0; a < 3; ++a) {
+      const bool stag = i != j && (a == i || a == j);
+      const bool point = kind == FLUX_FACE ? a == j : kind == FLUX_VOLUME ? false : a == i || (kind == FLUX_LINE && a == j);
+      t.t[a] = taps.add(d->c, stag, point, fd(d), nfd(d));
+    }
+    v.push_back(t);
+  }
+}
+
+// The fine-filtered velocities GDH u that the classic closure's sigma2 reads
+// at its LES centres and edges (src/N.jl:1117-1135, 1143-1145), in the order
+// classic_stress_kernel takes them; odd ratios only (the reference's top hat).
+// GDH is the centred box composed with the Gaussian: the taps of a centre
+// (stag false) moved to the sample point.
+void classic_targets(exc_dnsaid* d, double* out, SepTaps& taps, std::vector<SepTarget>& v) {
+  const long long M = (long long)d->m * d->m * d->m;
+  const int c = d->c, a = c / 2;
+  const int six[6][2] = {{0, 0}, {1, 1}, {2, 2}, {0, 1}, {1, 2}, {2, 0}};
+  auto add = [&](int comp, const int pos[3], int axis, int step) {
+    SepTarget t{SEP_U + comp, -1, {}, out + (long long)(v.size()) * M};
+    for (int q = 0; q < 3; ++q)
+      t.t[q] = taps.add(c, false, false, fd(d), nfd(d), pos[q] - a + (q == axis ? step : 0));
+    v.push_back(t);
+  };
+  for (const auto& ij : six) {
+    const int i = ij[0], j = ij[1];
+    int pos[3];
+    for (int q = 0; q < 3; ++q) pos[q] = i != j && (q == i || q == j) ? c - 1 : a;
+    if (i == j) {
+      add(i, pos, i, 0);
+      add(i, pos, i, -1);
+    } else {
+      add(i, pos, j, 1);
+      add(i, pos, j, 0);
+      add(j, pos, i, 1);
+      add(j, pos, i, 0);
+    }
+  }
+}
+
 // `apply_ΔHπ` (src/N.jl:1228-1237): volume filter, coarse-grain at the
 // faces, project on the LES grid.
 int apply_dhpi(exc_dnsaid* d, double* out) {
-  int rc = filter_vector<double>(d->n, d->c, EXC_FILTER_VOLUME, fd(d), nfd(d), d->u, out, d->st);
+  SepTaps taps;
+  std::vector<SepTarget> v;
+  velocity_targets(d, false, out, taps, v);
+  int rc = run_filters(d, taps, v);
   if (rc) return rc;
   return cuda_rc(project(&d->psl, out, d->st));
 }
@@ -168,7 +264,7 @@ int forward_euler(exc_dnsaid* d, exc_poisson* ps, int n, double h, double* v, do
 
 // One lockstep step (src/N.jl:1295-1320).
 int lockstep(exc_dnsaid* d, double dt) {
-  const int n = d->n, m = d->m, c = d->c;
+  const int n = d->n, m = d->m;
   const long long N3 = 3LL * n * n * n, M = (long long)m * m * m;
   cudaStream_t st = d->st;
   // DNS right-hand side, projected; its pressure enters r = sigma + p I.
@@ -176,11 +272,28 @@ int lockstep(exc_dnsaid* d, double dt) {
   if (e == cudaSuccess) e = project(&d->psd, d->du, st);
   if (e == cudaSuccess) e = copy_pressure<double>(&d->psd, d->p, st);
   if (e != cudaSuccess) return cuda_rc(e);
-  int rc = closure_flux<double>(n, c, d->l, d->visc, fd(d), nfd(d), d->u, d->p, d->r9, st);
-  if (!rc) rc = filtered_stress<double>(n, c, d->l, d->visc, fd(d), nfd(d), d->u, d->sdh, st);
-  if (!rc) rc = classic_stress<double>(n, c, d->l, d->visc, fd(d), nfd(d), d->u, d->s2, st);
-  if (!rc) rc = apply_dhpi(d, d->ub);
+  // filters of the DNS: rDHi and sigmaDH; the classic closure's velocities
+  // and ubar = apply_ΔHπ(u)
+  int rc;
+  {
+    SepTaps taps;
+    std::vector<SepTarget> v;
+    flux_targets(d, FLUX_FACE, true, d->r9, taps, v);
+    flux_targets(d, FLUX_VOLUME, false, d->sdh, taps, v);
+    rc = run_filters(d, taps, v);
+  }
+  if (!rc) {
+    SepTaps taps;
+    std::vector<SepTarget> v;
+    classic_targets(d, d->uf, taps, v);
+    velocity_targets(d, false, d->ub, taps, v);
+    rc = run_filters(d, taps, v);
+  }
   if (rc) return rc;
+  classic_stress_kernel<<<gridsz(M), 256, 0, st>>>(M, d->uf, 1.0 / d->h, d->visc, d->s2);
+  e = cudaGetLastError();
+  if (e == cudaSuccess) e = project(&d->psl, d->ub, st);
+  if (e != cudaSuccess) return cuda_rc(e);
   // no model
   rc = forward_euler(d, &d->psl, m, d->H, d->les[0], d->dul, dt);
   if (rc) return rc;
@@ -219,8 +332,10 @@ int lockstep(exc_dnsaid* d, double dt) {
 // (src/NavierStokes.jl:333, 449): the face filter, divergence free on the
 // LES grid and never projected.
 int paper_target(exc_dnsaid* d, double* out) {
-  int rc = filter_vector<double>(d->n, d->c, d->surface ? EXC_FILTER_FACE : EXC_FILTER_VOLUME, fd(d), nfd(d), d->u,
-                                 out, d->st);
+  SepTaps taps;
+  std::vector<SepTarget> v;
+  velocity_targets(d, d->surface, out, taps, v);
+  const int rc = run_filters(d, taps, v);
   if (rc || !d->doproject || d->surface) return rc;
   return cuda_rc(project(&d->psl, out, d->st));
 }
@@ -228,7 +343,7 @@ int paper_target(exc_dnsaid* d, double* out) {
 // One step of dns_aid_volavg (src/NavierStokes.jl:186-288) or of
 // dns_aid_surface (src/NavierStokes.jl:350-452).
 int lockstep_paper(exc_dnsaid* d, double dt) {
-  const int n = d->n, m = d->m, c = d->c;
+  const int n = d->n, m = d->m;
   const long long N3 = 3LL * n * n * n, M = (long long)m * m * m;
   cudaStream_t st = d->st;
   // DNS right-hand side, projected; its pressure enters r = sigma + p I
@@ -239,14 +354,12 @@ int lockstep_paper(exc_dnsaid* d, double dt) {
   // volume: fru = volume-filtered r (sdh), firu = face-filtered r (r9);
   // surface: firu = surface-filtered r (rc9), swap flux = firu on the
   // diagonal, line-filtered r off it (r9)
-  int rc;
-  if (d->surface) {
-    rc = surface_flux<double>(n, c, d->l, d->visc, fd(d), nfd(d), d->u, d->p, d->rc9, false, st);
-    if (!rc) rc = surface_flux<double>(n, c, d->l, d->visc, fd(d), nfd(d), d->u, d->p, d->r9, true, st);
-  } else {
-    rc = filtered_stress<double>(n, c, d->l, d->visc, fd(d), nfd(d), d->u, d->sdh, st, d->p);
-    if (!rc) rc = closure_flux<double>(n, c, d->l, d->visc, fd(d), nfd(d), d->u, d->p, d->r9, st);
-  }
+  SepTaps taps;
+  std::vector<SepTarget> v;
+  if (d->surface) flux_targets(d, FLUX_SURFACE, true, d->rc9, taps, v);
+  else flux_targets(d, FLUX_VOLUME, true, d->sdh, taps, v);
+  flux_targets(d, d->surface ? FLUX_LINE : FLUX_FACE, true, d->r9, taps, v);
+  int rc = run_filters(d, taps, v);
   // fu and rfu = sigma_H(fu) + p_H I, p_H from the LES right-hand side of fu
   if (!rc) rc = paper_target(d, d->ub);
   if (rc) return rc;
@@ -333,7 +446,7 @@ int exc_dnsaid_create(const exc_dnsaid_desc* desc, void* stream, exc_dnsaid** ou
                 dalloc(&d->sl, 6 * M) || dalloc(&d->sc, 6 * M) || dalloc(&d->zero, M) || dalloc(&d->scal, 16) ||
                 dalloc(&d->part, (size_t)SHELL_BLOCKS * 1024 + 2048 + RED_PARTS) || dalloc(&d->spec, spec);
   for (int k = 0; k < 5 && !rc; ++k) rc = dalloc(&d->les[k], 3 * M);
-  if (!rc) rc = dalloc(&d->pl, M) || dalloc(&d->dsig, 3 * M);
+  if (!rc) rc = dalloc(&d->pl, M) || dalloc(&d->dsig, 3 * M) || dalloc(&d->uf, 18 * M);
   if (rc) { exc_dnsaid_destroy(d); return rc; }
   cudaMemsetAsync(d->zero, 0, M * sizeof(double), d->st);
   cudaMemsetAsync(d->u, 0, 3 * N * sizeof(double), d->st);
@@ -349,8 +462,9 @@ int exc_dnsaid_destroy(exc_dnsaid* d) {
   poisson_free(&d->psd);
   poisson_free(&d->psl);
   double* bufs[] = {d->u, d->du, d->p, d->ub, d->dul, d->sdh, d->s2, d->r9, d->sl, d->sc, d->zero, d->scal,
-                    d->part, d->spec, d->pl, d->dsig, d->rc9};
+                    d->part, d->spec, d->pl, d->dsig, d->rc9, d->uf};
   for (double* b : bufs) cudaFree(b);
+  sep_free(&d->sep);
   for (double* b : d->les) cudaFree(b);
   delete d;
   return EXC_OK;

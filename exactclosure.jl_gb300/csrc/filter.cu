@@ -258,36 +258,6 @@ int closure_flux(int n, int c, double l, double visc, const double* fdelta, int 
   return EXC_OK;
 }
 
-// Surface-filtered flux of the paper's face-average driver (dns_aid_surface,
-// src/NavierStokes.jl:368-369): component (i, j) = r_ij point-sampled along i
-// (the face of the velocity u_i it updates) and boxed along the other two
-// axes (Turbulox's surfacefilter!(firu, ru, c, true)); with `line`, the
-// off-diagonal components are point-sampled along j too and boxed along the
-// third axis only (linefilter!), the diagonal unchanged.  Sampled at the LES
-// centre (i == j) or edge (i, j); order s11,s21,s31,s12,... like rDHi.
-template <typename T>
-int surface_flux(int n, int c, double l, double visc, const double* fdelta, int nfd, const T* u, const T* p,
-                 T* r9, bool line, cudaStream_t st) {
-  const int m = n / c;
-  const long long M = (long long)m * m * m;
-  for (int j = 0; j < 3; ++j)
-    for (int i = 0; i < 3; ++i) {
-      bool stag[3], point[3];
-      for (int d = 0; d < 3; ++d) {
-        stag[d] = (i != j) && (d == i || d == j);
-        point[d] = (d == i) || (line && d == j);
-      }
-      Taps3 taps;
-      int rc = make_taps3(c, stag, point, fdelta, nfd, &taps);
-      if (rc) return rc;
-      launch_flux_filter_rt<T>(i, j, u, p, n, (T)(1.0 / (l / n)), (T)visc, c, taps, r9 + (long long)(3 * j + i) * M, M,
-                               st);
-    }
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
-  return EXC_OK;
-}
-
 // sigmaDH (src/N.jl:1088-1115): volume filter GDH of each stress component,
 // sampled at LES centres/edges; order s11,s22,s33,s12,s23,s31.  With p the
 // total flux r = sigma + p I is filtered (the paper driver's volume-filtered
@@ -460,104 +430,12 @@ cudaError_t filter_vector_box(int n, int c, int kind, const T* u, T* ub, T* tb, 
   return e;
 }
 
-// Stress of the fine-grid filtered velocity, uf = lazyfilter(u, GDH) on the
-// DNS grid (centred box of odd width c, composed with FDelta), at fine cell
-// (x, y, z): the field that `step_ΔHπ_classic!` (src/N.jl:1137-1162) samples
-// at the LES centres and edges.  Each uf value is evaluated on the fly.
-// sigma_ij of the fine-filtered velocity GDH u at fine cell (x, y, z); the
-// components (I, J) are compile-time and every index wraps by comparison (tap
-// offsets stay within (-n, 2n)).
-template <typename T, int I, int J>
-struct FineFilteredStressSrc {
-  const T* u;
-  int n;
-  T inv_h, visc;
-  Taps1D ft;  // centred fine-filter taps (same along every axis)
-  __device__ __forceinline__ int wrap(int q) const { return q < 0 ? q + n : (q >= n ? q - n : q); }
-  __device__ __forceinline__ double uf(int comp, int x, int y, int z) const {
-    const long long N = (long long)n * n * n;
-    const T* f = u + comp * N;
-    double acc = 0.0;
-    for (int tz = 0; tz < ft.cnt; ++tz) {
-      const int zz = wrap(z + ft.off[tz]);
-      double az = 0.0;
-      for (int ty = 0; ty < ft.cnt; ++ty) {
-        const T* row = f + ((long long)zz * n + wrap(y + ft.off[ty])) * n;
-        double ay = 0.0;
-        for (int tx = 0; tx < ft.cnt; ++tx) ay += ft.w[tx] * (double)row[wrap(x + ft.off[tx])];
-        az += ft.w[ty] * ay;
-      }
-      acc += ft.w[tz] * az;
-    }
-    return acc;
-  }
-  template <int A>
-  __device__ __forceinline__ double uf_at(int comp, int x, int y, int z, int s) const {
-    if (A == 0) x = wrap(x + s);
-    if (A == 1) y = wrap(y + s);
-    if (A == 2) z = wrap(z + s);
-    return uf(comp, x, y, z);
-  }
-  __device__ __forceinline__ double operator()(int x, int y, int z) const {
-    constexpr int off = (I != J);
-    const double uir = uf_at<J>(I, x, y, z, off), uil = uf_at<J>(I, x, y, z, off - 1);
-    // on the diagonal the two pairs are the same filtered values
-    const double ujr = I == J ? uir : uf_at<I>(J, x, y, z, off);
-    const double ujl = I == J ? uil : uf_at<I>(J, x, y, z, off - 1);
-    const double etaj_ui = (uir + uil) / 2, etai_uj = (ujr + ujl) / 2;
-    const double dj_ui = (uir - uil) * (double)inv_h, di_uj = (ujr - ujl) * (double)inv_h;
-    return etaj_ui * etai_uj - (double)visc * (dj_ui + di_uj);
-  }
-};
-
-template <typename T, int I, int J>
-static void launch_classic(const T* u, int n, T inv_h, T visc, const Taps1D& ft, int c, const Taps3& taps, T* out,
-                           long long M, cudaStream_t st) {
-  FineFilteredStressSrc<T, I, J> src{u, n, inv_h, visc, ft};
-  filter_kernel<T><<<grid_for(M), 256, 0, st>>>(src, n, c, taps, out);
-}
-
-// sigma2 of `step_ΔHπ_classic!`: `lazytensorcoarsegrain(g_les,
-// stresstensor(lazyfilter(u, GDH)))` (src/N.jl:1117-1135, 1143-1145); order
-// s11, s22, s33, s12, s23, s31.  Odd ratios only (the reference's top hat).
-template <typename T>
-int classic_stress(int n, int c, double l, double visc, const double* fdelta, int nfd, const T* u, T* s6,
-                   cudaStream_t st) {
-  if (c % 2 == 0) { set_last_error("the classic closure's fine-grid filter needs an odd ratio"); return EXC_ERR_RATIO; }
-  const int m = n / c;
-  const long long M = (long long)m * m * m;
-  Taps1D ft = build_taps(c, false, false, fdelta, nfd);
-  if (ft.cnt < 0) { set_last_error("filter stencil longer than MAX_TAPS"); return EXC_ERR_ARG; }
-  for (int k = 0; k < ft.cnt; ++k) ft.off[k] -= c / 2;  // centre the box on the fine cell
-  const int comps[6][2] = {{0, 0}, {1, 1}, {2, 2}, {0, 1}, {1, 2}, {2, 0}};
-  for (int k = 0; k < 6; ++k) {
-    const int i = comps[k][0], j = comps[k][1];
-    bool stag[3], point[3] = {true, true, true};
-    for (int d = 0; d < 3; ++d) stag[d] = (i != j) && (d == i || d == j);
-    Taps3 taps;
-    int rc = make_taps3(c, stag, point, nullptr, 0, &taps);
-    if (rc) return rc;
-    const T inv_h = (T)(1.0 / (l / n));
-    T* out = s6 + (long long)k * M;
-#define EXC_CLASSIC(I, J) \
-  if (i == I && j == J) launch_classic<T, I, J>(u, n, inv_h, (T)visc, ft, c, taps, out, M, st);
-    EXC_CLASSIC(0, 0) EXC_CLASSIC(1, 1) EXC_CLASSIC(2, 2) EXC_CLASSIC(0, 1) EXC_CLASSIC(1, 2) EXC_CLASSIC(2, 0)
-#undef EXC_CLASSIC
-  }
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
-  return EXC_OK;
-}
-
 #define INST(T)                                                                                          \
-  template int classic_stress<T>(int, int, double, double, const double*, int, const T*, T*, cudaStream_t); \
   template cudaError_t filter_vector_box<T>(int, int, int, const T*, T*, T*, cudaStream_t);              \
   template cudaError_t box_tb<T>(int, int, const T*, T*, cudaStream_t);                                  \
   template cudaError_t box_tb_coarsen<T>(int, int, int, const T*, T*, cudaStream_t);                     \
   template cudaError_t box_oa<T>(int, int, int, const T*, T*, cudaStream_t);                             \
   template int filter_vector<T>(int, int, int, const double*, int, const T*, T*, cudaStream_t);          \
-  template int surface_flux<T>(int, int, double, double, const double*, int, const T*, const T*, T*, bool, \
-                               cudaStream_t);                                                             \
   template int closure_flux<T>(int, int, double, double, const double*, int, const T*, const T*, T*,     \
                                cudaStream_t);                                                            \
   template int filtered_stress<T>(int, int, double, double, const double*, int, const T*, T*, cudaStream_t, const T*);

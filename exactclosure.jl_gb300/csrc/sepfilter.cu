@@ -1,0 +1,319 @@
+// Separable filter-and-sample of the DNS quantities the LES drivers need each
+// step (`lazycoarsegrain(lazyfilter(.))`, src/N.jl:592-698): the fluxes r_ij =
+// sigma_ij(u) + delta_ij p with their face and volume filters
+// (src/N.jl:1038-1115), the volume-filtered velocity (src/N.jl:1228-1237) and
+// the fine-filtered velocity at the sample points of the classic closure
+// (src/N.jl:1143-1145).
+//
+// The kernels of these filters are products of 1-D ones, so a target is three
+// passes: along x at every fine (y, z), along y at every fine z, along z.  A
+// target with T taps per axis and ratio c then costs about T (1/c + 1/c^2 +
+// 1/c^3) FP64 operations per fine cell instead of T^3 / c^3 times the cost of
+// evaluating the source: 17 taps at ratio 5 (the box of 5 convolved with the
+// reference's Gaussian of width 2H) are 4 instead of 39 source evaluations.
+// The FP64 pipe (two operations per clock per SM) bounds the x pass, which
+// evaluates every source once per fine cell and shares it between all filters
+// of it; all targets of a batch go through three launches.
+//
+// One lockstep step of dnsaid_project, DNS 250^3, ratio 5, that Gaussian: 165
+// -> 11.7 ms, the filters (sums over T^3 taps per LES cell before) 155 -> 4.4
+// ms: x pass 2.8 ms = 85 FP64 operations per fine cell at the pipe's rate, y
+// 0.7, z 0.3.  Without the Gaussian (5 taps) 10.7 -> 9.8 ms, ratio 3 at 240^3
+// 11.0 -> 10.3, 60^3 1.50 -> 1.22.
+#include <cstring>
+
+#include "internal.cuh"
+#include "sepfilter.cuh"
+
+namespace exc {
+namespace {
+
+constexpr int SEP_MAX_TAPSETS = 16;  // distinct 1-D stencils of one batch
+constexpr int SEP_MAX_XV = 12;       // x-filtered arrays
+constexpr int SEP_MAX_YV = 32;       // xy-filtered arrays
+constexpr int SEP_MAX_OUT = 32;      // targets
+constexpr int SEP_ROWS = 8;          // x rows per CTA
+constexpr int SEP_THREADS = 256;
+
+struct XVar {
+  int taps;
+  double* out;
+};
+struct XArgs {
+  Taps1D taps[SEP_MAX_TAPSETS];
+  int nsrc;
+  int src[SEP_SOURCES];    // source of blockIdx.y
+  int first[SEP_SOURCES];  // its variants are v[first .. first + count)
+  int count[SEP_SOURCES];
+  XVar v[SEP_MAX_XV];
+  const double* u;
+  const double* p;
+  int n, m, c, rows;
+  int pad;  // ghost cells on either side of a staged row
+  double vh;  // visc / h
+};
+
+// sigma_ij at fine cell (x, y, z): a b / 4 - (visc / h) d with a, b the
+// two-point sums of u_i along j and of u_j along i, d the sum of the two
+// differences (src/N.jl:106-118; the form of flux_filter_kernel).
+__device__ __forceinline__ double sep_value(const XArgs& A, int src, int x, int y, int z) {
+  const int n = A.n;
+  const long long nn = (long long)n * n, N = nn * n;
+  const long long at = (long long)z * nn + (long long)y * n + x;
+  if (src < SEP_SIGMA) return A.u[src * N + at];
+  if (src == SEP_P) return A.p[at];
+  const int k = src - SEP_SIGMA;
+  // step of one cell along axis d from (x, y, z), periodic
+  auto up = [&](int d) -> long long {
+    return d == 0 ? (x + 1 == n ? 1 - n : 1) : d == 1 ? (y + 1 == n ? (long long)(1 - n) * n : n)
+                                                      : (z + 1 == n ? (1 - n) * nn : nn);
+  };
+  auto dn = [&](int d) -> long long {
+    return d == 0 ? (x == 0 ? n - 1 : -1) : d == 1 ? (y == 0 ? (long long)(n - 1) * n : -n)
+                                                   : (z == 0 ? (n - 1) * nn : -nn);
+  };
+  if (k < 3) {
+    const double* f = A.u + k * N + at;
+    const double r = f[0], l = f[dn(k)];
+    const double s = r + l;
+    return fma(-2.0 * A.vh, r - l, 0.25 * (s * s));
+  }
+  const int i = k - 3, j = k == 5 ? 0 : k - 2;  // s12, s23, s31
+  const double* fi = A.u + i * N + at;
+  const double* fj = A.u + j * N + at;
+  const double il = fi[0], ir = fi[up(j)], jl = fj[0], jr = fj[up(i)];
+  return fma(-A.vh, (ir + jr) - (il + jl), 0.25 * ((ir + il) * (jr + jl)));
+}
+
+// Along x.  A CTA stages `rows` rows of one source with ghosts, then applies
+// every tap list of that source.
+__global__ void __launch_bounds__(SEP_THREADS) sep_x_kernel(const __grid_constant__ XArgs A) {
+  extern __shared__ double row[];
+  const int n = A.n, m = A.m, c = A.c, pitch = n + 2 * A.pad;
+  const int src = A.src[blockIdx.y];
+  const int nn = n * n;
+  const int r0 = blockIdx.x * A.rows;
+  const int rows = min(A.rows, nn - r0);
+  for (int t = threadIdx.x; t < rows * pitch; t += SEP_THREADS) {
+    const int r = t / pitch;
+    const int z = (r0 + r) / n, y = r0 + r - z * n;
+    int x = t - r * pitch - A.pad;
+    while (x < 0) x += n;
+    while (x >= n) x -= n;
+    row[t] = sep_value(A, src, x, y, z);
+  }
+  __syncthreads();
+  const int v0 = A.first[blockIdx.y], vn = A.count[blockIdx.y];
+  for (int q = threadIdx.x; q < rows * m; q += SEP_THREADS) {
+    const int r = q / m, ix = q - r * m;
+    const double* f = row + r * pitch + A.pad + c * ix;
+    for (int v = v0; v < v0 + vn; ++v) {
+      const Taps1D& T = A.taps[A.v[v].taps];
+      double acc = 0.0;
+      for (int t = 0; t < T.cnt; ++t) acc = fma(T.w[t], f[T.off[t]], acc);
+      A.v[v].out[(long long)(r0 + r) * m + ix] = acc;
+    }
+  }
+}
+
+struct YVar {
+  int taps;
+  const double* in;
+  double* out;
+};
+struct YArgs {
+  Taps1D taps[SEP_MAX_TAPSETS];
+  YVar v[SEP_MAX_YV];
+  int n, m, c;
+};
+
+// Along y: [z][y][ix] -> [z][iy][ix].  The tap offsets of the y and z passes
+// are reduced to [0, n) on the host, so one comparison wraps them.
+__global__ void __launch_bounds__(SEP_THREADS) sep_y_kernel(const __grid_constant__ YArgs A) {
+  const int n = A.n, m = A.m;
+  const YVar V = A.v[blockIdx.y];
+  const Taps1D& T = A.taps[V.taps];
+  const long long tot = (long long)n * m * m;
+  const IdxDiv dm(m);
+  for (long long g = blockIdx.x * (long long)SEP_THREADS + threadIdx.x; g < tot; g += (long long)gridDim.x * SEP_THREADS) {
+    const long long r = dm.div(g);
+    const int ix = (int)(g - r * m);
+    const int z = (int)dm.div(r), iy = (int)(r - (long long)z * m);
+    const double* f = V.in + (long long)z * n * m + ix;
+    double acc = 0.0;
+    for (int t = 0; t < T.cnt; ++t) {
+      const int q = A.c * iy + T.off[t], y = q >= n ? q - n : q;
+      acc = fma(T.w[t], f[(long long)y * m], acc);
+    }
+    V.out[g] = acc;
+  }
+}
+
+struct ZVar {
+  int taps;
+  const double* in;
+  const double* in2;  // second source of the target, or null
+  double* out;
+};
+struct ZArgs {
+  Taps1D taps[SEP_MAX_TAPSETS];
+  ZVar v[SEP_MAX_OUT];
+  int n, m, c;
+};
+
+// Along z: [z][iy][ix] -> [iz][iy][ix].
+__global__ void __launch_bounds__(SEP_THREADS) sep_z_kernel(const __grid_constant__ ZArgs A) {
+  const int n = A.n, m = A.m;
+  const ZVar V = A.v[blockIdx.y];
+  const Taps1D& T = A.taps[V.taps];
+  const int mm = m * m;
+  const long long tot = (long long)mm * m;
+  const IdxDiv dmm(mm);
+  for (long long g = blockIdx.x * (long long)SEP_THREADS + threadIdx.x; g < tot; g += (long long)gridDim.x * SEP_THREADS) {
+    const int iz = (int)dmm.div(g), r = (int)(g - (long long)iz * mm);
+    double acc = 0.0, acc2 = 0.0;
+    for (int t = 0; t < T.cnt; ++t) {
+      const int q = A.c * iz + T.off[t], z = q >= n ? q - n : q;
+      acc = fma(T.w[t], V.in[(long long)z * mm + r], acc);
+      if (V.in2) acc2 = fma(T.w[t], V.in2[(long long)z * mm + r], acc2);
+    }
+    V.out[g] = acc + acc2;
+  }
+}
+
+int sep_reserve(double** p, size_t* have, size_t want) {
+  if (*have >= want) return EXC_OK;
+  cudaFree(*p);
+  *p = nullptr;
+  *have = 0;
+  if (cudaMalloc(p, want * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+    set_last_error("out of device memory (filter scratch)");
+    return EXC_ERR_OOM;
+  }
+  *have = want;
+  return EXC_OK;
+}
+
+}  // namespace
+
+void sep_free(SepWork* w) {
+  cudaFree(w->a);
+  cudaFree(w->b);
+  *w = SepWork();
+}
+
+int SepTaps::add(int c, bool stag, bool point, const double* fdelta, int nfd, int shift) {
+  Taps1D t = build_taps(c, stag, point, fdelta, nfd);
+  if (t.cnt < 0) { bad = true; return 0; }
+  for (int k = 0; k < t.cnt; ++k) t.off[k] += shift;
+  for (size_t i = 0; i < list.size(); ++i)
+    if (list[i].cnt == t.cnt && !std::memcmp(list[i].off, t.off, t.cnt * sizeof(int)) &&
+        !std::memcmp(list[i].w, t.w, t.cnt * sizeof(double)))
+      return (int)i;
+  list.push_back(t);
+  return (int)list.size() - 1;
+}
+
+int sep_filter(SepWork* w, int n, int c, double inv_h, double visc, const SepTaps& taps,
+               const std::vector<SepTarget>& targets, const double* u, const double* p, cudaStream_t st) {
+  if (taps.bad) { set_last_error("filter stencil longer than MAX_TAPS"); return EXC_ERR_ARG; }
+  const int m = n / c;
+  // distinct (source, x taps) and (x variant, y taps) pairs
+  struct XV { int src, t; };
+  struct YV { int x, t; };
+  std::vector<XV> xv;
+  std::vector<YV> yv;
+  auto xvar = [&](int src, int t) {
+    for (size_t i = 0; i < xv.size(); ++i)
+      if (xv[i].src == src && xv[i].t == t) return (int)i;
+    xv.push_back({src, t});
+    return (int)xv.size() - 1;
+  };
+  auto yvar = [&](int x, int t) {
+    for (size_t i = 0; i < yv.size(); ++i)
+      if (yv[i].x == x && yv[i].t == t) return (int)i;
+    yv.push_back({x, t});
+    return (int)yv.size() - 1;
+  };
+  std::vector<int> y1, y2;
+  for (const SepTarget& T : targets) {
+    y1.push_back(yvar(xvar(T.src, T.t[0]), T.t[1]));
+    y2.push_back(T.src2 >= 0 ? yvar(xvar(T.src2, T.t[0]), T.t[1]) : -1);
+  }
+  if (taps.list.size() > SEP_MAX_TAPSETS || xv.size() > SEP_MAX_XV || yv.size() > SEP_MAX_YV ||
+      targets.size() > SEP_MAX_OUT) {
+    set_last_error("too many filters in one batch");
+    return EXC_ERR_ARG;
+  }
+  const size_t xw = (size_t)n * n * m, yw = (size_t)n * m * m;
+  int rc = sep_reserve(&w->a, &w->na, xv.size() * xw);
+  if (!rc) rc = sep_reserve(&w->b, &w->nb, yv.size() * yw);
+  if (rc) return rc;
+
+  XArgs X{};
+  YArgs Y{};
+  ZArgs Z{};
+  int pad = 0;
+  for (size_t i = 0; i < taps.list.size(); ++i) {
+    X.taps[i] = Y.taps[i] = taps.list[i];
+    for (int k = 0; k < Y.taps[i].cnt; ++k) Y.taps[i].off[k] = ((Y.taps[i].off[k] % n) + n) % n;
+    Z.taps[i] = Y.taps[i];
+  }
+  X.u = u;
+  X.p = p;
+  X.n = Y.n = Z.n = n;
+  X.m = Y.m = Z.m = m;
+  X.c = Y.c = Z.c = c;
+  X.vh = visc * inv_h;
+  // sources in order, the variants of one source together
+  std::vector<int> slot(xv.size());
+  int used = 0;
+  for (int s = 0; s < SEP_SOURCES; ++s) {
+    int cnt = 0;
+    for (size_t i = 0; i < xv.size(); ++i)
+      if (xv[i].src == s) {
+        const Taps1D& T = taps.list[xv[i].t];
+        for (int k = 0; k < T.cnt; ++k) {
+          // farthest reach beyond the row: c ix + off over ix < m
+          if (-T.off[k] > pad) pad = -T.off[k];
+          if (T.off[k] - (c - 1) > pad) pad = T.off[k] - (c - 1);
+        }
+        slot[i] = used + cnt;
+        X.v[used + cnt] = {xv[i].t, w->a + (size_t)(used + cnt) * xw};
+        ++cnt;
+      }
+    if (!cnt) continue;
+    X.src[X.nsrc] = s;
+    X.first[X.nsrc] = used;
+    X.count[X.nsrc] = cnt;
+    ++X.nsrc;
+    used += cnt;
+  }
+  X.pad = pad;
+  for (size_t i = 0; i < yv.size(); ++i)
+    Y.v[i] = {yv[i].t, w->a + (size_t)slot[yv[i].x] * xw, w->b + i * yw};
+  for (size_t i = 0; i < targets.size(); ++i)
+    Z.v[i] = {targets[i].t[2], w->b + (size_t)y1[i] * yw, y2[i] >= 0 ? w->b + (size_t)y2[i] * yw : nullptr,
+              targets[i].out};
+
+  // rows that fit the default 48 KB of shared memory (one row of 1024 cells
+  // and its ghosts is 9 KB at most)
+  const size_t rowb = (size_t)(n + 2 * pad) * sizeof(double);
+  int rows = (int)((48 * 1024) / rowb);
+  rows = rows < 1 ? 1 : rows > SEP_ROWS ? SEP_ROWS : rows;
+  X.rows = rows;
+  auto blocks = [](size_t cnt) {
+    const size_t b = (cnt + SEP_THREADS - 1) / SEP_THREADS;
+    return (unsigned)(b < 152 * 16 ? b : 152 * 16);
+  };
+  sep_x_kernel<<<dim3((unsigned)((n * n + rows - 1) / rows), X.nsrc), SEP_THREADS, rows * rowb, st>>>(X);
+  sep_y_kernel<<<dim3(blocks(yw), (unsigned)yv.size()), SEP_THREADS, 0, st>>>(Y);
+  sep_z_kernel<<<dim3(blocks((size_t)m * m * m), (unsigned)targets.size()), SEP_THREADS, 0, st>>>(Z);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
+  return EXC_OK;
+}
+
+}  // namespace exc

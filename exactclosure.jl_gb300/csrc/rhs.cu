@@ -46,6 +46,15 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned 
       : "memory");
   return ok != 0;
 }
+// 4-D tiled TMA load of one box (x, y, z, component)
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, int x, int y, int z, int c,
+                                            unsigned long long* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(
+          smem_u32(dst)),
+      "l"(reinterpret_cast<unsigned long long>(map)), "r"(x), "r"(y), "r"(z), "r"(c), "r"(smem_u32(bar))
+      : "memory");
+}
 // 3-D tiled TMA load of one box (x, y, z) of the tensor map into shared memory
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,
                                             unsigned long long* bar) {
@@ -92,70 +101,52 @@ constexpr size_t plane_smem_bytes() {
   return sizeof(PlaneSmem<T, NC>) + 128;
 }
 
-// Stress values.  FP32 form (SC false): 4 sigma of the velocities in shared
-// memory, the divergence takes 1/(4h).  FP64 form (SC true): the planes in
-// shared memory hold w = s u - q (s = sqrt(kd), kd = 1/(4h), rho = rv s, q =
-// rho/2, rv = 4 visc/h) and the stresses are -kd 4 sigma up to a constant per
-// component, which the divergence's differences cancel:
-//   -kd 4 sigma_ii = -(w_i + w_i(-e_i))^2 - 4 rho w_i(-e_i) - rho^2,
-//   -kd 4 sigma_ij = -(w_i + w_i(+e_j)) (w_j + w_j(+e_i)) - 2 rho (w_i + w_j) - rho^2,
-// (expand 4 sigma_ii = (a + b)^2 - 2 rv (a - b), 4 sigma_ij = (a + b)(c + d)
-// - rv ((b - a) + (d - c)) with a = (w_a + q) / s ...): 3 and 5 FP64
-// operations instead of 4 and 7, and no scaling in the divergence -- the FP64
-// pipe, about two operations per clock per SM, bounds this sweep.
-// Diagonal: a at the cell, b its lower neighbour along i; cd = rv2 (FP32
-// form) or -4 rho (FP64 form).
-template <bool SC, typename T>
+// Stress values, kept as 4 sigma; the divergence takes 1/(4h).  Diagonal: a
+// at the cell, b its lower neighbour along i; cd = 2 rv, rv = 4 visc / h.
+template <typename T>
 __device__ __forceinline__ T sdiag_of(T a, T b, T cd) {
-  const T s = a + b;
-  if constexpr (SC) {
-    return fma(-s, s, cd * b);
-  } else {
-    const T d = a - b;
-    return s * s - cd * d;
-  }
+  const T s = a + b, d = a - b;
+  return s * s - cd * d;
 }
-// Off-diagonal: a = u_i, b = u_i(+e_j), c = u_j, d = u_j(+e_i); co = rv (FP32
-// form) or -2 rho (FP64 form).
-template <bool SC, typename T>
+// Off-diagonal: a = u_i, b = u_i(+e_j), c = u_j, d = u_j(+e_i); co = rv.
+template <typename T>
 __device__ __forceinline__ T soff_of(T a, T b, T c, T d, T co) {
-  if constexpr (SC) return fma(-(a + b), c + d, co * (a + c));
-  else return (a + b) * (c + d) - co * ((b - a) + (d - c));
+  return (a + b) * (c + d) - co * ((b - a) + (d - c));
 }
 // sigma_ii at box (bx, by) of plane buffer b (uses u_i at the cell and at -e_i)
-template <bool SC, typename T, int I, typename U>
+template <typename T, int I, typename U>
 __device__ __forceinline__ T sdiag(const U& u, int bx, int by, T cd) {
   bx += SH<T>;
-  return sdiag_of<SC>(u[I][by][bx], I == 0 ? u[0][by][bx - 1] : u[1][by - 1][bx], cd);
+  return sdiag_of(u[I][by][bx], I == 0 ? u[0][by][bx - 1] : u[1][by - 1][bx], cd);
 }
 // sigma_12 at box (bx, by): u1, u1(+y), u2, u2(+x)
-template <bool SC, typename T, typename U>
+template <typename T, typename U>
 __device__ __forceinline__ T s12(const U& u, int bx, int by, T co) {
   bx += SH<T>;
-  return soff_of<SC>(u[0][by][bx], u[0][by + 1][bx], u[1][by][bx], u[1][by][bx + 1], co);
+  return soff_of(u[0][by][bx], u[0][by + 1][bx], u[1][by][bx], u[1][by][bx + 1], co);
 }
 // sigma_13 at box (bx, by): u1, u1(+z) [next plane], u3, u3(+x)
-template <bool SC, typename T, typename U>
+template <typename T, typename U>
 __device__ __forceinline__ T s13(const U& uc, const U& un, int bx, int by, T co) {
   bx += SH<T>;
-  return soff_of<SC>(uc[0][by][bx], un[0][by][bx], uc[2][by][bx], uc[2][by][bx + 1], co);
+  return soff_of(uc[0][by][bx], un[0][by][bx], uc[2][by][bx], uc[2][by][bx + 1], co);
 }
 // sigma_23 at box (bx, by): u2, u2(+z) [next plane], u3, u3(+y)
-template <bool SC, typename T, typename U>
+template <typename T, typename U>
 __device__ __forceinline__ T s23(const U& uc, const U& un, int bx, int by, T co) {
   bx += SH<T>;
-  return soff_of<SC>(uc[1][by][bx], un[1][by][bx], uc[2][by][bx], uc[2][by + 1][bx], co);
+  return soff_of(uc[1][by][bx], un[1][by][bx], uc[2][by][bx], uc[2][by + 1][bx], co);
 }
 // sigma_33 between planes: u3 of the upper plane and of the lower plane
-template <bool SC, typename T>
+template <typename T>
 __device__ __forceinline__ T s33(T up, T lo, T cd) {
-  return sdiag_of<SC>(up, lo, cd);
+  return sdiag_of(up, lo, cd);
 }
 
 template <typename T, int NC, bool DOADD>
-__global__ void __launch_bounds__(PTX * NWARP, sizeof(T) == 4 ? 4 : 3)
+__global__ void __launch_bounds__(PTX * NWARP, 4)
 rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, SlotBatch sb, int zblocks, int ptz,
-           const __grid_constant__ CUtensorMap umap, int have_map, int pre_shifted) {
+           const __grid_constant__ CUtensorMap umap, int have_map) {
   constexpr int PTY = PTYT<NC>, PBY = PBYT<NC>;
   constexpr int CSTRIDE = (int)(sizeof(CompPlane<T, NC>) / sizeof(T));
   extern __shared__ __align__(128) unsigned char rhs_smem[];
@@ -172,18 +163,10 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int lane = tx, warp = ty;
   const int x0 = blockIdx.x * PTX, y0 = blockIdx.y * PTY, z0 = zb * ptz;
-  // FP32: stresses kept as 4 sigma (rv = 4 visc / h), the divergence takes
-  // 1/(4h).  FP64 (SC): shared memory holds w = s u - q, stresses are -kd 4
-  // sigma up to constants (see sdiag_of / soff_of)
-  constexpr bool SC = sizeof(T) == 8;
+  // stresses kept as 4 sigma (rv = 4 visc / h), the divergence takes 1/(4h)
   const T kd = (T)0.25 * inv_h;
   const T rv = (T)4 * visc * inv_h;
-  const Fp64Shift fs = fp64_shift((double)inv_h, (double)visc);
-  const T sq = SC ? (T)fs.sq : (T)1;
-  const T rho = (T)fs.rho;
-  const T qs = (T)fs.qs;
-  const T cd = SC ? (T)-4 * rho : (T)2 * rv;
-  const T co = SC ? (T)-2 * rho : rv;
+  const T cd = (T)2 * rv, co = rv;
   auto wrap = [n](int g) { return g < 0 ? g + n : (g >= n ? g - n : g); };
   auto wrapm = [n](int g) { return ((g % n) + n) % n; };
   const bool big = n >= PBX;
@@ -287,63 +270,20 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
     }
     parity ^= 1u << buf;
   };
-  // FP64 form: w = s u - q in place over what this thread may touch of
-  // buffer buf after its wait -- the whole plane for TMA tiles (the mbarrier
-  // wait makes every copy visible to every waiting thread), else its own
-  // 16-byte pieces or words; the barrier after the wait publishes the result
-  auto shift_plane = [&](int buf) {
-    if constexpr (SC) {
-      if (pre_shifted) return;  // the field is stored in the shifted form already
-      if (tma) {
-        constexpr int HALF = PBY * UROW<T> / 2;  // 16-byte pairs per component plane
-        static_assert(PBY * UROW<T> % 2 == 0, "component plane of whole pairs");
-        for (int i = tid; i < 3 * HALF; i += PTX * NWARP) {
-          const int c = i / HALF;
-          double2* const p2 = reinterpret_cast<double2*>(&sm.u[buf][c].r[0][0]) + (i - c * HALF);
-          double2 v = *p2;
-          v.x = fma(sq, v.x, -qs);
-          v.y = fma(sq, v.y, -qs);
-          *p2 = v;
-        }
-      } else if (vec) {
-        T* const sb0 = &sm.u[buf][0].r[0][0];
-#pragma unroll
-        for (int i = 0; i < NSLOT; ++i)
-          if (goff[i] >= 0) {
-            double2* const p2 = reinterpret_cast<double2*>(sb0 + soff[i]);
-            double2 v = *p2;
-            v.x = fma(sq, v.x, -qs);
-            v.y = fma(sq, v.y, -qs);
-            *p2 = v;
-          }
-      } else {
-        for (int rr = ty; rr < PBY; rr += NWARP)
-          for (int bxx = tx; bxx < PBX; bxx += PTX)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              T& w = sm.u[buf][c][rr][bxx + SH<T>];
-              w = fma(sq, w, -qs);
-            }
-      }
-    }
-  };
   load_plane(0, zwrap(z0 - 1));
   load_plane(1, zwrap(z0));
   load_plane(2, zwrap(z0 + 1));
   wait_plane(0);
   wait_plane(1);
   wait_plane(2);
-  shift_plane(0);
-  shift_plane(1);
-  shift_plane(2);
   __syncthreads();
   T s13_prev[NC], s23_prev[NC], s33_cur[NC];
 #pragma unroll
   for (int i = 0; i < NC; ++i) {
     const int by = NC * ty + 1 + i;
-    s13_prev[i] = s13<SC, T>(sm.u[0], sm.u[1], bx, by, co);
-    s23_prev[i] = s23<SC, T>(sm.u[0], sm.u[1], bx, by, co);
-    s33_cur[i] = s33<SC, T>(sm.u[1][2][by][bx + SH<T>], sm.u[0][2][by][bx + SH<T>], cd);
+    s13_prev[i] = s13<T>(sm.u[0], sm.u[1], bx, by, co);
+    s23_prev[i] = s23<T>(sm.u[0], sm.u[1], bx, by, co);
+    s33_cur[i] = s33<T>(sm.u[1][2][by][bx + SH<T>], sm.u[0][2][by][bx + SH<T>], cd);
   }
   __syncthreads();  // buffer 0 is refilled by the first prefetch
   // buffers: cur = plane z, nxt = plane z + 1, pre = the free one
@@ -365,12 +305,12 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
 #pragma unroll
     for (int i = 0; i < NC; ++i) {
       const int by = NC * ty + 1 + i;
-      v11[i] = sdiag<SC, T, 0>(uc, bx, by, cd);
-      v22[i] = sdiag<SC, T, 1>(uc, bx, by, cd);
-      v12[i] = s12<SC, T>(uc, bx, by, co);
-      v13[i] = s13<SC, T>(uc, un, bx, by, co);
-      v23[i] = s23<SC, T>(uc, un, bx, by, co);
-      v33n[i] = s33<SC, T>(un[2][by][bx + SH<T>], uc[2][by][bx + SH<T>], cd);
+      v11[i] = sdiag<T, 0>(uc, bx, by, cd);
+      v22[i] = sdiag<T, 1>(uc, bx, by, cd);
+      v12[i] = s12<T>(uc, bx, by, co);
+      v13[i] = s13<T>(uc, un, bx, by, co);
+      v23[i] = s23<T>(uc, un, bx, by, co);
+      v33n[i] = s33<T>(un[2][by][bx + SH<T>], uc[2][by][bx + SH<T>], cd);
       // s22 is read from the row above and s23 from the row below: inside a
       // thread's rows they stay in registers
       sm.s[0][by][bx] = v11[i];
@@ -383,17 +323,17 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
     // on the upper halo row, s12 and s13 on the left halo column, s11 on the
     // right halo column
     if (warp == 0) {
-      sm.s[2][0][lane + 1] = s12<SC, T>(uc, lane + 1, 0, co);
+      sm.s[2][0][lane + 1] = s12<T>(uc, lane + 1, 0, co);
     } else if (warp == 1) {
-      sm.s[4][0][lane + 1] = s23<SC, T>(uc, un, lane + 1, 0, co);
+      sm.s[4][0][lane + 1] = s23<T>(uc, un, lane + 1, 0, co);
     } else if (warp == 2) {
-      sm.s[1][PTY + 1][lane + 1] = sdiag<SC, T, 1>(uc, lane + 1, PTY + 1, cd);
+      sm.s[1][PTY + 1][lane + 1] = sdiag<T, 1>(uc, lane + 1, PTY + 1, cd);
     } else if (warp == 3) {
-      for (int r = lane; r <= PTY; r += 32) sm.s[2][r][0] = s12<SC, T>(uc, 0, r, co);
+      for (int r = lane; r <= PTY; r += 32) sm.s[2][r][0] = s12<T>(uc, 0, r, co);
     } else if (warp == 4) {
-      for (int r = lane + 1; r <= PTY; r += 32) sm.s[3][r][0] = s13<SC, T>(uc, un, 0, r, co);
+      for (int r = lane + 1; r <= PTY; r += 32) sm.s[3][r][0] = s13<T>(uc, un, 0, r, co);
     } else if (warp == 5) {
-      for (int r = lane + 1; r <= PTY; r += 32) sm.s[0][r][PTX + 1] = sdiag<SC, T, 0>(uc, PTX + 1, r, cd);
+      for (int r = lane + 1; r <= PTY; r += 32) sm.s[0][r][PTX + 1] = sdiag<T, 0>(uc, PTX + 1, r, cd);
     }
     __syncthreads();
     if (gx < n) {
@@ -412,17 +352,7 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
           const T d2 = (v12[i] - S[2][by][bx - 1]) + (s22_above - v22[i]) + (v23[i] - s23_prev[i]);
           const T d3 = (v13[i] - S[3][by][bx - 1]) + (v23[i] - s23_below) + (v33n[i] - s33_cur[i]);
           const long long g = ((long long)z * n + gy) * n + gx;
-          if constexpr (SC) {  // the stresses carry -kd
-            if (DOADD) {
-              du1[g] += d1;
-              du2[g] += d2;
-              du3[g] += d3;
-            } else {
-              du1[g] = d1;
-              du2[g] = d2;
-              du3[g] = d3;
-            }
-          } else if (DOADD) {
+          if (DOADD) {
             du1[g] -= kd * d1;
             du2[g] -= kd * d2;
             du3[g] -= kd * d3;
@@ -437,11 +367,458 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
         s33_cur[i] = v33n[i];
       }
     }
-    if (kz + 1 < ptz && z + 1 < n) {
-      wait_plane(pre);
-      shift_plane(pre);
-    }
+    if (kz + 1 < ptz && z + 1 < n) wait_plane(pre);
     __syncthreads();
+    const int freed = cur;
+    cur = nxt;
+    nxt = pre;
+    pre = freed;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 sweep on the integer pipe.
+//
+// GB300 retires two FP64 operations per clock and SM but 55 widening integer
+// multiply-adds (32 x 32 + 64 -> 64) and about 100 integer additions (all
+// measured), so this sweep forms the stresses and their divergence in fixed
+// point, with more bits than FP64 carries, and rounds once at the end.
+//
+// Fixed point.  All values a CTA holds share one scale 2^(57 - E), |u| + S <
+// 2^E: a velocity becomes an integer U, |U| <= 2^57, split as U = h 2^29 + l
+// with h and l int32 and l in [-2^28, 2^28].  A double whose exponent is within
+// five of the largest value's converts exactly; smaller ones round to 2^-58
+// of the scale.  E follows the planes: it is the exponent of the largest
+// value of the three planes held plus one, kept while the next plane fits and
+// is not much smaller, else the planes are loaded and converted again.
+//
+// Arithmetic.  With S = 2 visc/h (an integer in the same scale), A = u_i +
+// u_i(+e_j) - 2S, B = u_j + u_j(+e_i) - 2S,
+//   4 sigma_ij = A B + 4S (u_i + u_j) + const,
+//   4 sigma_ii = (u_i + u_i(-e_i) - 2S)^2 + 8S u_i(-e_i) + const
+// (the shifted stress form, constants cancel in the divergence), so
+//   -4h du_i = D_i S_i + sum_{j != i} [A B - (A B)(-e_j)]
+//              + 4S [sum_j (u_i - u_i(-e_j)) + sum_j (u_j - u_j(-e_j))],
+//   D_i = u_i(+e_i) - u_i(-e_i),  S_i = u_i(+e_i) + 2 u_i + u_i(-e_i) - 4S.
+// Products of (h, l) pairs accumulate in three int64 sums of weight 2^58,
+// 2^29 and 1 -- the addition is part of the multiply-add, no carries travel --
+// and the bounds above keep every sum below 2^63:
+//   in weight 2^29, the largest of the three, the four A B give at most 3 2^60
+//   (|A.h| <= 2^29, |A.l| <= 3 2^28), D_i S_i 1.2 2^60 and the three groups of
+//   the linear term 1.5 2^60 (4S < 2^57): 5.7 2^60 in all.
+// The sum is exact to 2^-85 of the squared scale; converted to a double with
+// one rounding and multiplied by -1/(4h), it is closer to the exact sum than
+// the FP64 operations it replaces wherever a cell's own velocity is within
+// 2^-7 of the tile's largest.  Cells below that, and planes with values that
+// are not finite or out of range, take rhs_cell_f64.
+//
+// Per cell 650 instructions, 88 of them the multiply-adds, 57 shared-memory
+// accesses per 32 cells and 6 FP64 operations (45 before).  512^3: 11.4 -> 3.46
+// ms (HBM floor 0.95), 250^3 1470 -> 492 us, 128^3 215 -> 80, 90^3 102 -> 41,
+// 32^3 47 -> 10.  Bound by the latency of the multiply-add pipe (66% busy) at 8
+// warps per scheduler.  Error against 113-bit arithmetic, relative L2: white
+// noise 0.7-1.1e-16 (FP64 form 1.7-2.1e-16), smooth fields 0.8e-16 (1.2e-15), a
+// mean flow of 100 7e-17 (1.3e-14), visc 0.1 1.4e-16 (7.7e-16).
+// ---------------------------------------------------------------------------
+struct Fx { int h, l; };
+__device__ __forceinline__ Fx operator+(Fx a, Fx b) { return {a.h + b.h, a.l + b.l}; }
+__device__ __forceinline__ Fx operator-(Fx a, Fx b) { return {a.h - b.h, a.l - b.l}; }
+__device__ __forceinline__ Fx operator-(Fx a) { return {-a.h, -a.l}; }
+struct FxSum { long long hh, m, ll; };
+__device__ __forceinline__ void fx_mac(FxSum& s, Fx a, Fx b) {
+  s.hh += (long long)a.h * b.h;
+  s.m += (long long)a.h * b.l;
+  s.m += (long long)a.l * b.h;
+  s.ll += (long long)a.l * b.l;
+}
+constexpr int FX_BITS = 57, FX_LOW = 29;
+// E of the fixed-point path: well inside the range of the FP32 bound that
+// finds it, and squares and their scaling stay normal doubles
+constexpr int FX_EMIN = -100, FX_EMAX = FX_BITS;
+
+// x (|x| < 2^E) in units of 2^(E - 57), rounded to nearest; kexp = (57 - E) <<
+// 20.  On the integer pipe: the FP64 pipe's own conversion measured slower
+// (512^3 3.93 against 3.57 ms), it shares the pipe with fx_to_double's.
+__device__ __forceinline__ Fx fx_from_double(double x, int kexp) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const int e = (int)((hi >> 20) & 0x7ffu);
+  const unsigned mh = (hi & 0xfffffu) | 0x100000u;
+  // mantissa with five more bits (one of them the rounding bit); shr.b64 gives
+  // 0 for counts of 64 and more (small values, zero)
+  const unsigned long long m5 = ((unsigned long long)__funnelshift_l(lo, mh, 5) << 32) | (lo << 5);
+  unsigned long long t;
+  asm("shr.u64 %0, %1, %2;" : "=l"(t) : "l"(m5), "r"(1022 + FX_BITS - (kexp >> 20) - e));
+  const long long U = (long long)((t + 1) >> 1);
+  const int h = (int)((U + (1 << (FX_LOW - 1))) >> FX_LOW);
+  const int l = (int)(unsigned)U - (h << FX_LOW);
+  const int sg = ((int)hi >> 31) | 1;
+  return {h * sg, l * sg};
+}
+
+// (hh 2^58 + m 2^29 + ll) in units of 2^58 times `scale`, with ten more bits
+// (and 2^-10 of scale, by its exponent field) while they fit: to 2^-95 of the
+// squared scale, or to half a unit of the double.
+__device__ __forceinline__ double fx_to_double(const FxSum& s, double scale) {
+  const long long mm = s.m + (s.ll >> FX_LOW);
+  const long long hi = s.hh + (mm >> FX_LOW);
+  const int low10 = ((int)mm >> (FX_LOW - 10)) & 0x3ff;
+  const bool big = (unsigned)((int)(hi >> 32) + 0x200000) >= 0x400000u;  // |hi| >= 2^53
+  const long long v = big ? hi : (hi << 10) | low10;
+  return (double)v * __hiloint2double(__double2hiint(scale) - (big ? 0 : 10 << 20), __double2loint(scale));
+}
+
+// The reference's arithmetic for one cell, from global memory: the cells the
+// fixed-point sweep leaves out.
+__device__ __noinline__ double3 rhs_cell_f64(const double* __restrict__ u, int n, int x, int y, int z, double inv_h,
+                                             double visc) {
+  const long long nn = (long long)n * n, N = nn * n;
+  const double* const a = u + z * nn + (long long)y * n + x;
+  const double *const b = a + N, *const c = b + N;
+  const long long xp = x + 1 == n ? 1 - n : 1, xm = x == 0 ? n - 1 : -1;
+  const long long yp = y + 1 == n ? -(nn - n) : n, ym = y == 0 ? nn - n : -n;
+  const long long zp = z + 1 == n ? -(N - nn) : nn, zm = z == 0 ? N - nn : -nn;
+  const double rv = 4.0 * visc * inv_h;
+  auto diag = [rv](double p, double q) { return (p + q) * (p + q) - 2.0 * rv * (p - q); };
+  auto off = [rv](double p, double q, double r, double t) { return (p + q) * (r + t) - rv * ((q - p) + (t - r)); };
+  // all loads first: they are independent
+  const double a0 = a[0], axp = a[xp], axm = a[xm], ayp = a[yp], aym = a[ym], azp = a[zp], azm = a[zm];
+  const double b0 = b[0], bxp = b[xp], bxm = b[xm], byp = b[yp], bym = b[ym], bzp = b[zp], bzm = b[zm];
+  const double c0 = c[0], cxp = c[xp], cxm = c[xm], cyp = c[yp], cym = c[ym], czp = c[zp], czm = c[zm];
+  const double axmyp = a[xm + yp], axmzp = a[xm + zp], bxpym = b[xp + ym], bymzp = b[ym + zp], cxpzm = c[xp + zm],
+               cypzm = c[yp + zm];
+  const double s12 = off(a0, ayp, b0, bxp), s13 = off(a0, azp, c0, cxp), s23 = off(b0, bzp, c0, cyp);
+  const double k = -0.25 * inv_h;
+  const double d1 = (diag(axp, a0) - diag(a0, axm)) + (s12 - off(aym, a0, bym, bxpym)) + (s13 - off(azm, a0, czm, cxpzm));
+  const double d2 = (s12 - off(axm, axmyp, bxm, b0)) + (diag(byp, b0) - diag(b0, bym)) + (s23 - off(bzm, b0, czm, cypzm));
+  const double d3 = (s13 - off(axm, axmzp, cxm, c0)) + (s23 - off(bym, bymzp, cym, c0)) + (diag(czp, c0) - diag(c0, czm));
+  return make_double3(k * d1, k * d2, k * d3);
+}
+
+// Tile of the fixed-point sweep: 32 x 16 cells, FXC rows per thread, FX_CTAS
+// CTAs per SM (64 registers).  512^3 / 250^3 / 128^3 / 32^3: 3.43 ms / 488 / 78
+// / 10 us; three CTAs (80 registers) 3.75 / 497 / 84 / 10; one row per thread 5.3
+// ms / 701 / 108 / 10 (every shared value loaded once per cell); four rows, five
+// CTAs 3.27 ms / 462 / 88 / 12: the larger tile of work per thread loses on the
+// LES grids and on 128^3.
+constexpr int FXC = 2, FX_CTAS = 4, FXY = 16, FXW = FXY / FXC, FXBY = FXY + 2, FXROW = 36;  // box rows and words per row
+constexpr int FXPIECES = 3 * FXBY * FXROW / 2;                                      // 16-byte pieces of a plane
+constexpr int FXTHREADS = PTX * FXW;
+
+struct FixedSmem {
+  // plane buffers: the box of each component, row after row (one 4-D TMA box),
+  // x = x0 - 2 first; doubles on arrival, then Fx pairs
+  double u[3][3 * FXBY * FXROW + 8];
+  unsigned piece[FXPIECES];      // word offset in the field of each 16-byte piece of a plane
+  unsigned red[3][FXW];          // largest magnitude (high word) per plane buffer and warp
+  unsigned long long bar[3];     // TMA completion of each plane buffer
+};
+static_assert(sizeof(FixedSmem::u[0]) % 128 == 0, "TMA destinations");
+constexpr size_t FIXED_SMEM = sizeof(FixedSmem) + 128;
+
+template <bool DOADD>
+__global__ void __launch_bounds__(FXTHREADS, FX_CTAS)
+rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u, double* __restrict__ du, SlotBatch sb,
+                 int zblocks, int ptz, const __grid_constant__ CUtensorMap umap, int have_map) {
+  using T = double;
+  constexpr int NC = FXC;
+  extern __shared__ __align__(128) unsigned char rhs_smem[];
+  FixedSmem& sm = *reinterpret_cast<FixedSmem*>(rhs_smem + ((128u - (smem_u32(rhs_smem) & 127u)) & 127u));
+  const long long N = (long long)n * n * n, nn = (long long)n * n;
+  const int slot = blockIdx.z / zblocks;
+  const int zb = blockIdx.z - slot * zblocks;
+  if (sb.active && !sb.active[slot]) return;
+  u += slot * sb.ustride;
+  du += slot * sb.ustride;
+  if (sb.visc) visc = reinterpret_cast<const T*>(sb.visc)[slot];
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * PTX + tx;
+  const int x0 = blockIdx.x * PTX, y0 = blockIdx.y * FXY, z0 = zb * ptz;
+  auto wrapm = [n](int g) { return ((g % n) + n) % n; };
+  // plane copies: one TMA box where the box lies inside the grid, else 16-byte
+  // pieces (n is even, so a piece never straddles the periodic boundary), or
+  // words when the field is not 16-byte aligned
+  const bool vec = (reinterpret_cast<uintptr_t>(u) & 15) == 0;
+  const bool tma = vec && have_map && x0 >= 2 && x0 - 2 + FXROW <= n && y0 >= 1 && y0 + FXY + 1 <= n;
+  unsigned parity = 0;
+  const bool drill = tma && g_rhs_drill != 0;
+  const int poll_limit = drill ? RHS_DRILL_POLLS : RHS_POLLS;
+  if (tma) {
+    if (tid == 0) {
+#pragma unroll
+      for (int b = 0; b < 3; ++b) mbar_init(&sm.bar[b], 1);
+      asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+  } else {
+    for (int t = tid; t < FXPIECES; t += FXTHREADS) {
+      const int c = t / (FXBY * FXROW / 2), rem = t - c * (FXBY * FXROW / 2);
+      const int rr = rem / (FXROW / 2), j = rem - rr * (FXROW / 2);
+      // 3 n^3 <= 3 2^30 words: an unsigned offset
+      sm.piece[t] = (unsigned)(c * N) + (unsigned)wrapm(y0 - 1 + rr) * n + wrapm(x0 - 2 + 2 * j);
+    }
+  }
+  __syncthreads();
+  constexpr int NSLOT = (FXPIECES + FXTHREADS - 1) / FXTHREADS;
+  auto load_plane = [&](int buf, int gz) {
+    if (tma) {
+      if (tid == 0 && !drill) {
+        mbar_expect_tx(&sm.bar[buf], 3u * FXBY * FXROW * sizeof(T));
+        tma_load_4d(sm.u[buf], &umap, x0 - 2, y0 - 1, gz, 3 * slot, &sm.bar[buf]);
+      }
+      return;
+    }
+    const T* const ub = u + gz * nn;
+#pragma unroll
+    for (int i = 0; i < NSLOT; ++i) {
+      const int t = tid + i * FXTHREADS;
+      if (t < FXPIECES) {
+        T* const d = sm.u[buf] + 2 * t;
+        const T* const g = ub + sm.piece[t];
+        if (vec) {
+          cp_async_16(d, g);
+        } else {
+          cp_async_word(d, g);
+          cp_async_word(d + 1, g + 1);
+        }
+      }
+    }
+    cp_async_commit();
+  };
+  auto wait_plane = [&](int buf) {
+    if (!tma) {
+      cp_async_wait_all();
+      return;
+    }
+    int polls = 0;
+    while (!mbar_try_wait(&sm.bar[buf], (parity >> buf) & 1u)) {
+      if (++polls > poll_limit) {
+        if (tid == 0) atomicExch(&g_rhs_tma_fault, 1);
+        break;
+      }
+    }
+    parity ^= 1u << buf;
+  };
+  // f(value) over this thread's pieces of plane buffer buf, after its wait (a
+  // TMA plane's mbarrier wait makes every copy visible, else it copied them)
+  auto each_value = [&](int buf, auto f) {
+#pragma unroll
+    for (int i = 0; i < NSLOT; ++i) {
+      const int t = tid + i * FXTHREADS;
+      if (t < FXPIECES) {
+        double2* const p2 = reinterpret_cast<double2*>(sm.u[buf]) + t;
+        double2 v = *p2;
+        f(v.x);
+        f(v.y);
+        *p2 = v;
+      }
+    }
+  };
+  // largest magnitude of a plane (high words), this warp's part, into sm.red
+  auto scan_plane = [&](int buf) {
+    unsigned m = 0;
+    each_value(buf, [&](double& v) { m = max(m, (unsigned)__double2hiint(v) & 0x7fffffffu); });
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (tx == 0) sm.red[buf][ty] = m;
+  };
+  auto plane_max = [&](int buf) {
+    return __reduce_max_sync(0xffffffffu, tx < FXW ? sm.red[buf][tx] : 0u);
+  };
+  int E = 0;                     // |u| + S < 2^E for the planes held
+  int kexp = 0;                  // (57 - E) << 20
+  double scale = 0;              // -1/(4h) 2^58 in fixed-point units squared
+  auto convert_plane = [&](int buf) {
+    each_value(buf, [&](double& v) {
+      const Fx q = fx_from_double(v, kexp);
+      v = __hiloint2double(q.h, q.l);
+    });
+  };
+  Fx S2{}, S4{};  // 2S and 4S in fixed point
+  int tiny = 0;   // cells whose h words are all below this take the FP64 path
+  bool slow = false;
+  unsigned pm1 = 0, pm2 = 0;  // largest magnitudes of the upper two planes held
+  // E for planes whose largest magnitude has high word mx: above |u| + S
+  // (and above 4S, so that 4S converts); the FP64 path if it is out of range
+  // (in FP32, whose range covers the path's; bounds rounded up)
+  float Sf = 2.0 * visc * inv_h < 1e30 ? __double2float_ru(2.0 * visc * inv_h) : 1e30f;
+  asm volatile("" : "+f"(Sf));  // kept, not recomputed on the FP64 pipe
+  auto exponent_for = [&](unsigned mx) {
+    const unsigned m = mx < 0x39000000u ? 0u : mx >= 0x47000000u ? 0x7f000000u : ((mx - 0x38000000u) << 3) + 8u;
+    const float bound = fmaxf(__fadd_ru(__uint_as_float(m), Sf), 4.0f * Sf);
+    return (int)(__float_as_uint(bound) >> 23) - 126;
+  };
+  auto fxat = [&](int buf, int c, int row, int col) {
+    const double v = sm.u[buf][(c * FXBY + row) * FXROW + col];
+    return Fx{__double2hiint(v), __double2loint(v)};
+  };
+  const int col = tx + 2;
+  // previous plane at this thread's cells: the velocities and B of s13, s23
+  Fx pw1[NC], pw2[NC], pw3[NC], pb13[NC], pb23[NC];
+  auto keep = [&](int buf) {
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      const int r = NC * ty + 1 + i;
+      pw1[i] = fxat(buf, 0, r, col);
+      pw2[i] = fxat(buf, 1, r, col);
+      pw3[i] = fxat(buf, 2, r, col);
+      pb13[i] = pw3[i] + fxat(buf, 2, r, col + 1) - S2;
+      pb23[i] = pw3[i] + fxat(buf, 2, r + 1, col) - S2;
+    }
+  };
+  // planes z - 1, z, z + 1 into buffers 0, 1, 2, the scale for them, and the
+  // previous plane's values
+  int cur = 1, nxt = 2, pre = 0;
+  auto start = [&](int z) {
+    load_plane(0, wrapm(z - 1));
+    load_plane(1, wrapm(z));
+    load_plane(2, wrapm(z + 1));
+#pragma unroll 1
+    for (int b = 0; b < 3; ++b) wait_plane(b);
+#pragma unroll 1
+    for (int b = 0; b < 3; ++b) scan_plane(b);
+    __syncthreads();
+    pm1 = plane_max(1);
+    pm2 = plane_max(2);
+    const unsigned mx = max(plane_max(0), max(pm1, pm2));
+    const double S = 2.0 * visc * inv_h;
+    E = exponent_for(mx);
+    slow = mx >= 0x7fe00000u || !(S < 1e300) || E > FX_EMAX || E < FX_EMIN;
+    if (!slow) {
+      kexp = (FX_BITS - E) << 20;
+      scale = ldexp(-0.25 * inv_h, 2 * FX_LOW + 2 * (E - FX_BITS));
+      const Fx s = fx_from_double(4.0 * S, kexp);
+      // 4S to a multiple of four units, so that S and 2S are the same S
+      const long long s4 = (((long long)s.h << FX_LOW) + s.l + 2) >> 2 << 2;
+      const long long s2 = s4 >> 1;
+      S4 = {(int)((s4 + (1 << (FX_LOW - 1))) >> FX_LOW), 0};
+      S4.l = (int)(s4 - ((long long)S4.h << FX_LOW));
+      S2 = {(int)((s2 + (1 << (FX_LOW - 1))) >> FX_LOW), 0};
+      S2.l = (int)(s2 - ((long long)S2.h << FX_LOW));
+      // 2^-7 of the top of the largest magnitude's binade, in units of h (the
+      // FP64 path at 2^-5 costs 250^3 27% of its time, at 2^-7 nothing)
+      const int q = FX_BITS - FX_LOW - 7 - (E - (int)((mx >> 20) & 0x7ff) + 1022);
+      tiny = mx == 0 ? 0 : q < 0 ? 0 : 1 << q;
+#pragma unroll 1
+      for (int b = 0; b < 3; ++b) convert_plane(b);
+    }
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    __syncthreads();
+    if (!slow) keep(0);
+    __syncthreads();  // buffer 0 is refilled by the first prefetch
+    cur = 1;
+    nxt = 2;
+    pre = 0;
+  };
+  start(z0);
+  const int gx = x0 + tx;
+  for (int kz = 0; kz < ptz; ++kz) {
+    const int z = z0 + kz;
+    if (z >= n) break;  // uniform across the CTA
+    const bool more = kz + 1 < ptz && z + 1 < n;
+    if (more && !slow) load_plane(pre, wrapm(z + 2));
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      const int r = NC * ty + 1 + i, gy = y0 + NC * ty + i;
+      const Fx a = fxat(cur, 0, r, col), b = fxat(cur, 1, r, col), c = fxat(cur, 2, r, col);
+      double o1, o2, o3;
+      bool direct = slow || (max(abs(a.h), max(abs(b.h), abs(c.h))) < tiny);
+      if (!slow) {
+        // u1: neighbours along x, y, z and (-x, +y), (-x, +z)
+        const Fx axp = fxat(cur, 0, r, col + 1), axm = fxat(cur, 0, r, col - 1);
+        const Fx ayp = fxat(cur, 0, r + 1, col), aym = fxat(cur, 0, r - 1, col);
+        const Fx axmyp = fxat(cur, 0, r + 1, col - 1);
+        const Fx azp = fxat(nxt, 0, r, col), axmzp = fxat(nxt, 0, r, col - 1);
+        // u2: along x, y, z and (+x, -y), (-y, +z)
+        const Fx bxp = fxat(cur, 1, r, col + 1), bxm = fxat(cur, 1, r, col - 1);
+        const Fx byp = fxat(cur, 1, r + 1, col), bym = fxat(cur, 1, r - 1, col);
+        const Fx bxpym = fxat(cur, 1, r - 1, col + 1);
+        const Fx bzp = fxat(nxt, 1, r, col), bymzp = fxat(nxt, 1, r - 1, col);
+        // u3: along x, y, z
+        const Fx cxp = fxat(cur, 2, r, col + 1), cxm = fxat(cur, 2, r, col - 1);
+        const Fx cyp = fxat(cur, 2, r + 1, col), cym = fxat(cur, 2, r - 1, col);
+        const Fx czp = fxat(nxt, 2, r, col);
+        // the linear term's group common to the components
+        FxSum s0{0, 0, 0};
+        fx_mac(s0, (a - axm) + (b - bym), S4);
+        const Fx dz3 = c - pw3[i];
+        const Fx A12 = a + ayp - S2, B12 = b + bxp - S2;
+        const Fx A13 = a + azp - S2, B13 = c + cxp - S2;
+        const Fx A23 = b + bzp - S2, B23 = c + cyp - S2;
+        {
+          FxSum s = s0;
+          fx_mac(s, dz3 + (a - axm), S4);
+          fx_mac(s, (a - aym) + (a - pw1[i]), S4);
+          fx_mac(s, axp - axm, (axp + axm) + (a + a) - S4);
+          fx_mac(s, A12, B12);
+          fx_mac(s, S2 - a - aym, bym + bxpym - S2);
+          fx_mac(s, A13, B13);
+          fx_mac(s, S2 - a - pw1[i], pb13[i]);
+          o1 = fx_to_double(s, scale);
+        }
+        {
+          FxSum s = s0;
+          fx_mac(s, dz3 + (b - bxm), S4);
+          fx_mac(s, (b - bym) + (b - pw2[i]), S4);
+          fx_mac(s, byp - bym, (byp + bym) + (b + b) - S4);
+          fx_mac(s, A12, B12);
+          fx_mac(s, S2 - axm - axmyp, bxm + b - S2);
+          fx_mac(s, A23, B23);
+          fx_mac(s, S2 - b - pw2[i], pb23[i]);
+          o2 = fx_to_double(s, scale);
+        }
+        {
+          FxSum s = s0;
+          fx_mac(s, dz3 + (c - cxm), S4);
+          fx_mac(s, (c - cym) + dz3, S4);
+          fx_mac(s, czp - pw3[i], (czp + pw3[i]) + (c + c) - S4);
+          fx_mac(s, A13, B13);
+          fx_mac(s, S2 - axm - axmzp, cxm + c - S2);
+          fx_mac(s, A23, B23);
+          fx_mac(s, S2 - bym - bymzp, cym + c - S2);
+          o3 = fx_to_double(s, scale);
+        }
+        pw1[i] = a;
+        pw2[i] = b;
+        pw3[i] = c;
+        pb13[i] = B13;
+        pb23[i] = B23;
+      }
+      if (gx < n && gy < n) {
+        if (direct) {
+          const double3 o = rhs_cell_f64(u, n, gx, gy, z, inv_h, visc);
+          o1 = o.x;
+          o2 = o.y;
+          o3 = o.z;
+        }
+        double* const d = du + ((long long)z * n + gy) * n + gx;
+        if (DOADD) {
+          d[0] += o1;
+          d[N] += o2;
+          d[2 * N] += o3;
+        } else {
+          d[0] = o1;
+          d[N] = o2;
+          d[2 * N] = o3;
+        }
+      }
+    }
+    if (!more) break;
+    if (slow) {
+      __syncthreads();
+      start(z + 1);
+      continue;
+    }
+    wait_plane(pre);
+    scan_plane(pre);
+    __syncthreads();
+    const unsigned pm = plane_max(pre);
+    const int En = exponent_for(max(pm, max(pm1, pm2)));
+    if (pm >= 0x7fe00000u || En > E || En < E - 2) {
+      start(z + 1);
+      continue;
+    }
+    convert_plane(pre);
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    __syncthreads();
+    pm1 = pm2;
+    pm2 = pm;
     const int freed = cur;
     cur = nxt;
     nxt = pre;
@@ -796,60 +1173,86 @@ static bool field_tensor_map(const T* u, int n, int nslots, const SlotBatch& sb,
              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename T>
-cudaError_t launch_rhs(int n, T h, T visc, const T* u, T* du, bool doadd, cudaStream_t st, const SlotBatch& sb,
-                       int nslots, bool pre_shifted) {
-  constexpr int NC = CYT<T>;
-  // planes per CTA (4 to 32): the fewest waves of resident CTAs (`per_sm`
-  // per SM) times the planes each CTA walks plus one for its start (three
-  // planes loaded, the previous plane's stresses), ties to more planes -- so
-  // small grids and single solves still fill the GPU without a nearly empty
-  // last wave.  The split changes no cell's arithmetic.
-  auto zsplit = [&](long long columns, int per_sm, int& ptz, int& zblocks) {
-    const long long slots = (long long)per_sm * 152;
-    long long best = -1;
-    for (int c = 32; c >= 4; --c) {
-      const int zb = (n + c - 1) / c;
-      const long long waves = (columns * zb * nslots + slots - 1) / slots;
-      if (best < 0 || waves * (c + 1) < best) {
-        best = waves * (c + 1);
-        ptz = c;
-        zblocks = zb;
-      }
-    }
-    return columns * zblocks * nslots;
-  };
-  int ptz, zblocks;
-  if constexpr (sizeof(T) == 4) {
-    // grids of 64-multiples with 16-byte aligned fields and at least one full
-    // wave of CTAs (three per SM): the 2 x 2 kernel
-    if (n % QX == 0 && (reinterpret_cast<uintptr_t>(u) & 15) == 0 && (reinterpret_cast<uintptr_t>(du) & 15) == 0 &&
-        zsplit((long long)(n / QX) * (n / QY), 3, ptz, zblocks) >= 3LL * 152) {
-      dim3 gq(n / QX, n / QY, zblocks * nslots);
-      const float ih = (float)(1.0 / (double)h);
-      CUtensorMap map;
-      const int have = field_tensor_map<float>((const float*)u, n, nslots, sb, QROW, QBY, &map) ? 1 : 0;
-      if (doadd)
-        rhs_quad_kernel<true><<<gq, dim3(32, 8), QUAD_SMEM, st>>>(n, ih, (float)visc, (const float*)u, (float*)du, sb,
-                                                                  zblocks, ptz, map, have);
-      else
-        rhs_quad_kernel<false><<<gq, dim3(32, 8), QUAD_SMEM, st>>>(n, ih, (float)visc, (const float*)u, (float*)du, sb,
-                                                                   zblocks, ptz, map, have);
-      return cudaGetLastError();
+// Planes per CTA (cmin to 32): the fewest waves of resident CTAs (`per_sm` per
+// SM) times the planes each CTA walks plus `start` for its start (three planes
+// loaded, the previous plane's part), ties to more planes -- so small grids and
+// single solves still fill the GPU without a nearly empty last wave.  The split
+// changes no cell's arithmetic.  Returns the CTAs of the launch.
+static long long zsplit(int n, int nslots, long long columns, int per_sm, int cmin, int start, int& ptz,
+                        int& zblocks) {
+  const long long slots = (long long)per_sm * 152;
+  long long best = -1;
+  for (int c = 32; c >= cmin; --c) {
+    const int zb = (n + c - 1) / c;
+    const long long waves = (columns * zb * nslots + slots - 1) / slots;
+    if (best < 0 || waves * (c + start) < best) {
+      best = waves * (c + start);
+      ptz = c;
+      zblocks = zb;
     }
   }
-  const int gxb = (n + PTX - 1) / PTX, gyb = (n + PTYT<NC> - 1) / PTYT<NC>;
-  zsplit((long long)gxb * gyb, sizeof(T) == 4 ? 4 : 3, ptz, zblocks);
-  dim3 grid(gxb, gyb, zblocks * nslots);
-  const size_t sh = plane_smem_bytes<T, NC>();
-  CUtensorMap map;
-  const int have = field_tensor_map<T>(u, n, nslots, sb, UROW<T>, PBYT<NC>, &map) ? 1 : 0;
+  return columns * zblocks * nslots;
+}
+
+// FP64: the fixed-point sweep, one plane per CTA and up (a 32^3 grid takes 64
+// CTAs of one plane: 10 us, 16 us with four).
+template <>
+cudaError_t launch_rhs<double>(int n, double h, double visc, const double* u, double* du, bool doadd, cudaStream_t st,
+                               const SlotBatch& sb, int nslots) {
+  int ptz, zblocks;
+  dim3 grid((n + PTX - 1) / PTX, (n + FXY - 1) / FXY, 1);
+  zsplit(n, nslots, (long long)grid.x * grid.y, FX_CTAS, 1, 2, ptz, zblocks);
+  grid.z = zblocks * nslots;
+  // the field as (x, y, z, slot * 3 + component), boxes of one plane of the
+  // three components
+  CUtensorMap map{};
+  const long long N = (long long)n * n * n;
+  const cuuint64_t dims[4] = {(cuuint64_t)n, (cuuint64_t)n, (cuuint64_t)n, (cuuint64_t)nslots * 3};
+  const cuuint64_t strides[3] = {(cuuint64_t)n * 8, (cuuint64_t)n * n * 8, (cuuint64_t)N * 8};
+  const cuuint32_t box[4] = {FXROW, FXBY, 1, 3};
+  const int have = (nslots == 1 || sb.ustride == 3 * N) && (reinterpret_cast<uintptr_t>(u) & 15) == 0 && n >= FXROW &&
+                   encode_tiled_map(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, u, dims, strides, box);
+  const dim3 block(PTX, FXW);
   if (doadd)
-    rhs_kernel<T, NC, true><<<grid, dim3(PTX, NWARP), sh, st>>>(n, (T)(1.0 / (double)h), visc, u, du, sb, zblocks, ptz,
-                                                                map, have, pre_shifted ? 1 : 0);
+    rhs_fixed_kernel<true><<<grid, block, FIXED_SMEM, st>>>(n, 1.0 / h, visc, u, du, sb, zblocks, ptz, map, have);
   else
-    rhs_kernel<T, NC, false><<<grid, dim3(PTX, NWARP), sh, st>>>(n, (T)(1.0 / (double)h), visc, u, du, sb, zblocks,
-                                                                 ptz, map, have, pre_shifted ? 1 : 0);
+    rhs_fixed_kernel<false><<<grid, block, FIXED_SMEM, st>>>(n, 1.0 / h, visc, u, du, sb, zblocks, ptz, map, have);
+  return cudaGetLastError();
+}
+
+template <>
+cudaError_t launch_rhs<float>(int n, float h, float visc, const float* u, float* du, bool doadd, cudaStream_t st,
+                              const SlotBatch& sb, int nslots) {
+  constexpr int NC = CYT<float>;
+  int ptz, zblocks;
+  // grids of 64-multiples with 16-byte aligned fields and at least one full
+  // wave of CTAs (three per SM): the 2 x 2 kernel
+  if (n % QX == 0 && (reinterpret_cast<uintptr_t>(u) & 15) == 0 && (reinterpret_cast<uintptr_t>(du) & 15) == 0 &&
+      zsplit(n, nslots, (long long)(n / QX) * (n / QY), 3, 4, 1, ptz, zblocks) >= 3LL * 152) {
+    dim3 gq(n / QX, n / QY, zblocks * nslots);
+    const float ih = (float)(1.0 / (double)h);
+    CUtensorMap map;
+    const int have = field_tensor_map<float>(u, n, nslots, sb, QROW, QBY, &map) ? 1 : 0;
+    if (doadd)
+      rhs_quad_kernel<true><<<gq, dim3(32, 8), QUAD_SMEM, st>>>(n, ih, visc, u, du, sb,
+                                                                zblocks, ptz, map, have);
+    else
+      rhs_quad_kernel<false><<<gq, dim3(32, 8), QUAD_SMEM, st>>>(n, ih, visc, u, du, sb,
+                                                                 zblocks, ptz, map, have);
+    return cudaGetLastError();
+  }
+  const int gxb = (n + PTX - 1) / PTX, gyb = (n + PTYT<NC> - 1) / PTYT<NC>;
+  zsplit(n, nslots, (long long)gxb * gyb, 4, 4, 1, ptz, zblocks);
+  dim3 grid(gxb, gyb, zblocks * nslots);
+  const size_t sh = plane_smem_bytes<float, NC>();
+  CUtensorMap map;
+  const int have = field_tensor_map<float>(u, n, nslots, sb, UROW<float>, PBYT<NC>, &map) ? 1 : 0;
+  if (doadd)
+    rhs_kernel<float, NC, true><<<grid, dim3(PTX, NWARP), sh, st>>>(n, (float)(1.0 / (double)h), visc, u, du, sb, zblocks, ptz,
+                                                                map, have);
+  else
+    rhs_kernel<float, NC, false><<<grid, dim3(PTX, NWARP), sh, st>>>(n, (float)(1.0 / (double)h), visc, u, du, sb, zblocks,
+                                                                 ptz, map, have);
   return cudaGetLastError();
 }
 
@@ -869,14 +1272,12 @@ cudaError_t configure_stencil() {
     e = cudaFuncSetAttribute(rhs_quad_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)QUAD_SMEM);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(rhs_quad_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)QUAD_SMEM);
-  if (e == cudaSuccess) e = configure_rhs_t<double>();
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(rhs_fixed_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FIXED_SMEM);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(rhs_fixed_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FIXED_SMEM);
   return e;
 }
-
-template cudaError_t launch_rhs<double>(int, double, double, const double*, double*, bool, cudaStream_t,
-                                        const SlotBatch&, int, bool);
-template cudaError_t launch_rhs<float>(int, float, float, const float*, float*, bool, cudaStream_t, const SlotBatch&,
-                                       int, bool);
 
 }  // namespace exc
 

@@ -1,6 +1,7 @@
 // FFT Poisson solver: R2C along x, complex passes along y and z with the
 // spectral divide of `project!` (src/N.jl:272-298) fused between the forward
 // and inverse z transforms, then C2R along x back into the work array.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -390,10 +391,11 @@ cudaError_t poisson_solve_inplace(exc_poisson* ps, const T* src, bool src_is_vec
                                   const SlotBatch& sb, int nslots) {
   if constexpr (sizeof(T) == 8) {
     if (ps->engine == 0 && ps->mix && nslots == 1 && !sb.active)
-      return fftmix_solve(ps, reinterpret_cast<const double*>(src), src_is_vector, st);
+      return ps->mix->gen ? gen_mix_solve(ps, src, src_is_vector, st) : fftmix_solve(ps, src, src_is_vector, st);
   }
   if (ps->engine != 1 && ps->twl_n && ps->twl_h && ps->invlap)
-    return fftreg_solve(ps, src, src_is_vector, st, sb, nslots);
+    return ps->gen ? gen_solve(ps, src, src_is_vector, st, sb, nslots)
+                   : fftreg_solve(ps, src, src_is_vector, st, sb, nslots);
   if (plan_ext(ps->plan_n) || plan_ext(ps->plan_h))
     return stockham_solve<T, true>(ps, src, src_is_vector, st, sb, nslots);
   return stockham_solve<T, false>(ps, src, src_is_vector, st, sb, nslots);
@@ -498,6 +500,7 @@ cudaError_t configure_fft() {
   if (e == cudaSuccess) e = configure_fftreg_f64();
   if (e == cudaSuccess) e = configure_fftreg_f32();
   if (e == cudaSuccess) e = configure_fftmix();
+  if (e == cudaSuccess) e = configure_gen();
   return e;
 }
 
@@ -520,10 +523,10 @@ static std::vector<C> level_table(int L, int N1) {
 }
 
 template <typename C>
-static int alloc_level_tables(exc_poisson* ps) {
+static int alloc_level_tables(exc_poisson* ps, int n1, int h1) {
   const int n = ps->n;
-  const std::vector<C> tn = level_table<C>(n, reg_split_host(n));
-  const std::vector<C> th = level_table<C>(n / 2, reg_split_host(n / 2));
+  const std::vector<C> tn = level_table<C>(n, n1);
+  const std::vector<C> th = level_table<C>(n / 2, h1);
   if (cudaMalloc(&ps->twl_n, tn.size() * sizeof(C)) != cudaSuccess ||
       cudaMalloc(&ps->twl_h, th.size() * sizeof(C)) != cudaSuccess) {
     set_last_error("out of device memory (poisson level twiddles)");
@@ -532,6 +535,21 @@ static int alloc_level_tables(exc_poisson* ps) {
   cudaMemcpy(ps->twl_n, tn.data(), tn.size() * sizeof(C), cudaMemcpyHostToDevice);
   cudaMemcpy(ps->twl_h, th.data(), th.size() * sizeof(C), cudaMemcpyHostToDevice);
   return EXC_OK;
+}
+
+// FP64 grids that solve by mixed-precision refinement: those with a compiled
+// plan, and the others with an FP32 run-time plan where its 16 launches beat
+// the 5 of the FP64 run-time plan.  Projection, FP64 plan against mixed: 72^3
+// 130 / 143 us, 80^3 159 / 170, 84^3 185 / 179, 90^3 224 / 189, 250^3 (Stockham)
+// 3.90 / 1.60 ms, 500^3 33.1 / 11.4.  Its pressure is closer to 113-bit
+// arithmetic than the FP64 transforms' (90^3 white noise 4.4e-16 against
+// 1.1e-15, velocity 1.1e-16 against 4.6e-16).
+constexpr int GEN_MIX_MIN = 84;
+static bool mix_wanted(int n) {
+  return fftmix_supported(n) || (n >= GEN_MIX_MIN && !fftreg_supported(n, EXC_F32) && gen_supported(n, EXC_F32));
+}
+static long long mix_part_words(int n) {
+  return fftmix_supported(n) ? fftmix_part_words(n) : std::max(gen_mix_parts(n), (long long)MIX_SUM_CTAS) + 2;
 }
 
 int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work) {
@@ -584,11 +602,14 @@ int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work) {
     if (precision == EXC_F32)
       invlap_split_kernel<<<(int)std::min<long long>((tot + 255) / 256, 152LL * 32), 256>>>(tot, ps->invlap);
   }
-  if (fftreg_supported(n, precision)) {
-    const int rc = precision == EXC_F64 ? alloc_level_tables<double2>(ps) : alloc_level_tables<float2>(ps);
+  ps->gen = !fftreg_supported(n, precision) && gen_supported(n, precision);
+  if (ps->gen || fftreg_supported(n, precision)) {
+    int n1 = reg_split_host(n), h1 = reg_split_host(n / 2);
+    if (ps->gen) gen_splits(n, precision, &n1, &h1);
+    const int rc = precision == EXC_F64 ? alloc_level_tables<double2>(ps, n1, h1) : alloc_level_tables<float2>(ps, n1, h1);
     if (rc) { poisson_free(ps); return rc; }
   }
-  if (precision == EXC_F64 && !work && fftmix_supported(n)) {
+  if (precision == EXC_F64 && !work && mix_wanted(n)) {
     // the mixed-precision solve's FP32 inner solver, with the factor 1/h of
     // the unscaled FP64 divergence folded into its divide table
     ps->mix = new exc_poisson;
@@ -602,7 +623,7 @@ int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work) {
     if (cudaMalloc(&ps->mix_d, (size_t)n * n * n * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&ps->mix_q, (size_t)n * n * n * sizeof(float)) != cudaSuccess ||
         cudaMalloc(&ps->mix_q2, (size_t)n * n * n * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&ps->mix_part, (size_t)fftmix_part_words(n) * sizeof(double)) != cudaSuccess) {
+        cudaMalloc(&ps->mix_part, (size_t)mix_part_words(n) * sizeof(double)) != cudaSuccess) {
       set_last_error("out of device memory (mixed-precision poisson buffers)");
       poisson_free(ps);
       return EXC_ERR_OOM;

@@ -1,0 +1,30 @@
+// Run-time register plans (fftgen.cuh): x passes, float.
+#include "fftgen.cuh"
+
+namespace exc {
+
+template <>
+void gen_r2c<float>(const GenArgs<float>& a, const GenSrc<float>& s) {
+  using C = cplx<float>;
+  const int n = a.ps->n;
+  gr2c_kernel<float><<<dim3((unsigned)((n * n + a.rw - 1) / a.rw), a.nslots), GEN_THREADS, (size_t)a.rw * gen_xs(a.half) * sizeof(C), a.st>>>(
+      s, a.half, n, a.rw, reinterpret_cast<C*>(a.ps->work), a.ps->P, reinterpret_cast<const C*>(a.ps->tw),
+      reinterpret_cast<const C*>(a.ps->twl_h), a.sb);
+}
+
+template <>
+void gen_c2r<float>(const GenArgs<float>& a, const GenDst& d) {
+  using C = cplx<float>;
+  const int n = a.ps->n;
+  gc2r_kernel<float><<<dim3((unsigned)((n * n + a.rw - 1) / a.rw), a.nslots), GEN_THREADS, (size_t)a.rw * gen_xs(a.half) * sizeof(C), a.st>>>(
+      reinterpret_cast<C*>(a.ps->work), a.half, n, a.rw, a.ps->P, reinterpret_cast<const C*>(a.ps->tw),
+      reinterpret_cast<const C*>(a.ps->twl_h), d, a.sb);
+}
+
+template <>
+cudaError_t configure_gen_x<float>() {
+  cudaError_t e = cudaFuncSetAttribute(gr2c_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEN_SMEM_MAX);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(gc2r_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEN_SMEM_MAX);
+}
+
+}  // namespace exc

@@ -96,7 +96,7 @@ struct ComposedDft {
 template <int R, bool INV, typename C>
 __device__ __forceinline__ void dft_reg(C* v) {
   if constexpr (R == 1) {
-  } else if constexpr (R == 2 || R == 3 || R == 4 || R == 5 || R == 8) {
+  } else if constexpr (R == 2 || R == 3 || R == 4 || R == 5 || R == 7 || R == 8 || R == 11 || R == 13 || R == 17) {
     dft_small<R, INV, C>(v);
   } else {
     constexpr int A = reg_radix_a(R);

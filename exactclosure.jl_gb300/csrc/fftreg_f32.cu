@@ -13,7 +13,8 @@ int reg_split_host(int L) { return reg_split(L); }
 void fftreg_geometry_f64(int n, int* col_w, int* x_rows);
 void fftreg_geometry_f32(int n, int* col_w, int* x_rows);
 void fftreg_geometry(int n, int precision, int* col_w, int* x_rows) {
-  if (precision == EXC_F32) fftreg_geometry_f32(n, col_w, x_rows);
+  if (!fftreg_supported(n, precision) && gen_supported(n, precision)) gen_geometry(n, precision, col_w, x_rows);
+  else if (precision == EXC_F32) fftreg_geometry_f32(n, col_w, x_rows);
   else fftreg_geometry_f64(n, col_w, x_rows);
 }
 

@@ -23,8 +23,9 @@ struct exc_poisson {
   // shared-memory passes
   void* twl_n = nullptr;
   void* twl_h = nullptr;
+  bool gen = false;  // those tables are of a run-time plan (fftgen.cuh), not of a compiled one
   // engine 0: the mixed-precision solve where built (FP64 grids with an FP32
-  // register plan, fftmix.cu), else the register passes, else Stockham;
+  // register plan, mix_wanted), else the register passes, else Stockham;
   // 1: the FP64 shared-memory Stockham passes; 2: the FP64 register passes
   // where planned, else Stockham (no mixed precision)
   int engine = 0;
@@ -81,6 +82,24 @@ bool fftmix_supported(int n);
 long long fftmix_part_words(int n);
 cudaError_t fftmix_solve(exc_poisson* ps, const double* src, bool src_is_vector, cudaStream_t st);
 cudaError_t configure_fftmix();
+// Fixed-order means of the mixed solves: of a dense field (part[0], its
+// MIX_SUM_CTAS partial sums after it), and of a field given its CTA sums.
+constexpr int MIX_SUM_CTAS = 1024;
+void launch_mix_mean_of(const double* src, long long count, double* part, cudaStream_t st);
+void launch_mix_mean(const double* part, int nparts, double invN, double* mean, cudaStream_t st);
+// The same two solves on run-time register plans (fftgen.cu), for the grids
+// without a compiled one: grids they cover, first factors of the columns and
+// the x lines, geometry, partial sums of the mixed solve.
+bool gen_supported(int n, int precision);
+void gen_splits(int n, int precision, int* n1, int* h1);
+void gen_geometry(int n, int precision, int* col_w, int* x_rows);
+cudaError_t gen_solve(exc_poisson* ps, const float* src, bool src_is_vector, cudaStream_t st, const SlotBatch& sb,
+                      int nslots);
+cudaError_t gen_solve(exc_poisson* ps, const double* src, bool src_is_vector, cudaStream_t st, const SlotBatch& sb,
+                      int nslots);
+long long gen_mix_parts(int n);
+cudaError_t gen_mix_solve(exc_poisson* ps, const double* src, bool src_is_vector, cudaStream_t st);
+cudaError_t configure_gen();
 // Lines per column tile and rows per x-pass CTA of a grid's register plan.
 void fftreg_geometry(int n, int precision, int* col_w, int* x_rows);
 // Read and clear the learned closure's tensor-core wait fault flag.

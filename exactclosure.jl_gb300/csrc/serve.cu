@@ -415,11 +415,14 @@ static int tune_chunk(exc_server* sv, Chunk<T>* ck) {
   cudaEventCreate(&a);
   cudaEventCreate(&b);
   // candidates: the register-resident passes (where the grid has a plan) and
-  // the Stockham passes over the tile shapes above
+  // the Stockham passes over the tile shapes above; a run-time plan measured
+  // faster at every size it covers, and alone it gives a solve the case path's
+  // bits whatever the batch
   std::vector<Tuned> cands;
   if (ck->ps.twl_n && ck->ps.twl_h) cands.push_back({0, 0, 0});
-  for (int w : ws)
-    for (int r : rs) cands.push_back({1, w, r});
+  if (!ck->ps.gen)
+    for (int w : ws)
+      for (int r : rs) cands.push_back({1, w, r});
   float best = 1e30f;
   Tuned bc = cands.front();
   for (const Tuned& c : cands) {

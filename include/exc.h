@@ -110,15 +110,17 @@ int exc_device_sync(void* stream, int* flags);
 int exc_debug_wait_drill(int flags);
 
 /* FFT engine of a solver (no counterpart in the reference).  0 (the
- * default): in FP64 on grids n = 128, 192, 256, 384, 512, 1024 a
+ * default): in FP64 on grids n = 128, 192, 256 and on grids n >= 84 without a
+ * compiled FP64 plan whose n and n/2 split into two factors of at most 34 a
  * mixed-precision solve (three FP32 register-pass solves refined by residuals
  * formed in FP64: the pressure agrees with the FP64 FFT solve to FP64
  * rounding); otherwise register-resident two-level passes where the grid has
- * a plan (n = 32, 48, 64, 96, 128, 192, 256 and, in FP32, 384, 512, 1024),
- * shared-memory Stockham passes for the rest.  1 = FP64/FP32 Stockham passes
- * for every grid.  2 = register passes where planned, else Stockham, in the
- * solver's own precision throughout.  Results agree to round-off; the
- * autotuner of the serving form picks per grid. */
+ * a plan (compiled for n = 32, 48, 64, 96, 128, 192, 256 and, in FP32, 384,
+ * 512, 1024; at run time where n and n/2 split into two factors of at most 34
+ * in FP32, of at most 17 in FP64 for n < 160), shared-memory Stockham passes for the rest.  1 =
+ * FP64/FP32 Stockham passes for every grid.  2 = register passes where
+ * planned, else Stockham, in the solver's own precision throughout.  Results
+ * agree to round-off; the autotuner of the serving form picks per grid. */
 int exc_poisson_set_engine(exc_poisson* ps, int engine);
 /* p with L_h p = d, mean(p) = 0 (src/N.jl:262-301).  d and p may alias. */
 int exc_poisson_solve(exc_poisson* ps, const void* d, void* p, void* stream);

@@ -9,13 +9,15 @@
 // closure terms go through L2.  Samples advance with their own time step
 // (src/Burgers.jl:307 loops over samples, each with its own `cfl`), so the
 // CTAs never wait on each other; a CTA finishing one sample takes the next.
-// Everything is FP64 like the reference, which makes the kernels FP64-pipe
-// bound on GB300.
+// States and updates are FP64 like the reference.  The DNS-aided loop keeps
+// the velocity in registers and filters in fixed point on the integer pipe
+// (advance_les_kernel); the plain DNS loop is bound by the FP64 pipe.
 //
 // Indexing: sample-major [ns][nh], x fastest (the reference's zeros(nh, ns)
 // column-major matrices).  Fine index j (0-based) is the reference's j+1.
 // Coarse cell I (0-based) reads the fine face (I+1)c - 1 and the fine centre
 // (I+1)c - a - 1, a = c / 2 (`lazycoarsegrain`, src/Burgers.jl:174-180).
+#include "fixed.cuh"
 #include "internal.cuh"
 
 #include <cmath>
@@ -182,10 +184,10 @@ struct AdvanceArgs {
   int* err;
 };
 
-// Per-sample time step (src/Burgers.jl:97-101, :383-385); false = stop.
-__device__ __forceinline__ bool sample_dt(const AdvanceArgs& A, double lmax, double tt, double* red, double& dt) {
+// Per-sample time step (src/Burgers.jl:97-101, :383-385) from the largest |u|
+// m; false = stop.
+__device__ __forceinline__ bool step_of(const AdvanceArgs& A, double m, double tt, double& dt) {
   const Geo& g = A.g;
-  const double m = block_max(lmax, red);
   const double dtc = A.cfl * fmin(g.h / m, g.h * g.h / g.visc);
   dt = fmin(dtc, A.tstop - tt);
   // A non-finite field, or a CFL step that collapsed, ends the sample with a
@@ -197,10 +199,9 @@ __device__ __forceinline__ bool sample_dt(const AdvanceArgs& A, double lmax, dou
   return true;
 }
 
-// `dns_aided_les` (src/Burgers.jl:350-445) when LES, else the DNS loop of
-// `create_dns` (src/Burgers.jl:522-545) with `timestep!` or, when RK4,
-// `rk4_timestep!` (src/Burgers.jl:112-142).
-template <bool LES, bool RK4>
+// The DNS loop of `create_dns` (src/Burgers.jl:522-545) with `timestep!` or,
+// when RK4, `rk4_timestep!` (src/Burgers.jl:112-142).
+template <bool RK4>
 __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
   extern __shared__ double smem[];
   __shared__ double red[40];
@@ -208,65 +209,24 @@ __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
   const int np = padded(g);
   double* ue = smem;
   double* se = ue + np;
-  double* wd = se + np;
-  double* wl = wd + 2 * g.Rd + 1;
-  if (LES) {
-    for (int r = threadIdx.x; r < 2 * g.Rd + 1; r += blockDim.x) wd[r] = A.wd[r];
-    for (int r = threadIdx.x; r < 2 * g.Rl + 1; r += blockDim.x) wl[r] = A.wl[r];
-  }
   const int tid = threadIdx.x;
-  const size_t vs = (size_t)4 * g.nH;
   for (int s = blockIdx.x; s < g.ns; s += gridDim.x) {
     double* us = A.u + (size_t)s * g.nh;
     load_sample(g, us, ue);
     double tt = A.t[s];
-    int done = 0, par = 0;
+    int done = 0;
     __syncthreads();
     // |u| maximum of this thread's cells, kept up to date by the updates.
     double lmax = 0.0;
     for (int j = tid; j < g.nh; j += blockDim.x) lmax = nanmax(lmax, fabs(ue[g.G + j]));
     while (tt < A.tstop && done < A.max_steps) {
       double dt;
-      if (!sample_dt(A, lmax, tt, red, dt)) break;
-      const double dth = dt * g.ih, dtH = dt * g.iH;
+      if (!step_of(A, block_max(lmax, red), tt, dt)) break;
+      const double dth = dt * g.ih;
       lmax = 0.0;
       if (!RK4) {
         fill_stress(g, ue, se);
         __syncthreads();
-        if (LES) {
-          double* vc = (par ? A.v1 : A.v0) + s * vs;
-          double* vn = (par ? A.v0 : A.v1) + s * vs;
-          double* tm = A.tmp + (size_t)s * 5 * g.nH;
-          for (int I = tid; I < g.nH; I += blockDim.x) {
-            const Terms c = coarse_terms(g, I, ue, se, wd, wl);
-            tm[I] = c.fsu;
-            tm[g.nH + I] = c.vsu;
-            tm[2 * g.nH + I] = c.vu;
-            tm[3 * g.nH + I] = c.sVU;
-          }
-          __syncthreads();
-          // LES steps: stress of each LES plus its correction
-          // (src/Burgers.jl:414-430), forward Euler with the DNS time step.
-          for (int i = tid; i < g.nH; i += blockDim.x) {
-            const int im = i == 0 ? g.nH - 1 : i - 1, ip = i + 1 == g.nH ? 0 : i + 1;
-            const double vum = tm[2 * g.nH + im], vui = tm[2 * g.nH + i], vup = tm[2 * g.nH + ip];
-            const double svi = bstress(vum, vui, g.vH), svp = bstress(vui, vup, g.vH);
-            const double fi = tm[i], fp = tm[ip];
-            const double vsi = tm[g.nH + i], vsp = tm[g.nH + ip];
-            const double Si = tm[3 * g.nH + i], Sp = tm[3 * g.nH + ip];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const double* x = vc + k * g.nH;
-              const double xm = x[im], xi = x[i], xp = x[ip];
-              double si = bstress(xm, xi, g.vH), sp = bstress(xi, xp, g.vH);
-              if (k == 1) { si = (si + vsi) - Si; sp = (sp + vsp) - Sp; }    // classic
-              if (k == 2) { si = (si + vsi) - svi; sp = (sp + vsp) - svp; }  // classic + flux
-              if (k == 3) { si = (si + fi) - svi; sp = (sp + fp) - svp; }    // + div (exact)
-              vn[k * g.nH + i] = fma(dtH, sp - si, xi);
-            }
-          }
-          par ^= 1;
-        }
         for (int j = tid; j < g.nh; j += blockDim.x) {
           const int p = g.G + j;
           const double x = fma(dth, se[p + 1] - se[p], ue[p]);
@@ -311,17 +271,229 @@ __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
       ++done;
     }
     for (int j = tid; j < g.nh; j += blockDim.x) us[j] = ue[g.G + j];
-    if (LES && par) {
-      const double* src = A.v1 + s * vs;
-      double* dst = A.v0 + s * vs;
-      for (size_t i = tid; i < vs; i += blockDim.x) dst[i] = src[i];
-    }
     if (tid == 0) {
       A.t[s] = tt;
       A.steps[s] += done;
     }
     __syncthreads();
   }
+}
+
+// `dns_aided_les` (src/Burgers.jl:350-445): the forward-Euler DNS with its four
+// LES in lockstep, one sample per CTA.
+//
+// The coarse filters (67 taps of the double kernel for four quantities, 53 of
+// the LES kernel for one, at nh = 13500, nH = 900, Delta = 2H: 321 FP64
+// operations per coarse cell) bounded this loop on the FP64 pipe.  They run in
+// fixed point here (fixed.cuh): velocity, stress and weights as 54-bit integers
+// below the step's largest |u|, a bound of the largest stress and the largest
+// weight, the weighted sums exact, one rounding each.  The integers live in
+// shared memory; the velocity itself stays in registers, NC consecutive cells
+// per thread (NC odd: the strided shared stores hit every bank), so the DNS
+// update keeps the FP64 values and their bits.  Sums below 2^63: |x.h| <= 2^27,
+// |x.l| <= 2^26, |w.l| <= 2^26, and the weights' scale is at least 2^-4, so the
+// w.h sum to at most 2^31: 2^58, 2^53 T + 2^57 and 2^52 T for T taps (T < 512).
+//
+// The four LES stresses of a cell are formed once, into the spare LES buffer,
+// and read by both cells they border.  One warp forms the step's scalars: FP64
+// work of all 16 warps would take the pipe 16 times.  A step of 152 samples at
+// nh = 13500 by taps of shared loads in flight:
+//   nH               900      300     2700    nh 1500, nH 300
+//   FP64 filters   209 us
+//   one tap a time  82       79      104      13.3
+//   four taps       71       66       94      12.7
+// What is left is the FP64 pipe for the DNS update (five operations a cell,
+// 2 cells a clock: 18 us), the conversions of 2 x nh values and the taps.
+constexpr int BX_BITS = 54, BX_LOW = 27;
+
+__device__ __forceinline__ Fx as_fx(int2 v) { return {v.x, v.y}; }
+__device__ __forceinline__ int2 as_int2(Fx v) { return make_int2(v.h, v.l); }
+// E with |x| <= 2^E for the magnitude x >= 0
+__device__ __forceinline__ int exponent_above(double x) { return ((__double2hiint(x) >> 20) & 0x7ff) - 1022; }
+__device__ __forceinline__ int clamp_exponent(int e) { return min(max(e, -900), 1000); }
+// 2^e for |e| <= 1020
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+
+struct LesStep {
+  double dt, dth, dtH;
+  int Eu, Es;
+  bool go;
+};
+
+template <int NC>
+__global__ void __launch_bounds__(BT, 1) advance_les_kernel(AdvanceArgs A) {
+  static_assert(NC % 2 == 1, "odd: conflict-free strided stores");
+  extern __shared__ double smem[];
+  __shared__ double red[40];
+  __shared__ double wfirst[BT / 32], wlast[BT / 32], last_cell;
+  __shared__ unsigned long long wmax[BT / 32];
+  __shared__ LesStep step;
+  const Geo g = A.g;
+  const int np = padded(g);
+  int2* const ui = reinterpret_cast<int2*>(smem);
+  int2* const si = ui + np;
+  int2* const wd = si + np;
+  int2* const wl = wd + 2 * g.Rd + 1;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // weights: one scale for both kernels, from the largest |w|
+  double wm = 0.0;
+  for (int r = tid; r < 2 * g.Rd + 1; r += BT) wm = fmax(wm, fabs(A.wd[r]));
+  for (int r = tid; r < 2 * g.Rl + 1; r += BT) wm = fmax(wm, fabs(A.wl[r]));
+  wm = block_max(wm, red);
+  const int Ew = max(exponent_above(wm), -4), kw = (BX_BITS - Ew) << 20;
+  for (int r = tid; r < 2 * g.Rd + 1; r += BT) wd[r] = as_int2(fx_from_double<BX_BITS, BX_LOW>(A.wd[r], kw));
+  for (int r = tid; r < 2 * g.Rl + 1; r += BT) wl[r] = as_int2(fx_from_double<BX_BITS, BX_LOW>(A.wl[r], kw));
+  const int j0 = tid * NC, cnt = max(0, min(NC, g.nh - j0));
+  const size_t vs = (size_t)4 * g.nH;
+  for (int s = blockIdx.x; s < g.ns; s += gridDim.x) {
+    double* const us = A.u + (size_t)s * g.nh;
+    double* const vc = A.v0 + s * vs;  // LES states, updated in place
+    double* const st = A.v1 + s * vs;  // their stresses
+    double* const tm = A.tmp + (size_t)s * 5 * g.nH;
+    double u[NC];
+    unsigned long long lmax = 0;  // magnitude bits: their order is the values'
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      u[k] = k < cnt ? us[j0 + k] : 0.0;
+      lmax = max(lmax, mag_bits(u[k]));
+    }
+    double tt = A.t[s];
+    int done = 0;
+    __syncthreads();
+    while (tt < A.tstop && done < A.max_steps) {
+      // the largest |u| on the integer pipe; the step and the scales by one
+      // warp (every warp's FP64 instruction takes the pipe 16 cycles)
+      for (int o = 16; o > 0; o >>= 1) lmax = max(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
+      if (lane == 0) wmax[warp] = lmax;
+      __syncthreads();
+      if (warp == 0) {
+        unsigned long long q = lane < BT / 32 ? wmax[lane] : 0ull;
+        for (int o = 16; o > 0; o >>= 1) q = max(q, __shfl_xor_sync(0xffffffffu, q, o));
+        const double m = from_mag_bits<double>(q);
+        double dt;
+        const bool go = step_of(A, m, tt, dt);
+        // scales: |u| <= m, |stress| <= m^2 / 2 + 2 (visc/h) m (clamped where 2^E
+        // would leave the doubles: values below 2^-955 count as zero, above
+        // 2^1000 the DNS overflows and the next step stops)
+        if (lane == 0) {
+          step = {go ? dt : 0.0, dt * g.ih, dt * g.iH, clamp_exponent(exponent_above(m)),
+                  clamp_exponent(exponent_above((0.5 * m + 2.0 * g.vh) * m * (1.0 + 0x1p-40))), go};
+        }
+      }
+      __syncthreads();
+      if (!step.go) break;
+      const double dt = step.dt, dth = step.dth, dtH = step.dtH;
+      const int Eu = step.Eu, Es = step.Es;
+      const int ku = (BX_BITS - Eu) << 20, ks = (BX_BITS - Es) << 20;
+      // cells beside this thread's: the previous thread's last and the next
+      // thread's first, across warps through shared memory; cell nh - 1 and
+      // cell 0 are neighbours
+      double lastv = u[0];
+#pragma unroll
+      for (int k = 1; k < NC; ++k)
+        if (k < cnt) lastv = u[k];
+      if (lane == 31) wlast[warp] = lastv;
+      if (lane == 0) wfirst[warp] = u[0];
+      if (cnt > 0 && j0 + cnt == g.nh) last_cell = lastv;
+      __syncthreads();
+      double left = __shfl_up_sync(0xffffffffu, lastv, 1), right = __shfl_down_sync(0xffffffffu, u[0], 1);
+      if (lane == 0) left = warp ? wlast[warp - 1] : last_cell;
+      if (lane == 31 && warp + 1 < BT / 32) right = wfirst[warp + 1];
+      if (j0 + cnt == g.nh) right = wfirst[0];
+      lmax = 0;
+      double sl = bstress(left, u[0], g.vh);
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {
+        if (k < cnt) {
+          const double x = u[k];
+          const double sr = bstress(x, k + 1 < NC && k + 1 < cnt ? u[k + 1 < NC ? k + 1 : k] : right, g.vh);
+          ui[g.G + j0 + k] = as_int2(fx_from_double<BX_BITS, BX_LOW>(x, ku));
+          si[g.G + j0 + k] = as_int2(fx_from_double<BX_BITS, BX_LOW>(sl, ks));
+          u[k] = fma(dth, sr - sl, x);
+          lmax = max(lmax, mag_bits(u[k]));
+          sl = sr;
+        }
+      }
+      __syncthreads();
+      for (int p = tid; p < g.G; p += BT) {
+        ui[p] = ui[p + g.nh];
+        si[p] = si[p + g.nh];
+        ui[g.G + g.nh + p] = ui[g.G + p];
+        si[g.G + g.nh + p] = si[g.G + p];
+      }
+      __syncthreads();
+      const double cu = pow2(Eu + Ew - 2 * BX_BITS + 2 * BX_LOW), cs = pow2(Es + Ew - 2 * BX_BITS + 2 * BX_LOW);
+      for (int I = tid; I < g.nH; I += BT) {
+        // coarse_terms' sums
+        const int pc = g.G + (I + 1) * g.comp - g.a - 1, pf = pc + g.a;
+        FxSum vsu{0, 0, 0}, fsu{0, 0, 0}, vl{0, 0, 0}, vr{0, 0, 0}, vu{0, 0, 0};
+        Fx prev = as_fx(ui[pc - 1 - g.Rd]);
+#pragma unroll 4
+        for (int r = -g.Rd; r <= g.Rd; ++r) {
+          const Fx w = as_fx(wd[r + g.Rd]), x = as_fx(ui[pc + r]);
+          fx_mac(vsu, w, as_fx(si[pc + r]));
+          fx_mac(vl, w, prev);
+          fx_mac(vr, w, x);
+          fx_mac(vu, w, as_fx(ui[pf + r]));
+          prev = x;
+        }
+#pragma unroll 4
+        for (int r = -g.Rl; r <= g.Rl; ++r) fx_mac(fsu, as_fx(wl[r + g.Rl]), as_fx(si[pc + r]));
+        tm[I] = fx_to_double<BX_LOW>(fsu, cs);
+        tm[g.nH + I] = fx_to_double<BX_LOW>(vsu, cs);
+        tm[2 * g.nH + I] = fx_to_double<BX_LOW>(vu, cu);
+        tm[3 * g.nH + I] = bstress(fx_to_double<BX_LOW>(vl, cu), fx_to_double<BX_LOW>(vr, cu), g.vh);
+      }
+      __syncthreads();
+      // LES steps: stress of each LES plus its correction
+      // (src/Burgers.jl:414-430), forward Euler with the DNS time step
+      for (int i = tid; i < g.nH; i += BT) {
+        const int im = i == 0 ? g.nH - 1 : i - 1;
+        const double svi = bstress(tm[2 * g.nH + im], tm[2 * g.nH + i], g.vH);
+        const double fi = tm[i], vsi = tm[g.nH + i], Si = tm[3 * g.nH + i];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const double* x = vc + k * g.nH;
+          double q = bstress(x[im], x[i], g.vH);
+          if (k == 1) q = (q + vsi) - Si;   // classic
+          if (k == 2) q = (q + vsi) - svi;  // classic + flux
+          if (k == 3) q = (q + fi) - svi;   // + div (exact)
+          st[k * g.nH + i] = q;
+        }
+      }
+      __syncthreads();
+      for (int i = tid; i < g.nH; i += BT) {
+        const int ip = i + 1 == g.nH ? 0 : i + 1;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const double* q = st + k * g.nH;
+          vc[k * g.nH + i] = fma(dtH, q[ip] - q[i], vc[k * g.nH + i]);
+        }
+      }
+      tt += dt;
+      ++done;
+    }
+#pragma unroll
+    for (int k = 0; k < NC; ++k)
+      if (k < cnt) us[j0 + k] = u[k];
+    if (tid == 0) {
+      A.t[s] = tt;
+      A.steps[s] += done;
+    }
+    __syncthreads();
+  }
+}
+
+// The kernel with enough cells per thread for nh; 29 x 512 is above the
+// shared-memory limit of a resident sample.
+const void* les_kernel(int nh) {
+  const int c = (nh + BT - 1) / BT;
+  return c <= 5    ? (const void*)advance_les_kernel<5>
+         : c <= 11 ? (const void*)advance_les_kernel<11>
+         : c <= 17 ? (const void*)advance_les_kernel<17>
+         : c <= 23 ? (const void*)advance_les_kernel<23>
+         : c <= 27 ? (const void*)advance_les_kernel<27>
+                   : (const void*)advance_les_kernel<29>;
 }
 
 struct TermsArgs {
@@ -1035,14 +1207,13 @@ int exc_burgers_advance(exc_burgers* b, double tstop, double cfl, int scheme, in
   A.acc = b->scr + (size_t)b->nh * b->ns;
   A.err = b->err;
   const size_t sm = sample_smem(A.g);
-  const void* fn = b->les_on ? (const void*)advance_kernel<true, false>
-                             : scheme == EXC_BURGERS_RK4 ? (const void*)advance_kernel<false, true>
-                                                         : (const void*)advance_kernel<false, false>;
+  const void* fn = b->les_on ? les_kernel(b->nh)
+                             : scheme == EXC_BURGERS_RK4 ? (const void*)advance_kernel<true>
+                                                         : (const void*)advance_kernel<false>;
   if (allow_smem(fn, sm) != cudaSuccess) { cudaGetLastError(); set_last_error("shared memory opt-in failed"); return EXC_ERR_CUDA; }
   const int grid = grid_for(fn, sm, b->ns);
-  if (b->les_on) advance_kernel<true, false><<<grid, BT, sm, b->st>>>(A);
-  else if (scheme == EXC_BURGERS_RK4) advance_kernel<false, true><<<grid, BT, sm, b->st>>>(A);
-  else advance_kernel<false, false><<<grid, BT, sm, b->st>>>(A);
+  void* args[] = {&A};
+  cudaLaunchKernel(fn, dim3(grid), dim3(BT), args, sm, b->st);
   int rc = launch_err(b);
   if (rc) return rc;
   rc = check_flag(b);

@@ -16,6 +16,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "fixed.cuh"
 #include "internal.cuh"
 
 namespace exc {
@@ -379,10 +380,9 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
 // ---------------------------------------------------------------------------
 // FP64 sweep on the integer pipe.
 //
-// GB300 retires two FP64 operations per clock and SM but 55 widening integer
-// multiply-adds (32 x 32 + 64 -> 64) and about 100 integer additions (all
-// measured), so this sweep forms the stresses and their divergence in fixed
-// point, with more bits than FP64 carries, and rounds once at the end.
+// The FP64 pipe bounds the sweep, so it forms the stresses and their divergence
+// in fixed point (fixed.cuh), with more bits than FP64 carries, and rounds once
+// at the end.
 //
 // Fixed point.  All values a CTA holds share one scale 2^(57 - E), |u| + S <
 // 2^E: a velocity becomes an integer U, |U| <= 2^57, split as U = h 2^29 + l
@@ -420,52 +420,10 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
 // noise 0.7-1.1e-16 (FP64 form 1.7-2.1e-16), smooth fields 0.8e-16 (1.2e-15), a
 // mean flow of 100 7e-17 (1.3e-14), visc 0.1 1.4e-16 (7.7e-16).
 // ---------------------------------------------------------------------------
-struct Fx { int h, l; };
-__device__ __forceinline__ Fx operator+(Fx a, Fx b) { return {a.h + b.h, a.l + b.l}; }
-__device__ __forceinline__ Fx operator-(Fx a, Fx b) { return {a.h - b.h, a.l - b.l}; }
-__device__ __forceinline__ Fx operator-(Fx a) { return {-a.h, -a.l}; }
-struct FxSum { long long hh, m, ll; };
-__device__ __forceinline__ void fx_mac(FxSum& s, Fx a, Fx b) {
-  s.hh += (long long)a.h * b.h;
-  s.m += (long long)a.h * b.l;
-  s.m += (long long)a.l * b.h;
-  s.ll += (long long)a.l * b.l;
-}
 constexpr int FX_BITS = 57, FX_LOW = 29;
 // E of the fixed-point path: well inside the range of the FP32 bound that
 // finds it, and squares and their scaling stay normal doubles
 constexpr int FX_EMIN = -100, FX_EMAX = FX_BITS;
-
-// x (|x| < 2^E) in units of 2^(E - 57), rounded to nearest; kexp = (57 - E) <<
-// 20.  On the integer pipe: the FP64 pipe's own conversion measured slower
-// (512^3 3.93 against 3.57 ms), it shares the pipe with fx_to_double's.
-__device__ __forceinline__ Fx fx_from_double(double x, int kexp) {
-  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-  const int e = (int)((hi >> 20) & 0x7ffu);
-  const unsigned mh = (hi & 0xfffffu) | 0x100000u;
-  // mantissa with five more bits (one of them the rounding bit); shr.b64 gives
-  // 0 for counts of 64 and more (small values, zero)
-  const unsigned long long m5 = ((unsigned long long)__funnelshift_l(lo, mh, 5) << 32) | (lo << 5);
-  unsigned long long t;
-  asm("shr.u64 %0, %1, %2;" : "=l"(t) : "l"(m5), "r"(1022 + FX_BITS - (kexp >> 20) - e));
-  const long long U = (long long)((t + 1) >> 1);
-  const int h = (int)((U + (1 << (FX_LOW - 1))) >> FX_LOW);
-  const int l = (int)(unsigned)U - (h << FX_LOW);
-  const int sg = ((int)hi >> 31) | 1;
-  return {h * sg, l * sg};
-}
-
-// (hh 2^58 + m 2^29 + ll) in units of 2^58 times `scale`, with ten more bits
-// (and 2^-10 of scale, by its exponent field) while they fit: to 2^-95 of the
-// squared scale, or to half a unit of the double.
-__device__ __forceinline__ double fx_to_double(const FxSum& s, double scale) {
-  const long long mm = s.m + (s.ll >> FX_LOW);
-  const long long hi = s.hh + (mm >> FX_LOW);
-  const int low10 = ((int)mm >> (FX_LOW - 10)) & 0x3ff;
-  const bool big = (unsigned)((int)(hi >> 32) + 0x200000) >= 0x400000u;  // |hi| >= 2^53
-  const long long v = big ? hi : (hi << 10) | low10;
-  return (double)v * __hiloint2double(__double2hiint(scale) - (big ? 0 : 10 << 20), __double2loint(scale));
-}
 
 // The reference's arithmetic for one cell, from global memory: the cells the
 // fixed-point sweep leaves out.
@@ -626,7 +584,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
   double scale = 0;              // -1/(4h) 2^58 in fixed-point units squared
   auto convert_plane = [&](int buf) {
     each_value(buf, [&](double& v) {
-      const Fx q = fx_from_double(v, kexp);
+      const Fx q = fx_from_double<FX_BITS, FX_LOW>(v, kexp);
       v = __hiloint2double(q.h, q.l);
     });
   };
@@ -683,7 +641,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     if (!slow) {
       kexp = (FX_BITS - E) << 20;
       scale = ldexp(-0.25 * inv_h, 2 * FX_LOW + 2 * (E - FX_BITS));
-      const Fx s = fx_from_double(4.0 * S, kexp);
+      const Fx s = fx_from_double<FX_BITS, FX_LOW>(4.0 * S, kexp);
       // 4S to a multiple of four units, so that S and 2S are the same S
       const long long s4 = (((long long)s.h << FX_LOW) + s.l + 2) >> 2 << 2;
       const long long s2 = s4 >> 1;
@@ -750,7 +708,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
           fx_mac(s, S2 - a - aym, bym + bxpym - S2);
           fx_mac(s, A13, B13);
           fx_mac(s, S2 - a - pw1[i], pb13[i]);
-          o1 = fx_to_double(s, scale);
+          o1 = fx_to_double<FX_LOW>(s, scale);
         }
         {
           FxSum s = s0;
@@ -761,7 +719,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
           fx_mac(s, S2 - axm - axmyp, bxm + b - S2);
           fx_mac(s, A23, B23);
           fx_mac(s, S2 - b - pw2[i], pb23[i]);
-          o2 = fx_to_double(s, scale);
+          o2 = fx_to_double<FX_LOW>(s, scale);
         }
         {
           FxSum s = s0;
@@ -772,7 +730,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
           fx_mac(s, S2 - axm - axmzp, cxm + c - S2);
           fx_mac(s, A23, B23);
           fx_mac(s, S2 - bym - bymzp, cym + c - S2);
-          o3 = fx_to_double(s, scale);
+          o3 = fx_to_double<FX_LOW>(s, scale);
         }
         pw1[i] = a;
         pw2[i] = b;

@@ -646,7 +646,7 @@ static int case_create(exc_case* cs) {
   ci->n = d.n;
   ci->N = (long long)d.n * d.n * d.n;
   ci->h = d.l / d.n;
-  int rc = poisson_init(&ci->ps, cs->precision, d.n, d.l, nullptr);
+  int rc = poisson_init(&ci->ps, cs->precision, d.n, d.l, nullptr, steppers_use_run_time_plans(cs->precision));
   if (rc) return rc;
   // the DNS pressure enters only through its gradient (RK stage): its
   // additive constant need not be removed
@@ -673,7 +673,7 @@ static int case_create(exc_case* cs) {
     L.kind = d.les[li].kind;
     L.m = d.n / L.c;
     L.M = (long long)L.m * L.m * L.m;
-    rc = poisson_init(&L.ps, cs->precision, L.m, d.l, nullptr);
+    rc = poisson_init(&L.ps, cs->precision, L.m, d.l, nullptr, steppers_use_run_time_plans(cs->precision));
     if (rc) return rc;
     size_t nb = 21 * 3 * L.M * sizeof(T);
     if (cudaMalloc(&L.buf, nb) != cudaSuccess) { set_last_error("out of device memory (LES fields)"); return EXC_ERR_OOM; }

@@ -552,7 +552,7 @@ static long long mix_part_words(int n) {
   return fftmix_supported(n) ? fftmix_part_words(n) : std::max(gen_mix_parts(n), (long long)MIX_SUM_CTAS) + 2;
 }
 
-int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work) {
+int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bool run_time_plans) {
   if (!fft_size_ok(n)) { set_last_error("grid size must be 2^a 3^b 5^c 7^d 11^e 13^f 17^g, a >= 1, 4 <= n <= 1024"); return EXC_ERR_SHAPE; }
   if (!(l > 0)) { set_last_error("domain size must be positive"); return EXC_ERR_ARG; }
   if (precision != EXC_F64 && precision != EXC_F32) { set_last_error("bad precision"); return EXC_ERR_ARG; }
@@ -602,7 +602,7 @@ int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work) {
     if (precision == EXC_F32)
       invlap_split_kernel<<<(int)std::min<long long>((tot + 255) / 256, 152LL * 32), 256>>>(tot, ps->invlap);
   }
-  ps->gen = !fftreg_supported(n, precision) && gen_supported(n, precision);
+  ps->gen = run_time_plans && !fftreg_supported(n, precision) && gen_supported(n, precision);
   if (ps->gen || fftreg_supported(n, precision)) {
     int n1 = reg_split_host(n), h1 = reg_split_host(n / 2);
     if (ps->gen) gen_splits(n, precision, &n1, &h1);

@@ -503,7 +503,8 @@ static int make_chunk(exc_server* sv, int n, double l, double cfl, ChunkBase** o
   using C = cplx<T>;
   const long long wst = (long long)n * n * spec_pitch(n);
   if (cudaMalloc(&ck->work, S * wst * sizeof(C)) != cudaSuccess) { set_last_error("out of device memory (chunk work)"); return EXC_ERR_OOM; }
-  int rc = poisson_init(&ck->ps, sizeof(T) == 8 ? EXC_F64 : EXC_F32, n, l, ck->work);
+  const int precision = sizeof(T) == 8 ? EXC_F64 : EXC_F32;
+  int rc = poisson_init(&ck->ps, precision, n, l, ck->work, steppers_use_run_time_plans(precision));
   if (rc) return rc;
   if (cudaMalloc(&ck->big, 4 * S * 3 * ck->N * sizeof(T)) != cudaSuccess) { set_last_error("out of device memory (chunk fields)"); return EXC_ERR_OOM; }
   cudaMemsetAsync(ck->big, 0, 4 * S * 3 * ck->N * sizeof(T), ck->stream);

@@ -117,7 +117,8 @@ int exc_debug_wait_drill(int flags);
  * rounding); otherwise register-resident two-level passes where the grid has
  * a plan (compiled for n = 32, 48, 64, 96, 128, 192, 256 and, in FP32, 384,
  * 512, 1024; at run time where n and n/2 split into two factors of at most 34
- * in FP32, of at most 17 in FP64 for n < 160), shared-memory Stockham passes for the rest.  1 =
+ * in FP32, of at most 17 in FP64 for n < 160; FP32 cases and served solves do
+ * without run-time plans), shared-memory Stockham passes for the rest.  1 =
  * FP64/FP32 Stockham passes for every grid.  2 = register passes where
  * planned, else Stockham, in the solver's own precision throughout.  Results
  * agree to round-off; the autotuner of the serving form picks per grid. */

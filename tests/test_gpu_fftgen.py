@@ -65,17 +65,18 @@ def test_large_factors_match_stockham(NS, n):
         assert float((a - b).norm() / b.norm()) < 1e-12
 
 
-def test_served_batch_equals_the_case(NS, built_lib):
+@pytest.mark.parametrize("precision", [0, 1])
+def test_served_batch_equals_the_case(NS, built_lib, precision):
     """Several slots of one run-time-planned grid (the batched passes)."""
     from exactclosure_gb300.serving import Server
 
     n, steps = 50, 6
-    sv = Server(precision=1, autotune=False, slots_per_chunk=3)
+    sv = Server(precision=precision, autotune=False, slots_per_chunk=3)
     ids = [sv.submit(n, 1 / 2000, steps, seed=s, keep_field=True) for s in range(3)]
     sv.drain()
     got = {r["id"]: r["field"] for r in sv.poll()}
     for s, i in enumerate(ids):
-        cs = NS.Case(n, 1.0, 1 / 2000, 0.3, precision=1)
+        cs = NS.Case(n, 1.0, 1 / 2000, 0.3, precision=precision)
         cs.init_random(4.0, 1.0, s)
         cs.step(steps)
         assert (cs.velocity() == got[i]).all()

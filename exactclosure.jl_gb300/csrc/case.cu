@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "lesstep.cuh"
 #include "fields.cuh"
 #include "filter.cuh"
 
@@ -43,11 +44,15 @@ struct LesState {
   // overlapped FP64 stepper: the stage-state sums (targets of the next stage),
   // apart from tb, which holds k's sums while the LES streams read them
   T* tbs = nullptr;
-  T *ub, *fk, *mcl, *mlast, *rtmp;
-  T *ve[2], *ves, *ke;  // exact LES: state (ping-pong), stage, k
-  T *vn[2], *vns, *kn;  // no-model LES
-  T* ublast;            // target at stage 0 of the last step (pairs with mlast)
-  T *vl[2], *vls, *kl, *nn;  // LES driven by the learned closure (when a net is attached)
+  // Batches of a stage, slot after slot (3M words): [target, exact, no-model,
+  // learned] at the step's start (ping-pong) and at a stage, and their
+  // right-hand sides with two more fields to project (LesStage::k)
+  T *g[2], *gs, *k;
+  long long wstride = 0;  // words between the solver's slots
+  T* ub;                  // target at a stage (in gs)
+  T *ve[2], *vn[2], *vl[2];  // states of the exact, no-model and learned LES (in g)
+  T *mlast, *ublast;      // closure and target at stage 0 of the last step
+  T* nn;                  // closure of the learned LES (when a net is attached)
   T* vgood;                  // its last state inside the energy band (fallback)
   // fallback of the learned LES (device, 8 doubles): [0] engaged (0/1), [1]
   // lower and [2] upper bound of its kinetic energy, [3] sum of squares of
@@ -117,14 +122,6 @@ __global__ void learned_guard_kernel(long long count, T* __restrict__ v, T* __re
 }
 
 // y += x unless the fallback is engaged (the net's closure term).
-template <typename T>
-__global__ void add_unless_kernel(long long count, T* __restrict__ y, const T* __restrict__ x,
-                                  const double* __restrict__ fb) {
-  if (fb[0] != 0.0) return;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x)
-    y[i] += x[i];
-}
-
 static int grid_for_count(long long cnt) {
   long long b = (cnt + 255) / 256;
   return (int)(b < 152LL * 8 ? b : 152LL * 8);
@@ -247,77 +244,64 @@ static int les_target(CaseImpl<T>* ci, LesState<T>& L, const T* src, T* out, cud
 
 // One LES grid's work of RK stage s once the box sums of k_s (ksums) are
 // ready, on stream sl: the closure m_s, then the exact, no-model and learned
-// LES stages.
+// LES stages, and the targets of stage s + 1 where its sums (ssums) are ready
+// too.
+//   m_s = P_H(filter(k_s) - RHS_H(ubar_s)); the unprojected difference is used:
+//   the projection is linear, so the exact LES projects it together with its
+//   own RHS, k = P_H(RHS_H(v_s) + filter(k_s) - RHS_H(ubar_s)), one solve
+//   instead of two; m_0 itself (snapshot pairs, diagnostics) is a slot of
+//   stage 0.
 template <typename T>
 static int les_stage(exc_case* cs, CaseImpl<T>* ci, LesState<T>& L, int s, int cur, const double* dt,
-                     const T* ksums, cudaStream_t sl) {
-  const T visc = (T)cs->desc.visc;
-  cudaError_t e;
+                     const T* ksums, const T* ssums, cudaStream_t sl) {
   const int m = L.m;
   const T H = (T)(cs->desc.l / m);
-  // m_s = P_H(filter(k_s) - RHS_H(ubar_s)); mcl keeps the unprojected
-  // difference (the projection is linear: the exact LES projects it
-  // together with its own RHS, one solve instead of two)
-  e = box_oa<T>(ci->n, L.c, L.kind, ksums, L.mcl, sl);
-  if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
-  int rc;
-  e = launch_rhs<T>(m, H, visc, L.ub, L.rtmp, false, sl);
-  if (e == cudaSuccess) e = launch_axpy<T>(3 * L.M, L.mcl, L.rtmp, (T)-1, sl);
-  if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
-  if (s == 0) {
-    // the closure of stage 0 (snapshot pairs, diagnostics): m_0 itself
-    e = cudaMemcpyAsync(L.mlast, L.mcl, 3 * L.M * sizeof(T), cudaMemcpyDeviceToDevice, sl);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(L.ublast, L.ub, 3 * L.M * sizeof(T), cudaMemcpyDeviceToDevice, sl);
-    if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
-    rc = project_vec<T>(&L.ps, L.mlast, sl);
+  const T* const src = s == 0 ? L.g[cur] : L.gs;
+  SlotBatch sb;
+  sb.ustride = 3 * L.M;
+  sb.wstride = L.wstride;
+  LesStage<T> a{};
+  a.n = ci->n; a.c = L.c; a.kind = L.kind; a.m = m;
+  a.s = s;
+  a.nst = L.net ? 3 : 2;
+  a.ksums = ksums;
+  a.ssums = ssums;
+  a.k = L.k;
+  a.ub = src;
+  a.ublast = L.ublast;
+  a.mlast = L.mlast;
+  a.next = L.ub;
+  a.net = L.net ? L.nn : nullptr;
+  a.fb = L.fb;
+  a.x0 = L.g[cur] + 3 * L.M;
+  a.xs = L.gs + 3 * L.M;
+  a.xfin = L.g[cur ^ 1] + 3 * L.M;
+  a.dt = dt;
+  cudaError_t e = launch_rhs<T>(m, H, (T)cs->desc.visc, src, L.k, false, sl, sb, 1 + a.nst);
+  if (e == cudaSuccess && L.net) {
+    const int rc = exc_net_forward(L.net, cs->precision, 1, m, src + 9 * L.M, L.nn, sl);
     if (rc) return rc;
   }
-  // exact-closure LES: k = P_H(RHS_H(v_s) + filter(k_s) - RHS_H(ubar_s))
-  T* ve0 = L.ve[cur];
-  T* vefin = L.ve[cur ^ 1];
-  e = launch_rhs<T>(m, H, visc, s == 0 ? ve0 : L.ves, L.ke, false, sl);
-  if (e == cudaSuccess) e = launch_axpy<T>(3 * L.M, L.ke, L.mcl, (T)1, sl);
-  if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
-  rc = project_vec<T>(&L.ps, L.ke, sl);
-  if (rc) return rc;
-  e = launch_rk_stage<T>(m, H, L.ke, nullptr, 0, ve0, L.ves, vefin, s, dt, sl);
-  // no-model LES
-  T* vn0 = L.vn[cur];
-  T* vnfin = L.vn[cur ^ 1];
-  if (e == cudaSuccess) e = launch_rhs<T>(m, H, visc, s == 0 ? vn0 : L.vns, L.kn, false, sl);
-  if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
-  rc = project_vec<T>(&L.ps, L.kn, sl);
-  if (rc) return rc;
-  e = launch_rk_stage<T>(m, H, L.kn, nullptr, 0, vn0, L.vns, vnfin, s, dt, sl);
-  if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
-  if (L.net) {
-    // learned-closure LES: k = P_H(RHS_H(v_s) + net(v_s))
-    T* vl0 = L.vl[cur];
-    T* vlfin = L.vl[cur ^ 1];
-    const T* vsrc = s == 0 ? vl0 : L.vls;
-    e = launch_rhs<T>(m, H, visc, vsrc, L.kl, false, sl);
-    if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
-    rc = exc_net_forward(L.net, cs->precision, 1, m, vsrc, L.nn, sl);
-    if (rc) return rc;
-    add_unless_kernel<T><<<grid_for_count(3 * L.M), 256, 0, sl>>>(3 * L.M, L.kl, L.nn, L.fb);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
-    rc = project_vec<T>(&L.ps, L.kl, sl);
-    if (rc) return rc;
-    e = launch_rk_stage<T>(m, H, L.kl, nullptr, 0, vl0, L.vls, vlfin, s, dt, sl);
-    if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
+  if (e == cudaSuccess) e = launch_les_combine<T>(a, sl);
+  // one batched solve, or one after the other where the grid has the
+  // mixed-precision solve (one work array)
+  const int slots = les_slots(a), each = L.ps.mix ? 1 : slots;
+  const T* const p = reinterpret_cast<const T*>(L.ps.work);
+  for (int i = 0; i < slots && e == cudaSuccess; i += each) {
+    e = poisson_solve_inplace<T>(&L.ps, L.k + 3 * L.M * (1 + i), true, sl, sb, each);
+    if (e == cudaSuccess) e = launch_les_apply<T>(a, H, p, 2 * L.ps.P, 2 * L.wstride, i, each, sl);
   }
+  if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
   return EXC_OK;
 }
 
 // ubar_s of one LES from the box sums of the stage state (own-axis taps, then
 // the projection for the volume filter), on stream sl.
 template <typename T>
-static int les_target_from(CaseImpl<T>* ci, LesState<T>& L, const T* ssums, cudaStream_t sl) {
-  cudaError_t e = box_oa<T>(ci->n, L.c, L.kind, ssums, L.ub, sl);
+static int les_target_from(CaseImpl<T>* ci, LesState<T>& L, const T* ssums, T* ub, cudaStream_t sl) {
+  cudaError_t e = box_oa<T>(ci->n, L.c, L.kind, ssums, ub, sl);
   if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
-  return L.kind == EXC_FILTER_VOLUME ? project_vec<T>(&L.ps, L.ub, sl) : EXC_OK;
+  return L.kind == EXC_FILTER_VOLUME ? project_vec<T>(&L.ps, ub, sl) : EXC_OK;
 }
 
 // Stage sums of LES L (shared by LES of the same ratio).
@@ -354,7 +338,8 @@ static int enqueue_stages_overlap(exc_case* cs, CaseImpl<T>* ci, int cur, T* u0,
   }
   if (!rc) rc = cuda_rc(cudaEventRecord(ci->ev_s, st));
   if (!rc) rc = cuda_rc(cudaStreamWaitEvent(sl, ci->ev_s, 0));
-  for (int li = 0; li < ci->nles && !rc; ++li) rc = les_target_from<T>(ci, ci->les[li], les_tbs(ci, ci->les[li]), sl);
+  for (int li = 0; li < ci->nles && !rc; ++li)
+    rc = les_target_from<T>(ci, ci->les[li], les_tbs(ci, ci->les[li]), ci->les[li].g[cur], sl);
   if (!rc) rc = cuda_rc(cudaEventRecord(ci->ev_t0, sl));
   for (int s = 0; s < 4 && !rc; ++s) {
     const T* src = s == 0 ? u0 : ci->us;
@@ -378,10 +363,9 @@ static int enqueue_stages_overlap(exc_case* cs, CaseImpl<T>* ci, int cur, T* u0,
     }
     if (!rc) rc = cuda_rc(cudaEventRecord(ci->ev_k[s], st));
     if (!rc) rc = cuda_rc(cudaStreamWaitEvent(sl, ci->ev_k[s], 0));
-    for (int li = 0; li < ci->nles && !rc; ++li) rc = les_stage<T>(cs, ci, ci->les[li], s, cur, dt, les_tb(ci, ci->les[li]), sl);
-    if (s < 3)
-      for (int li = 0; li < ci->nles && !rc; ++li)
-        rc = les_target_from<T>(ci, ci->les[li], les_tbs(ci, ci->les[li]), sl);
+    for (int li = 0; li < ci->nles && !rc; ++li)
+      rc = les_stage<T>(cs, ci, ci->les[li], s, cur, dt, les_tb(ci, ci->les[li]),
+                        s < 3 ? les_tbs(ci, ci->les[li]) : nullptr, sl);
     if (!rc) rc = cuda_rc(cudaEventRecord(ci->ev_rd[s], sl));
   }
   if (!rc) rc = cuda_rc(cudaStreamWaitEvent(st, ci->ev_rd[3], 0));
@@ -426,7 +410,7 @@ static int enqueue_stages_overlap_fused(exc_case* cs, CaseImpl<T>* ci, int cur, 
   if (!rc) rc = cuda_rc(cudaEventRecord(ci->ev_s, st));
   if (!rc) rc = cuda_rc(cudaStreamWaitEvent(sl, ci->ev_s, 0));
   for (int li = 0; li < ci->nles && !rc; ++li)
-    rc = les_target_from<T>(ci, ci->les[li], les_tbs_fused(ci, ci->les[li]), sl);
+    rc = les_target_from<T>(ci, ci->les[li], les_tbs_fused(ci, ci->les[li]), ci->les[li].g[cur], sl);
   if (!rc) rc = cuda_rc(cudaEventRecord(ci->ev_t0, sl));
   for (int s = 0; s < 4 && !rc; ++s) {
     const T* src = s == 0 ? u0 : ci->us;
@@ -442,10 +426,8 @@ static int enqueue_stages_overlap_fused(exc_case* cs, CaseImpl<T>* ci, int cur, 
     if (!rc) rc = cuda_rc(cudaEventRecord(ci->ev_k[s], st));
     if (!rc) rc = cuda_rc(cudaStreamWaitEvent(sl, ci->ev_k[s], 0));
     for (int li = 0; li < ci->nles && !rc; ++li)
-      rc = les_stage<T>(cs, ci, ci->les[li], s, cur, dt, les_tb_from_root(ci, ci->les[li], root_k), sl);
-    if (s < 3)
-      for (int li = 0; li < ci->nles && !rc; ++li)
-        rc = les_target_from<T>(ci, ci->les[li], les_tbs_fused(ci, ci->les[li]), sl);
+      rc = les_stage<T>(cs, ci, ci->les[li], s, cur, dt, les_tb_from_root(ci, ci->les[li], root_k),
+                        s < 3 ? les_tbs_fused(ci, ci->les[li]) : nullptr, sl);
     if (!rc) rc = cuda_rc(cudaEventRecord(ci->ev_rd[s], sl));
   }
   if (!rc) rc = cuda_rc(cudaStreamWaitEvent(st, ci->ev_rd[3], 0));
@@ -506,7 +488,8 @@ static int enqueue_step(exc_case* cs, CaseImpl<T>* ci, int cur, double dt_fixed)
     }
     for (int li = 0; li < ci->nles; ++li) {
       LesState<T>& L = ci->les[li];
-      const int rc = les_target_from<T>(ci, L, fused ? les_tb_from_root(ci, L, troot) : les_tb(ci, L), st);
+      const int rc = les_target_from<T>(ci, L, fused ? les_tb_from_root(ci, L, troot) : les_tb(ci, L),
+                                        s == 0 ? L.g[cur] : L.ub, st);
       if (rc) return rc;
     }
     if (fused) {
@@ -523,7 +506,8 @@ static int enqueue_step(exc_case* cs, CaseImpl<T>* ci, int cur, double dt_fixed)
     }
     for (int li = 0; li < ci->nles; ++li) {
       LesState<T>& L = ci->les[li];
-      const int rc = les_stage<T>(cs, ci, L, s, cur, dt, fused ? les_tb_from_root(ci, L, root_k) : les_tb(ci, L), st);
+      const int rc = les_stage<T>(cs, ci, L, s, cur, dt, fused ? les_tb_from_root(ci, L, root_k) : les_tb(ci, L),
+                                  nullptr, st);
       if (rc) return rc;
     }
   }
@@ -673,21 +657,26 @@ static int case_create(exc_case* cs) {
     L.kind = d.les[li].kind;
     L.m = d.n / L.c;
     L.M = (long long)L.m * L.m * L.m;
-    rc = poisson_init(&L.ps, cs->precision, L.m, d.l, nullptr, steppers_use_run_time_plans(cs->precision));
+    // a stage projects up to three states, the closure and the next target
+    rc = poisson_init(&L.ps, cs->precision, L.m, d.l, nullptr, steppers_use_run_time_plans(cs->precision), 5);
     if (rc) return rc;
-    size_t nb = 21 * 3 * L.M * sizeof(T);
+    L.wstride = (long long)L.m * L.m * L.ps.P;
+    size_t nb = 22 * 3 * L.M * sizeof(T);
     if (cudaMalloc(&L.buf, nb) != cudaSuccess) { set_last_error("out of device memory (LES fields)"); return EXC_ERR_OOM; }
     cudaMemset(L.buf, 0, nb);
     size_t tbb = 3 * (size_t)d.n * L.m * L.m * sizeof(T);
     if (cudaMalloc(&L.tb, tbb) != cudaSuccess) { set_last_error("out of device memory (LES filter scratch)"); return EXC_ERR_OOM; }
     T* p = L.buf;
     auto take = [&]() { T* q = p; p += 3 * L.M; return q; };
-    L.ub = take(); L.fk = take(); L.mcl = take(); L.mlast = take(); L.rtmp = take();
-    L.ve[0] = take(); L.ve[1] = take(); L.ves = take(); L.ke = take();
-    L.vn[0] = take(); L.vn[1] = take(); L.vns = take(); L.kn = take();
-    L.ublast = take();
-    L.vl[0] = take(); L.vl[1] = take(); L.vls = take(); L.kl = take(); L.nn = take();
-    L.vgood = take();
+    auto batch = [&](int slots) { T* q = p; p += (long long)slots * 3 * L.M; return q; };
+    L.g[0] = batch(4); L.g[1] = batch(4); L.gs = batch(4); L.k = batch(6);
+    L.ub = L.gs;
+    for (int k = 0; k < 2; ++k) {
+      L.ve[k] = L.g[k] + 3 * L.M;
+      L.vn[k] = L.g[k] + 6 * L.M;
+      L.vl[k] = L.g[k] + 9 * L.M;
+    }
+    L.mlast = take(); L.ublast = take(); L.nn = take(); L.vgood = take();
     // 8 doubles: fb[3..4] receive the two-word result of the sum of squares
     if (cudaMalloc(&L.fb, 8 * sizeof(double)) != cudaSuccess) { set_last_error("out of device memory (LES fallback)"); return EXC_ERR_OOM; }
     const double fb0[8] = {0.0, 0.0, INFINITY, 0.0, 0.0, 0.0, 0.0, 0.0};

@@ -552,7 +552,7 @@ static long long mix_part_words(int n) {
   return fftmix_supported(n) ? fftmix_part_words(n) : std::max(gen_mix_parts(n), (long long)MIX_SUM_CTAS) + 2;
 }
 
-int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bool run_time_plans) {
+int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bool run_time_plans, int slots) {
   if (!fft_size_ok(n)) { set_last_error("grid size must be 2^a 3^b 5^c 7^d 11^e 13^f 17^g, a >= 1, 4 <= n <= 1024"); return EXC_ERR_SHAPE; }
   if (!(l > 0)) { set_last_error("domain size must be positive"); return EXC_ERR_ARG; }
   if (precision != EXC_F64 && precision != EXC_F32) { set_last_error("bad precision"); return EXC_ERR_ARG; }
@@ -629,7 +629,7 @@ int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bo
       return EXC_ERR_OOM;
     }
   }
-  size_t wbytes = (size_t)n * n * ps->P * csz;
+  size_t wbytes = (size_t)n * n * ps->P * csz * (ps->mix ? 1 : slots);
   if (work) {
     ps->work = work;
     ps->external_work = true;

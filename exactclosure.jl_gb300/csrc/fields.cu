@@ -22,7 +22,7 @@ static inline int grid_for(long long N, int threads = 256) {
 // ---------------------------------------------------------------------------
 // With STORE_K the projected k is written back (the LES closures filter it);
 // without, k is consumed here and the write is skipped.
-template <typename T, bool GRAD, bool STORE_K = true>
+template <typename T, bool STORE_K>
 __global__ void rk_stage_kernel(int n, T inv_h, T* __restrict__ k, const T* __restrict__ p, int ppitch,
                                 const T* __restrict__ x0, T* __restrict__ xs, T* __restrict__ xfin, int stage,
                                 const double* __restrict__ dtp, SlotBatch sb) {
@@ -33,30 +33,28 @@ __global__ void rk_stage_kernel(int n, T inv_h, T* __restrict__ k, const T* __re
   x0 += slot * sb.ustride;
   xs += slot * sb.ustride;
   xfin += slot * sb.ustride;
-  if (GRAD) p += slot * 2 * sb.wstride;
+  p += slot * 2 * sb.wstride;
   const double dt = dtp[slot];
   const T cf = (T)((stage == 0 || stage == 3) ? dt / 6.0 : dt / 3.0);
   const T cs = (T)(stage == 2 ? dt : 0.5 * dt);
   const IdxDiv dn(n);
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
     T k0 = k[g], k1 = k[N + g], k2 = k[2 * N + g];
-    if (GRAD) {
-      const long long r = dn.div(g);
-      int x = (int)(g - r * n);
-      int z = (int)dn.div(r);
-      int y = (int)(r - (long long)z * n);
-      T pc = p[r * ppitch + x];
-      T px = p[r * ppitch + wrap_up(x, n)];
-      T py = p[((long long)z * n + wrap_up(y, n)) * ppitch + x];
-      T pz = p[((long long)wrap_up(z, n) * n + y) * ppitch + x];
-      k0 -= (px - pc) * inv_h;
-      k1 -= (py - pc) * inv_h;
-      k2 -= (pz - pc) * inv_h;
-      if (STORE_K) {
-        k[g] = k0;
-        k[N + g] = k1;
-        k[2 * N + g] = k2;
-      }
+    const long long r = dn.div(g);
+    int x = (int)(g - r * n);
+    int z = (int)dn.div(r);
+    int y = (int)(r - (long long)z * n);
+    T pc = p[r * ppitch + x];
+    T px = p[r * ppitch + wrap_up(x, n)];
+    T py = p[((long long)z * n + wrap_up(y, n)) * ppitch + x];
+    T pz = p[((long long)wrap_up(z, n) * n + y) * ppitch + x];
+    k0 -= (px - pc) * inv_h;
+    k1 -= (py - pc) * inv_h;
+    k2 -= (pz - pc) * inv_h;
+    if (STORE_K) {
+      k[g] = k0;
+      k[N + g] = k1;
+      k[2 * N + g] = k2;
     }
     T a0 = 0, a1 = 0, a2 = 0;  // x0 is not read at stage 3
     if (stage < 3) {
@@ -81,7 +79,7 @@ __global__ void rk_stage_kernel(int n, T inv_h, T* __restrict__ k, const T* __re
   }
 }
 
-// FP32 form of rk_stage_kernel with GRAD for n % 4 == 0: four consecutive
+// FP32 form of rk_stage_kernel for n % 4 == 0: four consecutive
 // x cells per thread with 16-byte loads and stores (same arithmetic per
 // element, so the results are bitwise those of the scalar kernel).
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -339,7 +337,7 @@ cudaError_t launch_rk_stage(int n, T h, T* k, const T* p, int ppitch, const T* x
   long long N = (long long)n * n * n;
   dim3 grid(nslots > 1 ? std::min(grid_for(N), 152 * 8) : grid_for(N), nslots);
   if constexpr (sizeof(T) == 4) {
-    if (p && n % 4 == 0) {
+    if (n % 4 == 0) {
       dim3 g4(nslots > 1 ? std::min(grid_for(N / 4), 152 * 8) : grid_for(N / 4), nslots);
       const float ih = (float)(1.0 / (double)h);
       if (store_k)
@@ -351,7 +349,7 @@ cudaError_t launch_rk_stage(int n, T h, T* k, const T* p, int ppitch, const T* x
       return cudaGetLastError();
     }
   } else {
-    if (p && n % 2 == 0) {
+    if (n % 2 == 0) {
       dim3 g2(nslots > 1 ? std::min(grid_for(N / 2), 152 * 8) : grid_for(N / 2), nslots);
       const double ih = 1.0 / (double)h;
       if (store_k)
@@ -363,13 +361,10 @@ cudaError_t launch_rk_stage(int n, T h, T* k, const T* p, int ppitch, const T* x
       return cudaGetLastError();
     }
   }
-  if (p && store_k)
+  if (store_k)
     rk_stage_kernel<T, true><<<grid, 256, 0, st>>>(n, (T)(1.0 / (double)h), k, p, ppitch, x0, xs, xfin, stage, dtp, sb);
-  else if (p)
-    rk_stage_kernel<T, true, false><<<grid, 256, 0, st>>>(n, (T)(1.0 / (double)h), k, p, ppitch, x0, xs, xfin, stage,
-                                                          dtp, sb);
   else
-    rk_stage_kernel<T, false><<<grid, 256, 0, st>>>(n, (T)0, k, nullptr, 0, x0, xs, xfin, stage, dtp, sb);
+    rk_stage_kernel<T, false><<<grid, 256, 0, st>>>(n, (T)(1.0 / (double)h), k, p, ppitch, x0, xs, xfin, stage, dtp, sb);
   return cudaGetLastError();
 }
 

@@ -339,22 +339,7 @@ __global__ void oa_kernel(const T* __restrict__ tb3, int n, int c, Taps1D taps, 
   const T* __restrict__ tb = tb3 + comp * Mt;
   const IdxDiv dm(m);
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < M; g += (long long)gridDim.x * blockDim.x) {
-    const long long r = dm.div(g);
-    const int ix = (int)(g - r * m);
-    const int iz = (int)dm.div(r), iy = (int)(r - (long long)iz * m);
-    const int own = comp == 0 ? ix : (comp == 1 ? iy : iz);
-    // accumulate in the field's word type (FP32 form: no FP64-pipe work)
-    T acc = (T)0;
-    for (int t = 0; t < taps.cnt; ++t) {
-      int fi = c * own + taps.off[t];
-      fi = fi >= n ? fi - n : (fi < 0 ? fi + n : fi);
-      long long idx;
-      if (comp == 0) idx = ((long long)iz * m + iy) * n + fi;
-      else if (comp == 1) idx = ((long long)iz * n + fi) * m + ix;
-      else idx = ((long long)fi * m + iy) * m + ix;
-      acc += (T)taps.w[t] * tb[idx];
-    }
-    out3[comp * M + g] = acc * (T)scale;
+    out3[comp * M + g] = oa_value<T>(tb, n, c, m, taps, scale, OaCell(dm, m, g, comp), comp);
   }
 }
 

@@ -57,8 +57,11 @@ __host__ __device__ __forceinline__ long long invlap_index(int n, int kz, int ky
 
 // Allocate/free the device tables of a solver; `work` may be supplied by the
 // caller (external_work) and is otherwise allocated here.  run_time_plans =
-// false leaves grids without a compiled plan on the Stockham passes.
-int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bool run_time_plans = true);
+// false leaves grids without a compiled plan on the Stockham passes.  `slots`:
+// batched solves the own work array is for (n n P complex words each; a solver
+// with the mixed-precision solve takes one at a time).
+int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bool run_time_plans = true,
+                 int slots = 1);
 // Cases and served solves take the run-time plans in FP64 alone.  In FP32 the
 // sub-filter stress of a 2:1 LES is a difference of fields 4e-5 above their
 // rounding (400^3, ten steps: 4.3e-5 off 64-bit arithmetic with either

@@ -77,16 +77,23 @@ __global__ void slot_maxabs_partial(long long count, const T* __restrict__ u, lo
 
 // per-slot dt = min(cfl h/umax, cfl h^2/visc/6) (propose_timestep,
 // src/N.jl:348-356); a non-finite umax flags the slot and freezes it (dt = 0)
-__global__ void slot_set_dt(int S, const int* __restrict__ active, const double* __restrict__ part, double h,
-                            double cfl, const double* __restrict__ viscd, double* __restrict__ dt,
-                            double* __restrict__ clock, int* __restrict__ flag) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= S || !active[s]) return;
-  double m = 0.0;
-  for (int b = 0; b < SRV_RED; ++b) {
-    double v = part[s * SRV_RED + b];
-    m = (v > m || v != v) ? v : m;
-  }
+// One block of SRV_RED threads per slot (one thread folding the partials held
+// every step's start for 256 loads one after the other); the partials are
+// magnitudes or NaN, so the maximum of their bits is theirs.
+__global__ void __launch_bounds__(SRV_RED)
+    slot_set_dt(const int* __restrict__ active, const double* __restrict__ part, double h, double cfl,
+                const double* __restrict__ viscd, double* __restrict__ dt, double* __restrict__ clock,
+                int* __restrict__ flag) {
+  const int s = blockIdx.x;
+  if (!active[s]) return;
+  __shared__ unsigned long long red[SRV_RED / 32];
+  unsigned long long q = mag_bits(part[s * SRV_RED + threadIdx.x]);
+  for (int o = 16; o > 0; o >>= 1) q = max(q, __shfl_xor_sync(0xffffffffu, q, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = q;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < SRV_RED / 32; ++w) q = max(q, red[w]);
+  const double m = from_mag_bits<double>(q);
   double a = cfl * h / m, v = cfl * h * h / viscd[s] / 6.0;
   double d = a < v ? a : v;
   if (!(m < 1e300)) { flag[s] = 1; d = 0.0; }
@@ -259,12 +266,16 @@ class Chunk : public ChunkBase {
   int *active = nullptr, *flag = nullptr;
   SlotCtl* ctl = nullptr;  // device control block
   int cur = 0;             // 0: every active slot's state is in u[0] between launches
-  cudaGraphExec_t loop = nullptr;
-  int kernels_per_step = 0;
+  // Step loops by the slots they cover (the first `ns`).  A loop over all S
+  // slots starts the blocks of the empty ones and splits the sweeps of the few
+  // active ones for S: 100 steps of one 128^3 solve of 8 slots 46.6 ms, of a
+  // loop over its own slot 34.9; one 64^3 of 16 23.5 / 14.6, three 27.3 / 20.5.
+  // Built when first needed, for LOOP_SLOTS counts.
+  std::map<int, cudaGraphExec_t> loops;
 
   ~Chunk() override {
     if (stream) cudaStreamSynchronize(stream);
-    if (loop) cudaGraphExecDestroy(loop);
+    for (auto& l : loops) cudaGraphExecDestroy(l.second);
     if (ctl) cudaFree(ctl);
     if (mirror) cudaFreeHost(mirror);
     if (done_ev) cudaEventDestroy(done_ev);
@@ -286,22 +297,35 @@ class Chunk : public ChunkBase {
     return sb;
   }
 
-  // one batched RK4 step (same tableau and projection as the case stepper)
-  cudaError_t enqueue_step(int c) {
+  // Slots the next loop has to cover: free slots are taken from the lowest, so
+  // the active ones lie close together; rounded up to a few counts.
+  int loop_slots() const {
+    static constexpr int LOOP_SLOTS[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64};
+    int hi = 0;
+    for (int s = 0; s < S; ++s)
+      if (slot_id[s] >= 0) hi = s + 1;
+    for (int c : LOOP_SLOTS)
+      if (c >= hi) return std::min(c, S);
+    return S;
+  }
+
+  // one batched RK4 step of the first ns slots (same tableau and projection as
+  // the case stepper)
+  cudaError_t enqueue_step(int c, int ns) {
     const SlotBatch sb = batch();
     const T h = (T)(l / n);
     T* u0 = u[c];
     T* ufin = u[c ^ 1];
-    slot_maxabs_partial<T><<<dim3(SRV_RED, S), 256, 0, stream>>>(3 * N, u0, 3 * N, active, part);
-    slot_set_dt<<<(S + 63) / 64, 64, 0, stream>>>(S, active, part, l / n, cfl, viscd, dt, clock, flag);
+    slot_maxabs_partial<T><<<dim3(SRV_RED, ns), 256, 0, stream>>>(3 * N, u0, 3 * N, active, part);
+    slot_set_dt<<<ns, SRV_RED, 0, stream>>>(active, part, l / n, cfl, viscd, dt, clock, flag);
     cudaError_t e = cudaGetLastError();
     for (int s = 0; s < 4 && e == cudaSuccess; ++s) {
       const T* src = s == 0 ? u0 : us;
-      e = launch_rhs<T>(n, h, (T)0, src, rhs, false, stream, sb, S);
-      if (e == cudaSuccess) e = poisson_solve_inplace<T>(&ps, rhs, true, stream, sb, S);
+      e = launch_rhs<T>(n, h, (T)0, src, rhs, false, stream, sb, ns);
+      if (e == cudaSuccess) e = poisson_solve_inplace<T>(&ps, rhs, true, stream, sb, ns);
       if (e == cudaSuccess)
         e = launch_rk_stage<T>(n, h, rhs, reinterpret_cast<const T*>(ps.work), 2 * ps.P, u0, us, ufin, s, dt, stream,
-                               sb, S, false);
+                               sb, ns, false);
     }
     return e;
   }
@@ -309,7 +333,7 @@ class Chunk : public ChunkBase {
   // The device-side loop: WHILE (condition set by slot_ctl_kernel) { step
   // from u[0]; control; step from u[1]; control }, then the energies of the
   // retired slots and the copy of the control block to the pinned mirror.
-  cudaError_t build_loop() {
+  cudaError_t build_loop(int ns, cudaGraphExec_t* loop) {
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaGraphCreate(&g, 0);
     cudaGraphConditionalHandle h;
@@ -325,32 +349,27 @@ class Chunk : public ChunkBase {
       cudaGraph_t body = cp.conditional.phGraph_out[0];
       e = cudaStreamBeginCaptureToGraph(stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
       if (e == cudaSuccess) {
-        cudaError_t e2 = enqueue_step(0);
-        slot_ctl_kernel<<<1, SRV_MAXS, 0, stream>>>(S, 1, 0, kpairs, ctl, active, clock, h);
-        if (e2 == cudaSuccess) e2 = enqueue_step(1);
-        slot_ctl_kernel<<<1, SRV_MAXS, 0, stream>>>(S, 0, 1, kpairs, ctl, active, clock, h);
+        cudaError_t e2 = enqueue_step(0, ns);
+        slot_ctl_kernel<<<1, SRV_MAXS, 0, stream>>>(ns, 1, 0, kpairs, ctl, active, clock, h);
+        if (e2 == cudaSuccess) e2 = enqueue_step(1, ns);
+        slot_ctl_kernel<<<1, SRV_MAXS, 0, stream>>>(ns, 0, 1, kpairs, ctl, active, clock, h);
         if (e2 == cudaSuccess) e2 = cudaGetLastError();
         e = cudaStreamEndCapture(stream, &body);
         if (e2 != cudaSuccess) e = e2;
-      }
-      if (e == cudaSuccess) {
-        size_t num = 0;
-        cudaGraphGetNodes(body, nullptr, &num);
-        kernels_per_step = (int)num / 2;
       }
     }
     if (e == cudaSuccess)
       e = cudaStreamBeginCaptureToGraph(stream, g, &wnode, nullptr, 1, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-      slot_energy_partial<T><<<dim3(SRV_RED, S), 256, 0, stream>>>(3 * N, u[0], u[1], 3 * N, ctl, part);
-      slot_energy_fold<<<1, SRV_MAXS, 0, stream>>>(S, ctl, part);
+      slot_energy_partial<T><<<dim3(SRV_RED, ns), 256, 0, stream>>>(3 * N, u[0], u[1], 3 * N, ctl, part);
+      slot_energy_fold<<<1, SRV_MAXS, 0, stream>>>(ns, ctl, part);
       cudaError_t e2 = cudaMemcpyAsync(mirror, ctl, sizeof(SlotCtl), cudaMemcpyDeviceToHost, stream);
       if (e2 == cudaSuccess) e2 = cudaGetLastError();
       cudaGraph_t g2 = g;
       e = cudaStreamEndCapture(stream, &g2);
       if (e2 != cudaSuccess) e = e2;
     }
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&loop, g, 0);
+    if (e == cudaSuccess) e = cudaGraphInstantiate(loop, g, 0);
     if (g) cudaGraphDestroy(g);
     return e;
   }
@@ -532,11 +551,6 @@ static int make_chunk(exc_server* sv, int n, double l, double cfl, ChunkBase** o
     rc = tune_chunk<T>(sv, ck.get());
     if (rc) return rc;
   }
-  // capture the device-side step loop
-  {
-    cudaError_t e = ck->build_loop();
-    if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
-  }
   ck->bytes = need;
   sv->used += need;
   *out = ck.get();
@@ -666,9 +680,19 @@ template <typename T>
 static int launch_chunk(exc_server* sv, Chunk<T>* ck) {
   (void)sv;
   if (ck->in_flight || ck->active_count() == 0) return EXC_OK;
-  loop_begin_kernel<<<1, SRV_MAXS, 0, ck->stream>>>(ck->S, ck->ctl, ck->active);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaGraphLaunch(ck->loop, ck->stream);
+  const int ns = ck->loop_slots();
+  cudaError_t e = cudaSuccess;
+  auto loop = ck->loops.find(ns);
+  if (loop == ck->loops.end()) {
+    cudaGraphExec_t g = nullptr;
+    e = ck->build_loop(ns, &g);
+    if (e == cudaSuccess) loop = ck->loops.emplace(ns, g).first;
+  }
+  if (e == cudaSuccess) {
+    loop_begin_kernel<<<1, SRV_MAXS, 0, ck->stream>>>(ck->S, ck->ctl, ck->active);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaGraphLaunch(loop->second, ck->stream);
   if (e == cudaSuccess) e = cudaEventRecord(ck->done_ev, ck->stream);
   if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
   ck->in_flight = true;

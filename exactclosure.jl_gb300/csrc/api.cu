@@ -160,12 +160,10 @@ int exc_project(exc_poisson* ps, void* u, void* p_out, void* stream) {
   cudaError_t e;
   if (ps->precision == EXC_F64) {
     e = poisson_solve_inplace<double>(ps, (const double*)u, true, st);
-    if (e == cudaSuccess) e = launch_gradient<double>(ps->n, ps->h, (double*)u, (const double*)ps->work, 2 * ps->P, st);
-    if (e == cudaSuccess && p_out) e = copy_pressure<double>(ps, (double*)p_out, st);
+    if (e == cudaSuccess) e = finish_projection<double>(ps, (double*)u, (double*)p_out, st);
   } else {
     e = poisson_solve_inplace<float>(ps, (const float*)u, true, st);
-    if (e == cudaSuccess) e = launch_gradient<float>(ps->n, (float)ps->h, (float*)u, (const float*)ps->work, 2 * ps->P, st);
-    if (e == cudaSuccess && p_out) e = copy_pressure<float>(ps, (float*)p_out, st);
+    if (e == cudaSuccess) e = finish_projection<float>(ps, (float*)u, (float*)p_out, st);
   }
   return cuda_status(e);
 }

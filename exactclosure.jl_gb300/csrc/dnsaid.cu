@@ -135,10 +135,10 @@ const double* fd(const exc_dnsaid* d) { return d->fdelta.size() > 1 ? d->fdelta.
 int nfd(const exc_dnsaid* d) { return d->fdelta.size() > 1 ? (int)d->fdelta.size() : 0; }
 
 // project!(v, poisson) (src/N.jl:256-307) in place; the pressure stays in the
-// solver's work array.
-cudaError_t project(exc_poisson* ps, double* v, cudaStream_t st) {
+// solver's work array and goes to p if given.
+cudaError_t project(exc_poisson* ps, double* v, cudaStream_t st, double* p = nullptr) {
   cudaError_t e = poisson_solve_inplace<double>(ps, v, true, st);
-  if (e == cudaSuccess) e = launch_gradient<double>(ps->n, ps->h, v, (const double*)ps->work, 2 * ps->P, st);
+  if (e == cudaSuccess) e = finish_projection<double>(ps, v, p, st);
   return e;
 }
 
@@ -269,8 +269,7 @@ int lockstep(exc_dnsaid* d, double dt) {
   cudaStream_t st = d->st;
   // DNS right-hand side, projected; its pressure enters r = sigma + p I.
   cudaError_t e = launch_rhs<double>(n, d->h, d->visc, d->u, d->du, false, st);
-  if (e == cudaSuccess) e = project(&d->psd, d->du, st);
-  if (e == cudaSuccess) e = copy_pressure<double>(&d->psd, d->p, st);
+  if (e == cudaSuccess) e = project(&d->psd, d->du, st, d->p);
   if (e != cudaSuccess) return cuda_rc(e);
   // filters of the DNS: rDHi and sigmaDH; the classic closure's velocities
   // and ubar = apply_ΔHπ(u)
@@ -348,8 +347,7 @@ int lockstep_paper(exc_dnsaid* d, double dt) {
   cudaStream_t st = d->st;
   // DNS right-hand side, projected; its pressure enters r = sigma + p I
   cudaError_t e = launch_rhs<double>(n, d->h, d->visc, d->u, d->du, false, st);
-  if (e == cudaSuccess) e = project(&d->psd, d->du, st);
-  if (e == cudaSuccess) e = copy_pressure<double>(&d->psd, d->p, st);
+  if (e == cudaSuccess) e = project(&d->psd, d->du, st, d->p);
   if (e != cudaSuccess) return cuda_rc(e);
   // volume: fru = volume-filtered r (sdh), firu = face-filtered r (r9);
   // surface: firu = surface-filtered r (rc9), swap flux = firu on the

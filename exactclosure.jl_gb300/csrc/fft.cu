@@ -470,6 +470,19 @@ cudaError_t copy_pressure(const exc_poisson* ps, T* p, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+template <typename T>
+cudaError_t finish_projection(const exc_poisson* ps, T* u, T* p_out, cudaStream_t st) {
+  const uintptr_t N = (uintptr_t)ps->n * ps->n * ps->n * sizeof(T);
+  const uintptr_t a = reinterpret_cast<uintptr_t>(u), b = reinterpret_cast<uintptr_t>(p_out);
+  const bool apart = b + N <= a || a + 3 * N <= b;
+  cudaError_t e = launch_gradient<T>(ps->n, (T)ps->h, u, reinterpret_cast<const T*>(ps->work), 2 * ps->P, st,
+                                     apart ? p_out : nullptr);
+  if (e == cudaSuccess && p_out && !apart) e = copy_pressure<T>(ps, p_out, st);
+  return e;
+}
+template cudaError_t finish_projection<double>(const exc_poisson*, double*, double*, cudaStream_t);
+template cudaError_t finish_projection<float>(const exc_poisson*, float*, float*, cudaStream_t);
+
 template cudaError_t poisson_solve_inplace<double>(exc_poisson*, const double*, bool, cudaStream_t, const SlotBatch&,
                                                    int);
 template cudaError_t poisson_solve_inplace<float>(exc_poisson*, const float*, bool, cudaStream_t, const SlotBatch&,

@@ -154,15 +154,23 @@ constexpr int pow2_floor(int x) {
   return p;
 }
 
+constexpr int imin(int a, int b) { return a < b ? a : b; }
+constexpr int imax(int a, int b) { return a > b ? a : b; }
+
 // x-pass geometry: RW rows per CTA (a power of two, about 256 threads); the
 // exchange buffer row of XS complex words holds [k1][m2] with m2 stride 1 and
 // k1 stride N2 + 1 (odd: conflict-free level-B reads); XS = N2 (mod 16) so the
-// rows of a half warp start on different banks.
+// rows of a half warp start on different banks.  FP64 passes are bound by the
+// FP64 pipe of the SMs they reach: on grids under 96^3 fewer rows, so that some
+// 128 to 300 CTAs share the work, down to one warp each (32^3, 128 CTAs of 8
+// rows instead of 16 of 64: RHS and projection 65.6 -> 55.3 us; 48^3 77.8 ->
+// 75.8; 16 served 64^3 solves 3.82 -> 3.79 ms a step; FP32 measured no gain).
 template <typename T, int N1, int N2>
 struct XGeom {
   static constexpr int L = N1 * N2;
   static constexpr int NR = N1 > N2 ? N1 : N2;
-  static constexpr int RW = pow2_floor(256 / NR);
+  static constexpr int RW_FILL = sizeof(T) == 4 ? 256 : pow2_floor(imax(32 / NR, 4 * L * L / 256));
+  static constexpr int RW = imin(pow2_floor(256 / NR), RW_FILL);
   static constexpr int NT = RW * NR;
   static constexpr int XS0 = N1 * (N2 + 1);
   static constexpr int XS = XS0 + (((N2 - XS0) % 16) + 16) % 16;

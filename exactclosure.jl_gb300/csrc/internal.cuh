@@ -158,9 +158,14 @@ template <typename T>
 cudaError_t launch_tensordiv(int n, T h, int nsym, const T* s, T* du, bool doadd, cudaStream_t st);
 template <typename T>
 cudaError_t launch_divergence(int n, T h, const T* u, T* d, cudaStream_t st);
-// u_i -= (p[I+e_i] - p[I]) / h with p read at row pitch `ppitch` words.
+// u_i -= (p[I+e_i] - p[I]) / h with p read at row pitch `ppitch` words; pout
+// (may be null, not overlapping u) receives p densely.
 template <typename T>
-cudaError_t launch_gradient(int n, T h, T* u, const T* p, int ppitch, cudaStream_t st);
+cudaError_t launch_gradient(int n, T h, T* u, const T* p, int ppitch, cudaStream_t st, T* pout = nullptr);
+// The projection's last steps: u - grad p with the pressure in ps->work, and
+// the pressure to p_out if given (written after u where the two overlap).
+template <typename T>
+cudaError_t finish_projection(const exc_poisson* ps, T* u, T* p_out, cudaStream_t st);
 template <typename T>
 cudaError_t launch_max_abs(size_t count, const T* x, double* out_dev, double* partial, int npartial,
                            cudaStream_t st);

@@ -77,8 +77,7 @@ static int project_noalloc(int n, double l, T* u, T* p_out, cudaStream_t st) {
   ps.external_work = true;
   noalloc_tables_kernel<T><<<(n + 127) / 128, 128, 0, st>>>(n, reinterpret_cast<C*>(ps.tw), ps.sin2);
   cudaError_t e = poisson_solve_inplace<T>(&ps, u, true, st);
-  if (e == cudaSuccess) e = launch_gradient<T>(n, (T)ps.h, u, reinterpret_cast<const T*>(ps.work), 2 * ps.P, st);
-  if (e == cudaSuccess && p_out) e = copy_pressure<T>(&ps, p_out, st);
+  if (e == cudaSuccess) e = finish_projection<T>(&ps, u, p_out, st);
   if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
   return EXC_OK;
 }

@@ -95,6 +95,57 @@ struct SlotBatch {
   const void* visc = nullptr;     // per-slot viscosity (field word type), null = scalar argument
 };
 
+// Launches of the solver's kernel chains.  A chained kernel may be started while
+// the kernel before it in its stream still runs and waits on the device for that
+// kernel to end and its writes to be visible (chain_wait), so that the start of
+// a launch is not added to every link of the chain.  Every block of a kernel
+// launched with `chain` calls chain_wait before anything else, also before an
+// early return: the kernel after it relies on it having waited.  A kernel
+// without chain_wait is launched with <<<>>>.
+// Only launches of at most one block per SM outside a capture are chained so
+// (RHS and projection of 32^3 in FP64, eight launches: 51.2 -> 36.9 us).  Blocks
+// started beside the tail of a larger launch fill the SMs unevenly and the
+// FP64 passes wait for the fullest one (64^3: 101.6 us plain and up to 160
+// blocks, 109.6 with 310, 141.5 with 610), and captured graphs replay chains of
+// plain launches faster (ten steps of FP32 72^3 with two LES 12.2 / 13.9 ms).
+constexpr long long CHAIN_BLOCKS = 152;
+// The run-time FFT plans' passes and the general FP32 RHS up to 64 blocks: FP32
+// 24^3 48.3 -> 45.1 us, but with 152 44^3 49.4 -> 53.5 and 52^3 52.9 -> 56.9.
+constexpr long long CHAIN_BLOCKS_FEW = 64;
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+template <typename... P>
+struct ChainLaunch {
+  void (*kernel)(P...);
+  cudaLaunchConfig_t cfg;
+  long long most;
+  void operator()(P... args) const {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = cfg;
+    c.attrs = at;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    c.numAttrs = (long long)c.gridDim.x * c.gridDim.y * c.gridDim.z <= most &&
+                         cudaStreamIsCapturing(c.stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone
+                     ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, args...);
+  }
+};
+template <typename... P>
+inline ChainLaunch<P...> chain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                               long long most = CHAIN_BLOCKS) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  return {kernel, c, most};
+}
+
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 // Grid sizes the FFT supports: n = 2^a 3^b 5^c 7^d 11^e 13^f 17^g with a >= 1,

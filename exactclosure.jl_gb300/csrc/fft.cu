@@ -19,6 +19,7 @@ template <typename T, bool DIV, bool EXT = false>
 __global__ void __launch_bounds__(fft_threads<cplx<T>>(), 3)
 r2c_x_kernel(const T* __restrict__ src, int n, T inv_h, cplx<T>* __restrict__ out, int P,
              const cplx<T>* __restrict__ tw, FftPlan plan, int rows_per_cta, SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   extern __shared__ unsigned char smem_raw[];
   C* s = reinterpret_cast<C*>(smem_raw);
@@ -114,6 +115,7 @@ template <typename T, bool INV, bool EXT = false>
 __global__ void __launch_bounds__(fft_threads<cplx<T>>(), 3)
 cols_kernel(cplx<T>* __restrict__ g, int n, int nkx, int W, long long elem_stride,
             long long outer_stride, const cplx<T>* __restrict__ tw, FftPlan plan, SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   extern __shared__ unsigned char smem_raw[];
   C* const buf0 = reinterpret_cast<C*>(smem_raw);
@@ -203,6 +205,7 @@ __global__ void __launch_bounds__(fft_threads<cplx<T>>(), 3)
 zsolve_kernel(cplx<T>* __restrict__ g, int n, int nkx, int W, int P, const cplx<T>* __restrict__ tw,
               FftPlan plan, const double* __restrict__ sin2, double coef, const double* __restrict__ invlap,
               SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   extern __shared__ unsigned char smem_raw[];
   C* const buf0 = reinterpret_cast<C*>(smem_raw);
@@ -243,6 +246,7 @@ template <typename T, bool EXT = false>
 __global__ void __launch_bounds__(fft_threads<cplx<T>>(), 3)
 c2r_x_kernel(cplx<T>* __restrict__ g, int n, int P, const cplx<T>* __restrict__ tw, FftPlan plan,
              int rows_per_cta, SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   extern __shared__ unsigned char smem_raw[];
   C* s = reinterpret_cast<C*>(smem_raw);
@@ -290,6 +294,7 @@ c2r_x_kernel(cplx<T>* __restrict__ g, int n, int P, const cplx<T>* __restrict__ 
 
 template <typename T>
 __global__ void copy_pitched_kernel(const T* __restrict__ src, int pitch, T* __restrict__ dst, int n) {
+  chain_wait();
   long long N = (long long)n * n * n;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
        i += (long long)gridDim.x * blockDim.x) {
@@ -368,21 +373,21 @@ static cudaError_t stockham_solve(exc_poisson* ps, const T* src, bool src_is_vec
   size_t shx = (size_t)rows * padded_len(N2) * sizeof(C);
   dim3 gx((unsigned)((nn + rows - 1) / rows), nslots);
   if (src_is_vector)
-    r2c_x_kernel<T, true, EXT><<<gx, fft_threads<C>(), shx, st>>>(src, n, (T)(1.0 / ps->h), g, P, tw, ps->plan_h, rows, sb);
+    chain(r2c_x_kernel<T, true, EXT>, gx, fft_threads<C>(), shx, st)(src, n, (T)(1.0 / ps->h), g, P, tw, ps->plan_h, rows, sb);
   else
-    r2c_x_kernel<T, false, EXT><<<gx, fft_threads<C>(), shx, st>>>(src, n, (T)1, g, P, tw, ps->plan_h, rows, sb);
+    chain(r2c_x_kernel<T, false, EXT>, gx, fft_threads<C>(), shx, st)(src, n, (T)1, g, P, tw, ps->plan_h, rows, sb);
   // y forward
   const long long ntiles = (long long)((nkx + W - 1) / W) * n;
   size_t shc = 2 * (size_t)W * padded_len(n) * sizeof(C);
   dim3 gc(column_ctas(ntiles), 1, nslots);
-  cols_kernel<T, false, EXT><<<gc, fft_threads<C>(), shc, st>>>(g, n, nkx, W, P, (long long)n * P, tw, ps->plan_n, sb);
+  chain(cols_kernel<T, false, EXT>, gc, fft_threads<C>(), shc, st)(g, n, nkx, W, P, (long long)n * P, tw, ps->plan_n, sb);
   // z forward + divide + inverse; coef = 1/(lambda N) numerator: -h^2/(4 N)
   double coef = -ps->h * ps->h / (4.0 * (double)n * (double)n * (double)n);
-  zsolve_kernel<T, EXT><<<gc, fft_threads<C>(), shc, st>>>(g, n, nkx, W, P, tw, ps->plan_n, ps->sin2, coef, ps->invlap, sb);
+  chain(zsolve_kernel<T, EXT>, gc, fft_threads<C>(), shc, st)(g, n, nkx, W, P, tw, ps->plan_n, ps->sin2, coef, ps->invlap, sb);
   // y inverse
-  cols_kernel<T, true, EXT><<<gc, fft_threads<C>(), shc, st>>>(g, n, nkx, W, P, (long long)n * P, tw, ps->plan_n, sb);
+  chain(cols_kernel<T, true, EXT>, gc, fft_threads<C>(), shc, st)(g, n, nkx, W, P, (long long)n * P, tw, ps->plan_n, sb);
   // x inverse (in place)
-  c2r_x_kernel<T, EXT><<<gx, fft_threads<C>(), shx, st>>>(g, n, P, tw, ps->plan_h, rows, sb);
+  chain(c2r_x_kernel<T, EXT>, gx, fft_threads<C>(), shx, st)(g, n, P, tw, ps->plan_h, rows, sb);
   return cudaGetLastError();
 }
 
@@ -415,12 +420,12 @@ static cudaError_t fft3d_forward_t(exc_poisson* ps, const T* src, cudaStream_t s
   const SlotBatch one;
   size_t shx = (size_t)rows * padded_len(N2) * sizeof(C);
   int gx = (int)((nn + rows - 1) / rows);
-  r2c_x_kernel<T, false, EXT><<<gx, fft_threads<C>(), shx, st>>>(src, n, (T)1, g, P, tw, ps->plan_h, rows, one);
+  chain(r2c_x_kernel<T, false, EXT>, gx, fft_threads<C>(), shx, st)(src, n, (T)1, g, P, tw, ps->plan_h, rows, one);
   const long long ntiles = (long long)((nkx + W - 1) / W) * n;
   size_t shc = 2 * (size_t)W * padded_len(n) * sizeof(C);
   dim3 gc(column_ctas(ntiles));
-  cols_kernel<T, false, EXT><<<gc, fft_threads<C>(), shc, st>>>(g, n, nkx, W, P, (long long)n * P, tw, ps->plan_n, one);
-  cols_kernel<T, false, EXT><<<gc, fft_threads<C>(), shc, st>>>(g, n, nkx, W, (long long)n * P, P, tw, ps->plan_n, one);
+  chain(cols_kernel<T, false, EXT>, gc, fft_threads<C>(), shc, st)(g, n, nkx, W, P, (long long)n * P, tw, ps->plan_n, one);
+  chain(cols_kernel<T, false, EXT>, gc, fft_threads<C>(), shc, st)(g, n, nkx, W, (long long)n * P, P, tw, ps->plan_n, one);
   return cudaGetLastError();
 }
 
@@ -437,11 +442,11 @@ static cudaError_t fft3d_inverse_t(exc_poisson* ps, cudaStream_t st) {
   const long long ntiles = (long long)((nkx + W - 1) / W) * n;
   size_t shc = 2 * (size_t)W * padded_len(n) * sizeof(C);
   dim3 gc(column_ctas(ntiles));
-  cols_kernel<T, true, EXT><<<gc, fft_threads<C>(), shc, st>>>(g, n, nkx, W, (long long)n * P, P, tw, ps->plan_n, one);
-  cols_kernel<T, true, EXT><<<gc, fft_threads<C>(), shc, st>>>(g, n, nkx, W, P, (long long)n * P, tw, ps->plan_n, one);
+  chain(cols_kernel<T, true, EXT>, gc, fft_threads<C>(), shc, st)(g, n, nkx, W, (long long)n * P, P, tw, ps->plan_n, one);
+  chain(cols_kernel<T, true, EXT>, gc, fft_threads<C>(), shc, st)(g, n, nkx, W, P, (long long)n * P, tw, ps->plan_n, one);
   size_t shx = (size_t)rows * padded_len(N2) * sizeof(C);
   int gx = (int)((nn + rows - 1) / rows);
-  c2r_x_kernel<T, EXT><<<gx, fft_threads<C>(), shx, st>>>(g, n, P, tw, ps->plan_h, rows, one);
+  chain(c2r_x_kernel<T, EXT>, gx, fft_threads<C>(), shx, st)(g, n, P, tw, ps->plan_h, rows, one);
   return cudaGetLastError();
 }
 
@@ -466,7 +471,7 @@ template <typename T>
 cudaError_t copy_pressure(const exc_poisson* ps, T* p, cudaStream_t st) {
   long long N = (long long)ps->n * ps->n * ps->n;
   int blocks = (int)std::min<long long>((N + 255) / 256, 152LL * 16);
-  copy_pitched_kernel<T><<<blocks, 256, 0, st>>>(reinterpret_cast<const T*>(ps->work), 2 * ps->P, p, ps->n);
+  chain(copy_pitched_kernel<T>, blocks, 256, 0, st)(reinterpret_cast<const T*>(ps->work), 2 * ps->P, p, ps->n);
   return cudaGetLastError();
 }
 

@@ -77,6 +77,7 @@ template <typename T, bool INV>
 __global__ void __launch_bounds__(GEN_THREADS, 2)
 gcols_kernel(cplx<T>* __restrict__ g, GenLine ln, int nkx, int ntx, int wlog, long long es, long long outer_stride,
              const cplx<T>* __restrict__ tl, SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* const xs = reinterpret_cast<C*>(smem_raw);
@@ -122,6 +123,7 @@ template <typename T>
 __global__ void __launch_bounds__(GEN_THREADS, 2)
 gzsolve_kernel(cplx<T>* __restrict__ g, GenLine ln, int n, int nkx, int ntx, int wlog, int P,
                const cplx<T>* __restrict__ tl, const double* __restrict__ invlap, SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* const xs = reinterpret_cast<C*>(smem_raw);
@@ -266,6 +268,7 @@ template <typename T>
 __global__ void __launch_bounds__(GEN_THREADS, 2)
 gr2c_kernel(GenSrc<T> s, GenLine ln, int n, int rw, cplx<T>* __restrict__ out, int P, const cplx<T>* __restrict__ tw,
             const cplx<T>* __restrict__ tl, SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* const xs = reinterpret_cast<C*>(smem_raw);
@@ -367,6 +370,7 @@ template <typename T>
 __global__ void __launch_bounds__(GEN_THREADS, 2)
 gc2r_kernel(cplx<T>* g, GenLine ln, int n, int rw, int P, const cplx<T>* __restrict__ tw,
             const cplx<T>* __restrict__ tl, GenDst d, SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* const xs = reinterpret_cast<C*>(smem_raw);

@@ -7,7 +7,7 @@ template <>
 void gen_r2c<double>(const GenArgs<double>& a, const GenSrc<double>& s) {
   using C = cplx<double>;
   const int n = a.ps->n;
-  gr2c_kernel<double><<<dim3((unsigned)((n * n + a.rw - 1) / a.rw), a.nslots), GEN_THREADS, (size_t)a.rw * gen_xs(a.half) * sizeof(C), a.st>>>(
+  chain(gr2c_kernel<double>, dim3((unsigned)((n * n + a.rw - 1) / a.rw), a.nslots), GEN_THREADS, (size_t)a.rw * gen_xs(a.half) * sizeof(C), a.st, CHAIN_BLOCKS_FEW)(
       s, a.half, n, a.rw, reinterpret_cast<C*>(a.ps->work), a.ps->P, reinterpret_cast<const C*>(a.ps->tw),
       reinterpret_cast<const C*>(a.ps->twl_h), a.sb);
 }
@@ -16,7 +16,7 @@ template <>
 void gen_c2r<double>(const GenArgs<double>& a, const GenDst& d) {
   using C = cplx<double>;
   const int n = a.ps->n;
-  gc2r_kernel<double><<<dim3((unsigned)((n * n + a.rw - 1) / a.rw), a.nslots), GEN_THREADS, (size_t)a.rw * gen_xs(a.half) * sizeof(C), a.st>>>(
+  chain(gc2r_kernel<double>, dim3((unsigned)((n * n + a.rw - 1) / a.rw), a.nslots), GEN_THREADS, (size_t)a.rw * gen_xs(a.half) * sizeof(C), a.st, CHAIN_BLOCKS_FEW)(
       reinterpret_cast<C*>(a.ps->work), a.half, n, a.rw, a.ps->P, reinterpret_cast<const C*>(a.ps->tw),
       reinterpret_cast<const C*>(a.ps->twl_h), d, a.sb);
 }

@@ -194,6 +194,7 @@ template <typename T, int N1, int N2, bool INV>
 __global__ void __launch_bounds__(ColGeom<T, N1, N2>::NT, ColGeom<T, N1, N2>::MINB)
 rcols_kernel(cplx<T>* __restrict__ g, int nkx, int ntx, long long es, long long outer_stride,
              const cplx<T>* __restrict__ tl, SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   using G = ColGeom<T, N1, N2>;
   constexpr int W = G::W;
@@ -247,6 +248,7 @@ template <typename T, int N1, int N2>
 __global__ void __launch_bounds__(ColGeom<T, N1, N2>::NT, ColGeom<T, N1, N2>::MINB_Z)
 rzsolve_kernel(cplx<T>* __restrict__ g, int n, int nkx, int ntx, int P, const cplx<T>* __restrict__ tl,
                const double* __restrict__ invlap, SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   using G = ColGeom<T, N1, N2>;
   constexpr int W = G::W, L = N1 * N2;
@@ -388,6 +390,7 @@ template <typename T, int N1, int N2, bool INV>
 __global__ void __launch_bounds__(ColGeom<T, N1, N2>::NT, 3)
 rcols_pipe_kernel(cplx<T>* __restrict__ g, int nkx, int ntx, int ntiles, int P, long long es, long long outer_stride,
                   const cplx<T>* __restrict__ tl, SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   using G = ColGeom<T, N1, N2>;
   using Gp = PipeGeom<T, N1, N2>;
@@ -447,6 +450,7 @@ template <typename T, int N1, int N2>
 __global__ void __launch_bounds__(ColGeom<T, N1, N2>::NT, 2)
 rzsolve_pipe_kernel(cplx<T>* __restrict__ g, int n, int nkx, int ntx, int ntiles, int P,
                     const cplx<T>* __restrict__ tl, const double* __restrict__ invlap, SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   using G = ColGeom<T, N1, N2>;
   using Gp = PipeGeom<T, N1, N2>;
@@ -565,6 +569,7 @@ template <typename T, int N1, int N2, bool DIV, bool STAGE = false>
 __global__ void __launch_bounds__(XGeom<T, N1, N2>::NT)
 rr2c_kernel(const T* __restrict__ src, T inv_h, cplx<T>* __restrict__ out, int P, const cplx<T>* __restrict__ tw,
             const cplx<T>* __restrict__ tl, SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   using T2 = C;
   using G = XGeom<T, N1, N2>;
@@ -722,6 +727,7 @@ template <typename T, int N1, int N2>
 __global__ void __launch_bounds__(XGeom<T, N1, N2>::NT)
 rc2r_kernel(cplx<T>* __restrict__ g, int P, const cplx<T>* __restrict__ tw, const cplx<T>* __restrict__ tl,
             SlotBatch sb) {
+  chain_wait();
   using C = cplx<T>;
   using G = XGeom<T, N1, N2>;
   constexpr int L = N1 * N2, n = 2 * L, RW = G::RW, XS = G::XS;
@@ -811,16 +817,16 @@ struct RegSolve {
     if constexpr (PipeGeom<T, A1, A2>::OK) {
       using Gp = PipeGeom<T, A1, A2>;
       const dim3 gy((unsigned)pipe_ctas(ntiles, ns, 3), 1, ns), gz((unsigned)pipe_ctas(ntiles, ns, 4), 1, ns);
-      rcols_pipe_kernel<T, A1, A2, false><<<gy, CG::NT, Gp::SMEM_COLS, st>>>(g, nkx, ntx, ntiles, P, P,
+      chain(rcols_pipe_kernel<T, A1, A2, false>, gy, CG::NT, Gp::SMEM_COLS, st)(g, nkx, ntx, ntiles, P, P,
                                                                              (long long)n * P, tln, sb);
-      rzsolve_pipe_kernel<T, A1, A2><<<gz, CG::NT, Gp::SMEM_Z, st>>>(g, n, nkx, ntx, ntiles, P, tln, invlap, sb);
-      rcols_pipe_kernel<T, A1, A2, true><<<gy, CG::NT, Gp::SMEM_COLS, st>>>(g, nkx, ntx, ntiles, P, P,
+      chain(rzsolve_pipe_kernel<T, A1, A2>, gz, CG::NT, Gp::SMEM_Z, st)(g, n, nkx, ntx, ntiles, P, tln, invlap, sb);
+      chain(rcols_pipe_kernel<T, A1, A2, true>, gy, CG::NT, Gp::SMEM_COLS, st)(g, nkx, ntx, ntiles, P, P,
                                                                             (long long)n * P, tln, sb);
     } else {
       const dim3 gc((unsigned)ntiles, 1, ns);
-      rcols_kernel<T, A1, A2, false><<<gc, CG::NT, CG::SMEM, st>>>(g, nkx, ntx, P, (long long)n * P, tln, sb);
-      rzsolve_kernel<T, A1, A2><<<gc, CG::NT, CG::SMEM_Z, st>>>(g, n, nkx, ntx, P, tln, invlap, sb);
-      rcols_kernel<T, A1, A2, true><<<gc, CG::NT, CG::SMEM, st>>>(g, nkx, ntx, P, (long long)n * P, tln, sb);
+      chain(rcols_kernel<T, A1, A2, false>, gc, CG::NT, CG::SMEM, st)(g, nkx, ntx, P, (long long)n * P, tln, sb);
+      chain(rzsolve_kernel<T, A1, A2>, gc, CG::NT, CG::SMEM_Z, st)(g, n, nkx, ntx, P, tln, invlap, sb);
+      chain(rcols_kernel<T, A1, A2, true>, gc, CG::NT, CG::SMEM, st)(g, nkx, ntx, P, (long long)n * P, tln, sb);
     }
   }
 
@@ -838,17 +844,17 @@ struct RegSolve {
     if constexpr (XG::STAGE) {
       // 16-byte copies need a 16-byte aligned field (slot strides 3 n^3 words keep it)
       if (vec && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-        rr2c_kernel<T, B1, B2, true, true><<<gx, XG::NT, XG::SMEM_DIV, st>>>(src, (T)(1.0 / ps->h), g, P, tw, tlh, sb);
+        chain(rr2c_kernel<T, B1, B2, true, true>, gx, XG::NT, XG::SMEM_DIV, st)(src, (T)(1.0 / ps->h), g, P, tw, tlh, sb);
         staged = true;
       }
     }
     if (staged) {
     } else if (vec)
-      rr2c_kernel<T, B1, B2, true><<<gx, XG::NT, XG::SMEM, st>>>(src, (T)(1.0 / ps->h), g, P, tw, tlh, sb);
+      chain(rr2c_kernel<T, B1, B2, true>, gx, XG::NT, XG::SMEM, st)(src, (T)(1.0 / ps->h), g, P, tw, tlh, sb);
     else
-      rr2c_kernel<T, B1, B2, false><<<gx, XG::NT, XG::SMEM, st>>>(src, (T)1, g, P, tw, tlh, sb);
+      chain(rr2c_kernel<T, B1, B2, false>, gx, XG::NT, XG::SMEM, st)(src, (T)1, g, P, tw, tlh, sb);
     columns(g, nkx, P, tln, ps->invlap, st, sb, ns);
-    rc2r_kernel<T, B1, B2><<<gx, XG::NT, XG::SMEM, st>>>(g, P, tw, tlh, sb);
+    chain(rc2r_kernel<T, B1, B2>, gx, XG::NT, XG::SMEM, st)(g, P, tw, tlh, sb);
     return cudaGetLastError();
   }
 };

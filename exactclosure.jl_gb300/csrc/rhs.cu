@@ -148,6 +148,7 @@ template <typename T, int NC, bool DOADD>
 __global__ void __launch_bounds__(PTX * NWARP, 4)
 rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, SlotBatch sb, int zblocks, int ptz,
            const __grid_constant__ CUtensorMap umap, int have_map) {
+  chain_wait();
   constexpr int PTY = PTYT<NC>, PBY = PBYT<NC>;
   constexpr int CSTRIDE = (int)(sizeof(CompPlane<T, NC>) / sizeof(T));
   extern __shared__ __align__(128) unsigned char rhs_smem[];
@@ -477,6 +478,7 @@ template <bool DOADD>
 __global__ void __launch_bounds__(FXTHREADS, FX_CTAS)
 rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u, double* __restrict__ du, SlotBatch sb,
                  int zblocks, int ptz, const __grid_constant__ CUtensorMap umap, int have_map) {
+  chain_wait();
   using T = double;
   constexpr int NC = FXC;
   extern __shared__ __align__(128) unsigned char rhs_smem[];
@@ -824,6 +826,7 @@ template <bool DOADD>
 __global__ void __launch_bounds__(256, 3)
 rhs_quad_kernel(int n, float inv_h, float visc, const float* __restrict__ u, float* __restrict__ du, SlotBatch sb,
                 int zblocks, int ptz, const __grid_constant__ CUtensorMap umap, int have_map) {
+  chain_wait();
   extern __shared__ __align__(128) unsigned char quad_smem[];
   QuadSmem& sm = *reinterpret_cast<QuadSmem*>(quad_smem + ((128u - (smem_u32(quad_smem) & 127u)) & 127u));
   const long long N = (long long)n * n * n;
@@ -1172,9 +1175,9 @@ cudaError_t launch_rhs<double>(int n, double h, double visc, const double* u, do
                    encode_tiled_map(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, u, dims, strides, box);
   const dim3 block(PTX, FXW);
   if (doadd)
-    rhs_fixed_kernel<true><<<grid, block, FIXED_SMEM, st>>>(n, 1.0 / h, visc, u, du, sb, zblocks, ptz, map, have);
+    chain(rhs_fixed_kernel<true>, grid, block, FIXED_SMEM, st)(n, 1.0 / h, visc, u, du, sb, zblocks, ptz, map, have);
   else
-    rhs_fixed_kernel<false><<<grid, block, FIXED_SMEM, st>>>(n, 1.0 / h, visc, u, du, sb, zblocks, ptz, map, have);
+    chain(rhs_fixed_kernel<false>, grid, block, FIXED_SMEM, st)(n, 1.0 / h, visc, u, du, sb, zblocks, ptz, map, have);
   return cudaGetLastError();
 }
 
@@ -1192,10 +1195,10 @@ cudaError_t launch_rhs<float>(int n, float h, float visc, const float* u, float*
     CUtensorMap map;
     const int have = field_tensor_map<float>(u, n, nslots, sb, QROW, QBY, &map) ? 1 : 0;
     if (doadd)
-      rhs_quad_kernel<true><<<gq, dim3(32, 8), QUAD_SMEM, st>>>(n, ih, visc, u, du, sb,
+      chain(rhs_quad_kernel<true>, gq, dim3(32, 8), QUAD_SMEM, st)(n, ih, visc, u, du, sb,
                                                                 zblocks, ptz, map, have);
     else
-      rhs_quad_kernel<false><<<gq, dim3(32, 8), QUAD_SMEM, st>>>(n, ih, visc, u, du, sb,
+      chain(rhs_quad_kernel<false>, gq, dim3(32, 8), QUAD_SMEM, st)(n, ih, visc, u, du, sb,
                                                                  zblocks, ptz, map, have);
     return cudaGetLastError();
   }
@@ -1206,11 +1209,11 @@ cudaError_t launch_rhs<float>(int n, float h, float visc, const float* u, float*
   CUtensorMap map;
   const int have = field_tensor_map<float>(u, n, nslots, sb, UROW<float>, PBYT<NC>, &map) ? 1 : 0;
   if (doadd)
-    rhs_kernel<float, NC, true><<<grid, dim3(PTX, NWARP), sh, st>>>(n, (float)(1.0 / (double)h), visc, u, du, sb, zblocks, ptz,
-                                                                map, have);
+    chain(rhs_kernel<float, NC, true>, grid, dim3(PTX, NWARP), sh, st, CHAIN_BLOCKS_FEW)(
+        n, (float)(1.0 / (double)h), visc, u, du, sb, zblocks, ptz, map, have);
   else
-    rhs_kernel<float, NC, false><<<grid, dim3(PTX, NWARP), sh, st>>>(n, (float)(1.0 / (double)h), visc, u, du, sb, zblocks,
-                                                                 ptz, map, have);
+    chain(rhs_kernel<float, NC, false>, grid, dim3(PTX, NWARP), sh, st, CHAIN_BLOCKS_FEW)(
+        n, (float)(1.0 / (double)h), visc, u, du, sb, zblocks, ptz, map, have);
   return cudaGetLastError();
 }
 

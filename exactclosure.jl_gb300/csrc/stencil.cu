@@ -20,6 +20,7 @@ __device__ __forceinline__ void cell_of(long long g, int n, int& x, int& y, int&
 // The 6 stress components materialised (src/N.jl:94-118).
 template <typename T>
 __global__ void stress_kernel(int n, T h, T visc, const T* __restrict__ u, T* __restrict__ s6) {
+  chain_wait();
   const long long N = (long long)n * n * n;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
@@ -47,6 +48,7 @@ __global__ void stress_kernel(int n, T h, T visc, const T* __restrict__ u, T* __
 // du_i = doadd*du_i - sum_j delta_j s_ij with an explicit tensor (src/N.jl:120-200).
 template <typename T>
 __global__ void tensordiv_kernel(int n, T h, int nsym, const T* __restrict__ s, T* __restrict__ du, int doadd) {
+  chain_wait();
   const long long N = (long long)n * n * n;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
@@ -80,6 +82,7 @@ __global__ void tensordiv_kernel(int n, T h, int nsym, const T* __restrict__ s, 
 
 template <typename T>
 __global__ void divergence_kernel(int n, T h, const T* __restrict__ u, T* __restrict__ d) {
+  chain_wait();
   const long long N = (long long)n * n * n;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
@@ -96,6 +99,7 @@ __global__ void divergence_kernel(int n, T h, const T* __restrict__ u, T* __rest
 template <typename T>
 __global__ void gradient_kernel(int n, T inv_h, T* __restrict__ u, const T* __restrict__ p, int ppitch,
                                 T* __restrict__ pout) {
+  chain_wait();
   const long long N = (long long)n * n * n;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
@@ -118,6 +122,7 @@ __global__ void gradient_kernel(int n, T inv_h, T* __restrict__ u, const T* __re
 template <typename T>
 __global__ void gradient2_kernel(int n, T inv_h, T* __restrict__ u, const T* __restrict__ p, int ppitch,
                                  T* __restrict__ pout) {
+  chain_wait();
   using V2 = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
   const long long N = (long long)n * n * n;
   const int hx = n >> 1;
@@ -159,19 +164,19 @@ static inline int grid_for(long long N, int threads) {
 template <typename T>
 cudaError_t launch_stress(int n, T h, T visc, const T* u, T* s6, cudaStream_t st) {
   long long N = (long long)n * n * n;
-  stress_kernel<T><<<grid_for(N, 256), 256, 0, st>>>(n, h, visc, u, s6);
+  chain(stress_kernel<T>, grid_for(N, 256), 256, 0, st)(n, h, visc, u, s6);
   return cudaGetLastError();
 }
 template <typename T>
 cudaError_t launch_tensordiv(int n, T h, int nsym, const T* s, T* du, bool doadd, cudaStream_t st) {
   long long N = (long long)n * n * n;
-  tensordiv_kernel<T><<<grid_for(N, 256), 256, 0, st>>>(n, h, nsym, s, du, doadd ? 1 : 0);
+  chain(tensordiv_kernel<T>, grid_for(N, 256), 256, 0, st)(n, h, nsym, s, du, doadd ? 1 : 0);
   return cudaGetLastError();
 }
 template <typename T>
 cudaError_t launch_divergence(int n, T h, const T* u, T* d, cudaStream_t st) {
   long long N = (long long)n * n * n;
-  divergence_kernel<T><<<grid_for(N, 256), 256, 0, st>>>(n, h, u, d);
+  chain(divergence_kernel<T>, grid_for(N, 256), 256, 0, st)(n, h, u, d);
   return cudaGetLastError();
 }
 template <typename T>
@@ -181,9 +186,9 @@ cudaError_t launch_gradient(int n, T h, T* u, const T* p, int ppitch, cudaStream
                    (reinterpret_cast<uintptr_t>(p) % (2 * sizeof(T))) == 0 &&
                    (reinterpret_cast<uintptr_t>(pout) % (2 * sizeof(T))) == 0;
   if (vec)
-    gradient2_kernel<T><<<grid_for(N / 2, 256), 256, 0, st>>>(n, (T)(1.0 / (double)h), u, p, ppitch, pout);
+    chain(gradient2_kernel<T>, grid_for(N / 2, 256), 256, 0, st)(n, (T)(1.0 / (double)h), u, p, ppitch, pout);
   else
-    gradient_kernel<T><<<grid_for(N, 256), 256, 0, st>>>(n, (T)(1.0 / (double)h), u, p, ppitch, pout);
+    chain(gradient_kernel<T>, grid_for(N, 256), 256, 0, st)(n, (T)(1.0 / (double)h), u, p, ppitch, pout);
   return cudaGetLastError();
 }
 
@@ -193,6 +198,7 @@ cudaError_t launch_gradient(int n, T h, T* u, const T* p, int ppitch, cudaStream
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void maxabs_partial_kernel(size_t count, const T* __restrict__ x, double* __restrict__ partial) {
+  chain_wait();
   // the maximum of |x| is taken on the magnitude bits (unsigned integer order
   // equals the order of non-negative IEEE values, and NaN patterns sort above
   // infinity, so a NaN propagates): exact, on the integer pipe, and with
@@ -228,6 +234,7 @@ __global__ void maxabs_partial_kernel(size_t count, const T* __restrict__ x, dou
 }
 
 __global__ void maxabs_final_kernel(int np, const double* __restrict__ partial, double* __restrict__ out) {
+  chain_wait();
   __shared__ double red[32];
   double m = 0.0;
   for (int i = threadIdx.x; i < np; i += blockDim.x) {
@@ -255,8 +262,8 @@ cudaError_t launch_max_abs(size_t count, const T* x, double* out_dev, double* pa
                            cudaStream_t st) {
   int blocks = (int)std::min<size_t>((count + 255) / 256, (size_t)npartial);
   if (blocks < 1) blocks = 1;
-  maxabs_partial_kernel<T><<<blocks, 256, 0, st>>>(count, x, partial);
-  maxabs_final_kernel<<<1, 1024, 0, st>>>(blocks, partial, out_dev);
+  chain(maxabs_partial_kernel<T>, blocks, 256, 0, st)(count, x, partial);
+  chain(maxabs_final_kernel, 1, 1024, 0, st)(blocks, partial, out_dev);
   return cudaGetLastError();
 }
 

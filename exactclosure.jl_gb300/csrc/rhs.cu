@@ -787,8 +787,8 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
 }
 
 // ---------------------------------------------------------------------------
-// FP32 sweep with 2 x 2 cells per thread (64 x 16 tiles, grids that are
-// multiples of 64): each thread reads its u rows as aligned float pairs, takes
+// FP32 sweep with 2 x 2 cells per thread (64 x 16 tiles, the last ones ragged, of
+// rows of 16-byte multiples): each thread reads its u rows as aligned float pairs, takes
 // the x and y neighbour stresses of its own cells from registers and stores
 // float pairs, which halves the shared-memory and global instructions per
 // cell.  Same stress and divergence arithmetic, in the same order, as
@@ -855,7 +855,7 @@ rhs_quad_kernel(int n, float inv_h, float visc, const float* __restrict__ u, flo
       const int c = t / (QBY * 18), rem = t - c * (QBY * 18);
       const int rr = rem / 18, j = rem - rr * 18;
       const int gy = wrap(y0 - 1 + rr);
-      const int gx = j == 0 ? wrap(x0 - 4) : (j == 17 ? wrap(x0 + QX) : x0 + 4 * (j - 1));
+      const int gx = wrap(x0 + 4 * (j - 1));
       goff[i] = c * N + (long long)gy * n + gx;
       soff[i] = c * QCOMP + rr * QROW + 4 * j;
     }
@@ -1051,6 +1051,7 @@ rhs_quad_kernel(int n, float inv_h, float visc, const float* __restrict__ u, flo
         p23[j][i] = v23[j][i];
         p33[j][i] = v33[j][i];
       }
+      if (gx >= n || gy + j >= n) continue;  // outside a ragged tile's cells
       const long long g = ((long long)z * n + gy + j) * n + gx;
       float2* o1 = reinterpret_cast<float2*>(du1 + g);
       float2* o2 = reinterpret_cast<float2*>(du2 + g);
@@ -1186,11 +1187,19 @@ cudaError_t launch_rhs<float>(int n, float h, float visc, const float* u, float*
                               const SlotBatch& sb, int nslots) {
   constexpr int NC = CYT<float>;
   int ptz, zblocks;
-  // grids of 64-multiples with 16-byte aligned fields and at least one full
-  // wave of CTAs (three per SM): the 2 x 2 kernel
-  if (n % QX == 0 && (reinterpret_cast<uintptr_t>(u) & 15) == 0 && (reinterpret_cast<uintptr_t>(du) & 15) == 0 &&
-      zsplit(n, nslots, (long long)(n / QX) * (n / QY), 3, 4, 1, ptz, zblocks) >= 3LL * 152) {
-    dim3 gq(n / QX, n / QY, zblocks * nslots);
+  // the 2 x 2 kernel for 16-byte aligned fields whose rows are 16-byte
+  // multiples, its last tiles ragged.  Against the general kernel, which copies
+  // the last tile of a row that is no multiple of 32 word by word: 100^3 18.0 /
+  // 12.7 us, 180^3 56.3 / 38.1, 240^3 112 / 81, 500^3 704 / 583; not on fewer
+  // than 228 CTAs (72^3 9.9 / 10.1).  Without such tiles it wants a full wave
+  // (three CTAs per SM) and at most an eighth of padding: 128^3 16.7 / 15.5, 320^3
+  // 179 / 162, 512^3 691 / 622, but 96^3 9.4 / 10.0, 224^3 68.9 / 69.4.
+  const int qx = (n + QX - 1) / QX, qy = (n + QY - 1) / QY;
+  const long long qctas = zsplit(n, nslots, (long long)qx * qy, 3, 4, 1, ptz, zblocks);
+  const bool fits = n % PTX == 0 ? qctas >= 3LL * 152 && 8 * qx * QX <= 9 * n : qctas >= 228;
+  if (n % 4 == 0 && n >= QROW && fits && (reinterpret_cast<uintptr_t>(u) & 15) == 0 &&
+      (reinterpret_cast<uintptr_t>(du) & 15) == 0) {
+    dim3 gq(qx, qy, zblocks * nslots);
     const float ih = (float)(1.0 / (double)h);
     CUtensorMap map;
     const int have = field_tensor_map<float>(u, n, nslots, sb, QROW, QBY, &map) ? 1 : 0;

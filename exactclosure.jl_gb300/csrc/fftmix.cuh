@@ -69,7 +69,7 @@ mr2c_kernel(const double* __restrict__ src, double h, double* __restrict__ d, co
   const long long row0 = (long long)blockIdx.x * RW;
   const int tid = threadIdx.x;
   const int line = tid / N2, m2 = tid - line * N2;
-  double psum = 0.0;
+  SumF32 psum;
   C v[N1];
   if (tid < RW * N2) {
     const long long row = row0 + line;
@@ -134,7 +134,10 @@ mr2c_kernel(const double* __restrict__ src, double h, double* __restrict__ d, co
           if (store) d2[m] = rv;
           if constexpr (MODE == MIX_RES_MEAN) {
             const float2 pa = qp2[m];
-            psum += (f32_to_f64(pa.x) + f32_to_f64(qc.x)) + (f32_to_f64(pa.y) + f32_to_f64(qc.y));
+            psum.add(pa.x);
+            psum.add(qc.x);
+            psum.add(pa.y);
+            psum.add(qc.y);
           }
           v[m1] = to_f32c<C>(rv.x, rv.y);
         }
@@ -193,10 +196,11 @@ mr2c_kernel(const double* __restrict__ src, double h, double* __restrict__ d, co
   if constexpr (MODE == MIX_RES_MEAN) {
     // fixed-order block sum of p (deterministic for a fixed launch shape)
     __shared__ double red[32];
+    double ps = psum.value();
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) psum += __shfl_down_sync(0xffffffffu, psum, o);
+    for (int o = 16; o > 0; o >>= 1) ps += __shfl_down_sync(0xffffffffu, ps, o);
     const int warp = tid >> 5, lane = tid & 31;
-    if (lane == 0) red[warp] = psum;
+    if (lane == 0) red[warp] = ps;
     __syncthreads();
     if (tid == 0) {
       double s = 0.0;

@@ -83,6 +83,20 @@ __device__ __forceinline__ double stencil7_f32(float n0, float n1, float n2, flo
   return (f32_to_f64(h1) + f32_to_f64(h2)) + f32_to_f64(l2);
 }
 
+// Sum of FP32 values in two FP32 words (Knuth's TwoSum: six operations a term
+// on the FP32 pipe, where an FP64 addition takes the FP64 pipe as long as 64).
+// A thread sums a few hundred values of a CTA's rows: their sum is off by some
+// 2^-44 of one, the mean over all threads by less than 2^-53.
+struct SumF32 {
+  float hi = 0.0f, lo = 0.0f;
+  __device__ __forceinline__ void add(float x) {
+    const float s = __fadd_rn(hi, x), b = __fsub_rn(s, hi);
+    lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b)));
+    hi = s;
+  }
+  __device__ __forceinline__ double value() const { return f32_to_f64(hi) + f32_to_f64(lo); }
+};
+
 template <typename C>
 __device__ __forceinline__ C to_f32c(double a, double b) {
   C r;

@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
 // work of all 16 warps would take the pipe 16 times.  A step of 152 samples at
 // nh = 13500 by taps of shared loads in flight:
 //   nH               900      300     2700    nh 1500, nH 300
-//   FP64 filters   209 us
+//   FP64 filters   137 us  125      175      21.2
 //   one tap a time  82       79      104      13.3
 //   four taps       71       66       94      12.7
 // What is left is the FP64 pipe for the DNS update (five operations a cell,
@@ -983,6 +983,18 @@ int launch_err(exc_burgers* b) {
   return EXC_OK;
 }
 
+// One row of nH values per sample, `pitch` apart, to the host: gathered on the
+// device (the scratch rows are free between calls) and copied at once; 152
+// copies of one row took 1.4 ms.
+int rows_to_host(exc_burgers* b, double* host, const double* src, size_t pitch) {
+  const size_t row = (size_t)b->nH * sizeof(double);
+  cudaError_t e = cudaMemcpy2DAsync(b->scr, row, src, pitch * sizeof(double), row, b->ns, cudaMemcpyDeviceToDevice, b->st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(host, b->scr, row * b->ns, cudaMemcpyDeviceToHost, b->st);
+  if (e == cudaSuccess) return EXC_OK;
+  set_last_error(cudaGetErrorString(e));
+  return EXC_ERR_CUDA;
+}
+
 int max_steps_of(exc_burgers* b, int* out) {
   std::vector<int> s(b->ns);
   cudaError_t e = cudaMemcpyAsync(s.data(), b->steps, b->ns * sizeof(int), cudaMemcpyDeviceToHost, b->st);
@@ -1230,14 +1242,12 @@ int exc_burgers_get_les(exc_burgers* b, int which, double* host) {
   if (which == EXC_BURGERS_DNS_FIL) {
     int rc = run_terms(b, b->tmp, nullptr, nullptr, nullptr, nullptr);
     if (rc) return rc;
-    for (int s = 0; s < b->ns; ++s)
-      EXC_CHECK_CUDA(cudaMemcpyAsync(host + s * M, b->tmp + (size_t)s * 5 * M + 2 * M, M * sizeof(double),
-                                     cudaMemcpyDeviceToHost, b->st));
+    int rc2 = rows_to_host(b, host, b->tmp + 2 * M, 5 * M);
+    if (rc2) return rc2;
   } else if (which >= EXC_BURGERS_NOMODEL && which <= EXC_BURGERS_SWAPFIL) {
     const int k = which - EXC_BURGERS_NOMODEL;
-    for (int s = 0; s < b->ns; ++s)
-      EXC_CHECK_CUDA(cudaMemcpyAsync(host + s * M, b->v + (size_t)s * 4 * M + k * M, M * sizeof(double),
-                                     cudaMemcpyDeviceToHost, b->st));
+    int rc = rows_to_host(b, host, b->v + k * M, 4 * M);
+    if (rc) return rc;
   } else if (which == EXC_BURGERS_SMAG) {
     if (!b->smag_on) { set_last_error("no Smagorinsky solve has run"); return EXC_ERR_STATE; }
     EXC_CHECK_CUDA(cudaMemcpyAsync(host, b->smag, b->ns * M * sizeof(double), cudaMemcpyDeviceToHost, b->st));

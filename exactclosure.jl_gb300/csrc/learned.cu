@@ -23,6 +23,7 @@
 
 #include "internal.cuh"
 #include "fields.cuh"
+#include "fftmixops.cuh"
 
 #include <cuda_bf16.h>
 
@@ -31,6 +32,24 @@ namespace exc {
 constexpr int NET_TAPS = 27;
 constexpr int CONV_M = 64;  // voxels per CTA
 constexpr int CONV_THREADS = 128;
+constexpr int OUTP = 16;  // padded output channels
+constexpr int OUTS = 4;   // words of a voxel in the network's output (the three channels and a zero)
+
+// x * s rounded to float for a factor s given in 64 bits, as two floats on the
+// FP32 pipe: within 2^-24 ulp of the rounded FP64 product, which took three
+// FP64 instructions of 64 FP32 ones' time each.  Factors a float cannot hold
+// (`fast` false) and non-finite x take the plain forms.
+struct Scale {
+  float h, l;
+  bool fast;
+  double s;
+  explicit Scale(double v) : h((float)v), l((float)(v - (double)(float)v)), fast(std::fabs(v) > 0x1p-64 && std::fabs(v) < 0x1p64), s(v) {}
+  __device__ __forceinline__ float operator()(float x) const {
+    if (!fast) return (float)((double)x * s);
+    return fabsf(x) <= 3.402823466e38f ? fmaf(x, h, x * l) : x * h;
+  }
+  __device__ __forceinline__ float operator()(double x) const { return (float)(x * s); }
+};
 
 __device__ __forceinline__ float gelu_f(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_grad_f(float x) {
@@ -155,7 +174,7 @@ conv_mma_kernel(long long V, int n, const __nv_bfloat16* __restrict__ in, const 
           }
         } else if (EPI == 1) {
           x += bias[co];
-          pre_out[v * NP + co] = co < nout_valid ? x : 0.f;
+          if (co < OUTS) pre_out[v * OUTS + co] = co < nout_valid ? x : 0.f;
         } else {
           act_out[v * NP + co] = __float2bfloat16(x * __bfloat162float(dg[v * NP + co]));
         }
@@ -262,7 +281,7 @@ conv_tile_kernel(int n, const __nv_bfloat16* __restrict__ in, const __nv_bfloat1
           }
         } else if (EPI == 1) {
           x += bias[co];
-          pre_out[v * NP + co] = co < nout_valid ? x : 0.f;
+          if (co < OUTS) pre_out[v * OUTS + co] = co < nout_valid ? x : 0.f;
         } else {
           act_out[v * NP + co] = __float2bfloat16(x * __bfloat162float(dg[v * NP + co]));
         }
@@ -424,8 +443,9 @@ conv_res_kernel(int batch, int n, const __nv_bfloat16* __restrict__ in, const __
         } else if (EPI == 1) {
           x0v += bias[co];
           x1v += bias[co + 1];
-          *reinterpret_cast<float2*>(pre_out + v * NP + co) =
-              make_float2(co < nout_valid ? x0v : 0.f, co + 1 < nout_valid ? x1v : 0.f);
+          if (co < OUTS)
+            *reinterpret_cast<float2*>(pre_out + v * OUTS + co) =
+                make_float2(co < nout_valid ? x0v : 0.f, co + 1 < nout_valid ? x1v : 0.f);
         } else {
           const float2 dd = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(dg + v * NP + co));
           *reinterpret_cast<__nv_bfloat162*>(act_out + v * NP + co) =
@@ -584,7 +604,7 @@ template <int NP, int EPI>
 __global__ void __launch_bounds__(CU_THREADS, 1)
 conv_umma_kernel(int batch, const __grid_constant__ HaloMaps maps, const __nv_bfloat16* __restrict__ Wt,
                  const float* __restrict__ bias, float* __restrict__ pre_out, __nv_bfloat16* __restrict__ act_out,
-                 __nv_bfloat16* __restrict__ dg, int nout_valid) {
+                 __nv_bfloat16* __restrict__ dg, int nout_valid, Scale oscale) {
   constexpr int n = CU_N, KP = CU_KP, KC = CU_KC, NT = 3 * NP, NH = NP / 2;
   constexpr int HB = cu_halo_bytes, WB = cu_w_bytes<NP>();
   constexpr unsigned TCOLS = cu_tmem_cols<NP>();
@@ -726,9 +746,11 @@ conv_umma_kernel(int batch, const __grid_constant__ HaloMaps maps, const __nv_bf
     // 32 voxels of the same row
     const int q = warp & 3, k = (warp - 2) >> 2, et = k & 1, eh = k >> 1;
     const int erow = 2 * et + (q >> 1), x = 32 * (q & 1) + lane, cb = eh * NH;
+    constexpr bool OUT = EPI == 1 || EPI == 3;  // the last layer: the first OUTS channels
+    constexpr int NQ = OUT ? OUTS : NH;         // channels a thread finishes
     float bb[NH];
 #pragma unroll
-    for (int j = 0; j < NH; ++j) bb[j] = (EPI == 2) ? 0.f : __ldg(bias + cb + j);
+    for (int j = 0; j < NH; ++j) bb[j] = (EPI == 2 || (OUT && eh)) ? 0.f : __ldg(bias + cb + j);
     for (int i = 0; i < nb; ++i) {
       const int set = i & 1;
       if (!__all_sync(0xffffffffu, cu_wait(&afull[set], (unsigned)((i >> 1) & 1), polls))) {
@@ -737,6 +759,12 @@ conv_umma_kernel(int batch, const __grid_constant__ HaloMaps maps, const __nv_bf
       }
       if (*s_abort) break;
       tc_fence_after();
+      if (OUT && eh) {  // no output channel in this half: only release the set
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) cu_arrive(&aempty[set]);
+        continue;
+      }
       const unsigned ta = tmem + ((unsigned)(32 * q) << 16) + (unsigned)((set * 2 + et) * NT + cb);
       unsigned d0[NH], d1[NH], d2[NH];
       tmem_ld_nowait<NH>(ta, d0);
@@ -749,11 +777,11 @@ conv_umma_kernel(int batch, const __grid_constant__ HaloMaps maps, const __nv_bf
       const float* const other = xch + ((i & 1) * CU_EPI_WARPS + ((warp ^ 1) - 2)) * 2 * NH;
       if (lane == 31) {
 #pragma unroll
-        for (int j = 0; j < NH; ++j) mine[j] = __uint_as_float(d0[j]);
+        for (int j = 0; j < NQ; ++j) mine[j] = __uint_as_float(d0[j]);
       }
       if (lane == 0) {
 #pragma unroll
-        for (int j = 0; j < NH; ++j) mine[NH + j] = __uint_as_float(d2[j]);
+        for (int j = 0; j < NQ; ++j) mine[NH + j] = __uint_as_float(d2[j]);
       }
       __syncwarp();
       unsigned long long* const xb = &xbar[((warp - 2) >> 1) * 2 + (i & 1)];
@@ -762,9 +790,9 @@ conv_umma_kernel(int batch, const __grid_constant__ HaloMaps maps, const __nv_bf
         if (lane == 0) fault();
         break;
       }
-      float f[NH];
+      float f[NQ];
 #pragma unroll
-      for (int j = 0; j < NH; ++j) {
+      for (int j = 0; j < NQ; ++j) {
         // D[x - 1][0] from the lane below, D[x + 1][2] from the lane above
         float lo = __uint_as_float(__shfl_up_sync(0xffffffffu, d0[j], 1));
         float hi = __uint_as_float(__shfl_down_sync(0xffffffffu, d2[j], 1));
@@ -781,15 +809,15 @@ conv_umma_kernel(int batch, const __grid_constant__ HaloMaps maps, const __nv_bf
       int z0, y0;
       origin(blockIdx.x + (long long)i * gridDim.x, s, z0, y0);
       const long long g = s * N + ((long long)z0 * n + (y0 + erow)) * n + x;
-      if (EPI == 0 || EPI == 1) {
+      if (EPI != 2) {
 #pragma unroll
-        for (int j = 0; j < NH; j += 4) {
+        for (int j = 0; j < NQ; j += 4) {
           float4 v;
           v.x = f[j] + bb[j];
           v.y = f[j + 1] + bb[j + 1];
           v.z = f[j + 2] + bb[j + 2];
           v.w = f[j + 3] + bb[j + 3];
-          if (EPI == 1) {
+          if (OUT) {
             const int co = cb + j;
             v.x = co < nout_valid ? v.x : 0.f;
             v.y = co + 1 < nout_valid ? v.y : 0.f;
@@ -797,7 +825,13 @@ conv_umma_kernel(int batch, const __grid_constant__ HaloMaps maps, const __nv_bf
             v.w = co + 3 < nout_valid ? v.w : 0.f;
           }
           if (EPI == 1) {
-            *reinterpret_cast<float4*>(pre_out + g * NP + cb + j) = v;
+            *reinterpret_cast<float4*>(pre_out + g * OUTS) = v;
+          } else if (EPI == 3) {
+            // the scaled fields themselves, [sample][3][n^3]
+            float* const o = pre_out + 2 * s * N + g;
+            o[0] = oscale(v.x);
+            o[N] = oscale(v.y);
+            o[2 * N] = oscale(v.z);
           } else if (dg) {
             float ga, da, gb, db, gc, dc, gd, dd;
             gelu_and_grad(v.x, ga, da);
@@ -884,7 +918,7 @@ static void conv_launch(int engine, long long V, int n, const __nv_bfloat16* in,
         const long long nblk = (long long)batch * n * (n / CU_ROWS);
         const long long ctas = std::min<long long>(nblk, 152);
         conv_umma_kernel<NP, EPI><<<(unsigned)ctas, CU_THREADS, conv_umma_smem<NP>(), st>>>(
-            batch, maps, W, bias, pre_out, act_out, dg, nout_valid);
+            batch, maps, W, bias, pre_out, act_out, dg, nout_valid, Scale(1.0));
         return;
       }
     }
@@ -1432,7 +1466,7 @@ __global__ void wgrad_fold_kernel(int nchunk, const float* __restrict__ part, fl
   const int i = t >> 2, q = t & 3;
   double s = 0;
   if (i < NET_TAPS * PAIRS)
-    for (int c = q; c < nchunk; c += 4) s += (double)part[(long long)c * NET_TAPS * PAIRS + i];
+    for (int c = q; c < nchunk; c += 4) s += f32_to_f64(part[(long long)c * NET_TAPS * PAIRS + i]);
   s += __shfl_xor_sync(0xffffffffu, s, 1);
   s += __shfl_xor_sync(0xffffffffu, s, 2);
   if (q == 0 && i < NET_TAPS * PAIRS) dW[i] = (float)s;
@@ -1479,7 +1513,7 @@ __global__ void bgrad_fold_kernel(int nblk, const double* __restrict__ part, flo
 // ---------------------------------------------------------------------------
 // fields [b][3][n^3] (T) -> channel-last bf16 [b n^3][KP], scaled
 template <typename T>
-__global__ void pack_input_kernel(long long V, long long N, const T* __restrict__ f, double scale,
+__global__ void pack_input_kernel(long long V, long long N, const T* __restrict__ f, Scale scale,
                                   __nv_bfloat16* __restrict__ out, int KP) {
   // one voxel row per thread, written as 16-byte pieces (KP % 8 == 0)
   const IdxDiv dN(N);
@@ -1488,29 +1522,34 @@ __global__ void pack_input_kernel(long long V, long long N, const T* __restrict_
     __nv_bfloat16 row[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c)
-      row[c] = __float2bfloat16(c < 3 ? (float)((double)f[(b * 3 + c) * N + r] * scale) : 0.f);
+      row[c] = __float2bfloat16(c < 3 ? scale(f[(b * 3 + c) * N + r]) : 0.f);
     uint4* o = reinterpret_cast<uint4*>(out + v * KP);
     o[0] = *reinterpret_cast<const uint4*>(row);
     for (int c = 1; c < KP / 8; ++c) o[c] = make_uint4(0, 0, 0, 0);
   }
 }
 
-constexpr int OUTP = 16;  // padded output channels
-
-// net output [V][OUTP] (FP32, normalised) -> fields [b][3][n^3] (T) * scale
+// net output [V][OUTS] (FP32, normalised) -> fields [b][3][n^3] (T) * scale
 template <typename T>
-__global__ void unpack_output_kernel(long long V, long long N, const float* __restrict__ o, double scale,
+__global__ void unpack_output_kernel(long long V, long long N, const float* __restrict__ o, Scale scale,
                                      T* __restrict__ f) {
+  const IdxDiv dN(N);
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x) {
-    const long long b = v / N, r = v - b * N;
-    for (int c = 0; c < 3; ++c) f[(b * 3 + c) * N + r] = (T)((double)o[v * OUTP + c] * scale);
+    const long long b = dN.div(v), r = v - b * N;
+    const float4 w = *reinterpret_cast<const float4*>(o + v * OUTS);
+    const float c3[3] = {w.x, w.y, w.z};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      if constexpr (sizeof(T) == 8) f[(b * 3 + c) * N + r] = (double)c3[c] * scale.s;
+      else f[(b * 3 + c) * N + r] = scale(c3[c]);
+    }
   }
 }
 
-// g = 2 (out - target*tscale) / count (bf16, [V][OUTP]); per-block squared-error partials
+// g = 2 (out - target*tscale) / count (bf16, [V][OUTP]; out [V][OUTS]); per-block squared-error partials
 template <typename T>
 __global__ void loss_grad_kernel(long long V, long long N, const float* __restrict__ out, const T* __restrict__ tgt,
-                                 double tscale, double inv_count, __nv_bfloat16* __restrict__ g,
+                                 Scale tscale, double inv_count, __nv_bfloat16* __restrict__ g,
                                  double* __restrict__ part) {
   __shared__ double red[256];
   double s = 0;
@@ -1518,16 +1557,19 @@ __global__ void loss_grad_kernel(long long V, long long N, const float* __restri
   const float gs = (float)(2.0 * inv_count);
   for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < V; v += (long long)gridDim.x * blockDim.x) {
     const long long b = dN.div(v), r = v - b * N;
-    // the output row's first 4 words in one 16-byte load; the gradient row
+    // the output row in one 16-byte load; the gradient row
     // (3 values, then zeros) in 16-byte pieces
-    const float4 o4 = *reinterpret_cast<const float4*>(out + v * OUTP);
+    const float4 o4 = *reinterpret_cast<const float4*>(out + v * OUTS);
     const float oc[3] = {o4.x, o4.y, o4.z};
     __nv_bfloat16 row[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
       float d = 0.f;
-      if (c < 3) d = oc[c] - (float)((double)tgt[(b * 3 + c) * N + r] * tscale);
-      if (c < 3) s += (double)d * d;
+      if (c < 3) d = oc[c] - tscale(tgt[(b * 3 + c) * N + r]);
+      if (c < 3) {
+        const double dd = f32_to_f64(d);
+        s = fma(dd, dd, s);
+      }
       row[c] = __float2bfloat16(gs * d);
     }
     uint4* gr = reinterpret_cast<uint4*>(g + v * OUTP);
@@ -1654,7 +1696,7 @@ static int ensure_workspace(exc_net* net, long long V) {
             cudaMalloc(&net->gp1, V * exc_net::N1 * 2) == cudaSuccess &&
             cudaMalloc(&net->dg1, V * exc_net::N1 * 2) == cudaSuccess &&
             cudaMalloc(&net->dg2, V * exc_net::N2 * 2) == cudaSuccess &&
-            cudaMalloc(&net->out, V * exc_net::N3 * 4) == cudaSuccess &&
+            cudaMalloc(&net->out, V * OUTS * 4) == cudaSuccess &&
             cudaMalloc(&net->wpart, nchunk * 27 * 32 * 32 * 4 + (long long)WT_CTAS * 2 * 32 * sizeof(double)) == cudaSuccess &&
             cudaMalloc(&net->lpart, (1024 + 8) * sizeof(double)) == cudaSuccess;
   if (!ok) {
@@ -1682,11 +1724,13 @@ static cudaError_t refresh(exc_net* net, cudaStream_t st) {
 
 // forward from the packed input x0; leaves a1, a2, out and, for training,
 // the GELU derivatives dg1, dg2
-static cudaError_t forward_packed(exc_net* net, long long V, int n, bool train, cudaStream_t st) {
+// (`hidden` alone: without the last layer)
+static cudaError_t forward_packed(exc_net* net, long long V, int n, bool train, cudaStream_t st, bool hidden = false) {
   conv_launch<16, 32, 0>(net->conv_engine, V, n, net->x0, net->Wt(0), net->B(0), nullptr, net->a1,
                          train ? net->dg1 : nullptr, 32, st);
   conv_launch<32, 32, 0>(net->conv_engine, V, n, net->a1, net->Wt(1), net->B(1), nullptr, net->a2,
                          train ? net->dg2 : nullptr, 32, st);
+  if (hidden) return cudaGetLastError();
   conv_launch<32, 16, 1>(net->conv_engine, V, n, net->a2, net->Wt(2), net->B(2), net->out, nullptr, nullptr, 3, st);
   return cudaGetLastError();
 }
@@ -1737,7 +1781,7 @@ static cudaError_t wgrad(exc_net* net, int l, long long V, int n, const __nv_bfl
 template <typename T>
 static cudaError_t backward(exc_net* net, long long V, int n, long long N, const T* target, cudaStream_t st) {
   const int lb = (int)std::min<long long>((V + 255) / 256, 1024);
-  loss_grad_kernel<T><<<lb, 256, 0, st>>>(V, N, net->out, target, 1.0 / net->out_scale, 1.0 / (3.0 * (double)V),
+  loss_grad_kernel<T><<<lb, 256, 0, st>>>(V, N, net->out, target, Scale(1.0 / net->out_scale), 1.0 / (3.0 * (double)V),
                                           net->g3, net->lpart);
   sum_kernel<<<1, 256, 0, st>>>(lb, net->lpart, 1.0 / (3.0 * (double)V), net->lpart + 1024);
   cudaError_t e = wgrad<32, 16>(net, 2, V, n, net->a2, net->g3, st);
@@ -1756,10 +1800,29 @@ static int net_forward_t(exc_net* net, int batch, int n, const T* u, T* m, cudaS
   int rc = ensure_workspace(net, V);
   if (rc) return rc;
   const int gb = (int)std::min<long long>((V + 255) / 256, 152LL * 32);
-  pack_input_kernel<T><<<gb, 256, 0, st>>>(V, N, u, 1.0 / net->in_scale, net->x0, exc_net::K1);
-  cudaError_t e = forward_packed(net, V, n, false, st);
+  pack_input_kernel<T><<<gb, 256, 0, st>>>(V, N, u, Scale(1.0 / net->in_scale), net->x0, exc_net::K1);
+  cudaError_t e;
+  if (sizeof(T) == 4 && net->conv_engine == 0 && n == CU_N && batch > 0) {
+    // the last tcgen05 layer writes the scaled fields itself
+    e = forward_packed(net, V, n, false, st, true);
+    HaloMaps maps;
+    if (e == cudaSuccess && halo_maps(net->a2, batch, &maps)) {
+      const long long nblk = (long long)batch * n * (n / CU_ROWS);
+      conv_umma_kernel<16, 3><<<(unsigned)std::min<long long>(nblk, 152), CU_THREADS, conv_umma_smem<16>(), st>>>(
+          batch, maps, net->Wt(2), net->B(2), reinterpret_cast<float*>(m), nullptr, nullptr, 3, Scale(net->out_scale));
+      e = cudaGetLastError();
+      if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
+      return EXC_OK;
+    }
+    if (e == cudaSuccess) {
+      conv_launch<32, 16, 1>(net->conv_engine, V, n, net->a2, net->Wt(2), net->B(2), net->out, nullptr, nullptr, 3, st);
+      e = cudaGetLastError();
+    }
+  } else {
+    e = forward_packed(net, V, n, false, st);
+  }
   if (e == cudaSuccess) {
-    unpack_output_kernel<T><<<gb, 256, 0, st>>>(V, N, net->out, net->out_scale, m);
+    unpack_output_kernel<T><<<gb, 256, 0, st>>>(V, N, net->out, Scale(net->out_scale), m);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
@@ -1772,7 +1835,7 @@ static int net_grad_t(exc_net* net, int batch, int n, const T* u, const T* m, cu
   int rc = ensure_workspace(net, V);
   if (rc) return rc;
   const int gb = (int)std::min<long long>((V + 255) / 256, 152LL * 32);
-  pack_input_kernel<T><<<gb, 256, 0, st>>>(V, N, u, 1.0 / net->in_scale, net->x0, exc_net::K1);
+  pack_input_kernel<T><<<gb, 256, 0, st>>>(V, N, u, Scale(1.0 / net->in_scale), net->x0, exc_net::K1);
   cudaError_t e = forward_packed(net, V, n, true, st);
   if (e == cudaSuccess) e = backward<T>(net, V, n, N, m, st);
   if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
@@ -1840,6 +1903,7 @@ static int configure_learned() {
   if (e == cudaSuccess) e = conv_res_attr<32, 32, 2>();
   if (e == cudaSuccess) e = conv_umma_attr<32, 0>();
   if (e == cudaSuccess) e = conv_umma_attr<16, 1>();
+  if (e == cudaSuccess) e = conv_umma_attr<16, 3>();
   if (e == cudaSuccess) e = conv_umma_attr<32, 2>();
   if (e == cudaSuccess) e = wgrad_umma_attr<16, 32>();
   if (e == cudaSuccess) e = wgrad_umma_attr<32, 32>();

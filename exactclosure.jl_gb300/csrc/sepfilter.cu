@@ -11,17 +11,21 @@
 // 1/c^3) FP64 operations per fine cell instead of T^3 / c^3 times the cost of
 // evaluating the source: 17 taps at ratio 5 (the box of 5 convolved with the
 // reference's Gaussian of width 2H) are 4 instead of 39 source evaluations.
-// The FP64 pipe (two operations per clock per SM) bounds the x pass, which
-// evaluates every source once per fine cell and shares it between all filters
-// of it; all targets of a batch go through three launches.
+// The x pass evaluates every source once per fine cell (on the FP64 pipe, two
+// operations per clock per SM) and shares it between all filters of it, whose
+// products go to the integer pipe; all targets of a batch go through three
+// launches.
 //
 // One lockstep step of dnsaid_project, DNS 250^3, ratio 5, that Gaussian: 165
 // -> 11.7 ms, the filters (sums over T^3 taps per LES cell before) 155 -> 4.4
-// ms: x pass 2.8 ms = 85 FP64 operations per fine cell at the pipe's rate, y
-// 0.7, z 0.3.  Without the Gaussian (5 taps) 10.7 -> 9.8 ms, ratio 3 at 240^3
+// ms with an x pass of 2.8 ms in FP64 (85 operations per fine cell at the
+// pipe's rate), y 0.7, z 0.3; the step is 6.5 ms now.  Without the Gaussian (5 taps) 10.7 -> 9.8 ms, ratio 3 at 240^3
 // 11.0 -> 10.3, 60^3 1.50 -> 1.22.
 #include <cstring>
 
+#include <cmath>
+
+#include "fixed.cuh"
 #include "internal.cuh"
 #include "sepfilter.cuh"
 
@@ -39,8 +43,17 @@ struct XVar {
   int taps;
   double* out;
 };
+// Fixed-point form of the x pass: values as 57-bit integers below the CTA's
+// largest, weights below their list's largest, sums of at most MAX_TAPS
+// products below 2^63 (halves of 2^28: 40 x 2^57 for the two middle products).
+constexpr int SX_BITS = 57, SX_LOW = 29;
+static_assert(2 * (long long)MAX_TAPS < (1LL << (63 - 2 * (SX_BITS - SX_LOW))), "sums fit");
+
 struct XArgs {
   Taps1D taps[SEP_MAX_TAPSETS];
+  int2 wx[SEP_MAX_TAPSETS][MAX_TAPS];  // the weights in fixed point
+  int we[SEP_MAX_TAPSETS];             // their exponent
+  int fixed[SEP_SOURCES];              // source of blockIdx.y: fixed-point form
   int nsrc;
   int src[SEP_SOURCES];    // source of blockIdx.y
   int first[SEP_SOURCES];  // its variants are v[first .. first + count)
@@ -86,24 +99,68 @@ __device__ __forceinline__ double sep_value(const XArgs& A, int src, int x, int 
 }
 
 // Along x.  A CTA stages `rows` rows of one source with ghosts, then applies
-// every tap list of that source.
+// every tap list of that source: in FP64, or with the values turned into
+// integers in place (each word by the thread that wrote it) and the sums on the
+// integer pipe (fixed.cuh), one rounding each.  A CTA with a non-finite value
+// or outside the exponents the scales can hold stays in FP64.
+// Fixed point pays from about three products a fine cell on (the conversion is
+// some 40 integer instructions a cell): four steps of 250^3, ratio 5, Gaussian 30.5
+// -> 27.0 ms, 240^3, ratio 3, Gaussian 38.2 -> 36.6; without one (5 and 3 taps)
+// 22.9 / 23.3 and 31.2 / 31.6, which stay in FP64.
 __global__ void __launch_bounds__(SEP_THREADS) sep_x_kernel(const __grid_constant__ XArgs A) {
   extern __shared__ double row[];
+  __shared__ unsigned wmax[SEP_THREADS / 32];
   const int n = A.n, m = A.m, c = A.c, pitch = n + 2 * A.pad;
   const int src = A.src[blockIdx.y];
   const int nn = n * n;
   const int r0 = blockIdx.x * A.rows;
   const int rows = min(A.rows, nn - r0);
+  unsigned top = 0;  // largest high word of a magnitude
   for (int t = threadIdx.x; t < rows * pitch; t += SEP_THREADS) {
     const int r = t / pitch;
     const int z = (r0 + r) / n, y = r0 + r - z * n;
     int x = t - r * pitch - A.pad;
     while (x < 0) x += n;
     while (x >= n) x -= n;
-    row[t] = sep_value(A, src, x, y, z);
+    const double q = sep_value(A, src, x, y, z);
+    row[t] = q;
+    top = max(top, (unsigned)__double2hiint(q) & 0x7fffffffu);
+  }
+  const int v0 = A.first[blockIdx.y], vn = A.count[blockIdx.y];
+  if (A.fixed[blockIdx.y]) {
+    for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = top;
+    __syncthreads();
+    for (int w = 0; w < SEP_THREADS / 32; ++w) top = max(top, wmax[w]);
+    const int E = (int)(top >> 20) - 1022;  // |value| < 2^E
+    if (E > -800 && E < 800) {
+      int2* const xi = reinterpret_cast<int2*>(row);
+      const int kexp = (SX_BITS - E) << 20;
+      for (int t = threadIdx.x; t < rows * pitch; t += SEP_THREADS) {
+        const Fx q = fx_from_double<SX_BITS, SX_LOW>(row[t], kexp);
+        xi[t] = make_int2(q.h, q.l);
+      }
+      __syncthreads();
+      for (int q = threadIdx.x; q < rows * m; q += SEP_THREADS) {
+        const int r = q / m, ix = q - r * m;
+        const int2* f = xi + r * pitch + A.pad + c * ix;
+        for (int v = v0; v < v0 + vn; ++v) {
+          const int ts = A.v[v].taps;
+          const Taps1D& T = A.taps[ts];
+          FxSum acc{0, 0, 0};
+#pragma unroll 4
+          for (int t = 0; t < T.cnt; ++t) {
+            const int2 w = A.wx[ts][t], x = f[T.off[t]];
+            fx_mac(acc, Fx{w.x, w.y}, Fx{x.x, x.y});
+          }
+          const int e = E + A.we[ts] - 2 * SX_BITS + 2 * SX_LOW;
+          A.v[v].out[(long long)(r0 + r) * m + ix] = fx_to_double<SX_LOW>(acc, __hiloint2double((e + 1023) << 20, 0));
+        }
+      }
+      return;
+    }
   }
   __syncthreads();
-  const int v0 = A.first[blockIdx.y], vn = A.count[blockIdx.y];
   for (int q = threadIdx.x; q < rows * m; q += SEP_THREADS) {
     const int r = q / m, ix = q - r * m;
     const double* f = row + r * pitch + A.pad + c * ix;
@@ -256,10 +313,23 @@ int sep_filter(SepWork* w, int n, int c, double inv_h, double visc, const SepTap
   YArgs Y{};
   ZArgs Z{};
   int pad = 0;
+  bool ok[SEP_MAX_TAPSETS];
   for (size_t i = 0; i < taps.list.size(); ++i) {
     X.taps[i] = Y.taps[i] = taps.list[i];
     for (int k = 0; k < Y.taps[i].cnt; ++k) Y.taps[i].off[k] = ((Y.taps[i].off[k] % n) + n) % n;
     Z.taps[i] = Y.taps[i];
+    // |w| < 2^we; weights outside the range of the scales stay in FP64
+    double top = 0.0;
+    for (int k = 0; k < X.taps[i].cnt; ++k) top = std::max(top, std::fabs(X.taps[i].w[k]));
+    int e = 0;
+    if (top > 0.0 && std::isfinite(top)) std::frexp(top, &e);
+    X.we[i] = e;
+    ok[i] = std::isfinite(top) && e > -200 && e < 200;
+    for (int k = 0; ok[i] && k < X.taps[i].cnt; ++k) {
+      const long long W = std::llrint(std::ldexp(X.taps[i].w[k], SX_BITS - e));
+      const long long h = (W + (1LL << (SX_LOW - 1))) >> SX_LOW;
+      X.wx[i][k] = make_int2((int)h, (int)(W - h * (1LL << SX_LOW)));
+    }
   }
   X.u = u;
   X.p = p;
@@ -271,7 +341,8 @@ int sep_filter(SepWork* w, int n, int c, double inv_h, double visc, const SepTap
   std::vector<int> slot(xv.size());
   int used = 0;
   for (int s = 0; s < SEP_SOURCES; ++s) {
-    int cnt = 0;
+    int cnt = 0, products = 0;
+    bool fits = true;
     for (size_t i = 0; i < xv.size(); ++i)
       if (xv[i].src == s) {
         const Taps1D& T = taps.list[xv[i].t];
@@ -280,11 +351,14 @@ int sep_filter(SepWork* w, int n, int c, double inv_h, double visc, const SepTap
           if (-T.off[k] > pad) pad = -T.off[k];
           if (T.off[k] - (c - 1) > pad) pad = T.off[k] - (c - 1);
         }
+        products += T.cnt;
+        fits = fits && ok[xv[i].t];
         slot[i] = used + cnt;
         X.v[used + cnt] = {xv[i].t, w->a + (size_t)(used + cnt) * xw};
         ++cnt;
       }
     if (!cnt) continue;
+    X.fixed[X.nsrc] = fits && products > 3 * c;
     X.src[X.nsrc] = s;
     X.first[X.nsrc] = used;
     X.count[X.nsrc] = cnt;

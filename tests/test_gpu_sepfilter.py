@@ -63,3 +63,22 @@ def test_paper_step_with_gaussian(NS, filter, n, c):
     for key in ns.PAPER_NAMES:
         assert rel(d.get(key), les[key]) < 1e-12, key
     d.close()
+
+
+def test_step_of_a_field_with_still_rows(NS):
+    """Rows of zeros, which the x pass keeps in FP64, beside moving ones in fixed
+    point."""
+    n, c, l, visc, cfl = 50, 5, 1.0, 1e-3, 0.4
+    fdelta = ns.gaussian(l / n, 2 * l * c / n, 2)
+    u = ns.randomfield(n, l, -5 / 3, 5, 1.0, profile="power")
+    u[:, n // 2 :] = 0.0
+    d = NS.DnsAid(n, l, visc, c, fdelta)
+    d.set_velocity(u)
+    d.start()
+    les = ns.dnsaid_start(u, l, c, fdelta)
+    d.step(1.0, cfl, max_steps=1)
+    u, les, _, _ = ns.dnsaid_project_steps(u, les, visc, l, c, 1.0, cfl, fdelta, max_steps=1)
+    for key in ns.DNSAID_NAMES:
+        assert rel(d.get(key), les[key]) < 1e-12, key
+    assert rel(d.get("u_les"), ns.apply_DHpi(u, c, l, fdelta)) < 1e-12
+    d.close()

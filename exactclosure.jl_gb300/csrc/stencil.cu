@@ -17,63 +17,80 @@ __device__ __forceinline__ void cell_of(long long g, int n, int& x, int& y, int&
   y = (int)(r - (long long)z * n);
 }
 
-// The 6 stress components materialised (src/N.jl:94-118).
+// Steps to the neighbours of a cell along each axis, periodic.
+struct Neighbours {
+  long long up[3], dn[3];
+  __device__ __forceinline__ Neighbours(int n, int x, int y, int z) {
+    const long long s[3] = {1, n, (long long)n * n};
+    const int c[3] = {x, y, z};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      up[d] = c[d] + 1 == n ? (1 - n) * s[d] : s[d];
+      dn[d] = c[d] == 0 ? (n - 1) * s[d] : -s[d];
+    }
+  }
+};
+
+// a / h with rh = 1 / h rounded: quotient estimate, its exact remainder, one
+// correction, which rounds like the division (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34(1), 1990) in three FP64 operations; estimates near the ends of the
+// exponent range, zero and non-finite ones divide.
+__device__ __forceinline__ float div_by(float a, float h, float) { return a / h; }
+__device__ __forceinline__ double div_by(double a, double h, double rh) {
+  const double q = a * rh;
+  const unsigned e = ((unsigned)__double2hiint(q) >> 20) & 0x7ffu;
+  if (e - 100u >= 1800u) return a / h;
+  return fma(fma(-q, h, a), rh, q);
+}
+
+// The 6 stress components materialised (src/N.jl:94-118).  Bound by the FP64
+// divisions by h and index arithmetic: with div_by and the neighbour steps 41.1
+// -> 34.9 us at 50^3, 3.30 -> 2.14 ms at 250^3, the same bits.
 template <typename T>
 __global__ void stress_kernel(int n, T h, T visc, const T* __restrict__ u, T* __restrict__ s6) {
   chain_wait();
   const long long N = (long long)n * n * n;
+  const T rh = (T)1 / h;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
     cell_of(g, n, x, y, z);
-    int c[3] = {x, y, z};
+    const Neighbours nb(n, x, y, z);
     const int comps[6][2] = {{0, 0}, {1, 1}, {2, 2}, {0, 1}, {1, 2}, {2, 0}};
 #pragma unroll
     for (int m = 0; m < 6; ++m) {
-      int i = comps[m][0], j = comps[m][1];
-      auto idx = [&](int d, int s) {
-        int cc[3] = {c[0], c[1], c[2]};
-        cc[d] = (cc[d] + s + n) % n;
-        return ((long long)cc[2] * n + cc[1]) * n + cc[0];
-      };
-      int off = (i != j);
-      T uir = u[i * N + idx(j, off)], uil = u[i * N + idx(j, off - 1)];
-      T ujr = u[j * N + idx(i, off)], ujl = u[j * N + idx(i, off - 1)];
-      T etaj_ui = (uir + uil) / 2, etai_uj = (ujr + ujl) / 2;
-      T dj_ui = (uir - uil) / h, di_uj = (ujr - ujl) / h;
+      const int i = comps[m][0], j = comps[m][1];
+      const T* const ui = u + i * N + g;
+      const T* const uj = u + j * N + g;
+      const T uir = i == j ? ui[0] : ui[nb.up[j]], uil = i == j ? ui[nb.dn[j]] : ui[0];
+      const T ujr = i == j ? uir : uj[nb.up[i]], ujl = i == j ? uil : uj[0];
+      const T etaj_ui = (uir + uil) / 2, etai_uj = (ujr + ujl) / 2;
+      const T dj_ui = div_by(uir - uil, h, rh), di_uj = i == j ? dj_ui : div_by(ujr - ujl, h, rh);
       s6[m * N + g] = etaj_ui * etai_uj - visc * (dj_ui + di_uj);
     }
   }
 }
 
-// du_i = doadd*du_i - sum_j delta_j s_ij with an explicit tensor (src/N.jl:120-200).
+// du_i = doadd*du_i - sum_j delta_j s_ij with an explicit tensor (src/N.jl:120-200);
+// at 50^3 28.7 -> 21.3 us, at 250^3 2.48 -> 1.42 ms (div_by, neighbour steps).
 template <typename T>
 __global__ void tensordiv_kernel(int n, T h, int nsym, const T* __restrict__ s, T* __restrict__ du, int doadd) {
   chain_wait();
   const long long N = (long long)n * n * n;
+  const T rh = (T)1 / h;
+  const int sym[3][3] = {{0, 3, 5}, {3, 1, 4}, {5, 4, 2}};
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < N; g += (long long)gridDim.x * blockDim.x) {
     int x, y, z;
     cell_of(g, n, x, y, z);
-    int c[3] = {x, y, z};
-    auto nb = [&](int d, int sgn) {
-      int cc[3] = {c[0], c[1], c[2]};
-      cc[d] = (cc[d] + sgn + n) % n;
-      return ((long long)cc[2] * n + cc[1]) * n + cc[0];
-    };
+    const Neighbours nb(n, x, y, z);
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
       T acc = doadd ? du[i * N + g] : (T)0;
+#pragma unroll
       for (int j = 0; j < 3; ++j) {
-        int m;
-        if (nsym == 9) m = 3 * j + i;  // s11,s21,s31,s12,... (src/N.jl:181)
-        else {
-          if (i == j) m = i;
-          else {
-            int a = i < j ? i : j, b = i < j ? j : i;
-            m = (a == 0 && b == 1) ? 3 : (a == 1 && b == 2) ? 4 : 5;
-          }
-        }
-        const T* sc = s + (long long)m * N;
-        if (i == j) acc -= (sc[nb(j, 1)] - sc[g]) / h;
-        else acc -= (sc[g] - sc[nb(j, -1)]) / h;
+        const int m = nsym == 9 ? 3 * j + i : sym[i][j];  // s11,s21,s31,s12,... (src/N.jl:181)
+        const T* const sc = s + (long long)m * N + g;
+        acc -= div_by(i == j ? sc[nb.up[j]] - sc[0] : sc[0] - sc[nb.dn[j]], h, rh);
       }
       du[i * N + g] = acc;
     }

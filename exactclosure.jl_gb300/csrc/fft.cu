@@ -567,7 +567,9 @@ static bool mix_wanted(int n) {
   return fftmix_supported(n) || (n >= GEN_MIX_MIN && !fftreg_supported(n, EXC_F32) && gen_supported(n, EXC_F32));
 }
 static long long mix_part_words(int n) {
-  return fftmix_supported(n) ? fftmix_part_words(n) : std::max(gen_mix_parts(n), (long long)MIX_SUM_CTAS) + 2;
+  // run-time plans: the partial sums, the mean, an exponent per CTA and the shift
+  return fftmix_supported(n) ? fftmix_part_words(n)
+                             : std::max(gen_mix_parts(n), (long long)MIX_SUM_CTAS) + 2 + gen_mix_parts(n) / 2 + 1;
 }
 
 int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bool run_time_plans, int slots) {

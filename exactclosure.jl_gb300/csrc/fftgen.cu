@@ -122,10 +122,13 @@ long long gen_mix_parts(int n) {
 }
 
 cudaError_t gen_mix_solve(exc_poisson* ps, const double* src, bool vec, cudaStream_t st) {
-  const GenArgs<float> a = gen_args<float>(ps->mix, st, SlotBatch(), 1);
+  GenArgs<float> a = gen_args<float>(ps->mix, st, SlotBatch(), 1);
   const long long N = (long long)ps->n * ps->n * ps->n, parts = gen_mix_parts(ps->n);
   float *const q1 = ps->mix_q, *const q2 = ps->mix_q2;
   double* const mean = ps->mix_part + std::max(parts, (long long)MIX_SUM_CTAS);
+  GenRange range;
+  range.top = reinterpret_cast<int*>(mean + 1);
+  range.n = (int)parts;
   auto columns = [&] {
     gen_cols<float, false>(a);
     gen_zsolve<float>(a);
@@ -139,12 +142,17 @@ cudaError_t gen_mix_solve(exc_poisson* ps, const double* src, bool vec, cudaStre
   s.part = ps->mix_part;
   s.mode = vec ? GEN_MIX_DIV : GEN_MIX_SCAL;
   if (!vec) launch_mix_mean_of(src, N, ps->mix_part, st);
+  s.range = a.range = range;
   gen_r2c<float>(a, s);
   columns();
+  a.range = GenRange();
   GenDst d{};
   d.mode = GEN_MIX_Q;
   d.q = q1;
+  d.range = range;
+  d.first = 1;
   gen_c2r<float>(a, d);
+  d.first = 0;
   s.mode = GEN_MIX_RES;
   s.q = q1;
   s.store = 1;

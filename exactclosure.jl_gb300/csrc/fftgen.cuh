@@ -73,11 +73,38 @@ __host__ __device__ __forceinline__ int gen_xs(const GenLine& l) { return l.n1 *
 // Column passes: a tile is W = 2^wlog consecutive kx columns of one outer
 // index; blockIdx.x = outer * ntx + tile column, blockIdx.z = slot.
 // ---------------------------------------------------------------------------
+// Range of the mixed-precision solve.  Its transforms are FP32, its input FP64:
+// the first x pass leaves the largest biased exponent of its right-hand side per
+// CTA, the first y pass folds them into a shift, 0 for right-hand sides between
+// 2^-60 and 2^80 (every correction then stays within the floats).  With another
+// shift the first solve's correction is dropped (its input may not have fitted)
+// and the two that follow work on residuals scaled by 2^-shift.
+struct GenRange {
+  int* top = nullptr;    // the CTAs' exponents, then the shift
+  int n = 0;             // CTAs
+  __device__ __forceinline__ int shift() const { return top ? top[n] : 0; }
+};
+__device__ __forceinline__ double gen_pow2(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+__device__ __forceinline__ void gen_fold_range(const GenRange& rg) {
+  __shared__ int most;
+  if (threadIdx.x == 0) most = 0;
+  __syncthreads();
+  int m = 0;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < rg.n; i += GEN_THREADS) m = max(m, rg.top[i]);
+  atomicMax(&most, m);
+  __syncthreads();
+  // a zero or non-finite right-hand side goes through as it is
+  if (threadIdx.x == 0)
+    rg.top[rg.n] = most == 0 || most == 0x7ff || (most >= 1023 - 60 && most <= 1023 + 80) ? 0 : max(most - 1023, -1000);
+}
+
 template <typename T, bool INV>
 __global__ void __launch_bounds__(GEN_THREADS, 2)
 gcols_kernel(cplx<T>* __restrict__ g, GenLine ln, int nkx, int ntx, int wlog, long long es, long long outer_stride,
-             const cplx<T>* __restrict__ tl, SlotBatch sb) {
+             const cplx<T>* __restrict__ tl, SlotBatch sb, GenRange rg) {
   chain_wait();
+  if (!INV && sizeof(T) == 4 && rg.top && blockIdx.x == 0) gen_fold_range(rg);
   using C = cplx<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* const xs = reinterpret_cast<C*>(smem_raw);
@@ -251,6 +278,7 @@ struct GenSrc {
   const float *q, *qp;
   double* part;
   int store, mean;
+  GenRange range;
 };
 
 // Where the inverse x pass puts the reals: in place at pitch 2P, or
@@ -262,6 +290,8 @@ struct GenDst {
   double* p;               // GEN_MIX_FIN: ((q1 + q2) - mean) + c at pitch 2P
   const double* mean;      // null: no mean to remove
   const float *q1, *q2;
+  GenRange range;
+  int first;               // GEN_MIX_Q of the first solve
 };
 
 template <typename T>
@@ -317,6 +347,11 @@ gr2c_kernel(GenSrc<T> s, GenLine ln, int n, int rw, cplx<T>* __restrict__ out, i
   auto c_at = [](const T* f, int off, int m) { return reinterpret_cast<const C*>(f + off)[m]; };
   auto f_at = [](const float* f, int off, int m) { return reinterpret_cast<const float2*>(f + off)[m]; };
   auto d_at = [](const double* f, int off, int m) { return reinterpret_cast<const double2*>(f + off)[m]; };
+  // the largest biased exponent of the right-hand side (first pass)
+  int top = 0;
+  auto seen = [&](double2 v) {
+    top = max(top, max((__double2hiint(v.x) >> 20) & 0x7ff, (__double2hiint(v.y) >> 20) & 0x7ff));
+  };
   auto put_d = [&](const Pos& p, double2 v) { reinterpret_cast<double2*>(s.d + p.base)[p.m] = v; };
   if (s.mode == GEN_SCAL) {
     sweep([&](const Pos& p) { return c_at(src, p.base, p.m); }, [](const Pos&, const C& v) { return v; });
@@ -344,6 +379,7 @@ gr2c_kernel(GenSrc<T> s, GenLine ln, int n, int rw, cplx<T>* __restrict__ out, i
         dv.x = (w.a.x - w.l) + (w.b0.x - w.b1.x) + (w.c0.x - w.c1.x);
         dv.y = (w.a.y - w.a.x) + (w.b0.y - w.b1.y) + (w.c0.y - w.c1.y);
         put_d(p, dv);
+        seen(dv);
         return to_f32c<C>(dv.x, dv.y);
       });
     } else if (s.mode == GEN_MIX_SCAL) {
@@ -352,31 +388,53 @@ gr2c_kernel(GenSrc<T> s, GenLine ln, int n, int rw, cplx<T>* __restrict__ out, i
         dv.x = (dv.x - dm) * s.h;
         dv.y = (dv.y - dm) * s.h;
         put_d(p, dv);
+        seen(dv);
         return to_f32c<C>(dv.x, dv.y);
       });
     } else {
+      // with a shift the corrections are in units of 2^shift
+      const int shift = s.range.shift();
       struct W { float2 qc, a, b, c, e, pa; float qxm, qxp; double2 dv; };
-      sweep([&](const Pos& p) {
-        W w{f_at(s.q, p.base, p.m), f_at(s.q, p.by, p.m), f_at(s.q, p.uy, p.m), f_at(s.q, p.bz, p.m), f_at(s.q, p.uz, p.m),
-            make_float2(0.0f, 0.0f), s.q[p.xl], s.q[p.xr], d_at(s.d, p.base, p.m)};
-        if (s.mean) w.pa = f_at(s.qp, p.base, p.m);
-        return w;
-      }, [&](const Pos& p, const W& w) {
-        double2 dv;
-        dv.x = fma(-s.inv_h64, stencil7_f32(w.qxm, w.qc.y, w.a.x, w.b.x, w.c.x, w.e.x, w.qc.x), w.dv.x);
-        dv.y = fma(-s.inv_h64, stencil7_f32(w.qc.x, w.qxp, w.a.y, w.b.y, w.c.y, w.e.y, w.qc.y), w.dv.y);
-        if (s.store) put_d(p, dv);
-        if (s.mean) {
-          psum.add(w.pa.x);
-          psum.add(w.qc.x);
-          psum.add(w.pa.y);
-          psum.add(w.qc.y);
-        }
-        return to_f32c<C>(dv.x, dv.y);
-      });
+      auto residual = [&](auto shifted) {
+        const double ih = shifted ? s.inv_h64 * gen_pow2(shift) : s.inv_h64, down = shifted ? gen_pow2(-shift) : 1.0;
+        sweep([&](const Pos& p) {
+          W w{f_at(s.q, p.base, p.m), f_at(s.q, p.by, p.m), f_at(s.q, p.uy, p.m), f_at(s.q, p.bz, p.m), f_at(s.q, p.uz, p.m),
+              make_float2(0.0f, 0.0f), s.q[p.xl], s.q[p.xr], d_at(s.d, p.base, p.m)};
+          if (s.mean) w.pa = f_at(s.qp, p.base, p.m);
+          return w;
+        }, [&](const Pos& p, const W& w) {
+          double2 dv;
+          dv.x = fma(-ih, stencil7_f32(w.qxm, w.qc.y, w.a.x, w.b.x, w.c.x, w.e.x, w.qc.x), w.dv.x);
+          dv.y = fma(-ih, stencil7_f32(w.qc.x, w.qxp, w.a.y, w.b.y, w.c.y, w.e.y, w.qc.y), w.dv.y);
+          if (s.store) put_d(p, dv);
+          if (s.mean) {
+            psum.add(w.pa.x);
+            psum.add(w.qc.x);
+            psum.add(w.pa.y);
+            psum.add(w.qc.y);
+          }
+          if (shifted) {
+            dv.x *= down;
+            dv.y *= down;
+          }
+          return to_f32c<C>(dv.x, dv.y);
+        });
+      };
+      if (shift) residual(std::true_type());
+      else residual(std::false_type());
     }
   }
+  __shared__ int most[GEN_THREADS / 32];
+  const bool first = sizeof(T) == 4 && (s.mode == GEN_MIX_DIV || s.mode == GEN_MIX_SCAL);
+  if (first) {
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((threadIdx.x & 31) == 0) most[threadIdx.x >> 5] = top;
+  }
   __syncthreads();
+  if (first && threadIdx.x == 0) {
+    for (int w = 1; w < GEN_THREADS / 32; ++w) top = max(top, most[w]);
+    s.range.top[blockIdx.x] = top;
+  }
   gen_rows_fft<T, false>(xs, ln, rows, tl);
   // Z_k is at row k mod n1, word k / n1
   auto at = [&](const C* x, int k) {
@@ -449,40 +507,50 @@ gc2r_kernel(cplx<T>* g, GenLine ln, int n, int rw, int P, const cplx<T>* __restr
       g[(long long)row * P + m] = v;
     }
   } else if constexpr (sizeof(T) == 4) {
+    const int shift = d.range.shift();
     if (d.mode == GEN_MIX_Q) {
+      const bool drop = d.first && shift;
       for (int t = threadIdx.x; t < total; t += GEN_THREADS) {
         int m, row;
         const C v = word(t, m, row);
-        reinterpret_cast<float2*>(d.q + row * n)[m] = make_float2(f32_flush(v.x), f32_flush(v.y));
+        reinterpret_cast<float2*>(d.q + row * n)[m] = drop ? make_float2(0.0f, 0.0f) : make_float2(f32_flush(v.x), f32_flush(v.y));
       }
     } else {
       const bool rm = d.mean != nullptr;
       const double mu = rm ? *d.mean : 0.0;
-      for (int t0 = threadIdx.x; t0 < total; t0 += U * GEN_THREADS) {
-        float2 b1[U], b2[U];
-        C v[U];
-        int m[U], row[U];
+      auto sum = [&](auto shifted) {
+        for (int t0 = threadIdx.x; t0 < total; t0 += U * GEN_THREADS) {
+          float2 b1[U], b2[U];
+          C v[U];
+          int m[U], row[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          v[u] = word(min(t0 + u * GEN_THREADS, total - 1), m[u], row[u]);
-          b1[u] = reinterpret_cast<const float2*>(d.q1 + row[u] * n)[m[u]];
-          b2[u] = reinterpret_cast<const float2*>(d.q2 + row[u] * n)[m[u]];
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (t0 + u * GEN_THREADS >= total) continue;
-          double2 o;
-          o.x = f32_to_f64(b1[u].x) + f32_to_f64(b2[u].x);
-          o.y = f32_to_f64(b1[u].y) + f32_to_f64(b2[u].y);
-          if (rm) {
-            o.x -= mu;
-            o.y -= mu;
+          for (int u = 0; u < U; ++u) {
+            v[u] = word(min(t0 + u * GEN_THREADS, total - 1), m[u], row[u]);
+            b1[u] = reinterpret_cast<const float2*>(d.q1 + row[u] * n)[m[u]];
+            b2[u] = reinterpret_cast<const float2*>(d.q2 + row[u] * n)[m[u]];
           }
-          o.x += f32_to_f64(v[u].x);
-          o.y += f32_to_f64(v[u].y);
-          reinterpret_cast<double2*>(d.p + row[u] * 2LL * P)[m[u]] = o;
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            if (t0 + u * GEN_THREADS >= total) continue;
+            double2 o;
+            o.x = f32_to_f64(b1[u].x) + f32_to_f64(b2[u].x);
+            o.y = f32_to_f64(b1[u].y) + f32_to_f64(b2[u].y);
+            if (rm) {
+              o.x -= mu;
+              o.y -= mu;
+            }
+            o.x += f32_to_f64(v[u].x);
+            o.y += f32_to_f64(v[u].y);
+            if (shifted) {
+              o.x *= gen_pow2(shift);
+              o.y *= gen_pow2(shift);
+            }
+            reinterpret_cast<double2*>(d.p + row[u] * 2LL * P)[m[u]] = o;
+          }
         }
-      }
+      };
+      if (shift) sum(std::true_type());
+      else sum(std::false_type());
     }
   }
 }
@@ -508,6 +576,7 @@ struct GenArgs {  // what every pass of one solve shares
   int wlog, rw, nslots;
   SlotBatch sb;
   cudaStream_t st;
+  GenRange range;  // of a mixed solve's first y pass
 };
 // One pass each: y (INV: inverse), z with the divide, x forward, x inverse.
 template <typename T, bool INV>

@@ -82,3 +82,26 @@ def test_served_batch_equals_the_case(NS, built_lib, precision):
         assert (cs.velocity() == got[i]).all()
         cs.close()
     sv.close()
+
+
+@pytest.mark.parametrize("e", [-900, -300, -130, -70, -40, 60, 100, 140, 400])
+def test_mixed_solve_beyond_the_floats(NS, e):
+    """A solve is linear: inputs scaled by 2^e, far outside FP32's exponents too,
+    give the scaled results to 1e-12."""
+    import torch
+
+    n = 84
+    gen = torch.Generator("cuda").manual_seed(3)
+    u = torch.randn((3, n, n, n), generator=gen, dtype=torch.float64, device="cuda")
+    d = torch.randn((n, n, n), generator=gen, dtype=torch.float64, device="cuda")
+    d -= d.mean()
+    ps = NS.poissonsolver(NS.Grid(1.0, n), 0)
+    out = []
+    for k in (0, e):
+        a, p, q = u * 2.0**k, torch.empty_like(d), torch.empty_like(d)
+        ps.project(a, p)
+        ps.solve(q, d * 2.0**k)
+        out.append([x * 2.0**-k for x in (a, p, q)])
+    for x, y in zip(*out):
+        assert float((x - y).norm() / x.norm()) < 1e-12
+    ps.close()

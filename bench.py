@@ -870,10 +870,11 @@ def dgemm_peak(reps=5, size=8192):
 def roofline(cs, NS, n, prec, args, stream):
     """The dominant kernel of the step, the RHS sweep (stresstensor +
     tensordivergence), timed alone with CUDA events on its own stream, on the
-    case's device velocity.  In FP64 it is bound by the FP64 pipe: achieved
-    = algorithmic FP64 operations per launch / launch time, against the DGEMM
-    rate measured in the same run; its HBM figures sit beside.  In FP32 it
-    is bound by HBM: achieved = algorithmic bytes / launch time."""
+    case's device velocity: achieved = algorithmic bytes / launch time against
+    the measured copy.  The FP32 sweep is bound by HBM.  The FP64 sweep works in
+    fixed point and is bound by the integer pipe; `fp64` gives the reference's
+    FP64 operations per launch / launch time beside the DGEMM rate measured in
+    the same run (above 1: the operations do not run on the FP64 pipe)."""
     import torch
 
     hbm, src = peaks()
@@ -913,16 +914,16 @@ def roofline(cs, NS, n, prec, args, stream):
             traffic = d[key]
     hbm_part = {"achieved": gbs, "peak": hbm, "peak_source": src, "unit": "GB/s", "frac": gbs / hbm,
                 "algorithmic_bytes_per_launch": alg_bytes}
-    common = {"kernel": "rhs_kernel (stress + divergence sweep)", "ms_per_launch": ms, "traffic": traffic,
+    common = {"kernel": "stress + divergence sweep (rhs_fixed_kernel in FP64, rhs_quad_kernel in FP32)", "ms_per_launch": ms, "traffic": traffic,
               "traffic_note": "dram__bytes_read.sum + dram__bytes_write.sum of one launch at this size (ncu), "
                               "bytes per launch"}
     if prec == 0:
         dgemm, dclk, dsrc = dgemm_peak()
         ach = flops / (ms / 1e3) / 1e12
-        return {**common, "bound": "fp64", "achieved": ach, "peak": dgemm, "peak_source": dsrc,
-                "peak_clocks": dclk, "unit": "TFLOP/s", "frac": ach / dgemm,
-                "algorithmic_flops_per_launch": flops, "flops_per_cell": RHS_FLOPS_PER_CELL,
-                "hbm": hbm_part}
+        return {**common, "bound": "integer pipe", **hbm_part,
+                "fp64": {"achieved_tflops": ach, "dgemm_tflops": dgemm, "dgemm_source": dsrc, "dgemm_clocks": dclk,
+                         "ratio": ach / dgemm, "algorithmic_flops_per_launch": flops,
+                         "flops_per_cell": RHS_FLOPS_PER_CELL}}
     return {**common, "bound": "hbm", **hbm_part,
             "fp32": {"achieved_tflops": flops / (ms / 1e3) / 1e12, "flops_per_cell": RHS_FLOPS_PER_CELL}}
 

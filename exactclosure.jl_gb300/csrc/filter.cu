@@ -2,6 +2,7 @@
 // separable filter-and-sample operator of `lazycoarsegrain(lazyfilter(.))`
 // materialised on the LES grid, for velocities (volume or face average) and
 // for the closure fluxes r = sigma(u) + p I evaluated on the fly.
+#include <type_traits>
 #include <vector>
 
 #include "internal.cuh"
@@ -293,8 +294,49 @@ int filtered_stress(int n, int c, double l, double visc, const double* fdelta, i
 // point sample) and the transverse weight 1/c^2.  Both stages sum in a fixed
 // order, so the result is bit-reproducible.
 // ---------------------------------------------------------------------------
-template <typename T>
-__global__ void tb_kernel(const T* __restrict__ f3, int n, int c, T* __restrict__ tb3) {
+// Sum of K doubles on the integer pipe (an FP64 addition holds the FP64 pipe of
+// an SM for 16 cycles a warp): each value as a 53 + UP bit integer below the
+// largest one's exponent, the sum exact in 64 bits, rounded once.  Values near
+// the ends of the exponent range and non-finite ones are added in order.
+template <int K>
+__device__ __forceinline__ double sum_fixed(const double (&v)[K]) {
+  static_assert(K <= 32, "the sum of K integers below 2^(53 + UP) fits");
+  constexpr int UP = 5;
+  unsigned top = 0;
+#pragma unroll
+  for (int i = 0; i < K; ++i) top = max(top, (unsigned)__double2hiint(v[i]) & 0x7ff00000u);
+  if (top - (80u << 20) >= (1900u << 20)) {
+    double acc = 0.0;
+#pragma unroll
+    for (int i = 0; i < K; ++i) acc += v[i];
+    return acc;
+  }
+  const int e = (int)(top >> 20);
+  long long sum = 0;
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    const unsigned hi = (unsigned)__double2hiint(v[i]), lo = (unsigned)__double2loint(v[i]);
+    const unsigned mh = (hi & 0xfffffu) | 0x100000u;
+    const unsigned long long m = ((unsigned long long)__funnelshift_l(lo, mh, UP) << 32) | (lo << UP);
+    unsigned long long t;
+    asm("shr.u64 %0, %1, %2;" : "=l"(t) : "l"(m), "r"(e - (int)((hi >> 20) & 0x7ffu)));
+    const long long s = (int)hi >> 31;  // 0 or -1
+    sum += ((long long)t ^ s) - s;
+  }
+  // the unit: 2^(e - 1023 - 52 - UP)
+  return (double)sum * __hiloint2double((e - 52 - UP) << 20, 0);
+}
+
+// C = 0: any ratio.  With the ratio known the c x c loads of a sum are all in
+// flight (and pairs of words where C is even), which the loops of a run-time
+// ratio are not; the order of the sums is the same.
+// Per pass over the fine field: FP64 512^3 ratio 4 0.80 -> 0.49 ms (HBM; the FP64
+// additions alone took 0.69), 128^3 19.5 -> 13.2 us, 90^3 ratios 3 and 5 10.6 and
+// 10.9 -> 7.4; FP32 128^3 ratio 4 10.8 -> 8.0, 72^3 ratio 3 6.9 -> 4.6.  Four values
+// (ratio 2) stay on the FP64 pipe.
+template <typename T, int C>
+__global__ void tb_kernel(const T* __restrict__ f3, int n, int ratio, T* __restrict__ tb3) {
+  const int c = C ? C : ratio;
   const int comp = blockIdx.y;
   const int m = n / c;
   const long long N = (long long)n * n * n;
@@ -302,29 +344,59 @@ __global__ void tb_kernel(const T* __restrict__ f3, int n, int c, T* __restrict_
   const T* __restrict__ f = f3 + comp * N;
   T* __restrict__ tb = tb3 + comp * Mt;
   const IdxDiv dn(n), dm(m);
+  // sum of c rows `step` apart of c words each (`along` apart)
+  auto rows = [&](const T* p, long long step, auto along_x, long long along) {
+    if constexpr (C == 0) {
+      T acc = (T)0;
+      for (int a = 0; a < c; ++a)
+        for (int b = 0; b < c; ++b) acc += p[a * step + b * along];
+      return acc;
+    } else {
+      T w[C * C];
+      using V2 = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
+#pragma unroll
+      for (int a = 0; a < C; ++a) {
+        if constexpr (decltype(along_x)::value && C % 2 == 0) {
+#pragma unroll
+          for (int b = 0; b < C; b += 2) {
+            const V2 q = *reinterpret_cast<const V2*>(p + a * step + b);
+            w[a * C + b] = q.x;
+            w[a * C + b + 1] = q.y;
+          }
+        } else {
+#pragma unroll
+          for (int b = 0; b < C; ++b) w[a * C + b] = p[a * step + b * along];
+        }
+      }
+      if constexpr (sizeof(T) == 8 && C > 2) {
+        return sum_fixed(w);
+      } else {
+        T acc = (T)0;
+#pragma unroll
+        for (int i = 0; i < C * C; ++i) acc += w[i];
+        return acc;
+      }
+    }
+  };
+  using Yes = std::true_type;
+  using No = std::false_type;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < Mt; g += (long long)gridDim.x * blockDim.x) {
-    T acc = (T)0;
+    T acc;
     if (comp == 0) {
       const long long r = dn.div(g);
       const int x = (int)(g - r * n);
       const int Jz = (int)dm.div(r), Jy = (int)(r - (long long)Jz * m);
-      const T* p = f + ((long long)(c * Jz) * n + c * Jy) * n + x;
-      for (int dz = 0; dz < c; ++dz)
-        for (int dy = 0; dy < c; ++dy) acc += p[((long long)dz * n + dy) * n];
+      acc = rows(f + ((long long)(c * Jz) * n + c * Jy) * n + x, (long long)n * n, No(), n);
     } else if (comp == 1) {
       const long long r = dm.div(g);
       const int Jx = (int)(g - r * m);
       const int Jz = (int)dn.div(r), y = (int)(r - (long long)Jz * n);
-      const T* p = f + ((long long)(c * Jz) * n + y) * n + c * Jx;
-      for (int dz = 0; dz < c; ++dz)
-        for (int dx = 0; dx < c; ++dx) acc += p[(long long)dz * n * n + dx];
+      acc = rows(f + ((long long)(c * Jz) * n + y) * n + c * Jx, (long long)n * n, Yes(), 1);
     } else {
       const long long r = dm.div(g);
       const int Jx = (int)(g - r * m);
       const int z = (int)dm.div(r), Jy = (int)(r - (long long)z * m);
-      const T* p = f + ((long long)z * n + c * Jy) * n + c * Jx;
-      for (int dy = 0; dy < c; ++dy)
-        for (int dx = 0; dx < c; ++dx) acc += p[(long long)dy * n + dx];
+      acc = rows(f + ((long long)z * n + c * Jy) * n + c * Jx, n, Yes(), 1);
     }
     tb[g] = acc;
   }
@@ -384,7 +456,13 @@ template <typename T>
 cudaError_t box_tb(int n, int c, const T* u, T* tb, cudaStream_t st) {
   const int m = n / c;
   const long long Mt = (long long)n * m * m;
-  tb_kernel<T><<<dim3(grid_for(Mt), 3), 256, 0, st>>>(u, n, c, tb);
+  const dim3 grid(grid_for(Mt), 3);
+  const bool pairs = reinterpret_cast<uintptr_t>(u) % (2 * sizeof(T)) == 0;  // n is even
+  if (c == 2 && pairs) tb_kernel<T, 2><<<grid, 256, 0, st>>>(u, n, c, tb);
+  else if (c == 3) tb_kernel<T, 3><<<grid, 256, 0, st>>>(u, n, c, tb);
+  else if (c == 4 && pairs) tb_kernel<T, 4><<<grid, 256, 0, st>>>(u, n, c, tb);
+  else if (c == 5) tb_kernel<T, 5><<<grid, 256, 0, st>>>(u, n, c, tb);
+  else tb_kernel<T, 0><<<grid, 256, 0, st>>>(u, n, c, tb);
   return cudaGetLastError();
 }
 

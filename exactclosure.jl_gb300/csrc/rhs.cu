@@ -556,25 +556,22 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     }
     parity ^= 1u << buf;
   };
-  // f(value) over this thread's pieces of plane buffer buf, after its wait (a
+  // f(piece) over this thread's pieces of plane buffer buf, after its wait (a
   // TMA plane's mbarrier wait makes every copy visible, else it copied them)
-  auto each_value = [&](int buf, auto f) {
+  auto each_piece = [&](int buf, auto f) {
 #pragma unroll
     for (int i = 0; i < NSLOT; ++i) {
       const int t = tid + i * FXTHREADS;
-      if (t < FXPIECES) {
-        double2* const p2 = reinterpret_cast<double2*>(sm.u[buf]) + t;
-        double2 v = *p2;
-        f(v.x);
-        f(v.y);
-        *p2 = v;
-      }
+      if (t < FXPIECES) f(reinterpret_cast<double2*>(sm.u[buf])[t]);
     }
   };
-  // largest magnitude of a plane (high words), this warp's part, into sm.red
+  // largest magnitude of a plane (high words), this warp's part, into sm.red;
+  // the plane itself is only read
   auto scan_plane = [&](int buf) {
     unsigned m = 0;
-    each_value(buf, [&](double& v) { m = max(m, (unsigned)__double2hiint(v) & 0x7fffffffu); });
+    each_piece(buf, [&](const double2& v) {
+      m = max(m, max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu));
+    });
     m = __reduce_max_sync(0xffffffffu, m);
     if (tx == 0) sm.red[buf][ty] = m;
   };
@@ -585,9 +582,9 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
   int kexp = 0;                  // (57 - E) << 20
   double scale = 0;              // -1/(4h) 2^58 in fixed-point units squared
   auto convert_plane = [&](int buf) {
-    each_value(buf, [&](double& v) {
-      const Fx q = fx_from_double<FX_BITS, FX_LOW>(v, kexp);
-      v = __hiloint2double(q.h, q.l);
+    each_piece(buf, [&](double2& v) {
+      const Fx q = fx_from_double<FX_BITS, FX_LOW>(v.x, kexp), r = fx_from_double<FX_BITS, FX_LOW>(v.y, kexp);
+      v = make_double2(__hiloint2double(q.h, q.l), __hiloint2double(r.h, r.l));
     });
   };
   Fx S2{}, S4{};  // 2S and 4S in fixed point
@@ -665,6 +662,14 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     cur = 1;
     nxt = 2;
     pre = 0;
+  };
+  // The planes from another one on.  sm.red and the plane buffers belong to every
+  // warp until the last one has read this plane's values and maxima, and what was
+  // written to the buffers is ordered before the copies that come next.
+  auto restart = [&](int z) {
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    __syncthreads();
+    start(z);
   };
   start(z0);
   const int gx = x0 + tx;
@@ -761,8 +766,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     }
     if (!more) break;
     if (slow) {
-      __syncthreads();
-      start(z + 1);
+      restart(z + 1);
       continue;
     }
     wait_plane(pre);
@@ -771,7 +775,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     const unsigned pm = plane_max(pre);
     const int En = exponent_for(max(pm, max(pm1, pm2)));
     if (pm >= 0x7fe00000u || En > E || En < E - 2) {
-      start(z + 1);
+      restart(z + 1);
       continue;
     }
     convert_plane(pre);

@@ -200,8 +200,10 @@ __device__ __forceinline__ bool step_of(const AdvanceArgs& A, double m, double t
 }
 
 // The DNS loop of `create_dns` (src/Burgers.jl:522-545) with `timestep!` or,
-// when RK4, `rk4_timestep!` (src/Burgers.jl:112-142).
-template <bool RK4>
+// when RK4, `rk4_timestep!` (src/Burgers.jl:112-142); with LES, `dns_aided_les`
+// (src/Burgers.jl:350-445) in FP64 throughout, for what the fixed-point loop
+// below does not take.
+template <bool LES, bool RK4>
 __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
   extern __shared__ double smem[];
   __shared__ double red[40];
@@ -209,12 +211,19 @@ __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
   const int np = padded(g);
   double* ue = smem;
   double* se = ue + np;
+  double* wd = se + np;
+  double* wl = wd + 2 * g.Rd + 1;
+  if (LES) {
+    for (int r = threadIdx.x; r < 2 * g.Rd + 1; r += blockDim.x) wd[r] = A.wd[r];
+    for (int r = threadIdx.x; r < 2 * g.Rl + 1; r += blockDim.x) wl[r] = A.wl[r];
+  }
   const int tid = threadIdx.x;
+  const size_t vs = (size_t)4 * g.nH;
   for (int s = blockIdx.x; s < g.ns; s += gridDim.x) {
     double* us = A.u + (size_t)s * g.nh;
     load_sample(g, us, ue);
     double tt = A.t[s];
-    int done = 0;
+    int done = 0, par = 0;
     __syncthreads();
     // |u| maximum of this thread's cells, kept up to date by the updates.
     double lmax = 0.0;
@@ -222,11 +231,45 @@ __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
     while (tt < A.tstop && done < A.max_steps) {
       double dt;
       if (!step_of(A, block_max(lmax, red), tt, dt)) break;
-      const double dth = dt * g.ih;
+      const double dth = dt * g.ih, dtH = dt * g.iH;
       lmax = 0.0;
       if (!RK4) {
         fill_stress(g, ue, se);
         __syncthreads();
+        if (LES) {
+          double* vc = (par ? A.v1 : A.v0) + s * vs;
+          double* vn = (par ? A.v0 : A.v1) + s * vs;
+          double* tm = A.tmp + (size_t)s * 5 * g.nH;
+          for (int I = tid; I < g.nH; I += blockDim.x) {
+            const Terms c = coarse_terms(g, I, ue, se, wd, wl);
+            tm[I] = c.fsu;
+            tm[g.nH + I] = c.vsu;
+            tm[2 * g.nH + I] = c.vu;
+            tm[3 * g.nH + I] = c.sVU;
+          }
+          __syncthreads();
+          // LES steps: stress of each LES plus its correction
+          // (src/Burgers.jl:414-430), forward Euler with the DNS time step.
+          for (int i = tid; i < g.nH; i += blockDim.x) {
+            const int im = i == 0 ? g.nH - 1 : i - 1, ip = i + 1 == g.nH ? 0 : i + 1;
+            const double vum = tm[2 * g.nH + im], vui = tm[2 * g.nH + i], vup = tm[2 * g.nH + ip];
+            const double svi = bstress(vum, vui, g.vH), svp = bstress(vui, vup, g.vH);
+            const double fi = tm[i], fp = tm[ip];
+            const double vsi = tm[g.nH + i], vsp = tm[g.nH + ip];
+            const double Si = tm[3 * g.nH + i], Sp = tm[3 * g.nH + ip];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const double* x = vc + k * g.nH;
+              const double xm = x[im], xi = x[i], xp = x[ip];
+              double si = bstress(xm, xi, g.vH), sp = bstress(xi, xp, g.vH);
+              if (k == 1) { si = (si + vsi) - Si; sp = (sp + vsp) - Sp; }    // classic
+              if (k == 2) { si = (si + vsi) - svi; sp = (sp + vsp) - svp; }  // classic + flux
+              if (k == 3) { si = (si + fi) - svi; sp = (sp + fp) - svp; }    // + div (exact)
+              vn[k * g.nH + i] = fma(dtH, sp - si, xi);
+            }
+          }
+          par ^= 1;
+        }
         for (int j = tid; j < g.nh; j += blockDim.x) {
           const int p = g.G + j;
           const double x = fma(dth, se[p + 1] - se[p], ue[p]);
@@ -271,6 +314,11 @@ __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
       ++done;
     }
     for (int j = tid; j < g.nh; j += blockDim.x) us[j] = ue[g.G + j];
+    if (LES && par) {
+      const double* src = A.v1 + s * vs;
+      double* dst = A.v0 + s * vs;
+      for (size_t i = tid; i < vs; i += blockDim.x) dst[i] = src[i];
+    }
     if (tid == 0) {
       A.t[s] = tt;
       A.steps[s] += done;
@@ -292,7 +340,8 @@ __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
 // per thread (NC odd: the strided shared stores hit every bank), so the DNS
 // update keeps the FP64 values and their bits.  Sums below 2^63: |x.h| <= 2^27,
 // |x.l| <= 2^26, |w.l| <= 2^26, and the weights' scale is at least 2^-4, so the
-// w.h sum to at most 2^31: 2^58, 2^53 T + 2^57 and 2^52 T for T taps (T < 512).
+// w.h sum to at most 2^31: 2^58, 2^53 T + 2^57 and 2^52 T for T taps.  Stencils
+// of BX_MAX_TAPS and more take advance_kernel<true, false>.
 //
 // The four LES stresses of a cell are formed once, into the spare LES buffer,
 // and read by both cells they border.  One warp forms the step's scalars: FP64
@@ -304,7 +353,7 @@ __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
 //   four taps       71       66       94      12.7
 // What is left is the FP64 pipe for the DNS update (five operations a cell,
 // 2 cells a clock: 18 us), the conversions of 2 x nh values and the taps.
-constexpr int BX_BITS = 54, BX_LOW = 27;
+constexpr int BX_BITS = 54, BX_LOW = 27, BX_MAX_TAPS = 512;
 
 __device__ __forceinline__ Fx as_fx(int2 v) { return {v.x, v.y}; }
 __device__ __forceinline__ int2 as_int2(Fx v) { return make_int2(v.h, v.l); }
@@ -1219,9 +1268,10 @@ int exc_burgers_advance(exc_burgers* b, double tstop, double cfl, int scheme, in
   A.acc = b->scr + (size_t)b->nh * b->ns;
   A.err = b->err;
   const size_t sm = sample_smem(A.g);
-  const void* fn = b->les_on ? les_kernel(b->nh)
-                             : scheme == EXC_BURGERS_RK4 ? (const void*)advance_kernel<true>
-                                                         : (const void*)advance_kernel<false>;
+  const void* fn = b->les_on ? (2 * b->Rd + 1 < BX_MAX_TAPS ? les_kernel(b->nh)
+                                                            : (const void*)advance_kernel<true, false>)
+                             : scheme == EXC_BURGERS_RK4 ? (const void*)advance_kernel<false, true>
+                                                         : (const void*)advance_kernel<false, false>;
   if (allow_smem(fn, sm) != cudaSuccess) { cudaGetLastError(); set_last_error("shared memory opt-in failed"); return EXC_ERR_CUDA; }
   const int grid = grid_for(fn, sm, b->ns);
   void* args[] = {&A};

@@ -394,11 +394,14 @@ static cudaError_t stockham_solve(exc_poisson* ps, const T* src, bool src_is_vec
 template <typename T>
 cudaError_t poisson_solve_inplace(exc_poisson* ps, const T* src, bool src_is_vector, cudaStream_t st,
                                   const SlotBatch& sb, int nslots) {
+  // the register passes read pairs of words; the Stockham x pass reads words, so
+  // it takes a field that starts at an odd one
+  const bool pairs = reinterpret_cast<uintptr_t>(src) % (2 * sizeof(T)) == 0;
   if constexpr (sizeof(T) == 8) {
-    if (ps->engine == 0 && ps->mix && nslots == 1 && !sb.active)
+    if (ps->engine == 0 && pairs && ps->mix && nslots == 1 && !sb.active)
       return ps->mix->gen ? gen_mix_solve(ps, src, src_is_vector, st) : fftmix_solve(ps, src, src_is_vector, st);
   }
-  if (ps->engine != 1 && ps->twl_n && ps->twl_h && ps->invlap)
+  if (ps->engine != 1 && pairs && ps->twl_n && ps->twl_h && ps->invlap)
     return ps->gen ? gen_solve(ps, src, src_is_vector, st, sb, nslots)
                    : fftreg_solve(ps, src, src_is_vector, st, sb, nslots);
   if (plan_ext(ps->plan_n) || plan_ext(ps->plan_h))

@@ -39,6 +39,23 @@ constexpr int SEP_MAX_OUT = 32;      // targets
 constexpr int SEP_ROWS = 8;          // x rows per CTA
 constexpr int SEP_THREADS = 256;
 
+// Rows of n cells and `pad` ghosts on either side that an x-pass CTA stages
+// beside its static words in the default 48 KB of shared memory.
+constexpr size_t SEP_STATIC = SEP_THREADS / 32 * sizeof(unsigned);
+constexpr size_t sep_row_bytes(int n, int pad) { return (size_t)(n + 2 * pad) * sizeof(double); }
+constexpr int sep_rows(int n, int pad) {
+  const int rows = (int)((48 * 1024 - SEP_STATIC) / sep_row_bytes(n, pad));
+  return rows < 1 ? 1 : rows > SEP_ROWS ? SEP_ROWS : rows;
+}
+// every grid and every ghost width of MAX_TAPS taps
+constexpr bool sep_rows_fit() {
+  for (int n = 4; n <= 1024; ++n)
+    for (int pad = 0; pad <= 2 * MAX_TAPS; ++pad)
+      if (sep_rows(n, pad) * sep_row_bytes(n, pad) + SEP_STATIC > 48 * 1024) return false;
+  return true;
+}
+static_assert(sep_rows_fit(), "an x-pass CTA fits the default shared memory");
+
 struct XVar {
   int taps;
   double* out;
@@ -110,6 +127,7 @@ __device__ __forceinline__ double sep_value(const XArgs& A, int src, int x, int 
 __global__ void __launch_bounds__(SEP_THREADS) sep_x_kernel(const __grid_constant__ XArgs A) {
   extern __shared__ double row[];
   __shared__ unsigned wmax[SEP_THREADS / 32];
+  static_assert(sizeof(wmax) == SEP_STATIC, "counted by sep_rows");
   const int n = A.n, m = A.m, c = A.c, pitch = n + 2 * A.pad;
   const int src = A.src[blockIdx.y];
   const int nn = n * n;
@@ -372,17 +390,12 @@ int sep_filter(SepWork* w, int n, int c, double inv_h, double visc, const SepTap
     Z.v[i] = {targets[i].t[2], w->b + (size_t)y1[i] * yw, y2[i] >= 0 ? w->b + (size_t)y2[i] * yw : nullptr,
               targets[i].out};
 
-  // rows that fit the default 48 KB of shared memory (one row of 1024 cells
-  // and its ghosts is 9 KB at most)
-  const size_t rowb = (size_t)(n + 2 * pad) * sizeof(double);
-  int rows = (int)((48 * 1024) / rowb);
-  rows = rows < 1 ? 1 : rows > SEP_ROWS ? SEP_ROWS : rows;
-  X.rows = rows;
+  const int rows = X.rows = sep_rows(n, pad);
   auto blocks = [](size_t cnt) {
     const size_t b = (cnt + SEP_THREADS - 1) / SEP_THREADS;
     return (unsigned)(b < 152 * 16 ? b : 152 * 16);
   };
-  sep_x_kernel<<<dim3((unsigned)((n * n + rows - 1) / rows), X.nsrc), SEP_THREADS, rows * rowb, st>>>(X);
+  sep_x_kernel<<<dim3((unsigned)((n * n + rows - 1) / rows), X.nsrc), SEP_THREADS, rows * sep_row_bytes(n, pad), st>>>(X);
   sep_y_kernel<<<dim3(blocks(yw), (unsigned)yv.size()), SEP_THREADS, 0, st>>>(Y);
   sep_z_kernel<<<dim3(blocks((size_t)m * m * m), (unsigned)targets.size()), SEP_THREADS, 0, st>>>(Z);
   cudaError_t e = cudaGetLastError();

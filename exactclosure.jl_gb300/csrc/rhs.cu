@@ -407,11 +407,20 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
 //   in weight 2^29, the largest of the three, the four A B give at most 3 2^60
 //   (|A.h| <= 2^29, |A.l| <= 3 2^28), D_i S_i 1.2 2^60 and the three groups of
 //   the linear term 1.5 2^60 (4S < 2^57): 5.7 2^60 in all.
-// The sum is exact to 2^-85 of the squared scale; converted to a double with
-// one rounding and multiplied by -1/(4h), it is closer to the exact sum than
-// the FP64 operations it replaces wherever a cell's own velocity is within
-// 2^-7 of the tile's largest.  Cells below that, and planes with values that
-// are not finite or out of range, take rhs_cell_f64.
+// The sum is exact to 2^-85 of the squared scale, converted to a double with
+// one rounding and multiplied by -1/(4h).
+//
+// What remains is the rounding of the inputs to 2^-58 of the scale.  The FP64
+// operations it replaces round products of sums of u_i and S, so a component's
+// error goes with max(|u_i|, S) there and with the scale here: relative L2 of
+// the third component, white noise with that component 2^-k of the others, S
+// below it, FP64 form 2.2-2.9e-16 throughout:
+//   k = 0: 0.9e-16   3: 1.3e-16   4: 2.2e-16   5: 4.0e-16   7: 1.5e-15   10: 1e-14
+// So a component that is not zero and with S below 2^-FX_WEAK of the scale
+// in the three planes takes rhs_cell_f64.  So do the cells whose velocity is
+// below 2^-7 of the tile's largest (their error is below the larger cells' in
+// any norm over the tile), and planes with values that are not finite or out of
+// range.
 //
 // Per cell 650 instructions, 88 of them the multiply-adds, 57 shared-memory
 // accesses per 32 cells and 6 FP64 operations (45 before).  512^3: 11.4 -> 3.46
@@ -425,32 +434,34 @@ constexpr int FX_BITS = 57, FX_LOW = 29;
 // E of the fixed-point path: well inside the range of the FP32 bound that
 // finds it, and squares and their scaling stay normal doubles
 constexpr int FX_EMIN = -100, FX_EMAX = FX_BITS;
+constexpr int FX_WEAK = 4;
 
-// The reference's arithmetic for one cell, from global memory: the cells the
-// fixed-point sweep leaves out.
-__device__ __noinline__ double3 rhs_cell_f64(const double* __restrict__ u, int n, int x, int y, int z, double inv_h,
-                                             double visc) {
-  const long long nn = (long long)n * n, N = nn * n;
-  const double* const a = u + z * nn + (long long)y * n + x;
-  const double *const b = a + N, *const c = b + N;
-  const long long xp = x + 1 == n ? 1 - n : 1, xm = x == 0 ? n - 1 : -1;
-  const long long yp = y + 1 == n ? -(nn - n) : n, ym = y == 0 ? nn - n : -n;
-  const long long zp = z + 1 == n ? -(N - nn) : nn, zm = z == 0 ? N - nn : -nn;
-  const double rv = 4.0 * visc * inv_h;
-  auto diag = [rv](double p, double q) { return (p + q) * (p + q) - 2.0 * rv * (p - q); };
-  auto off = [rv](double p, double q, double r, double t) { return (p + q) * (r + t) - rv * ((q - p) + (t - r)); };
+// The reference's arithmetic for component I of one cell, from global memory:
+// what the fixed-point sweep leaves out.
+template <int I>
+__device__ __noinline__ double rhs_cell_f64(const double* __restrict__ u, int n, int x, int y, int z, double inv_h,
+                                            double visc) {
+  constexpr int J = I == 0 ? 1 : 0, K = I == 2 ? 1 : 2;
+  const long long N = (long long)n * n * n;
+  const int at[3] = {x, y, z};
+  const long long step[3] = {1, n, (long long)n * n};
+  auto up = [&](int d) { return at[d] + 1 == n ? (1 - n) * step[d] : step[d]; };
+  auto dn = [&](int d) { return at[d] == 0 ? (n - 1) * step[d] : -step[d]; };
+  const double* const p = u + I * N + z * step[2] + y * step[1] + x;
+  const double *const q = p + (J - I) * N, *const r = p + (K - I) * N;
+  const long long iu = up(I), id = dn(I), ju = up(J), jd = dn(J), ku = up(K), kd = dn(K);
   // all loads first: they are independent
-  const double a0 = a[0], axp = a[xp], axm = a[xm], ayp = a[yp], aym = a[ym], azp = a[zp], azm = a[zm];
-  const double b0 = b[0], bxp = b[xp], bxm = b[xm], byp = b[yp], bym = b[ym], bzp = b[zp], bzm = b[zm];
-  const double c0 = c[0], cxp = c[xp], cxm = c[xm], cyp = c[yp], cym = c[ym], czp = c[zp], czm = c[zm];
-  const double axmyp = a[xm + yp], axmzp = a[xm + zp], bxpym = b[xp + ym], bymzp = b[ym + zp], cxpzm = c[xp + zm],
-               cypzm = c[yp + zm];
-  const double s12 = off(a0, ayp, b0, bxp), s13 = off(a0, azp, c0, cxp), s23 = off(b0, bzp, c0, cyp);
-  const double k = -0.25 * inv_h;
-  const double d1 = (diag(axp, a0) - diag(a0, axm)) + (s12 - off(aym, a0, bym, bxpym)) + (s13 - off(azm, a0, czm, cxpzm));
-  const double d2 = (s12 - off(axm, axmyp, bxm, b0)) + (diag(byp, b0) - diag(b0, bym)) + (s23 - off(bzm, b0, czm, cypzm));
-  const double d3 = (s13 - off(axm, axmzp, cxm, c0)) + (s23 - off(bym, bymzp, cym, c0)) + (diag(czp, c0) - diag(c0, czm));
-  return make_double3(k * d1, k * d2, k * d3);
+  const double p0 = p[0], piu = p[iu], pid = p[id], pju = p[ju], pjd = p[jd], pku = p[ku], pkd = p[kd];
+  const double q0 = q[0], qiu = q[iu], qjd = q[jd], qjdiu = q[jd + iu];
+  const double r0 = r[0], riu = r[iu], rkd = r[kd], rkdiu = r[kd + iu];
+  const double rv = 4.0 * visc * inv_h;
+  auto diag = [rv](double a, double b) { return (a + b) * (a + b) - 2.0 * rv * (a - b); };
+  auto off = [rv](double a, double b, double c, double d) { return (a + b) * (c + d) - rv * ((b - a) + (d - c)); };
+  const double di = diag(piu, p0) - diag(p0, pid);
+  const double dj = off(p0, pju, q0, qiu) - off(pjd, p0, qjd, qjdiu);
+  const double dk = off(p0, pku, r0, riu) - off(pkd, p0, rkd, rkdiu);
+  const double sum = I == 2 ? (dj + dk) + di : (di + dj) + dk;
+  return -0.25 * inv_h * sum;
 }
 
 // Tile of the fixed-point sweep: 32 x 16 cells, FXC rows per thread, FX_CTAS
@@ -468,7 +479,7 @@ struct FixedSmem {
   // x = x0 - 2 first; doubles on arrival, then Fx pairs
   double u[3][3 * FXBY * FXROW + 8];
   unsigned piece[FXPIECES];      // word offset in the field of each 16-byte piece of a plane
-  unsigned red[3][FXW];          // largest magnitude (high word) per plane buffer and warp
+  unsigned red[3][3][FXW];       // largest magnitude (high word) per plane buffer, component and warp
   unsigned long long bar[3];     // TMA completion of each plane buffer
 };
 static_assert(sizeof(FixedSmem::u[0]) % 128 == 0, "TMA destinations");
@@ -565,18 +576,34 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
       if (t < FXPIECES) f(reinterpret_cast<double2*>(sm.u[buf])[t]);
     }
   };
-  // largest magnitude of a plane (high words), this warp's part, into sm.red;
-  // the plane itself is only read
+  // largest magnitude of each component of a plane (high words), this warp's
+  // part, into sm.red: of the pieces it copied itself, which it may read before the
+  // barrier; the plane is only read
   auto scan_plane = [&](int buf) {
-    unsigned m = 0;
-    each_piece(buf, [&](const double2& v) {
-      m = max(m, max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu));
-    });
-    m = __reduce_max_sync(0xffffffffu, m);
-    if (tx == 0) sm.red[buf][ty] = m;
+    constexpr int PC = FXPIECES / 3;  // pieces of a component
+    unsigned m[3] = {0, 0, 0};
+#pragma unroll
+    for (int i = 0; i < NSLOT; ++i) {
+      const int t = tid + i * FXTHREADS;
+      if (t < FXPIECES) {
+        const double2 v = reinterpret_cast<const double2*>(sm.u[buf])[t];
+        const unsigned q = max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)  // the components that slot i of any thread reaches
+          if (c * PC < (i + 1) * FXTHREADS && (c + 1) * PC > i * FXTHREADS)
+            m[c] = max(m[c], t >= c * PC && t < (c + 1) * PC ? q : 0u);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      m[c] = __reduce_max_sync(0xffffffffu, m[c]);
+      if (tx == 0) sm.red[buf][c][ty] = m[c];
+    }
   };
-  auto plane_max = [&](int buf) {
-    return __reduce_max_sync(0xffffffffu, tx < FXW ? sm.red[buf][tx] : 0u);
+  static_assert(3 * FXW <= 32, "a lane per warp and plane");
+  // a component's largest magnitude in the three planes held
+  auto held_max = [&](int c) {
+    return __reduce_max_sync(0xffffffffu, tx < 3 * FXW ? sm.red[tx / FXW][c][tx % FXW] : 0u);
   };
   int E = 0;                     // |u| + S < 2^E for the planes held
   int kexp = 0;                  // (57 - E) << 20
@@ -589,8 +616,9 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
   };
   Fx S2{}, S4{};  // 2S and 4S in fixed point
   int tiny = 0;   // cells whose h words are all below this take the FP64 path
+  int weak = 0;   // components (bits) that take it in every cell of the plane
+  unsigned below = 0;  // high word of 2^(E - FX_WEAK), 0 where S is above that
   bool slow = false;
-  unsigned pm1 = 0, pm2 = 0;  // largest magnitudes of the upper two planes held
   // E for planes whose largest magnitude has high word mx: above |u| + S
   // (and above 4S, so that 4S converts); the FP64 path if it is out of range
   // (in FP32, whose range covers the path's; bounds rounded up)
@@ -604,6 +632,17 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
   auto fxat = [&](int buf, int c, int row, int col) {
     const double v = sm.u[buf][(c * FXBY + row) * FXROW + col];
     return Fx{__double2hiint(v), __double2loint(v)};
+  };
+  // what the maxima m of the three planes held send to the FP64 path
+  auto choose = [&](const unsigned (&m)[3]) {
+    // 2^-7 of the top of the largest magnitude's binade, in units of h (the
+    // FP64 path at 2^-5 costs 250^3 27% of its time, at 2^-7 nothing)
+    const unsigned top = max(m[0], max(m[1], m[2]));
+    const int q = FX_BITS - FX_LOW - 7 - (E - (int)((top >> 20) & 0x7ff) + 1022);
+    tiny = top == 0 ? 0 : q < 0 ? 0 : 1 << q;
+    weak = 0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) weak |= m[c] != 0 && m[c] < below ? 1 << c : 0;
   };
   const int col = tx + 2;
   // previous plane at this thread's cells: the velocities and B of s13, s23
@@ -631,9 +670,8 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
 #pragma unroll 1
     for (int b = 0; b < 3; ++b) scan_plane(b);
     __syncthreads();
-    pm1 = plane_max(1);
-    pm2 = plane_max(2);
-    const unsigned mx = max(plane_max(0), max(pm1, pm2));
+    const unsigned m[3] = {held_max(0), held_max(1), held_max(2)};
+    const unsigned mx = max(m[0], max(m[1], m[2]));
     const double S = 2.0 * visc * inv_h;
     E = exponent_for(mx);
     slow = mx >= 0x7fe00000u || !(S < 1e300) || E > FX_EMAX || E < FX_EMIN;
@@ -648,10 +686,8 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
       S4.l = (int)(s4 - ((long long)S4.h << FX_LOW));
       S2 = {(int)((s2 + (1 << (FX_LOW - 1))) >> FX_LOW), 0};
       S2.l = (int)(s2 - ((long long)S2.h << FX_LOW));
-      // 2^-7 of the top of the largest magnitude's binade, in units of h (the
-      // FP64 path at 2^-5 costs 250^3 27% of its time, at 2^-7 nothing)
-      const int q = FX_BITS - FX_LOW - 7 - (E - (int)((mx >> 20) & 0x7ff) + 1022);
-      tiny = mx == 0 ? 0 : q < 0 ? 0 : 1 << q;
+      below = Sf < __int_as_float((E - FX_WEAK + 127) << 23) ? (unsigned)(E - FX_WEAK + 1023) << 20 : 0u;
+      choose(m);
 #pragma unroll 1
       for (int b = 0; b < 3; ++b) convert_plane(b);
     }
@@ -683,7 +719,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
       const int r = NC * ty + 1 + i, gy = y0 + NC * ty + i;
       const Fx a = fxat(cur, 0, r, col), b = fxat(cur, 1, r, col), c = fxat(cur, 2, r, col);
       double o1, o2, o3;
-      bool direct = slow || (max(abs(a.h), max(abs(b.h), abs(c.h))) < tiny);
+      const int direct = slow || max(abs(a.h), max(abs(b.h), abs(c.h))) < tiny ? 7 : weak;
       if (!slow) {
         // u1: neighbours along x, y, z and (-x, +y), (-x, +z)
         const Fx axp = fxat(cur, 0, r, col + 1), axm = fxat(cur, 0, r, col - 1);
@@ -746,12 +782,9 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
         pb23[i] = B23;
       }
       if (gx < n && gy < n) {
-        if (direct) {
-          const double3 o = rhs_cell_f64(u, n, gx, gy, z, inv_h, visc);
-          o1 = o.x;
-          o2 = o.y;
-          o3 = o.z;
-        }
+        if (direct & 1) o1 = rhs_cell_f64<0>(u, n, gx, gy, z, inv_h, visc);
+        if (direct & 2) o2 = rhs_cell_f64<1>(u, n, gx, gy, z, inv_h, visc);
+        if (direct & 4) o3 = rhs_cell_f64<2>(u, n, gx, gy, z, inv_h, visc);
         double* const d = du + ((long long)z * n + gy) * n + gx;
         if (DOADD) {
           d[0] += o1;
@@ -772,17 +805,17 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     wait_plane(pre);
     scan_plane(pre);
     __syncthreads();
-    const unsigned pm = plane_max(pre);
-    const int En = exponent_for(max(pm, max(pm1, pm2)));
-    if (pm >= 0x7fe00000u || En > E || En < E - 2) {
+    const unsigned m[3] = {held_max(0), held_max(1), held_max(2)};
+    const unsigned mx = max(m[0], max(m[1], m[2]));
+    const int En = exponent_for(mx);
+    if (mx >= 0x7fe00000u || En > E || En < E - 2) {
       restart(z + 1);
       continue;
     }
+    choose(m);
     convert_plane(pre);
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     __syncthreads();
-    pm1 = pm2;
-    pm2 = pm;
     const int freed = cur;
     cur = nxt;
     nxt = pre;

@@ -334,14 +334,13 @@ __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
 // the LES kernel for one, at nh = 13500, nH = 900, Delta = 2H: 321 FP64
 // operations per coarse cell) bounded this loop on the FP64 pipe.  They run in
 // fixed point here (fixed.cuh): velocity, stress and weights as 54-bit integers
-// below the step's largest |u|, a bound of the largest stress and the largest
-// weight, the weighted sums exact, one rounding each.  The integers live in
+// below the step's largest |u|, a bound of the largest stress and each kernel's
+// largest weight, the weighted sums exact, one rounding each.  The integers live in
 // shared memory; the velocity itself stays in registers, NC consecutive cells
 // per thread (NC odd: the strided shared stores hit every bank), so the DNS
-// update keeps the FP64 values and their bits.  Sums below 2^63: |x.h| <= 2^27,
-// |x.l| <= 2^26, |w.l| <= 2^26, and the weights' scale is at least 2^-4, so the
-// w.h sum to at most 2^31: 2^58, 2^53 T + 2^57 and 2^52 T for T taps.  Stencils
-// of BX_MAX_TAPS and more take advance_kernel<true, false>.
+// update keeps the FP64 values and their bits.  Sums below 2^63: with h words up to
+// 2^27 and l words up to 2^26, 2^54 T, 2^54 T and 2^52 T for T taps.  Stencils of
+// BX_MAX_TAPS and more take advance_kernel<true, false>.
 //
 // The four LES stresses of a cell are formed once, into the spare LES buffer,
 // and read by both cells they border.  One warp forms the step's scalars: FP64
@@ -384,14 +383,15 @@ __global__ void __launch_bounds__(BT, 1) advance_les_kernel(AdvanceArgs A) {
   int2* const wd = si + np;
   int2* const wl = wd + 2 * g.Rd + 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // weights: one scale for both kernels, from the largest |w|
-  double wm = 0.0;
-  for (int r = tid; r < 2 * g.Rd + 1; r += BT) wm = fmax(wm, fabs(A.wd[r]));
-  for (int r = tid; r < 2 * g.Rl + 1; r += BT) wm = fmax(wm, fabs(A.wl[r]));
-  wm = block_max(wm, red);
-  const int Ew = max(exponent_above(wm), -4), kw = (BX_BITS - Ew) << 20;
-  for (int r = tid; r < 2 * g.Rd + 1; r += BT) wd[r] = as_int2(fx_from_double<BX_BITS, BX_LOW>(A.wd[r], kw));
-  for (int r = tid; r < 2 * g.Rl + 1; r += BT) wl[r] = as_int2(fx_from_double<BX_BITS, BX_LOW>(A.wl[r], kw));
+  // weights, each kernel below its own largest
+  auto load_weights = [&](const double* w, int cnt, int2* to) {
+    double wm = 0.0;
+    for (int r = tid; r < cnt; r += BT) wm = fmax(wm, fabs(w[r]));
+    const int E = exponent_above(block_max(wm, red)), k = (BX_BITS - E) << 20;
+    for (int r = tid; r < cnt; r += BT) to[r] = as_int2(fx_from_double<BX_BITS, BX_LOW>(w[r], k));
+    return E;
+  };
+  const int Ewd = load_weights(A.wd, 2 * g.Rd + 1, wd), Ewl = load_weights(A.wl, 2 * g.Rl + 1, wl);
   const int j0 = tid * NC, cnt = max(0, min(NC, g.nh - j0));
   const size_t vs = (size_t)4 * g.nH;
   for (int s = blockIdx.x; s < g.ns; s += gridDim.x) {
@@ -471,7 +471,8 @@ __global__ void __launch_bounds__(BT, 1) advance_les_kernel(AdvanceArgs A) {
         si[g.G + g.nh + p] = si[g.G + p];
       }
       __syncthreads();
-      const double cu = pow2(Eu + Ew - 2 * BX_BITS + 2 * BX_LOW), cs = pow2(Es + Ew - 2 * BX_BITS + 2 * BX_LOW);
+      constexpr int UNIT = 2 * BX_LOW - 2 * BX_BITS;
+      const double cu = pow2(Eu + Ewd + UNIT), cs = pow2(Es + Ewd + UNIT), cl = pow2(Es + Ewl + UNIT);
       for (int I = tid; I < g.nH; I += BT) {
         // coarse_terms' sums
         const int pc = g.G + (I + 1) * g.comp - g.a - 1, pf = pc + g.a;
@@ -488,7 +489,7 @@ __global__ void __launch_bounds__(BT, 1) advance_les_kernel(AdvanceArgs A) {
         }
 #pragma unroll 4
         for (int r = -g.Rl; r <= g.Rl; ++r) fx_mac(fsu, as_fx(wl[r + g.Rl]), as_fx(si[pc + r]));
-        tm[I] = fx_to_double<BX_LOW>(fsu, cs);
+        tm[I] = fx_to_double<BX_LOW>(fsu, cl);
         tm[g.nH + I] = fx_to_double<BX_LOW>(vsu, cs);
         tm[2 * g.nH + I] = fx_to_double<BX_LOW>(vu, cu);
         tm[3 * g.nH + I] = bstress(fx_to_double<BX_LOW>(vl, cu), fx_to_double<BX_LOW>(vr, cu), g.vh);

@@ -15,6 +15,7 @@
 
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "fixed.cuh"
 #include "internal.cuh"
@@ -417,10 +418,14 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
 // below it, FP64 form 2.2-2.9e-16 throughout:
 //   k = 0: 0.9e-16   3: 1.3e-16   4: 2.2e-16   5: 4.0e-16   7: 1.5e-15   10: 1e-14
 // So a component that is not zero and with S below 2^-FX_WEAK of the scale
-// in the three planes takes rhs_cell_f64.  So do the cells whose velocity is
-// below 2^-7 of the tile's largest (their error is below the larger cells' in
-// any norm over the tile), and planes with values that are not finite or out of
-// range.
+// in the three planes takes rhs_cell_f64.  S is rounded with them: where it is
+// below 2^-FX_SMALL_S of the scale it stays out of the integers, and the linear
+// term is summed by itself, exactly, and multiplied by S in FP64 (a shear flow
+// u_1(y), whose advection vanishes, is nothing else: ten cells of noise at visc
+// 1e-5 2.9e-14 with S rounded, FP64 form 1.8e-16).
+// The cells whose velocity is below 2^-7 of the tile's largest take rhs_cell_f64
+// too (their error is below the larger cells' in any norm over the tile), and
+// planes with values that are not finite or out of range.
 //
 // Per cell 650 instructions, 88 of them the multiply-adds, 57 shared-memory
 // accesses per 32 cells and 6 FP64 operations (45 before).  512^3: 11.4 -> 3.46
@@ -434,7 +439,7 @@ constexpr int FX_BITS = 57, FX_LOW = 29;
 // E of the fixed-point path: well inside the range of the FP32 bound that
 // finds it, and squares and their scaling stay normal doubles
 constexpr int FX_EMIN = -100, FX_EMAX = FX_BITS;
-constexpr int FX_WEAK = 4;
+constexpr int FX_WEAK = 4, FX_SMALL_S = 6;
 
 // The reference's arithmetic for component I of one cell, from global memory:
 // what the fixed-point sweep leaves out.
@@ -481,6 +486,7 @@ struct FixedSmem {
   unsigned piece[FXPIECES];      // word offset in the field of each 16-byte piece of a plane
   unsigned red[3][3][FXW];       // largest magnitude (high word) per plane buffer, component and warp
   unsigned long long bar[3];     // TMA completion of each plane buffer
+  double by_s;                   // factor of the linear term of a small S
 };
 static_assert(sizeof(FixedSmem::u[0]) % 128 == 0, "TMA destinations");
 constexpr size_t FIXED_SMEM = sizeof(FixedSmem) + 128;
@@ -616,7 +622,8 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
   };
   Fx S2{}, S4{};  // 2S and 4S in fixed point
   int tiny = 0;   // cells whose h words are all below this take the FP64 path
-  int weak = 0;   // components (bits) that take it in every cell of the plane
+  int weak = 0;   // bits 0-2: components that take it in every cell of the plane
+  bool small_s = false;
   unsigned below = 0;  // high word of 2^(E - FX_WEAK), 0 where S is above that
   bool slow = false;
   // E for planes whose largest magnitude has high word mx: above |u| + S
@@ -643,6 +650,12 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     weak = 0;
 #pragma unroll
     for (int c = 0; c < 3; ++c) weak |= m[c] != 0 && m[c] < below ? 1 << c : 0;
+  };
+  // -4h du's linear term in units of S and of the velocity: its three groups, D
+  // and the two pair sums A + B - (A + B)(-e_j) without S; at most 48 2^57
+  auto linear = [](Fx g1, Fx g2, Fx g3, Fx d, Fx p, Fx q) {
+    auto word = [](Fx v) { return (long long)v.h * (1 << FX_LOW) + v.l; };
+    return (double)(4 * (word(g1) + word(g2) + word(g3) - word(d)) - 2 * (word(p) + word(q)));
   };
   const int col = tx + 2;
   // previous plane at this thread's cells: the velocities and B of s13, s23
@@ -678,7 +691,9 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     if (!slow) {
       kexp = (FX_BITS - E) << 20;
       scale = ldexp(-0.25 * inv_h, 2 * FX_LOW + 2 * (E - FX_BITS));
-      const Fx s = fx_from_double<FX_BITS, FX_LOW>(4.0 * S, kexp);
+      small_s = Sf < __int_as_float((E - FX_SMALL_S + 127) << 23);
+      if (small_s && tid == 0) sm.by_s = ldexp(-0.25 * inv_h * S, E - FX_BITS);
+      const Fx s = small_s ? Fx{0, 0} : fx_from_double<FX_BITS, FX_LOW>(4.0 * S, kexp);
       // 4S to a multiple of four units, so that S and 2S are the same S
       const long long s4 = (((long long)s.h << FX_LOW) + s.l + 2) >> 2 << 2;
       const long long s2 = s4 >> 1;
@@ -714,89 +729,105 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     if (z >= n) break;  // uniform across the CTA
     const bool more = kz + 1 < ptz && z + 1 < n;
     if (more && !slow) load_plane(pre, wrapm(z + 2));
+    auto cells = [&](auto s_is_small) {
+      constexpr bool SMALL_S = decltype(s_is_small)::value;
+      const Fx s2 = SMALL_S ? Fx{0, 0} : S2, s4 = SMALL_S ? Fx{0, 0} : S4;
 #pragma unroll
-    for (int i = 0; i < NC; ++i) {
-      const int r = NC * ty + 1 + i, gy = y0 + NC * ty + i;
-      const Fx a = fxat(cur, 0, r, col), b = fxat(cur, 1, r, col), c = fxat(cur, 2, r, col);
-      double o1, o2, o3;
-      const int direct = slow || max(abs(a.h), max(abs(b.h), abs(c.h))) < tiny ? 7 : weak;
-      if (!slow) {
-        // u1: neighbours along x, y, z and (-x, +y), (-x, +z)
-        const Fx axp = fxat(cur, 0, r, col + 1), axm = fxat(cur, 0, r, col - 1);
-        const Fx ayp = fxat(cur, 0, r + 1, col), aym = fxat(cur, 0, r - 1, col);
-        const Fx axmyp = fxat(cur, 0, r + 1, col - 1);
-        const Fx azp = fxat(nxt, 0, r, col), axmzp = fxat(nxt, 0, r, col - 1);
-        // u2: along x, y, z and (+x, -y), (-y, +z)
-        const Fx bxp = fxat(cur, 1, r, col + 1), bxm = fxat(cur, 1, r, col - 1);
-        const Fx byp = fxat(cur, 1, r + 1, col), bym = fxat(cur, 1, r - 1, col);
-        const Fx bxpym = fxat(cur, 1, r - 1, col + 1);
-        const Fx bzp = fxat(nxt, 1, r, col), bymzp = fxat(nxt, 1, r - 1, col);
-        // u3: along x, y, z
-        const Fx cxp = fxat(cur, 2, r, col + 1), cxm = fxat(cur, 2, r, col - 1);
-        const Fx cyp = fxat(cur, 2, r + 1, col), cym = fxat(cur, 2, r - 1, col);
-        const Fx czp = fxat(nxt, 2, r, col);
-        // the linear term's group common to the components
-        FxSum s0{0, 0, 0};
-        fx_mac(s0, (a - axm) + (b - bym), S4);
-        const Fx dz3 = c - pw3[i];
-        const Fx A12 = a + ayp - S2, B12 = b + bxp - S2;
-        const Fx A13 = a + azp - S2, B13 = c + cxp - S2;
-        const Fx A23 = b + bzp - S2, B23 = c + cyp - S2;
-        {
-          FxSum s = s0;
-          fx_mac(s, dz3 + (a - axm), S4);
-          fx_mac(s, (a - aym) + (a - pw1[i]), S4);
-          fx_mac(s, axp - axm, (axp + axm) + (a + a) - S4);
-          fx_mac(s, A12, B12);
-          fx_mac(s, S2 - a - aym, bym + bxpym - S2);
-          fx_mac(s, A13, B13);
-          fx_mac(s, S2 - a - pw1[i], pb13[i]);
-          o1 = fx_to_double<FX_LOW>(s, scale);
+      for (int i = 0; i < NC; ++i) {
+        const int r = NC * ty + 1 + i, gy = y0 + NC * ty + i;
+        const Fx a = fxat(cur, 0, r, col), b = fxat(cur, 1, r, col), c = fxat(cur, 2, r, col);
+        double o1, o2, o3;
+        const int direct = slow || max(abs(a.h), max(abs(b.h), abs(c.h))) < tiny ? 7 : weak;
+        if (!slow) {
+          // u1: neighbours along x, y, z and (-x, +y), (-x, +z)
+          const Fx axp = fxat(cur, 0, r, col + 1), axm = fxat(cur, 0, r, col - 1);
+          const Fx ayp = fxat(cur, 0, r + 1, col), aym = fxat(cur, 0, r - 1, col);
+          const Fx axmyp = fxat(cur, 0, r + 1, col - 1);
+          const Fx azp = fxat(nxt, 0, r, col), axmzp = fxat(nxt, 0, r, col - 1);
+          // u2: along x, y, z and (+x, -y), (-y, +z)
+          const Fx bxp = fxat(cur, 1, r, col + 1), bxm = fxat(cur, 1, r, col - 1);
+          const Fx byp = fxat(cur, 1, r + 1, col), bym = fxat(cur, 1, r - 1, col);
+          const Fx bxpym = fxat(cur, 1, r - 1, col + 1);
+          const Fx bzp = fxat(nxt, 1, r, col), bymzp = fxat(nxt, 1, r - 1, col);
+          // u3: along x, y, z
+          const Fx cxp = fxat(cur, 2, r, col + 1), cxm = fxat(cur, 2, r, col - 1);
+          const Fx cyp = fxat(cur, 2, r + 1, col), cym = fxat(cur, 2, r - 1, col);
+          const Fx czp = fxat(nxt, 2, r, col);
+          // the linear term's group common to the components
+          FxSum s0{0, 0, 0};
+          fx_mac(s0, (a - axm) + (b - bym), s4);
+          const Fx dz3 = c - pw3[i];
+          const Fx A12 = a + ayp - s2, B12 = b + bxp - s2;
+          const Fx A13 = a + azp - s2, B13 = c + cxp - s2;
+          const Fx A23 = b + bzp - s2, B23 = c + cyp - s2;
+          {
+            FxSum s = s0;
+            fx_mac(s, dz3 + (a - axm), s4);
+            fx_mac(s, (a - aym) + (a - pw1[i]), s4);
+            fx_mac(s, axp - axm, (axp + axm) + (a + a) - s4);
+            fx_mac(s, A12, B12);
+            fx_mac(s, s2 - a - aym, bym + bxpym - s2);
+            fx_mac(s, A13, B13);
+            fx_mac(s, s2 - a - pw1[i], pb13[i]);
+            o1 = fx_to_double<FX_LOW>(s, scale);
+            if constexpr (SMALL_S)
+              o1 = fma(sm.by_s, linear((a - axm) + (b - bym), dz3 + (a - axm), (a - aym) + (a - pw1[i]), axp - axm,
+                       (ayp - aym) + (b + bxp) - (bym + bxpym), (azp - pw1[i]) + (c + cxp) - (pb13[i] + s2)), o1);
+          }
+          {
+            FxSum s = s0;
+            fx_mac(s, dz3 + (b - bxm), s4);
+            fx_mac(s, (b - bym) + (b - pw2[i]), s4);
+            fx_mac(s, byp - bym, (byp + bym) + (b + b) - s4);
+            fx_mac(s, A12, B12);
+            fx_mac(s, s2 - axm - axmyp, bxm + b - s2);
+            fx_mac(s, A23, B23);
+            fx_mac(s, s2 - b - pw2[i], pb23[i]);
+            o2 = fx_to_double<FX_LOW>(s, scale);
+            if constexpr (SMALL_S)
+              o2 = fma(sm.by_s, linear((a - axm) + (b - bym), dz3 + (b - bxm), (b - bym) + (b - pw2[i]), byp - bym,
+                       (a + ayp) - (axm + axmyp) + (bxp - bxm), (bzp - pw2[i]) + (c + cyp) - (pb23[i] + s2)), o2);
+          }
+          {
+            FxSum s = s0;
+            fx_mac(s, dz3 + (c - cxm), s4);
+            fx_mac(s, (c - cym) + dz3, s4);
+            fx_mac(s, czp - pw3[i], (czp + pw3[i]) + (c + c) - s4);
+            fx_mac(s, A13, B13);
+            fx_mac(s, s2 - axm - axmzp, cxm + c - s2);
+            fx_mac(s, A23, B23);
+            fx_mac(s, s2 - bym - bymzp, cym + c - s2);
+            o3 = fx_to_double<FX_LOW>(s, scale);
+            if constexpr (SMALL_S)
+              o3 = fma(sm.by_s, linear((a - axm) + (b - bym), dz3 + (c - cxm), (c - cym) + dz3, czp - pw3[i],
+                       (a + azp) - (axm + axmzp) + (cxp - cxm), (b + bzp) - (bym + bymzp) + (cyp - cym)), o3);
+          }
+          pw1[i] = a;
+          pw2[i] = b;
+          pw3[i] = c;
+          pb13[i] = B13;
+          pb23[i] = B23;
         }
-        {
-          FxSum s = s0;
-          fx_mac(s, dz3 + (b - bxm), S4);
-          fx_mac(s, (b - bym) + (b - pw2[i]), S4);
-          fx_mac(s, byp - bym, (byp + bym) + (b + b) - S4);
-          fx_mac(s, A12, B12);
-          fx_mac(s, S2 - axm - axmyp, bxm + b - S2);
-          fx_mac(s, A23, B23);
-          fx_mac(s, S2 - b - pw2[i], pb23[i]);
-          o2 = fx_to_double<FX_LOW>(s, scale);
+        if (gx < n && gy < n) {
+          if (direct & 1) o1 = rhs_cell_f64<0>(u, n, gx, gy, z, inv_h, visc);
+          if (direct & 2) o2 = rhs_cell_f64<1>(u, n, gx, gy, z, inv_h, visc);
+          if (direct & 4) o3 = rhs_cell_f64<2>(u, n, gx, gy, z, inv_h, visc);
+          double* const d = du + ((long long)z * n + gy) * n + gx;
+          if (DOADD) {
+            d[0] += o1;
+            d[N] += o2;
+            d[2 * N] += o3;
+          } else {
+            d[0] = o1;
+            d[N] = o2;
+            d[2 * N] = o3;
+          }
         }
-        {
-          FxSum s = s0;
-          fx_mac(s, dz3 + (c - cxm), S4);
-          fx_mac(s, (c - cym) + dz3, S4);
-          fx_mac(s, czp - pw3[i], (czp + pw3[i]) + (c + c) - S4);
-          fx_mac(s, A13, B13);
-          fx_mac(s, S2 - axm - axmzp, cxm + c - S2);
-          fx_mac(s, A23, B23);
-          fx_mac(s, S2 - bym - bymzp, cym + c - S2);
-          o3 = fx_to_double<FX_LOW>(s, scale);
-        }
-        pw1[i] = a;
-        pw2[i] = b;
-        pw3[i] = c;
-        pb13[i] = B13;
-        pb23[i] = B23;
       }
-      if (gx < n && gy < n) {
-        if (direct & 1) o1 = rhs_cell_f64<0>(u, n, gx, gy, z, inv_h, visc);
-        if (direct & 2) o2 = rhs_cell_f64<1>(u, n, gx, gy, z, inv_h, visc);
-        if (direct & 4) o3 = rhs_cell_f64<2>(u, n, gx, gy, z, inv_h, visc);
-        double* const d = du + ((long long)z * n + gy) * n + gx;
-        if (DOADD) {
-          d[0] += o1;
-          d[N] += o2;
-          d[2 * N] += o3;
-        } else {
-          d[0] = o1;
-          d[N] = o2;
-          d[2 * N] = o3;
-        }
-      }
-    }
+    };
+    // two copies: the linear term by itself would cost the usual one registers
+    if (small_s) cells(std::true_type());
+    else cells(std::false_type());
     if (!more) break;
     if (slow) {
       restart(z + 1);

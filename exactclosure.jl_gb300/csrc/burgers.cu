@@ -43,6 +43,7 @@ struct exc_burgers {
   double* smag = nullptr;  // [ns][nH] Smagorinsky LES
   double* tsm = nullptr;   // [ns]
   int* ssm = nullptr;      // [ns]
+  int* left = nullptr;     // [2][ns] samples the fixed-point loop left, and their steps so far in the call
   bool les_on = false, smag_on = false;
   double* red = nullptr;   // [ns][8] per-sample partial sums
   double* sums = nullptr;  // [8]
@@ -181,7 +182,8 @@ struct AdvanceArgs {
   double* tmp;   // [ns][5][nH]
   double* uold;  // [ns][nh] (RK4)
   double* acc;   // [ns][nh] (RK4)
-  int* err;
+  int* err;      // bit 0: a sample stopped on a bad step; bit 1: one was left to the FP64 loop
+  int* left;     // [2][ns], null: every sample is this launch's from its start
 };
 
 // Per-sample time step (src/Burgers.jl:97-101, :383-385) from the largest |u|
@@ -193,7 +195,7 @@ __device__ __forceinline__ bool step_of(const AdvanceArgs& A, double m, double t
   // A non-finite field, or a CFL step that collapsed, ends the sample with a
   // flag instead of a NaN time or an unbounded loop.
   if (!(m == m) || isinf(m) || !(dtc > 1e-12 * A.tstop)) {
-    if (threadIdx.x == 0) atomicExch(A.err, 1);
+    if (threadIdx.x == 0) atomicOr(A.err, 1);
     return false;
   }
   return true;
@@ -220,10 +222,12 @@ __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
   const int tid = threadIdx.x;
   const size_t vs = (size_t)4 * g.nH;
   for (int s = blockIdx.x; s < g.ns; s += gridDim.x) {
+    if (LES && A.left && !A.left[s]) continue;
     double* us = A.u + (size_t)s * g.nh;
     load_sample(g, us, ue);
     double tt = A.t[s];
-    int done = 0, par = 0;
+    const int before = LES && A.left ? A.left[g.ns + s] : 0;
+    int done = before, par = 0;
     __syncthreads();
     // |u| maximum of this thread's cells, kept up to date by the updates.
     double lmax = 0.0;
@@ -321,7 +325,7 @@ __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
     }
     if (tid == 0) {
       A.t[s] = tt;
-      A.steps[s] += done;
+      A.steps[s] += done - before;
     }
     __syncthreads();
   }
@@ -342,6 +346,14 @@ __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
 // 2^27 and l words up to 2^26, 2^54 T, 2^54 T and 2^52 T for T taps.  Stencils of
 // BX_MAX_TAPS and more take advance_kernel<true, false>.
 //
+// The scales are the sample's, so values far below its largest keep fewer bits than
+// in FP64: a sample is left to advance_kernel<true, false>, from the step on that
+// meets it, when the largest |u| of a warp's cells (32 NC of them, 864 of 13500;
+// not all zero) is below 2^-BX_WEAK of the sample's.  One step against extended
+// precision, units of 2^-53 of the LES states: 0.4-1.1, FP64 sums 0.4-8.6, and a
+// stress far below its bound (a smooth field in a viscous fluid, 1/400 of it) the
+// same 0.4-0.9.
+//
 // The four LES stresses of a cell are formed once, into the spare LES buffer,
 // and read by both cells they border.  One warp forms the step's scalars: FP64
 // work of all 16 warps would take the pipe 16 times.  A step of 152 samples at
@@ -352,7 +364,7 @@ __global__ void __launch_bounds__(BT) advance_kernel(AdvanceArgs A) {
 //   four taps       71       66       94      12.7
 // What is left is the FP64 pipe for the DNS update (five operations a cell,
 // 2 cells a clock: 18 us), the conversions of 2 x nh values and the taps.
-constexpr int BX_BITS = 54, BX_LOW = 27, BX_MAX_TAPS = 512;
+constexpr int BX_BITS = 54, BX_LOW = 27, BX_MAX_TAPS = 512, BX_WEAK = 7;
 
 __device__ __forceinline__ Fx as_fx(int2 v) { return {v.x, v.y}; }
 __device__ __forceinline__ int2 as_int2(Fx v) { return make_int2(v.h, v.l); }
@@ -365,7 +377,7 @@ __device__ __forceinline__ double pow2(int e) { return __hiloint2double((1023 + 
 struct LesStep {
   double dt, dth, dtH;
   int Eu, Es;
-  bool go;
+  bool go, leave;
 };
 
 template <int NC>
@@ -408,6 +420,7 @@ __global__ void __launch_bounds__(BT, 1) advance_les_kernel(AdvanceArgs A) {
     }
     double tt = A.t[s];
     int done = 0;
+    bool leave = false;
     __syncthreads();
     while (tt < A.tstop && done < A.max_steps) {
       // the largest |u| on the integer pipe; the step and the scales by one
@@ -417,6 +430,8 @@ __global__ void __launch_bounds__(BT, 1) advance_les_kernel(AdvanceArgs A) {
       __syncthreads();
       if (warp == 0) {
         unsigned long long q = lane < BT / 32 ? wmax[lane] : 0ull;
+        // exponent of the smallest of the warps' maxima (full ones, not zero)
+        const unsigned low = __reduce_min_sync(0xffffffffu, q && (lane + 1) * 32 * NC <= g.nh ? (unsigned)(q >> 52) : ~0u >> 1);
         for (int o = 16; o > 0; o >>= 1) q = max(q, __shfl_xor_sync(0xffffffffu, q, o));
         const double m = from_mag_bits<double>(q);
         double dt;
@@ -425,12 +440,16 @@ __global__ void __launch_bounds__(BT, 1) advance_les_kernel(AdvanceArgs A) {
         // would leave the doubles: values below 2^-955 count as zero, above
         // 2^1000 the DNS overflows and the next step stops)
         if (lane == 0) {
+          const bool out = go && m > 0.0 && low + BX_WEAK < (unsigned)(q >> 52);
           step = {go ? dt : 0.0, dt * g.ih, dt * g.iH, clamp_exponent(exponent_above(m)),
-                  clamp_exponent(exponent_above((0.5 * m + 2.0 * g.vh) * m * (1.0 + 0x1p-40))), go};
+                  clamp_exponent(exponent_above((0.5 * m + 2.0 * g.vh) * m * (1.0 + 0x1p-40))), go && !out, out};
         }
       }
       __syncthreads();
-      if (!step.go) break;
+      if (!step.go) {
+        leave = step.leave;
+        break;
+      }
       const double dt = step.dt, dth = step.dth, dtH = step.dtH;
       const int Eu = step.Eu, Es = step.Es;
       const int ku = (BX_BITS - Eu) << 20, ks = (BX_BITS - Es) << 20;
@@ -529,6 +548,9 @@ __global__ void __launch_bounds__(BT, 1) advance_les_kernel(AdvanceArgs A) {
     if (tid == 0) {
       A.t[s] = tt;
       A.steps[s] += done;
+      A.left[s] = leave;
+      A.left[g.ns + s] = done;
+      if (leave) atomicOr(A.err, 2);
     }
     __syncthreads();
   }
@@ -1006,20 +1028,24 @@ int dalloc(T** p, size_t count) {
 
 void free_les(exc_burgers* b) {
   cudaFree(b->wd); cudaFree(b->wl); cudaFree(b->v); cudaFree(b->tmp);
-  cudaFree(b->smag); cudaFree(b->tsm); cudaFree(b->ssm);
+  cudaFree(b->smag); cudaFree(b->tsm); cudaFree(b->ssm); cudaFree(b->left);
   b->wd = b->wl = b->v = b->tmp = b->smag = b->tsm = nullptr;
-  b->ssm = nullptr;
+  b->ssm = b->left = nullptr;
   b->les_on = b->smag_on = false;
   b->nH = b->comp = b->a = b->Rd = b->Rl = 0;
 }
 
-int check_flag(exc_burgers* b) {
-  int f = 0;
-  cudaError_t e = cudaMemcpyAsync(&f, b->err, sizeof(int), cudaMemcpyDeviceToHost, b->st);
+int read_flag(exc_burgers* b, int* f) {
+  cudaError_t e = cudaMemcpyAsync(f, b->err, sizeof(int), cudaMemcpyDeviceToHost, b->st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->st);
   if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
-  if (f) {
-    cudaMemsetAsync(b->err, 0, sizeof(int), b->st);
+  return EXC_OK;
+}
+
+// Clears the flags read; an error if a sample stopped.
+int clear_flag(exc_burgers* b, int f) {
+  if (f) cudaMemsetAsync(b->err, 0, sizeof(int), b->st);
+  if (f & 1) {
     set_last_error("non-finite Burgers velocity or collapsed time step");
     return EXC_ERR_NONFINITE;
   }
@@ -1230,7 +1256,8 @@ int exc_burgers_les_setup(exc_burgers* b, int nH, double delta_ratio, int filter
   }
   const size_t M = (size_t)b->ns * nH;
   if (dalloc(&b->wd, wd.size()) || dalloc(&b->wl, wl.size()) || dalloc(&b->v, 8 * M) || dalloc(&b->tmp, 5 * M) ||
-      dalloc(&b->smag, M) || dalloc(&b->tsm, b->ns) || dalloc(&b->ssm, b->ns)) {
+      dalloc(&b->smag, M) || dalloc(&b->tsm, b->ns) || dalloc(&b->ssm, b->ns) ||
+      dalloc(&b->left, 2 * (size_t)b->ns)) {
     free_les(b);
     return EXC_ERR_OOM;
   }
@@ -1269,17 +1296,28 @@ int exc_burgers_advance(exc_burgers* b, double tstop, double cfl, int scheme, in
   A.acc = b->scr + (size_t)b->nh * b->ns;
   A.err = b->err;
   const size_t sm = sample_smem(A.g);
-  const void* fn = b->les_on ? (2 * b->Rd + 1 < BX_MAX_TAPS ? les_kernel(b->nh)
-                                                            : (const void*)advance_kernel<true, false>)
-                             : scheme == EXC_BURGERS_RK4 ? (const void*)advance_kernel<false, true>
-                                                         : (const void*)advance_kernel<false, false>;
-  if (allow_smem(fn, sm) != cudaSuccess) { cudaGetLastError(); set_last_error("shared memory opt-in failed"); return EXC_ERR_CUDA; }
-  const int grid = grid_for(fn, sm, b->ns);
-  void* args[] = {&A};
-  cudaLaunchKernel(fn, dim3(grid), dim3(BT), args, sm, b->st);
-  int rc = launch_err(b);
-  if (rc) return rc;
-  rc = check_flag(b);
+  auto launch = [&](const void* fn) {
+    if (allow_smem(fn, sm) != cudaSuccess) { cudaGetLastError(); set_last_error("shared memory opt-in failed"); return (int)EXC_ERR_CUDA; }
+    void* args[] = {&A};
+    cudaLaunchKernel(fn, dim3(grid_for(fn, sm, b->ns)), dim3(BT), args, sm, b->st);
+    return launch_err(b);
+  };
+  int rc, f = 0;
+  if (b->les_on && 2 * b->Rd + 1 < BX_MAX_TAPS) {
+    A.left = b->left;
+    rc = launch(les_kernel(b->nh));
+    if (!rc) rc = read_flag(b, &f);
+    if (!rc && (f & 2)) {  // the samples it left, to the end of the call
+      rc = launch((const void*)advance_kernel<true, false>);
+      if (!rc) rc = read_flag(b, &f);
+    }
+  } else {
+    rc = launch(b->les_on ? (const void*)advance_kernel<true, false>
+                : scheme == EXC_BURGERS_RK4 ? (const void*)advance_kernel<false, true>
+                                            : (const void*)advance_kernel<false, false>);
+    if (!rc) rc = read_flag(b, &f);
+  }
+  if (!rc) rc = clear_flag(b, f);
   if (rc) return rc;
   if (steps_max) return max_steps_of(b, steps_max);
   return EXC_OK;
@@ -1421,7 +1459,9 @@ int exc_burgers_smagorinsky_solve(exc_burgers* b, double theta, double tstop, do
   int rc = launch_err(b);
   if (rc) return rc;
   b->smag_on = true;
-  rc = check_flag(b);
+  int f = 0;
+  rc = read_flag(b, &f);
+  if (!rc) rc = clear_flag(b, f);
   if (rc) return rc;
   if (steps_max) {
     std::vector<int> s(b->ns);

@@ -41,7 +41,7 @@ constexpr int SEP_THREADS = 256;
 
 // Rows of n cells and `pad` ghosts on either side that an x-pass CTA stages
 // beside its static words in the default 48 KB of shared memory.
-constexpr size_t SEP_STATIC = SEP_THREADS / 32 * sizeof(unsigned);
+constexpr size_t SEP_STATIC = 2 * (SEP_THREADS / 32) * sizeof(unsigned);
 constexpr size_t sep_row_bytes(int n, int pad) { return (size_t)(n + 2 * pad) * sizeof(double); }
 constexpr int sep_rows(int n, int pad) {
   const int rows = (int)((48 * 1024 - SEP_STATIC) / sep_row_bytes(n, pad));
@@ -63,7 +63,7 @@ struct XVar {
 // Fixed-point form of the x pass: values as 57-bit integers below the CTA's
 // largest, weights below their list's largest, sums of at most MAX_TAPS
 // products below 2^63 (halves of 2^28: 40 x 2^57 for the two middle products).
-constexpr int SX_BITS = 57, SX_LOW = 29;
+constexpr int SX_BITS = 57, SX_LOW = 29, SX_WEAK = 7;
 static_assert(2 * (long long)MAX_TAPS < (1LL << (63 - 2 * (SX_BITS - SX_LOW))), "sums fit");
 
 struct XArgs {
@@ -118,40 +118,58 @@ __device__ __forceinline__ double sep_value(const XArgs& A, int src, int x, int 
 // Along x.  A CTA stages `rows` rows of one source with ghosts, then applies
 // every tap list of that source: in FP64, or with the values turned into
 // integers in place (each word by the thread that wrote it) and the sums on the
-// integer pipe (fixed.cuh), one rounding each.  A CTA with a non-finite value
-// or outside the exponents the scales can hold stays in FP64.
+// integer pipe (fixed.cuh), one rounding each.  A CTA stays in FP64 with a
+// non-finite value, outside the exponents the scales can hold, or where 32 words
+// of a row, not all zero, are below 2^-SX_WEAK of the largest: the scale would cost
+// them more than its four spare bits and three (three CTAs in a thousand of a
+// velocity field's quadratic stresses, none of the velocity's).
 // Fixed point pays from about three products a fine cell on (the conversion is
 // some 40 integer instructions a cell): four steps of 250^3, ratio 5, Gaussian 30.5
 // -> 27.0 ms, 240^3, ratio 3, Gaussian 38.2 -> 36.6; without one (5 and 3 taps)
 // 22.9 / 23.3 and 31.2 / 31.6, which stay in FP64.
 __global__ void __launch_bounds__(SEP_THREADS) sep_x_kernel(const __grid_constant__ XArgs A) {
   extern __shared__ double row[];
-  __shared__ unsigned wmax[SEP_THREADS / 32];
-  static_assert(sizeof(wmax) == SEP_STATIC, "counted by sep_rows");
+  __shared__ unsigned wmax[SEP_THREADS / 32], wmin[SEP_THREADS / 32];
+  static_assert(sizeof(wmax) + sizeof(wmin) == SEP_STATIC, "counted by sep_rows");
   const int n = A.n, m = A.m, c = A.c, pitch = n + 2 * A.pad;
   const int src = A.src[blockIdx.y];
   const int nn = n * n;
   const int r0 = blockIdx.x * A.rows;
   const int rows = min(A.rows, nn - r0);
-  unsigned top = 0;  // largest high word of a magnitude
-  for (int t = threadIdx.x; t < rows * pitch; t += SEP_THREADS) {
-    const int r = t / pitch;
-    const int z = (r0 + r) / n, y = r0 + r - z * n;
-    int x = t - r * pitch - A.pad;
-    while (x < 0) x += n;
-    while (x >= n) x -= n;
-    const double q = sep_value(A, src, x, y, z);
-    row[t] = q;
-    top = max(top, (unsigned)__double2hiint(q) & 0x7fffffffu);
+  // largest high word of a magnitude, and the smallest of the largest ones of 32
+  // words that are not all zero
+  unsigned top = 0, low = 0x7fffffffu;
+  for (int t0 = 0; t0 < rows * pitch; t0 += SEP_THREADS) {
+    const int t = t0 + threadIdx.x;
+    unsigned hi = 0;
+    if (t < rows * pitch) {
+      const int r = t / pitch;
+      const int z = (r0 + r) / n, y = r0 + r - z * n;
+      int x = t - r * pitch - A.pad;
+      while (x < 0) x += n;
+      while (x >= n) x -= n;
+      const double q = sep_value(A, src, x, y, z);
+      row[t] = q;
+      hi = (unsigned)__double2hiint(q) & 0x7fffffffu;
+    }
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    top = max(top, hi);
+    if (hi) low = min(low, hi);
   }
   const int v0 = A.first[blockIdx.y], vn = A.count[blockIdx.y];
   if (A.fixed[blockIdx.y]) {
-    for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
-    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = top;
+    if ((threadIdx.x & 31) == 0) {
+      wmax[threadIdx.x >> 5] = top;
+      wmin[threadIdx.x >> 5] = low;
+    }
     __syncthreads();
-    for (int w = 0; w < SEP_THREADS / 32; ++w) top = max(top, wmax[w]);
+    for (int w = 0; w < SEP_THREADS / 32; ++w) {
+      top = max(top, wmax[w]);
+      low = min(low, wmin[w]);
+    }
     const int E = (int)(top >> 20) - 1022;  // |value| < 2^E
-    if (E > -800 && E < 800) {
+    // the factor of the sums is 2^(E - 256) at the least: a normal double
+    if (E > -700 && E < 800 && (low >> 20) + SX_WEAK >= top >> 20) {
       int2* const xi = reinterpret_cast<int2*>(row);
       const int kexp = (SX_BITS - E) << 20;
       for (int t = threadIdx.x; t < rows * pitch; t += SEP_THREADS) {

@@ -77,8 +77,13 @@ __host__ __device__ __forceinline__ int gen_xs(const GenLine& l) { return l.n1 *
 // the first x pass leaves the largest biased exponent of its right-hand side per
 // CTA, the first y pass folds them into a shift, 0 for right-hand sides between
 // 2^-60 and 2^80 (every correction then stays within the floats).  With another
-// shift the first solve's correction is dropped (its input may not have fitted)
-// and the two that follow work on residuals scaled by 2^-shift.
+// shift the two solves that follow work on residuals scaled by 2^-shift, and the
+// first correction, of the unscaled input, is taken to their units.  Where it is
+// small its smallest parts may have been flushed, which the next ones make up for;
+// above 2^GEN_FIRST_MAX a spectrum of n^3 of them might not fit a float, and below
+// the smallest float there is none: then two corrections leave the pressure
+// 3e-13 off instead of 1e-15.
+constexpr int GEN_FIRST_MIN = -126, GEN_FIRST_MAX = 95;
 struct GenRange {
   int* top = nullptr;    // the CTAs' exponents, then the shift
   int n = 0;             // CTAs
@@ -509,11 +514,13 @@ gc2r_kernel(cplx<T>* g, GenLine ln, int n, int rw, int P, const cplx<T>* __restr
   } else if constexpr (sizeof(T) == 4) {
     const int shift = d.range.shift();
     if (d.mode == GEN_MIX_Q) {
-      const bool drop = d.first && shift;
+      const bool keep = shift >= GEN_FIRST_MIN && shift <= GEN_FIRST_MAX;
+      const float unit = !d.first || !shift ? 1.0f : keep ? __int_as_float((127 - shift) << 23) : 0.0f;
       for (int t = threadIdx.x; t < total; t += GEN_THREADS) {
         int m, row;
         const C v = word(t, m, row);
-        reinterpret_cast<float2*>(d.q + row * n)[m] = drop ? make_float2(0.0f, 0.0f) : make_float2(f32_flush(v.x), f32_flush(v.y));
+        reinterpret_cast<float2*>(d.q + row * n)[m] = unit != 0.0f ? make_float2(f32_flush(v.x * unit), f32_flush(v.y * unit))
+                                                                   : make_float2(0.0f, 0.0f);
       }
     } else {
       const bool rm = d.mean != nullptr;

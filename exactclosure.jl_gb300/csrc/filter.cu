@@ -295,12 +295,13 @@ int filtered_stress(int n, int c, double l, double visc, const double* fdelta, i
 // order, so the result is bit-reproducible.
 // ---------------------------------------------------------------------------
 // Sum of K doubles on the integer pipe (an FP64 addition holds the FP64 pipe of
-// an SM for 16 cycles a warp): each value as a 53 + UP bit integer below the
-// largest one's exponent, the sum exact in 64 bits, rounded once.  Values near
+// an SM for 16 cycles a warp): each value rounded to a 53 + UP bit integer below
+// the largest one's exponent, the integers' sum exact in 64 bits and rounded
+// once; off by at most K 2^-59 of the largest value and half a unit.  Values near
 // the ends of the exponent range and non-finite ones are added in order.
 template <int K>
 __device__ __forceinline__ double sum_fixed(const double (&v)[K]) {
-  static_assert(K <= 32, "the sum of K integers below 2^(53 + UP) fits");
+  static_assert(K < 32, "the sum of K integers up to 2^(53 + UP) fits");
   constexpr int UP = 5;
   unsigned top = 0;
 #pragma unroll
@@ -317,11 +318,12 @@ __device__ __forceinline__ double sum_fixed(const double (&v)[K]) {
   for (int i = 0; i < K; ++i) {
     const unsigned hi = (unsigned)__double2hiint(v[i]), lo = (unsigned)__double2loint(v[i]);
     const unsigned mh = (hi & 0xfffffu) | 0x100000u;
-    const unsigned long long m = ((unsigned long long)__funnelshift_l(lo, mh, UP) << 32) | (lo << UP);
+    // one bit more for the rounding
+    const unsigned long long m = ((unsigned long long)__funnelshift_l(lo, mh, UP + 1) << 32) | (lo << (UP + 1));
     unsigned long long t;
     asm("shr.u64 %0, %1, %2;" : "=l"(t) : "l"(m), "r"(e - (int)((hi >> 20) & 0x7ffu)));
     const long long s = (int)hi >> 31;  // 0 or -1
-    sum += ((long long)t ^ s) - s;
+    sum += ((long long)((t + 1) >> 1) ^ s) - s;
   }
   // the unit: 2^(e - 1023 - 52 - UP)
   return (double)sum * __hiloint2double((e - 52 - UP) << 20, 0);

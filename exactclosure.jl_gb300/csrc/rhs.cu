@@ -392,7 +392,9 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
 // five of the largest value's converts exactly; smaller ones round to 2^-58
 // of the scale.  E follows the planes: it is the exponent of the largest
 // value of the three planes held plus one, kept while the next plane fits and
-// is not much smaller, else the planes are loaded and converted again.
+// is not much smaller, else the planes are loaded and converted again.  Every
+// `block` planes of the grid it starts afresh, so that a cell's bits depend on
+// the field alone: a launch gives each CTA one block or several.
 //
 // Arithmetic.  With S = 2 visc/h (an integer in the same scale), A = u_i +
 // u_i(+e_j) - 2S, B = u_j + u_j(+e_i) - 2S,
@@ -494,7 +496,7 @@ constexpr size_t FIXED_SMEM = sizeof(FixedSmem) + 128;
 template <bool DOADD>
 __global__ void __launch_bounds__(FXTHREADS, FX_CTAS)
 rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u, double* __restrict__ du, SlotBatch sb,
-                 int zblocks, int ptz, const __grid_constant__ CUtensorMap umap, int have_map) {
+                 int zblocks, int ptz, int block, const __grid_constant__ CUtensorMap umap, int have_map) {
   chain_wait();
   using T = double;
   constexpr int NC = FXC;
@@ -839,7 +841,8 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     const unsigned m[3] = {held_max(0), held_max(1), held_max(2)};
     const unsigned mx = max(m[0], max(m[1], m[2]));
     const int En = exponent_for(mx);
-    if (mx >= 0x7fe00000u || En > E || En < E - 2) {
+    const int down = (kz + 1) % block == 0 ? 0 : 2;  // a block starts with its own exponent
+    if (mx >= 0x7fe00000u || En > E || En < E - down) {
       restart(z + 1);
       continue;
     }
@@ -1203,16 +1206,16 @@ static bool field_tensor_map(const T* u, int n, int nslots, const SlotBatch& sb,
              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Planes per CTA (cmin to 32): the fewest waves of resident CTAs (`per_sm` per
+// Planes per CTA (cmin to 32, a multiple of `mult`): the fewest waves of resident CTAs (`per_sm` per
 // SM) times the planes each CTA walks plus `start` for its start (three planes
 // loaded, the previous plane's part), ties to more planes -- so small grids and
-// single solves still fill the GPU without a nearly empty last wave.  The split
-// changes no cell's arithmetic.  Returns the CTAs of the launch.
+// single solves still fill the GPU without a nearly empty last wave.  Returns
+// the CTAs of the launch.
 static long long zsplit(int n, int nslots, long long columns, int per_sm, int cmin, int start, int& ptz,
-                        int& zblocks) {
+                        int& zblocks, int mult = 1) {
   const long long slots = (long long)per_sm * 152;
   long long best = -1;
-  for (int c = 32; c >= cmin; --c) {
+  for (int c = 32 / mult * mult; c >= cmin; c -= mult) {
     const int zb = (n + c - 1) / c;
     const long long waves = (columns * zb * nslots + slots - 1) / slots;
     if (best < 0 || waves * (c + start) < best) {
@@ -1225,13 +1228,16 @@ static long long zsplit(int n, int nslots, long long columns, int per_sm, int cm
 }
 
 // FP64: the fixed-point sweep, one plane per CTA and up (a 32^3 grid takes 64
-// CTAs of one plane: 10 us, 16 us with four).
+// CTAs of one plane: 10 us, 16 us with four).  A block of planes with one exponent
+// is what a CTA has in a launch of one field, and the CTAs of a batch take
+// multiples of it: a field's bits are the same alone and in any batch.
 template <>
 cudaError_t launch_rhs<double>(int n, double h, double visc, const double* u, double* du, bool doadd, cudaStream_t st,
                                const SlotBatch& sb, int nslots) {
-  int ptz, zblocks;
+  int block, ptz, zblocks;
   dim3 grid((n + PTX - 1) / PTX, (n + FXY - 1) / FXY, 1);
-  zsplit(n, nslots, (long long)grid.x * grid.y, FX_CTAS, 1, 2, ptz, zblocks);
+  zsplit(n, 1, (long long)grid.x * grid.y, FX_CTAS, 1, 2, block, zblocks);
+  zsplit(n, nslots, (long long)grid.x * grid.y, FX_CTAS, block, 2, ptz, zblocks, block);
   grid.z = zblocks * nslots;
   // the field as (x, y, z, slot * 3 + component), boxes of one plane of the
   // three components
@@ -1242,11 +1248,11 @@ cudaError_t launch_rhs<double>(int n, double h, double visc, const double* u, do
   const cuuint32_t box[4] = {FXROW, FXBY, 1, 3};
   const int have = (nslots == 1 || sb.ustride == 3 * N) && (reinterpret_cast<uintptr_t>(u) & 15) == 0 && n >= FXROW &&
                    encode_tiled_map(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, u, dims, strides, box);
-  const dim3 block(PTX, FXW);
+  const dim3 threads(PTX, FXW);
   if (doadd)
-    chain(rhs_fixed_kernel<true>, grid, block, FIXED_SMEM, st)(n, 1.0 / h, visc, u, du, sb, zblocks, ptz, map, have);
+    chain(rhs_fixed_kernel<true>, grid, threads, FIXED_SMEM, st)(n, 1.0 / h, visc, u, du, sb, zblocks, ptz, block, map, have);
   else
-    chain(rhs_fixed_kernel<false>, grid, block, FIXED_SMEM, st)(n, 1.0 / h, visc, u, du, sb, zblocks, ptz, map, have);
+    chain(rhs_fixed_kernel<false>, grid, threads, FIXED_SMEM, st)(n, 1.0 / h, visc, u, du, sb, zblocks, ptz, block, map, have);
   return cudaGetLastError();
 }
 

@@ -435,8 +435,9 @@ static int tune_chunk(exc_server* sv, Chunk<T>* ck) {
   cudaEventCreate(&b);
   // candidates: the register-resident passes (where the grid has a plan) and
   // the Stockham passes over the tile shapes above; a run-time plan measured
-  // faster at every size it covers, and alone it gives a solve the case path's
-  // bits whatever the batch
+  // faster at every size it covers.  Either gives a solve the same bits whatever
+  // the batch; an FP64 case has them too below 84^3 and at 96^3, where it does not
+  // solve in mixed precision
   std::vector<Tuned> cands;
   if (ck->ps.twl_n && ck->ps.twl_h) cands.push_back({0, 0, 0});
   if (!ck->ps.gen)

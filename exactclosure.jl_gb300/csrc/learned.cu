@@ -35,21 +35,43 @@ constexpr int CONV_THREADS = 128;
 constexpr int OUTP = 16;  // padded output channels
 constexpr int OUTS = 4;   // words of a voxel in the network's output (the three channels and a zero)
 
-// x * s rounded to float for a factor s given in 64 bits, as two floats on the
-// FP32 pipe: within 2^-24 ulp of the rounded FP64 product, which took three
-// FP64 instructions of 64 FP32 ones' time each.  Factors a float cannot hold
-// (`fast` false) and non-finite x take the plain forms.
+// x * s rounded to float for a factor s given in 64 bits: the bits of the rounded
+// FP64 product, whose three FP64 instructions take 64 FP32 ones' time each, by the
+// factor as two floats.  The product then lies within 2^-24 ulp of the exact one,
+// so where it is that close to the middle of two floats (or at a power of two,
+// whose neighbours are not evenly spaced) the FP64 product decides.  So it does for
+// factors a float cannot hold (`fast` false) and for values whose result would be
+// outside 2^-90 to 2^126, zero excepted.
 struct Scale {
   float h, l;
   bool fast;
+  unsigned lo, span;  // magnitude bits of the values inside
   double s;
-  explicit Scale(double v) : h((float)v), l((float)(v - (double)(float)v)), fast(std::fabs(v) > 0x1p-64 && std::fabs(v) < 0x1p64), s(v) {}
+  explicit Scale(double v) : h((float)v), l((float)(v - (double)(float)v)), fast(std::fabs(v) > 0x1p-64 && std::fabs(v) < 0x1p64), lo(0), span(0), s(v) {
+    if (!fast) return;
+    const float a = (float)std::fmax(0x1p-90 / std::fabs(v), 0x1p-126), b = (float)std::fmin(0x1p126 / std::fabs(v), 0x1p127);
+    unsigned hi;
+    std::memcpy(&lo, &a, sizeof lo);
+    std::memcpy(&hi, &b, sizeof hi);
+    span = hi - lo;
+  }
   __device__ __forceinline__ float operator()(float x) const {
-    if (!fast) return (float)((double)x * s);
-    return fabsf(x) <= 3.402823466e38f ? fmaf(x, h, x * l) : x * h;
+    const unsigned a = __float_as_uint(x) & 0x7fffffffu;
+    const float t = x * l, r = fmaf(x, h, t);
+    const unsigned b = __float_as_uint(r);
+    // distance from the middle, in parts of half an ulp of r
+    const float half = __uint_as_float((b & 0x7f800000u) - (24u << 23));
+    const bool middle = fabsf(fabsf(fmaf(x, h, -r) + t) - half) < half * 0x1p-16f || (b & 0x7fffffu) == 0;
+    if (!fast || ((a - lo >= span || middle) && a != 0)) return (float)((double)x * s);
+    return a != 0 ? r : x * h;
   }
   __device__ __forceinline__ float operator()(double x) const { return (float)(x * s); }
 };
+
+// (double)v on the integer pipe, subnormal values too (f32_to_f64 makes those zero)
+__device__ __forceinline__ double widen(float v) {
+  return (__float_as_uint(v) & 0x7fffffffu) - 1u < 0x007fffffu ? (double)v : f32_to_f64(v);
+}
 
 __device__ __forceinline__ float gelu_f(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_grad_f(float x) {
@@ -1466,7 +1488,7 @@ __global__ void wgrad_fold_kernel(int nchunk, const float* __restrict__ part, fl
   const int i = t >> 2, q = t & 3;
   double s = 0;
   if (i < NET_TAPS * PAIRS)
-    for (int c = q; c < nchunk; c += 4) s += f32_to_f64(part[(long long)c * NET_TAPS * PAIRS + i]);
+    for (int c = q; c < nchunk; c += 4) s += widen(part[(long long)c * NET_TAPS * PAIRS + i]);
   s += __shfl_xor_sync(0xffffffffu, s, 1);
   s += __shfl_xor_sync(0xffffffffu, s, 2);
   if (q == 0 && i < NET_TAPS * PAIRS) dW[i] = (float)s;
@@ -1567,7 +1589,7 @@ __global__ void loss_grad_kernel(long long V, long long N, const float* __restri
       float d = 0.f;
       if (c < 3) d = oc[c] - tscale(tgt[(b * 3 + c) * N + r]);
       if (c < 3) {
-        const double dd = f32_to_f64(d);
+        const double dd = widen(d);
         s = fma(dd, dd, s);
       }
       row[c] = __float2bfloat16(gs * d);

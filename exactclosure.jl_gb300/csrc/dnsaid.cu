@@ -47,7 +47,8 @@ struct exc_dnsaid {
   double* pl = nullptr;    // LES pressure M (paper mode)
   double* dsig = nullptr;  // closure divergence 3M (paper mode)
   double* rc9 = nullptr;   // surface-filtered flux 9M (surface mode)
-  double* uf = nullptr;    // fine-filtered velocity at the classic closure's sample points 18M
+  double* tmp = nullptr;   // dul, sl, sc and dsig, 18M; before the LES need them the fine-filtered velocity
+                           // at the classic closure's sample points
   exc::SepWork sep;        // scratch of the filters
   double t = 0;
   int steps = 0;
@@ -284,12 +285,12 @@ int lockstep(exc_dnsaid* d, double dt) {
   if (!rc) {
     SepTaps taps;
     std::vector<SepTarget> v;
-    classic_targets(d, d->uf, taps, v);
+    classic_targets(d, d->tmp, taps, v);
     velocity_targets(d, false, d->ub, taps, v);
     rc = run_filters(d, taps, v);
   }
   if (rc) return rc;
-  classic_stress_kernel<<<gridsz(M), 256, 0, st>>>(M, d->uf, 1.0 / d->h, d->visc, d->s2);
+  classic_stress_kernel<<<gridsz(M), 256, 0, st>>>(M, d->tmp, 1.0 / d->h, d->visc, d->s2);
   e = cudaGetLastError();
   if (e == cudaSuccess) e = project(&d->psl, d->ub, st);
   if (e != cudaSuccess) return cuda_rc(e);
@@ -440,12 +441,16 @@ int exc_dnsaid_create(const exc_dnsaid_desc* desc, void* stream, exc_dnsaid** ou
   rc = poisson_init(&d->psd, EXC_F64, n, d->l, nullptr);
   if (!rc) rc = poisson_init(&d->psl, EXC_F64, d->m, d->l, nullptr);
   if (!rc) rc = dalloc(&d->u, 3 * N) || dalloc(&d->du, 3 * N) || dalloc(&d->p, N) || dalloc(&d->ub, 3 * M) ||
-                dalloc(&d->dul, 3 * M) || dalloc(&d->sdh, 6 * M) || dalloc(&d->s2, 6 * M) || dalloc(&d->r9, 9 * M) ||
-                dalloc(&d->sl, 6 * M) || dalloc(&d->sc, 6 * M) || dalloc(&d->zero, M) || dalloc(&d->scal, 16) ||
+                dalloc(&d->tmp, 18 * M) || dalloc(&d->sdh, 6 * M) || dalloc(&d->s2, 6 * M) || dalloc(&d->r9, 9 * M) ||
+                dalloc(&d->zero, M) || dalloc(&d->scal, 16) ||
                 dalloc(&d->part, (size_t)SHELL_BLOCKS * 1024 + 2048 + RED_PARTS) || dalloc(&d->spec, spec);
   for (int k = 0; k < 5 && !rc; ++k) rc = dalloc(&d->les[k], 3 * M);
-  if (!rc) rc = dalloc(&d->pl, M) || dalloc(&d->dsig, 3 * M) || dalloc(&d->uf, 18 * M);
+  if (!rc) rc = dalloc(&d->pl, M);
   if (rc) { exc_dnsaid_destroy(d); return rc; }
+  d->dul = d->tmp;
+  d->sl = d->tmp + 3 * M;
+  d->sc = d->tmp + 9 * M;
+  d->dsig = d->tmp + 15 * M;
   cudaMemsetAsync(d->zero, 0, M * sizeof(double), d->st);
   cudaMemsetAsync(d->u, 0, 3 * N * sizeof(double), d->st);
   rc = cuda_rc(cudaGetLastError());
@@ -459,8 +464,8 @@ int exc_dnsaid_destroy(exc_dnsaid* d) {
   if (d->st) cudaStreamSynchronize(d->st); else cudaDeviceSynchronize();
   poisson_free(&d->psd);
   poisson_free(&d->psl);
-  double* bufs[] = {d->u, d->du, d->p, d->ub, d->dul, d->sdh, d->s2, d->r9, d->sl, d->sc, d->zero, d->scal,
-                    d->part, d->spec, d->pl, d->dsig, d->rc9, d->uf};
+  double* bufs[] = {d->u, d->du, d->p, d->ub, d->tmp, d->sdh, d->s2, d->r9, d->zero, d->scal,
+                    d->part, d->spec, d->pl, d->rc9};
   for (double* b : bufs) cudaFree(b);
   sep_free(&d->sep);
   for (double* b : d->les) cudaFree(b);

@@ -21,9 +21,9 @@
 // ms with an x pass of 2.8 ms in FP64 (85 operations per fine cell at the
 // pipe's rate), y 0.7, z 0.3; the step is 6.5 ms now.  Without the Gaussian (5 taps) 10.7 -> 9.8 ms, ratio 3 at 240^3
 // 11.0 -> 10.3, 60^3 1.50 -> 1.22.
-#include <cstring>
-
+#include <algorithm>
 #include <cmath>
+#include <cstring>
 
 #include "fixed.cuh"
 #include "internal.cuh"
@@ -79,6 +79,7 @@ struct XArgs {
   const double* u;
   const double* p;
   int n, m, c, rows;
+  int z0, planes;  // fine planes of the slab, from z0 on, periodic
   int pad;  // ghost cells on either side of a staged row
   double vh;  // visc / h
 };
@@ -133,9 +134,8 @@ __global__ void __launch_bounds__(SEP_THREADS) sep_x_kernel(const __grid_constan
   static_assert(sizeof(wmax) + sizeof(wmin) == SEP_STATIC, "counted by sep_rows");
   const int n = A.n, m = A.m, c = A.c, pitch = n + 2 * A.pad;
   const int src = A.src[blockIdx.y];
-  const int nn = n * n;
   const int r0 = blockIdx.x * A.rows;
-  const int rows = min(A.rows, nn - r0);
+  const int rows = min(A.rows, A.planes * n - r0);
   // largest high word of a magnitude, and the smallest of the largest ones of 32
   // words that are not all zero
   unsigned top = 0, low = 0x7fffffffu;
@@ -144,7 +144,8 @@ __global__ void __launch_bounds__(SEP_THREADS) sep_x_kernel(const __grid_constan
     unsigned hi = 0;
     if (t < rows * pitch) {
       const int r = t / pitch;
-      const int z = (r0 + r) / n, y = r0 + r - z * n;
+      const int zs = (r0 + r) / n, y = r0 + r - zs * n;
+      const int z = A.z0 + zs >= n ? A.z0 + zs - n : A.z0 + zs;
       int x = t - r * pitch - A.pad;
       while (x < 0) x += n;
       while (x >= n) x -= n;
@@ -217,16 +218,16 @@ struct YVar {
 struct YArgs {
   Taps1D taps[SEP_MAX_TAPSETS];
   YVar v[SEP_MAX_YV];
-  int n, m, c;
+  int n, m, c, planes;
 };
 
-// Along y: [z][y][ix] -> [z][iy][ix].  The tap offsets of the y and z passes
-// are reduced to [0, n) on the host, so one comparison wraps them.
+// Along y: [z][y][ix] -> [z][iy][ix] for the slab's planes.  The tap offsets of the
+// y pass are reduced to [0, n) on the host, so one comparison wraps them.
 __global__ void __launch_bounds__(SEP_THREADS) sep_y_kernel(const __grid_constant__ YArgs A) {
   const int n = A.n, m = A.m;
   const YVar V = A.v[blockIdx.y];
   const Taps1D& T = A.taps[V.taps];
-  const long long tot = (long long)n * m * m;
+  const long long tot = (long long)A.planes * m * m;
   const IdxDiv dm(m);
   for (long long g = blockIdx.x * (long long)SEP_THREADS + threadIdx.x; g < tot; g += (long long)gridDim.x * SEP_THREADS) {
     const long long r = dm.div(g);
@@ -251,26 +252,28 @@ struct ZVar {
 struct ZArgs {
   Taps1D taps[SEP_MAX_TAPSETS];
   ZVar v[SEP_MAX_OUT];
-  int n, m, c;
+  int m, c;
+  int i0, count;  // coarse planes of the slab
+  int wrap;       // fine planes after which the slab starts again: n where it holds them all
 };
 
-// Along z: [z][iy][ix] -> [iz][iy][ix].
+// Along z: [z][iy][ix] -> [iz][iy][ix].  Offsets from the slab's first fine plane.
 __global__ void __launch_bounds__(SEP_THREADS) sep_z_kernel(const __grid_constant__ ZArgs A) {
-  const int n = A.n, m = A.m;
+  const int m = A.m;
   const ZVar V = A.v[blockIdx.y];
   const Taps1D& T = A.taps[V.taps];
   const int mm = m * m;
-  const long long tot = (long long)mm * m;
+  const long long tot = (long long)mm * A.count;
   const IdxDiv dmm(mm);
   for (long long g = blockIdx.x * (long long)SEP_THREADS + threadIdx.x; g < tot; g += (long long)gridDim.x * SEP_THREADS) {
     const int iz = (int)dmm.div(g), r = (int)(g - (long long)iz * mm);
     double acc = 0.0, acc2 = 0.0;
     for (int t = 0; t < T.cnt; ++t) {
-      const int q = A.c * iz + T.off[t], z = q >= n ? q - n : q;
+      const int q = A.c * iz + T.off[t], z = q >= A.wrap ? q - A.wrap : q;
       acc = fma(T.w[t], V.in[(long long)z * mm + r], acc);
       if (V.in2) acc2 = fma(T.w[t], V.in2[(long long)z * mm + r], acc2);
     }
-    V.out[g] = acc + acc2;
+    V.out[(long long)A.i0 * mm + g] = acc + acc2;
   }
 }
 
@@ -282,7 +285,6 @@ int sep_reserve(double** p, size_t* have, size_t want) {
   if (cudaMalloc(p, want * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     *p = nullptr;
-    set_last_error("out of device memory (filter scratch)");
     return EXC_ERR_OOM;
   }
   *have = want;
@@ -340,10 +342,37 @@ int sep_filter(SepWork* w, int n, int c, double inv_h, double visc, const SepTap
     set_last_error("too many filters in one batch");
     return EXC_ERR_ARG;
   }
-  const size_t xw = (size_t)n * n * m, yw = (size_t)n * m * m;
-  int rc = sep_reserve(&w->a, &w->na, xv.size() * xw);
-  if (!rc) rc = sep_reserve(&w->b, &w->nb, yv.size() * yw);
-  if (rc) return rc;
+  // The whole grid at once while its scratch stays below SEP_SCRATCH, else slabs of
+  // `count` coarse planes with the fine planes their z taps reach, down to the
+  // memory there is
+  int zlo = 0, zhi = 0;
+  for (const SepTarget& T : targets) {
+    const Taps1D& z = taps.list[T.t[2]];
+    for (int k = 0; k < z.cnt; ++k) {
+      zlo = std::min(zlo, z.off[k]);
+      zhi = std::max(zhi, z.off[k]);
+    }
+  }
+  const size_t plane = xv.size() * n * m + yv.size() * m * m;  // words a fine plane
+  auto planes_of = [&](int count) { return c * (count - 1) + zhi - zlo + 1; };
+  int count = m;
+  bool whole = plane * n * sizeof(double) <= w->limit;
+  while (!whole && count > 1 && plane * planes_of(count) * sizeof(double) > w->limit) count = (count + 1) / 2;
+  for (;; whole = false, count = (count + 1) / 2) {
+    if (planes_of(count) >= n) whole = true;
+    const size_t planes = whole ? n : planes_of(count);
+    if (sep_reserve(&w->a, &w->na, xv.size() * planes * n * m) == EXC_OK &&
+        sep_reserve(&w->b, &w->nb, yv.size() * planes * m * m) == EXC_OK)
+      break;
+    cudaFree(w->a);
+    cudaFree(w->b);
+    w->a = w->b = nullptr;
+    w->na = w->nb = 0;
+    if (count == 1) { set_last_error("out of device memory (filter scratch)"); return EXC_ERR_OOM; }
+  }
+  const int planes = whole ? n : planes_of(count);
+  if (whole) count = m;
+  const size_t xw = (size_t)planes * n * m, yw = (size_t)planes * m * m;
 
   XArgs X{};
   YArgs Y{};
@@ -353,7 +382,8 @@ int sep_filter(SepWork* w, int n, int c, double inv_h, double visc, const SepTap
   for (size_t i = 0; i < taps.list.size(); ++i) {
     X.taps[i] = Y.taps[i] = taps.list[i];
     for (int k = 0; k < Y.taps[i].cnt; ++k) Y.taps[i].off[k] = ((Y.taps[i].off[k] % n) + n) % n;
-    Z.taps[i] = Y.taps[i];
+    Z.taps[i] = whole ? Y.taps[i] : X.taps[i];
+    for (int k = 0; !whole && k < Z.taps[i].cnt; ++k) Z.taps[i].off[k] -= zlo;
     // |w| < 2^we; weights outside the range of the scales stay in FP64
     double top = 0.0;
     for (int k = 0; k < X.taps[i].cnt; ++k) top = std::max(top, std::fabs(X.taps[i].w[k]));
@@ -369,7 +399,9 @@ int sep_filter(SepWork* w, int n, int c, double inv_h, double visc, const SepTap
   }
   X.u = u;
   X.p = p;
-  X.n = Y.n = Z.n = n;
+  X.n = Y.n = n;
+  X.planes = Y.planes = planes;
+  Z.wrap = whole ? n : planes;
   X.m = Y.m = Z.m = m;
   X.c = Y.c = Z.c = c;
   X.vh = visc * inv_h;
@@ -413,9 +445,14 @@ int sep_filter(SepWork* w, int n, int c, double inv_h, double visc, const SepTap
     const size_t b = (cnt + SEP_THREADS - 1) / SEP_THREADS;
     return (unsigned)(b < 152 * 16 ? b : 152 * 16);
   };
-  sep_x_kernel<<<dim3((unsigned)((n * n + rows - 1) / rows), X.nsrc), SEP_THREADS, rows * sep_row_bytes(n, pad), st>>>(X);
-  sep_y_kernel<<<dim3(blocks(yw), (unsigned)yv.size()), SEP_THREADS, 0, st>>>(Y);
-  sep_z_kernel<<<dim3(blocks((size_t)m * m * m), (unsigned)targets.size()), SEP_THREADS, 0, st>>>(Z);
+  for (int i0 = 0; i0 < m; i0 += count) {
+    X.z0 = whole ? 0 : (((c * i0 + zlo) % n) + n) % n;
+    Z.i0 = i0;
+    Z.count = std::min(count, m - i0);
+    sep_x_kernel<<<dim3((unsigned)((planes * n + rows - 1) / rows), X.nsrc), SEP_THREADS, rows * sep_row_bytes(n, pad), st>>>(X);
+    sep_y_kernel<<<dim3(blocks(yw), (unsigned)yv.size()), SEP_THREADS, 0, st>>>(Y);
+    sep_z_kernel<<<dim3(blocks((size_t)m * m * Z.count), (unsigned)targets.size()), SEP_THREADS, 0, st>>>(Z);
+  }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { set_last_error(cudaGetErrorString(e)); return EXC_ERR_CUDA; }
   return EXC_OK;

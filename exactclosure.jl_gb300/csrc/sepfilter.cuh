@@ -27,16 +27,18 @@ struct SepTarget {
 };
 
 // Scratch of the passes, grown to the largest batch asked for and freed by
-// the owner.
+// the owner.  A batch that would take more than `limit` bytes (some 600^3 with
+// ratio 5 for the five LES), or more than there is, goes slab by slab.
 struct SepWork {
-  double* a = nullptr;  // x-filtered sources, n^2 m words each
-  double* b = nullptr;  // xy-filtered ones, n m^2 words each
+  double* a = nullptr;  // x-filtered sources, n m words a fine plane each
+  double* b = nullptr;  // xy-filtered ones, m^2 words a fine plane each
   size_t na = 0, nb = 0;
+  size_t limit = size_t(4) << 30;
 };
 void sep_free(SepWork* w);
 
 // Fills every target from the velocity u (and the pressure p, if a target
-// uses it): three launches for the whole batch.  FP64.
+// uses it): three launches for the whole batch, or for each slab of it.  FP64.
 int sep_filter(SepWork* w, int n, int c, double inv_h, double visc, const SepTaps& taps,
                const std::vector<SepTarget>& targets, const double* u, const double* p, cudaStream_t st);
 

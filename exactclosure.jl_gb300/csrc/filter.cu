@@ -297,7 +297,7 @@ int filtered_stress(int n, int c, double l, double visc, const double* fdelta, i
 // Sum of K doubles on the integer pipe (an FP64 addition holds the FP64 pipe of
 // an SM for 16 cycles a warp): each value rounded to a 53 + UP bit integer below
 // the largest one's exponent, the integers' sum exact in 64 bits and rounded
-// once; off by at most K 2^-59 of the largest value and half a unit.  Values near
+// once; off by at most K 2^-58 of the largest value and half a unit.  Values near
 // the ends of the exponent range and non-finite ones are added in order.
 template <int K>
 __device__ __forceinline__ double sum_fixed(const double (&v)[K]) {

@@ -386,7 +386,7 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
 // in fixed point (fixed.cuh), with more bits than FP64 carries, and rounds once
 // at the end.
 //
-// Fixed point.  All values a CTA holds share one scale 2^(57 - E), |u| + S <
+// Fixed point.  All values a CTA holds share one scale 2^(57 - E), |u| + |S| <
 // 2^E: a velocity becomes an integer U, |U| <= 2^57, split as U = h 2^29 + l
 // with h and l int32 and l in [-2^28, 2^28].  A double whose exponent is within
 // five of the largest value's converts exactly; smaller ones round to 2^-58
@@ -628,10 +628,11 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
   bool small_s = false;
   unsigned below = 0;  // high word of 2^(E - FX_WEAK), 0 where S is above that
   bool slow = false;
-  // E for planes whose largest magnitude has high word mx: above |u| + S
-  // (and above 4S, so that 4S converts); the FP64 path if it is out of range
-  // (in FP32, whose range covers the path's; bounds rounded up)
-  float Sf = 2.0 * visc * inv_h < 1e30 ? __double2float_ru(2.0 * visc * inv_h) : 1e30f;
+  // E for planes whose largest magnitude has high word mx: above |u| + |S|
+  // (and above 4|S|, so that 4S converts; a negative viscosity is taken); the FP64
+  // path if it is out of range (in FP32, whose range covers the path's; bounds
+  // rounded up)
+  float Sf = 2.0 * fabs(visc) * inv_h < 1e30 ? __double2float_ru(2.0 * fabs(visc) * inv_h) : 1e30f;
   asm volatile("" : "+f"(Sf));  // kept, not recomputed on the FP64 pipe
   auto exponent_for = [&](unsigned mx) {
     const unsigned m = mx < 0x39000000u ? 0u : mx >= 0x47000000u ? 0x7f000000u : ((mx - 0x38000000u) << 3) + 8u;
@@ -689,7 +690,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     const unsigned mx = max(m[0], max(m[1], m[2]));
     const double S = 2.0 * visc * inv_h;
     E = exponent_for(mx);
-    slow = mx >= 0x7fe00000u || !(S < 1e300) || E > FX_EMAX || E < FX_EMIN;
+    slow = mx >= 0x7fe00000u || !(fabs(S) < 1e300) || E > FX_EMAX || E < FX_EMIN;
     if (!slow) {
       kexp = (FX_BITS - E) << 20;
       scale = ldexp(-0.25 * inv_h, 2 * FX_LOW + 2 * (E - FX_BITS));

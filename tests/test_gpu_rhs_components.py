@@ -73,3 +73,10 @@ def test_shear_flow(NS, visc, kind):
         u[0] = f[None, :, None]
         err = np.abs(run(NS, u, visc) - exact_rhs(u, visc)).max(axis=(1, 2, 3))
         assert (err <= 2 * 31 * 2.0**-53 * 4 * visc * n * np.abs(f).max() * n * np.array([1, 0, 0])).all(), err
+
+
+@pytest.mark.parametrize("visc", [-1e-4, -1 / 50, -0.1])
+def test_negative_viscosity(NS, visc):
+    """What a time reversal passes; r is its magnitude."""
+    for n in (16, 66):
+        check(NS, np.random.default_rng(n).standard_normal((3, n, n, n)), visc)

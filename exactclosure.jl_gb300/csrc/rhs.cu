@@ -420,11 +420,12 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
 // below it, FP64 form 2.2-2.9e-16 throughout:
 //   k = 0: 0.9e-16   3: 1.3e-16   4: 2.2e-16   5: 4.0e-16   7: 1.5e-15   10: 1e-14
 // So a component that is not zero and with S below 2^-FX_WEAK of the scale
-// in the three planes takes rhs_cell_f64.  S is rounded with them: where it is
-// below 2^-FX_SMALL_S of the scale it stays out of the integers, and the linear
-// term is summed by itself, exactly, and multiplied by S in FP64 (a shear flow
-// u_1(y), whose advection vanishes, is nothing else: ten cells of noise at visc
-// 1e-5 2.9e-14 with S rounded, FP64 form 1.8e-16).
+// in the three planes takes rhs_cell_f64.  S would be rounded with them, or the
+// velocity with a larger S: where |S| is below 2^-FX_SMALL_S of the velocities'
+// scale or above half of it, it stays out of the integers, and the linear term is
+// summed by itself, exactly, and multiplied by S in FP64 (a shear flow u_1(y),
+// whose advection vanishes, is nothing else: ten cells of noise at visc 1e-5
+// 2.9e-14 with S rounded, FP64 form 1.8e-16).
 // The cells whose velocity is below 2^-7 of the tile's largest take rhs_cell_f64
 // too (their error is below the larger cells' in any norm over the tile), and
 // planes with values that are not finite or out of range.
@@ -625,19 +626,27 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
   Fx S2{}, S4{};  // 2S and 4S in fixed point
   int tiny = 0;   // cells whose h words are all below this take the FP64 path
   int weak = 0;   // bits 0-2: components that take it in every cell of the plane
-  bool small_s = false;
+  bool s_out = false;  // S is not among the integers
   unsigned below = 0;  // high word of 2^(E - FX_WEAK), 0 where S is above that
   bool slow = false;
-  // E for planes whose largest magnitude has high word mx: above |u| + |S|
-  // (and above 4|S|, so that 4S converts; a negative viscosity is taken); the FP64
-  // path if it is out of range (in FP32, whose range covers the path's; bounds
-  // rounded up)
+  // |S| in FP32, whose range covers the fixed-point path's, rounded up (a
+  // negative viscosity is taken)
   float Sf = 2.0 * fabs(visc) * inv_h < 1e30 ? __double2float_ru(2.0 * fabs(visc) * inv_h) : 1e30f;
   asm volatile("" : "+f"(Sf));  // kept, not recomputed on the FP64 pipe
-  auto exponent_for = [&](unsigned mx) {
-    const unsigned m = mx < 0x39000000u ? 0u : mx >= 0x47000000u ? 0x7f000000u : ((mx - 0x38000000u) << 3) + 8u;
-    const float bound = fmaxf(__fadd_ru(__uint_as_float(m), Sf), 4.0f * Sf);
+  // E for planes whose largest magnitude has high word mx, bounds rounded up:
+  // above |u|, with S among the integers above |u| + |S| and 4|S|
+  auto exponent_for = [&](unsigned mx, bool out) {
+    if (mx == 0) return FX_EMIN;
+    const float m = __uint_as_float(mx < 0x39000000u ? 0u : mx >= 0x47000000u ? 0x7f000000u : ((mx - 0x38000000u) << 3) + 8u);
+    const float bound = out ? m : fmaxf(__fadd_ru(m, Sf), 4.0f * Sf);
     return (int)(__float_as_uint(bound) >> 23) - 126;
+  };
+  // and whether S stays out of them, for planes taken afresh
+  auto fresh = [&](unsigned mx, bool& out) {
+    const int e = exponent_for(mx, true);
+    // |u| < 2^e: S above 2^(e - 1), which may be above |u|, or far below
+    out = Sf > __int_as_float((e + 126) << 23) || Sf < __int_as_float((e - FX_SMALL_S + 127) << 23);
+    return out ? e : exponent_for(mx, false);
   };
   auto fxat = [&](int buf, int c, int row, int col) {
     const double v = sm.u[buf][(c * FXBY + row) * FXROW + col];
@@ -689,14 +698,13 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     const unsigned m[3] = {held_max(0), held_max(1), held_max(2)};
     const unsigned mx = max(m[0], max(m[1], m[2]));
     const double S = 2.0 * visc * inv_h;
-    E = exponent_for(mx);
+    E = fresh(mx, s_out);
     slow = mx >= 0x7fe00000u || !(fabs(S) < 1e300) || E > FX_EMAX || E < FX_EMIN;
     if (!slow) {
       kexp = (FX_BITS - E) << 20;
       scale = ldexp(-0.25 * inv_h, 2 * FX_LOW + 2 * (E - FX_BITS));
-      small_s = Sf < __int_as_float((E - FX_SMALL_S + 127) << 23);
-      if (small_s && tid == 0) sm.by_s = ldexp(-0.25 * inv_h * S, E - FX_BITS);
-      const Fx s = small_s ? Fx{0, 0} : fx_from_double<FX_BITS, FX_LOW>(4.0 * S, kexp);
+      if (s_out && tid == 0) sm.by_s = ldexp(-0.25 * inv_h * S, E - FX_BITS);
+      const Fx s = s_out ? Fx{0, 0} : fx_from_double<FX_BITS, FX_LOW>(4.0 * S, kexp);
       // 4S to a multiple of four units, so that S and 2S are the same S
       const long long s4 = (((long long)s.h << FX_LOW) + s.l + 2) >> 2 << 2;
       const long long s2 = s4 >> 1;
@@ -732,9 +740,9 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     if (z >= n) break;  // uniform across the CTA
     const bool more = kz + 1 < ptz && z + 1 < n;
     if (more && !slow) load_plane(pre, wrapm(z + 2));
-    auto cells = [&](auto s_is_small) {
-      constexpr bool SMALL_S = decltype(s_is_small)::value;
-      const Fx s2 = SMALL_S ? Fx{0, 0} : S2, s4 = SMALL_S ? Fx{0, 0} : S4;
+    auto cells = [&](auto s_outside) {
+      constexpr bool S_OUT = decltype(s_outside)::value;
+      const Fx s2 = S_OUT ? Fx{0, 0} : S2, s4 = S_OUT ? Fx{0, 0} : S4;
 #pragma unroll
       for (int i = 0; i < NC; ++i) {
         const int r = NC * ty + 1 + i, gy = y0 + NC * ty + i;
@@ -773,7 +781,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
             fx_mac(s, A13, B13);
             fx_mac(s, s2 - a - pw1[i], pb13[i]);
             o1 = fx_to_double<FX_LOW>(s, scale);
-            if constexpr (SMALL_S)
+            if constexpr (S_OUT)
               o1 = fma(sm.by_s, linear((a - axm) + (b - bym), dz3 + (a - axm), (a - aym) + (a - pw1[i]), axp - axm,
                        (ayp - aym) + (b + bxp) - (bym + bxpym), (azp - pw1[i]) + (c + cxp) - (pb13[i] + s2)), o1);
           }
@@ -787,7 +795,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
             fx_mac(s, A23, B23);
             fx_mac(s, s2 - b - pw2[i], pb23[i]);
             o2 = fx_to_double<FX_LOW>(s, scale);
-            if constexpr (SMALL_S)
+            if constexpr (S_OUT)
               o2 = fma(sm.by_s, linear((a - axm) + (b - bym), dz3 + (b - bxm), (b - bym) + (b - pw2[i]), byp - bym,
                        (a + ayp) - (axm + axmyp) + (bxp - bxm), (bzp - pw2[i]) + (c + cyp) - (pb23[i] + s2)), o2);
           }
@@ -801,7 +809,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
             fx_mac(s, A23, B23);
             fx_mac(s, s2 - bym - bymzp, cym + c - s2);
             o3 = fx_to_double<FX_LOW>(s, scale);
-            if constexpr (SMALL_S)
+            if constexpr (S_OUT)
               o3 = fma(sm.by_s, linear((a - axm) + (b - bym), dz3 + (c - cxm), (c - cym) + dz3, czp - pw3[i],
                        (a + azp) - (axm + axmzp) + (cxp - cxm), (b + bzp) - (bym + bymzp) + (cyp - cym)), o3);
           }
@@ -829,7 +837,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
       }
     };
     // two copies: the linear term by itself would cost the usual one registers
-    if (small_s) cells(std::true_type());
+    if (s_out) cells(std::true_type());
     else cells(std::false_type());
     if (!more) break;
     if (slow) {
@@ -841,9 +849,12 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     __syncthreads();
     const unsigned m[3] = {held_max(0), held_max(1), held_max(2)};
     const unsigned mx = max(m[0], max(m[1], m[2]));
-    const int En = exponent_for(mx);
-    const int down = (kz + 1) % block == 0 ? 0 : 2;  // a block starts with its own exponent
-    if (mx >= 0x7fe00000u || En > E || En < E - down) {
+    bool out;
+    const int Ef = fresh(mx, out);
+    const int En = out == s_out ? Ef : exponent_for(mx, s_out);
+    // a block starts with its own scale
+    const bool other = (kz + 1) % block == 0 ? Ef != E || out != s_out : En < E - 2;
+    if (mx >= 0x7fe00000u || En > E || other) {
       restart(z + 1);
       continue;
     }

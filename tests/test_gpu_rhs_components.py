@@ -80,3 +80,22 @@ def test_negative_viscosity(NS, visc):
     """What a time reversal passes; r is its magnitude."""
     for n in (16, 66):
         check(NS, np.random.default_rng(n).standard_normal((3, n, n, n)), visc)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-20])
+@pytest.mark.parametrize("visc", [1 / 500, 0.02, 0.1, 10.0, -10.0, 1e6])
+def test_viscosity_beside_a_weak_velocity(NS, visc, scale):
+    """2 visc/h about the velocity and far above it."""
+    for n in (16, 40, 66):
+        u = np.random.default_rng(n).standard_normal((3, n, n, n)) * scale
+        u[:, n // 2:] *= 0.01
+        check(NS, u, visc)
+
+
+def test_still_planes(NS):
+    """Zeros beside a moving half: no scale of their own."""
+    for n in (16, 66):
+        u = np.random.default_rng(n).standard_normal((3, n, n, n))
+        u[:, 2: n - 3] = 0
+        check(NS, u, 1 / 500)
+        assert (run(NS, u, 1 / 500)[:, 3: n - 4] == 0).all()

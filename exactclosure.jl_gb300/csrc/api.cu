@@ -117,6 +117,11 @@ int exc_poisson_create(int precision, int n, double l, exc_poisson** out) {
   if (rc) return rc;
   exc_poisson* ps = new exc_poisson();
   rc = poisson_init(ps, precision, n, l, nullptr);
+  if (rc == EXC_ERR_OOM) {
+    cudaGetLastError();
+    *ps = exc_poisson();
+    rc = poisson_init(ps, precision, n, l, nullptr, false);
+  }
   if (rc) { delete ps; return rc; }
   *out = ps;
   return EXC_OK;

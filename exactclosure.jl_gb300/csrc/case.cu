@@ -49,6 +49,7 @@ struct LesState {
   // right-hand sides with two more fields to project (LesStage::k)
   T *g[2], *gs, *k;
   long long wstride = 0;  // words between the solver's slots
+  bool batched = false;   // the solver has work for every slot
   T* ub;                  // target at a stage (in gs)
   T *ve[2], *vn[2], *vl[2];  // states of the exact, no-model and learned LES (in g)
   T *mlast, *ublast;      // closure and target at stage 0 of the last step
@@ -283,9 +284,9 @@ static int les_stage(exc_case* cs, CaseImpl<T>* ci, LesState<T>& L, int s, int c
     if (rc) return rc;
   }
   if (e == cudaSuccess) e = launch_les_combine<T>(a, sl);
-  // one batched solve, or one after the other where the grid has the
-  // mixed-precision solve (one work array)
-  const int slots = les_slots(a), each = L.ps.mix ? 1 : slots;
+  // one batched solve, or one after the other where there is one work array
+  // (grids with the mixed-precision solve, and where memory was short)
+  const int slots = les_slots(a), each = L.batched ? slots : 1;
   const T* const p = reinterpret_cast<const T*>(L.ps.work);
   for (int i = 0; i < slots && e == cudaSuccess; i += each) {
     e = poisson_solve_inplace<T>(&L.ps, L.k + 3 * L.M * (1 + i), true, sl, sb, each);
@@ -620,8 +621,9 @@ static int create_les_stream(CaseImpl<T>* ci) {
   return EXC_OK;
 }
 
+// `lean`: without what speeds the solves up at the price of memory
 template <typename T>
-static int case_create(exc_case* cs) {
+static int case_create(exc_case* cs, bool lean) {
   const exc_case_desc& d = cs->desc;
   CaseImpl<T>* ci = new CaseImpl<T>();
   cs->impl = ci;
@@ -630,7 +632,8 @@ static int case_create(exc_case* cs) {
   ci->n = d.n;
   ci->N = (long long)d.n * d.n * d.n;
   ci->h = d.l / d.n;
-  int rc = poisson_init(&ci->ps, cs->precision, d.n, d.l, nullptr, steppers_use_run_time_plans(cs->precision));
+  const bool plans = !lean && steppers_use_run_time_plans(cs->precision);
+  int rc = poisson_init(&ci->ps, cs->precision, d.n, d.l, nullptr, plans);
   if (rc) return rc;
   // the DNS pressure enters only through its gradient (RK stage): its
   // additive constant need not be removed
@@ -658,8 +661,9 @@ static int case_create(exc_case* cs) {
     L.m = d.n / L.c;
     L.M = (long long)L.m * L.m * L.m;
     // a stage projects up to three states, the closure and the next target
-    rc = poisson_init(&L.ps, cs->precision, L.m, d.l, nullptr, steppers_use_run_time_plans(cs->precision), 5);
+    rc = poisson_init(&L.ps, cs->precision, L.m, d.l, nullptr, plans, lean ? 1 : 5);
     if (rc) return rc;
+    L.batched = !lean && !L.ps.mix;
     L.wstride = (long long)L.m * L.m * L.ps.P;
     size_t nb = 22 * 3 * L.M * sizeof(T);
     if (cudaMalloc(&L.buf, nb) != cudaSuccess) { set_last_error("out of device memory (LES fields)"); return EXC_ERR_OOM; }
@@ -1077,7 +1081,12 @@ int exc_case_create(const exc_case_desc* desc, void* stream, exc_case** out) {
     cs->own_stream = true;
   }
   int rc = configure_device();
-  if (rc == EXC_OK) rc = DISPATCH(cs, case_create, cs);
+  if (rc == EXC_OK) rc = DISPATCH(cs, case_create, cs, false);
+  if (rc == EXC_ERR_OOM) {
+    cs->destroy_fn(cs);
+    cudaGetLastError();
+    rc = DISPATCH(cs, case_create, cs, true);
+  }
   if (rc) {
     if (cs->destroy_fn) cs->destroy_fn(cs);
     if (cs->own_stream) cudaStreamDestroy(cs->stream);

@@ -426,27 +426,34 @@ int exc_dnsaid_create(const exc_dnsaid_desc* desc, void* stream, exc_dnsaid** ou
   if (desc->nfdelta > 1 && (!desc->fdelta || desc->nfdelta % 2 == 0)) { set_last_error("fdelta must have odd length"); return EXC_ERR_ARG; }
   int rc = configure_device();
   if (rc) return rc;
-  exc_dnsaid* d = new exc_dnsaid();
-  d->n = n;
-  d->c = c;
-  d->m = n / c;
-  d->l = desc->l;
-  d->visc = desc->visc;
-  d->h = desc->l / n;
-  d->H = desc->l / d->m;
-  if (desc->nfdelta > 1) d->fdelta.assign(desc->fdelta, desc->fdelta + desc->nfdelta);
-  d->st = (cudaStream_t)stream;
-  const size_t N = (size_t)n * n * n, M = (size_t)d->m * d->m * d->m;
+  const size_t N = (size_t)n * n * n, M = (size_t)(n / c) * (n / c) * (n / c);
   const size_t spec = 3ull * n * n * spec_pitch(n) * 2;  // 3 complex spectral arrays, in doubles
-  rc = poisson_init(&d->psd, EXC_F64, n, d->l, nullptr);
-  if (!rc) rc = poisson_init(&d->psl, EXC_F64, d->m, d->l, nullptr);
-  if (!rc) rc = dalloc(&d->u, 3 * N) || dalloc(&d->du, 3 * N) || dalloc(&d->p, N) || dalloc(&d->ub, 3 * M) ||
-                dalloc(&d->tmp, 18 * M) || dalloc(&d->sdh, 6 * M) || dalloc(&d->s2, 6 * M) || dalloc(&d->r9, 9 * M) ||
-                dalloc(&d->zero, M) || dalloc(&d->scal, 16) ||
-                dalloc(&d->part, (size_t)SHELL_BLOCKS * 1024 + 2048 + RED_PARTS) || dalloc(&d->spec, spec);
-  for (int k = 0; k < 5 && !rc; ++k) rc = dalloc(&d->les[k], 3 * M);
-  if (!rc) rc = dalloc(&d->pl, M);
-  if (rc) { exc_dnsaid_destroy(d); return rc; }
+  exc_dnsaid* d = nullptr;
+  // without the run-time plans' memory if there is not enough for them
+  for (const bool plans : {true, false}) {
+    d = new exc_dnsaid();
+    d->n = n;
+    d->c = c;
+    d->m = n / c;
+    d->l = desc->l;
+    d->visc = desc->visc;
+    d->h = desc->l / n;
+    d->H = desc->l / d->m;
+    if (desc->nfdelta > 1) d->fdelta.assign(desc->fdelta, desc->fdelta + desc->nfdelta);
+    d->st = (cudaStream_t)stream;
+    rc = poisson_init(&d->psd, EXC_F64, n, d->l, nullptr, plans);
+    if (!rc) rc = poisson_init(&d->psl, EXC_F64, d->m, d->l, nullptr, plans);
+    if (!rc) rc = dalloc(&d->u, 3 * N) || dalloc(&d->du, 3 * N) || dalloc(&d->p, N) || dalloc(&d->ub, 3 * M) ||
+                  dalloc(&d->tmp, 18 * M) || dalloc(&d->sdh, 6 * M) || dalloc(&d->s2, 6 * M) || dalloc(&d->r9, 9 * M) ||
+                  dalloc(&d->zero, M) || dalloc(&d->scal, 16) ||
+                  dalloc(&d->part, (size_t)SHELL_BLOCKS * 1024 + 2048 + RED_PARTS) || dalloc(&d->spec, spec) ||
+                  dalloc(&d->pl, M);
+    for (int k = 0; k < 5 && !rc; ++k) rc = dalloc(&d->les[k], 3 * M);
+    if (!rc) break;
+    exc_dnsaid_destroy(d);
+    cudaGetLastError();
+  }
+  if (rc) return rc;
   d->dul = d->tmp;
   d->sl = d->tmp + 3 * M;
   d->sc = d->tmp + 9 * M;

@@ -632,7 +632,7 @@ int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bo
     const int rc = precision == EXC_F64 ? alloc_level_tables<double2>(ps, n1, h1) : alloc_level_tables<float2>(ps, n1, h1);
     if (rc) { poisson_free(ps); return rc; }
   }
-  if (precision == EXC_F64 && !work && mix_wanted(n)) {
+  if (precision == EXC_F64 && !work && mix_wanted(n) && (run_time_plans || fftmix_supported(n))) {
     // the mixed-precision solve's FP32 inner solver, with the factor 1/h of
     // the unscaled FP64 divergence folded into its divide table
     ps->mix = new exc_poisson;

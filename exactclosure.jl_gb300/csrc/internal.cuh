@@ -57,7 +57,9 @@ __host__ __device__ __forceinline__ long long invlap_index(int n, int kz, int ky
 
 // Allocate/free the device tables of a solver; `work` may be supplied by the
 // caller (external_work) and is otherwise allocated here.  run_time_plans =
-// false leaves grids without a compiled plan on the Stockham passes.  `slots`:
+// false leaves grids without a compiled plan on the Stockham passes, which in
+// FP64 from 84^3 on take 20 bytes a cell less: handles that memory does not
+// suffice for are made again that way.  `slots`:
 // batched solves the own work array is for (n n P complex words each; a solver
 // with the mixed-precision solve takes one at a time).
 int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bool run_time_plans = true,

@@ -1,30 +1,15 @@
 // Run-time register plans (fftgen.cuh): x passes, float.
-#include "fftgen.cuh"
+#include "fftgenpass.cuh"
 
 namespace exc {
 
-template <>
-void gen_r2c<float>(const GenArgs<float>& a, const GenSrc<float>& s) {
-  using C = cplx<float>;
-  const int n = a.ps->n;
-  chain(gr2c_kernel<float>, dim3((unsigned)((n * n + a.rw - 1) / a.rw), a.nslots), GEN_THREADS, (size_t)a.rw * gen_xs(a.half) * sizeof(C), a.st, CHAIN_BLOCKS_FEW)(
-      s, a.half, n, a.rw, reinterpret_cast<C*>(a.ps->work), a.ps->P, reinterpret_cast<const C*>(a.ps->tw),
-      reinterpret_cast<const C*>(a.ps->twl_h), a.sb);
-}
-
-template <>
-void gen_c2r<float>(const GenArgs<float>& a, const GenDst& d) {
-  using C = cplx<float>;
-  const int n = a.ps->n;
-  chain(gc2r_kernel<float>, dim3((unsigned)((n * n + a.rw - 1) / a.rw), a.nslots), GEN_THREADS, (size_t)a.rw * gen_xs(a.half) * sizeof(C), a.st, CHAIN_BLOCKS_FEW)(
-      reinterpret_cast<C*>(a.ps->work), a.half, n, a.rw, a.ps->P, reinterpret_cast<const C*>(a.ps->tw),
-      reinterpret_cast<const C*>(a.ps->twl_h), d, a.sb);
-}
+template void gen_r2c<float>(const GenArgs<float>&, const GenSrc<float>&);
+template void gen_c2r<float>(const GenArgs<float>&, const GenDst&);
 
 template <>
 cudaError_t configure_gen_x<float>() {
-  cudaError_t e = cudaFuncSetAttribute(gr2c_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEN_SMEM_MAX);
-  return e != cudaSuccess ? e : cudaFuncSetAttribute(gc2r_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEN_SMEM_MAX);
+  const cudaError_t e = gen_opt_in(gr2c_kernel<float>);
+  return e != cudaSuccess ? e : gen_opt_in(gc2r_kernel<float>);
 }
 
 }  // namespace exc

@@ -68,7 +68,6 @@ int closure_flux(int n, int c, double l, double visc, const double* fdelta, int 
                  T* r9, cudaStream_t st);
 template <typename T>
 int filtered_stress(int n, int c, double l, double visc, const double* fdelta, int nfd, const T* u, T* s6,
-                    cudaStream_t st,
-                    const T* p = nullptr);
+                    cudaStream_t st);
 
 }  // namespace exc

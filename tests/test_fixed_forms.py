@@ -2,11 +2,12 @@
 restated in Python integers:
 
 * the FP64 sweep (csrc/rhs.cu): velocities as integers of 57 bits below a power of
-  two, split in halves of 29 bits; stress and divergence in three sums, with a
-  small 2 visc/h outside them.  Every partial sum stays below 2^63, every half
-  in 32 bits, and a component's error against exact rationals is no larger than
-  that of the FP64 arithmetic (test_fp64_forms.shifted_rhs) down to 2^-4 of the
-  scale, where the sweep leaves a weak component to FP64;
+  two, split in halves of 29 bits; stress and divergence in three sums, 2 visc/h
+  outside them where it is far from the velocities.  Every partial sum stays
+  below 2^63, every half in 32 bits, and a component's error against exact
+  rationals is no larger than that of the FP64 arithmetic
+  (test_fp64_forms.shifted_rhs) down to 2^-4 of the scale, where the sweep
+  leaves a weak component to FP64;
 * the Burgers filters (csrc/burgers.cu): sums of 511 taps stay below 2^63, of 3001
   they do not;
 * the box sums (csrc/filter.cu): K values rounded to 58 bits below the largest, off by at
@@ -62,11 +63,13 @@ def to_int(u, e, bits):
 
 def sweep(u, visc, h, bits=57, low=29):
     """du of the fixed-point sweep with the scale of the whole grid, as rationals."""
-    S = 2 * visc / h
-    E = exponent(max(np.abs(u).max() + abs(S), 4 * abs(S)))
-    small = abs(S) < 2.0 ** (E - 6)
+    S, m = 2 * visc / h, np.abs(u).max()
+    E = exponent(m)
+    apart = abs(S) > 2.0 ** (E - 1) or abs(S) < 2.0 ** (E - 6)  # S outside the integers
+    if not apart:
+        E = exponent(max(m + abs(S), 4 * abs(S)))
     U = to_int(u, E, bits)
-    S4 = 0 if small else (round(Fraction(4 * S) * Fraction(2) ** (bits - E)) + 2) >> 2 << 2
+    S4 = 0 if apart else (round(Fraction(4 * S) * Fraction(2) ** (bits - E)) + 2) >> 2 << 2
     S2 = S4 >> 1
     full = lambda v: v + 0 * U[0]
     out = []
@@ -84,13 +87,13 @@ def sweep(u, visc, h, bits=57, low=29):
             s.mac(A, B)
             s.mac(-at(A, j, -1), at(B, j, -1))
             linear = linear - 2 * (A + B - at(A + B, j, -1))
-            if not small:
+            if not apart:
                 s.mac((a - at(a, j, -1)) + (U[j] - at(U[j], j, -1)), full(S4))
-        if not small:
+        if not apart:
             s.mac(2 * (a - at(a, i, -1)), full(S4))
         linear = linear + 4 * group
         unit = Fraction(2) ** (E - bits)
-        r = np.frompyfunc(lambda v, l: -(v * unit * unit + (Fraction(S) * unit * l if small else 0)) / (4 * Fraction(h)), 2, 1)
+        r = np.frompyfunc(lambda v, l: -(v * unit * unit + (Fraction(S) * unit * l if apart else 0)) / (4 * Fraction(h)), 2, 1)
         out.append(r(s.value(), linear))
     return np.array(out)
 
@@ -145,7 +148,7 @@ def test_sweep_sums_at_their_largest():
     for s in range(8):
         u = np.array([(-1.0) ** (((s >> c) & 1) + np.indices((4, 4, 4)).sum(axis=0) * (c != s % 3)) for c in range(3)])
         u *= 1 - 2.0**-40
-        for visc in (0.0, 0.124 / 4, -0.124 / 4):
+        for visc in (0.0, 0.06, -0.06, 0.002, 1.0):
             sweep(u, visc, 0.25)
 
 

@@ -431,9 +431,11 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
 // planes with values that are not finite or out of range.
 //
 // Per cell 650 instructions, 88 of them the multiply-adds, 57 shared-memory
-// accesses per 32 cells and 6 FP64 operations (45 before).  512^3: 11.4 -> 3.46
-// ms (HBM floor 0.95), 250^3 1470 -> 492 us, 128^3 215 -> 80, 90^3 102 -> 41,
-// 32^3 47 -> 10.  Bound by the latency of the multiply-add pipe (66% busy) at 8
+// accesses per 32 cells and 6 FP64 operations (45 before).  512^3: 11.4 -> 3.72
+// ms (HBM floor 0.95), 250^3 1470 -> 530 us, 128^3 215 -> 86, 90^3 102 -> 46,
+// 32^3 47 -> 14; with the linear term by itself 4.53 ms, 627, 99, 51 and 15 us; with
+// a third component weak everywhere 15.1 ms, 2.02, 0.29, 0.13 and 0.02 (its cells
+// share nothing).  Bound by the latency of the multiply-add pipe (66% busy) at 8
 // warps per scheduler.  Error against 113-bit arithmetic, relative L2: white
 // noise 0.7-1.1e-16 (FP64 form 1.7-2.1e-16), smooth fields 0.8e-16 (1.2e-15), a
 // mean flow of 100 7e-17 (1.3e-14), visc 0.1 1.4e-16 (7.7e-16).
@@ -473,7 +475,8 @@ __device__ __noinline__ double rhs_cell_f64(const double* __restrict__ u, int n,
 }
 
 // Tile of the fixed-point sweep: 32 x 16 cells, FXC rows per thread, FX_CTAS
-// CTAs per SM (64 registers).  512^3 / 250^3 / 128^3 / 32^3: 3.43 ms / 488 / 78
+// CTAs per SM (64 registers).  512^3 / 250^3 / 128^3 / 32^3, before the weak
+// components and the viscous term had paths of their own: 3.43 ms / 488 / 78
 // / 10 us; three CTAs (80 registers) 3.75 / 497 / 84 / 10; one row per thread 5.3
 // ms / 701 / 108 / 10 (every shared value loaded once per cell); four rows, five
 // CTAs 3.27 ms / 462 / 88 / 12: the larger tile of work per thread loses on the
@@ -734,6 +737,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     start(z);
   };
   start(z0);
+  int walked = 0;  // planes of the block behind
   const int gx = x0 + tx;
   for (int kz = 0; kz < ptz; ++kz) {
     const int z = z0 + kz;
@@ -841,6 +845,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     else cells(std::false_type());
     if (!more) break;
     if (slow) {
+      if (++walked == block) walked = 0;
       restart(z + 1);
       continue;
     }
@@ -849,12 +854,14 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     __syncthreads();
     const unsigned m[3] = {held_max(0), held_max(1), held_max(2)};
     const unsigned mx = max(m[0], max(m[1], m[2]));
-    bool out;
-    const int Ef = fresh(mx, out);
-    const int En = out == s_out ? Ef : exponent_for(mx, s_out);
-    // a block starts with its own scale
-    const bool other = (kz + 1) % block == 0 ? Ef != E || out != s_out : En < E - 2;
-    if (mx >= 0x7fe00000u || En > E || other) {
+    const int En = exponent_for(mx, s_out);
+    bool other = En > E || En < E - 2;
+    if (++walked == block) {  // a block starts with its own scale
+      bool out;
+      walked = 0;
+      other = fresh(mx, out) != E || out != s_out;
+    }
+    if (mx >= 0x7fe00000u || other) {
       restart(z + 1);
       continue;
     }

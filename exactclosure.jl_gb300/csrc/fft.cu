@@ -525,29 +525,40 @@ cudaError_t configure_fft() {
   return e;
 }
 
-// Level twiddles of a length-L register plan with first factor N1:
-// tl[k1 N2 + m2] = W_L^(m2 k1), from long double.
-template <typename C>
-static std::vector<C> level_table(int L, int N1) {
-  const int N2 = L / N1;
-  std::vector<C> t((size_t)L);
-  const long double pi_l = 3.141592653589793238462643383279502884L;
-  for (int k1 = 0; k1 < N1; ++k1)
-    for (int m2 = 0; m2 < N2; ++m2) {
-      const long double a = -2.0L * pi_l * (long double)((m2 * k1) % L) / (long double)L;
-      C w;
-      w.x = (decltype(w.x))cosl(a);
-      w.y = (decltype(w.y))sinl(a);
-      t[(size_t)k1 * N2 + m2] = w;
+// Twiddles W_n^m and sin^2(pi m / n), from long double on the host (software on Arm:
+// once for a solver, its level tables and its mixed solve).
+struct Tables {
+  std::vector<double2> d;
+  std::vector<float2> f;
+  std::vector<double> sin2;
+  explicit Tables(int n) : d(n), f(n), sin2(n) {
+    const long double pi_l = 3.141592653589793238462643383279502884L;
+    for (int m = 0; m < n; ++m) {
+      const long double a = -2.0L * pi_l * (long double)m / (long double)n;
+      const long double c = cosl(a), s = sinl(a);
+      d[m] = make_double2((double)c, (double)s);
+      f[m] = make_float2((float)c, (float)s);
+      const long double sn = sinl(pi_l * (long double)std::min(m, n - m) / (long double)n);
+      sin2[m] = (double)(sn * sn);  // mirrored: sin2[n - m] == sin2[m]
     }
+  }
+};
+
+// Level twiddles W_L^(m2 k1) laid out [k1][m2] of a register plan for L = n / part,
+// from the table of W_n.
+template <typename C>
+static std::vector<C> level_table(const std::vector<C>& tw, int part, int N1) {
+  const int L = (int)tw.size() / part, N2 = L / N1;
+  std::vector<C> t((size_t)L);
+  for (int k1 = 0; k1 < N1; ++k1)
+    for (int m2 = 0; m2 < N2; ++m2) t[(size_t)k1 * N2 + m2] = tw[(size_t)part * ((m2 * k1) % L)];
   return t;
 }
 
 template <typename C>
-static int alloc_level_tables(exc_poisson* ps, int n1, int h1) {
-  const int n = ps->n;
-  const std::vector<C> tn = level_table<C>(n, n1);
-  const std::vector<C> th = level_table<C>(n / 2, h1);
+static int alloc_level_tables(exc_poisson* ps, const std::vector<C>& tw, int n1, int h1) {
+  const std::vector<C> tn = level_table(tw, 1, n1);
+  const std::vector<C> th = level_table(tw, 2, h1);
   if (cudaMalloc(&ps->twl_n, tn.size() * sizeof(C)) != cudaSuccess ||
       cudaMalloc(&ps->twl_h, th.size() * sizeof(C)) != cudaSuccess) {
     set_last_error("out of device memory (poisson level twiddles)");
@@ -575,10 +586,8 @@ static long long mix_part_words(int n) {
                              : std::max(gen_mix_parts(n), (long long)MIX_SUM_CTAS) + 2 + gen_mix_parts(n) / 2 + 1;
 }
 
-int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bool run_time_plans, int slots) {
-  if (!fft_size_ok(n)) { set_last_error("grid size must be 2^a 3^b 5^c 7^d 11^e 13^f 17^g, a >= 1, 4 <= n <= 1024"); return EXC_ERR_SHAPE; }
-  if (!(l > 0)) { set_last_error("domain size must be positive"); return EXC_ERR_ARG; }
-  if (precision != EXC_F64 && precision != EXC_F32) { set_last_error("bad precision"); return EXC_ERR_ARG; }
+static int init_with(exc_poisson* ps, const Tables& tables, int precision, int n, double l, void* work,
+                     bool run_time_plans, int slots) {
   ps->precision = precision;
   ps->n = n;
   ps->l = l;
@@ -589,27 +598,14 @@ int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bo
   size_t csz = precision == EXC_F64 ? sizeof(double2) : sizeof(float2);
   int crc = configure_device();
   if (crc) return crc;
-  // twiddles W_n^m and sin^2 table, from long double on the host
-  std::vector<double2> twd(n);
-  std::vector<float2> twf(n);
-  std::vector<double> s2(n);
-  const long double pi_l = 3.141592653589793238462643383279502884L;
-  for (int m = 0; m < n; ++m) {
-    long double a = -2.0L * pi_l * (long double)m / (long double)n;
-    double c = (double)cosl(a), s = (double)sinl(a);
-    twd[m] = make_double2(c, s);
-    twf[m] = make_float2((float)cosl(a), (float)sinl(a));
-    long double sn = sinl(pi_l * (long double)std::min(m, n - m) / (long double)n);
-    s2[m] = (double)(sn * sn);  // mirrored: s2[n - m] == s2[m]
-  }
   if (cudaMalloc(&ps->tw, n * csz) != cudaSuccess || cudaMalloc(&ps->sin2, n * sizeof(double)) != cudaSuccess) {
     set_last_error("out of device memory (poisson tables)");
     poisson_free(ps);
     return EXC_ERR_OOM;
   }
-  cudaMemcpy(ps->tw, precision == EXC_F64 ? (const void*)twd.data() : (const void*)twf.data(), n * csz,
+  cudaMemcpy(ps->tw, precision == EXC_F64 ? (const void*)tables.d.data() : (const void*)tables.f.data(), n * csz,
              cudaMemcpyHostToDevice);
-  cudaMemcpy(ps->sin2, s2.data(), n * sizeof(double), cudaMemcpyHostToDevice);
+  cudaMemcpy(ps->sin2, tables.sin2.data(), n * sizeof(double), cudaMemcpyHostToDevice);
   {
     // 1/(lambda N) per mode with ky, kz folded to <= n/2 (lambda is even in
     // each wavenumber), from an exact float64 division
@@ -629,28 +625,31 @@ int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bo
   if (ps->gen || fftreg_supported(n, precision)) {
     int n1 = reg_split_host(n), h1 = reg_split_host(n / 2);
     if (ps->gen) gen_splits(n, precision, &n1, &h1);
-    const int rc = precision == EXC_F64 ? alloc_level_tables<double2>(ps, n1, h1) : alloc_level_tables<float2>(ps, n1, h1);
+    const int rc = precision == EXC_F64 ? alloc_level_tables(ps, tables.d, n1, h1) : alloc_level_tables(ps, tables.f, n1, h1);
     if (rc) { poisson_free(ps); return rc; }
   }
   if (precision == EXC_F64 && !work && mix_wanted(n) && (run_time_plans || fftmix_supported(n))) {
     // the mixed-precision solve's FP32 inner solver, with the factor 1/h of
     // the unscaled FP64 divergence folded into its divide table
     ps->mix = new exc_poisson;
-    int rc = poisson_init(ps->mix, EXC_F32, n, l, nullptr);
+    int rc = init_with(ps->mix, tables, EXC_F32, n, l, nullptr, true, 1);
     if (rc) { poisson_free(ps); return rc; }
     const long long tot = (long long)(n / 2 + 1) * (n / 2 + 1) * (n / 2 + 1);
     const double coef_mix = -ps->h / (4.0 * (double)n * (double)n * (double)n);
     const int blocks = (int)std::min<long long>((tot + 255) / 256, 152LL * 32);
     invlap_kernel<<<blocks, 256>>>(n, ps->mix->sin2, coef_mix, ps->mix->invlap);
     invlap_split_kernel<<<blocks, 256>>>(tot, ps->mix->invlap);
-    if (cudaMalloc(&ps->mix_d, (size_t)n * n * n * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&ps->mix_q, (size_t)n * n * n * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&ps->mix_q2, (size_t)n * n * n * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&ps->mix_part, (size_t)mix_part_words(n) * sizeof(double)) != cudaSuccess) {
+    // one allocation: d, the two corrections, the partial sums (n is even, so each
+    // starts on a 64-byte boundary)
+    const size_t N = (size_t)n * n * n;
+    if (cudaMalloc(&ps->mix_d, (2 * N + (size_t)mix_part_words(n)) * sizeof(double)) != cudaSuccess) {
       set_last_error("out of device memory (mixed-precision poisson buffers)");
       poisson_free(ps);
       return EXC_ERR_OOM;
     }
+    ps->mix_q = reinterpret_cast<float*>(ps->mix_d + N);
+    ps->mix_q2 = ps->mix_q + N;
+    ps->mix_part = ps->mix_d + 2 * N;
   }
   size_t wbytes = (size_t)n * n * ps->P * csz * (ps->mix ? 1 : slots);
   if (work) {
@@ -669,6 +668,13 @@ int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bo
   return EXC_OK;
 }
 
+int poisson_init(exc_poisson* ps, int precision, int n, double l, void* work, bool run_time_plans, int slots) {
+  if (!fft_size_ok(n)) { set_last_error("grid size must be 2^a 3^b 5^c 7^d 11^e 13^f 17^g, a >= 1, 4 <= n <= 1024"); return EXC_ERR_SHAPE; }
+  if (!(l > 0)) { set_last_error("domain size must be positive"); return EXC_ERR_ARG; }
+  if (precision != EXC_F64 && precision != EXC_F32) { set_last_error("bad precision"); return EXC_ERR_ARG; }
+  return init_with(ps, Tables(n), precision, n, l, work, run_time_plans, slots);
+}
+
 void poisson_free(exc_poisson* ps) {
   if (ps->mix) {
     poisson_free(ps->mix);
@@ -676,9 +682,6 @@ void poisson_free(exc_poisson* ps) {
     ps->mix = nullptr;
   }
   if (ps->mix_d) cudaFree(ps->mix_d);
-  if (ps->mix_q) cudaFree(ps->mix_q);
-  if (ps->mix_q2) cudaFree(ps->mix_q2);
-  if (ps->mix_part) cudaFree(ps->mix_part);
   ps->mix_d = ps->mix_part = nullptr;
   ps->mix_q = ps->mix_q2 = nullptr;
   if (ps->tw) cudaFree(ps->tw);

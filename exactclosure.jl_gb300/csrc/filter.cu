@@ -332,7 +332,8 @@ __device__ __forceinline__ double sum_fixed(const double (&v)[K]) {
 // Per pass over the fine field: FP64 512^3 ratio 4 0.80 -> 0.49 ms (HBM; the FP64
 // additions alone took 0.69), 128^3 19.5 -> 13.2 us, 90^3 ratios 3 and 5 10.6 and
 // 10.9 -> 7.4; FP32 128^3 ratio 4 10.8 -> 8.0, 72^3 ratio 3 6.9 -> 4.6.  Four values
-// (ratio 2) stay on the FP64 pipe.
+// (ratio 2) stay on the FP64 pipe.  From ratio 6 on a sum has more than the 31
+// values that sum_fixed's integers hold, so those ratios keep the loops.
 template <typename T, int C>
 __global__ void tb_kernel(const T* __restrict__ f3, int n, int ratio, T* __restrict__ tb3) {
   const int c = C ? C : ratio;

@@ -121,7 +121,10 @@ int exc_debug_wait_drill(int flags);
  * without run-time plans), shared-memory Stockham passes for the rest.  1 =
  * FP64/FP32 Stockham passes for every grid.  2 = register passes where
  * planned, else Stockham, in the solver's own precision throughout.  Results
- * agree to round-off; the autotuner of the serving form picks per grid. */
+ * agree to round-off; the autotuner of the serving form picks per grid.
+ * A field that starts at an odd word takes the Stockham passes whatever the
+ * engine, and a handle (solver, case, Euler driver) for which the device's
+ * memory does not suffice otherwise is made without run-time plans. */
 int exc_poisson_set_engine(exc_poisson* ps, int engine);
 /* p with L_h p = d, mean(p) = 0 (src/N.jl:262-301).  d and p may alias. */
 int exc_poisson_solve(exc_poisson* ps, const void* d, void* p, void* stream);

@@ -431,11 +431,11 @@ rhs_kernel(int n, T inv_h, T visc, const T* __restrict__ u, T* __restrict__ du, 
 // planes with values that are not finite or out of range.
 //
 // Per cell 650 instructions, 88 of them the multiply-adds, 57 shared-memory
-// accesses per 32 cells and 6 FP64 operations (45 before).  512^3: 11.4 -> 3.72
-// ms (HBM floor 0.95), 250^3 1470 -> 530 us, 128^3 215 -> 86, 90^3 102 -> 46,
-// 32^3 47 -> 14; with the linear term by itself 4.53 ms, 627, 99, 51 and 15 us; with
-// a third component weak everywhere 15.1 ms, 2.02, 0.29, 0.13 and 0.02 (its cells
-// share nothing).  Bound by the latency of the multiply-add pipe (66% busy) at 8
+// accesses per 32 cells and 6 FP64 operations (45 before).  512^3: 11.4 -> 3.64
+// ms (HBM floor 0.95), 250^3 1470 -> 518 us, 128^3 215 -> 85, 90^3 102 -> 46,
+// 32^3 47 -> 14; with the linear term by itself 4.14 ms, 579, 93, 48 and 15 us; with
+// a third component weak everywhere 11.2 ms, 1560, 236, 108 and 20 (its cells share
+// nothing).  Bound by the latency of the multiply-add pipe (66% busy) at 8
 // warps per scheduler.  Error against 113-bit arithmetic, relative L2: white
 // noise 0.7-1.1e-16 (FP64 form 1.7-2.1e-16), smooth fields 0.8e-16 (1.2e-15), a
 // mean flow of 100 7e-17 (1.3e-14), visc 0.1 1.4e-16 (7.7e-16).
@@ -446,9 +446,11 @@ constexpr int FX_BITS = 57, FX_LOW = 29;
 constexpr int FX_EMIN = -100, FX_EMAX = FX_BITS;
 constexpr int FX_WEAK = 4, FX_SMALL_S = 6;
 
-// The reference's arithmetic for component I of one cell, from global memory:
-// what the fixed-point sweep leaves out.
-template <int I>
+// Component I of one cell in FP64, from global memory: what the fixed-point sweep
+// leaves out.  WEAK: a weak component, whose S is small beside the velocities: the
+// products as differences of sums and the viscous term of the sums at hand (31 FP64
+// operations); else the reference's arithmetic (42).
+template <int I, bool WEAK>
 __device__ __noinline__ double rhs_cell_f64(const double* __restrict__ u, int n, int x, int y, int z, double inv_h,
                                             double visc) {
   constexpr int J = I == 0 ? 1 : 0, K = I == 2 ? 1 : 2;
@@ -464,13 +466,26 @@ __device__ __noinline__ double rhs_cell_f64(const double* __restrict__ u, int n,
   const double p0 = p[0], piu = p[iu], pid = p[id], pju = p[ju], pjd = p[jd], pku = p[ku], pkd = p[kd];
   const double q0 = q[0], qiu = q[iu], qjd = q[jd], qjdiu = q[jd + iu];
   const double r0 = r[0], riu = r[iu], rkd = r[kd], rkdiu = r[kd + iu];
-  const double rv = 4.0 * visc * inv_h;
-  auto diag = [rv](double a, double b) { return (a + b) * (a + b) - 2.0 * rv * (a - b); };
-  auto off = [rv](double a, double b, double c, double d) { return (a + b) * (c + d) - rv * ((b - a) + (d - c)); };
-  const double di = diag(piu, p0) - diag(p0, pid);
-  const double dj = off(p0, pju, q0, qiu) - off(pjd, p0, qjd, qjdiu);
-  const double dk = off(p0, pku, r0, riu) - off(pkd, p0, rkd, rkdiu);
-  const double sum = I == 2 ? (dj + dk) + di : (di + dj) + dk;
+  double sum;
+  if constexpr (WEAK) {
+    const double t = fma(2.0, p0, piu + pid), aj = p0 + pju, bj = p0 + pjd, ak = p0 + pku, bk = p0 + pkd;
+    sum = (piu - pid) * t;
+    sum = fma(aj, q0 + qiu, sum);
+    sum = fma(-bj, qjd + qjdiu, sum);
+    sum = fma(ak, r0 + riu, sum);
+    sum = fma(-bk, rkd + rkdiu, sum);
+    const double lin = fma(-16.0, p0, fma(2.0, t, (aj + bj) + (ak + bk))) + ((qiu - q0) - (qjdiu - qjd)) +
+                       ((riu - r0) - (rkdiu - rkd));
+    sum = fma(-4.0 * visc * inv_h, lin, sum);
+  } else {
+    const double rv = 4.0 * visc * inv_h;
+    auto diag = [rv](double a, double b) { return (a + b) * (a + b) - 2.0 * rv * (a - b); };
+    auto off = [rv](double a, double b, double c, double d) { return (a + b) * (c + d) - rv * ((b - a) + (d - c)); };
+    const double di = diag(piu, p0) - diag(p0, pid);
+    const double dj = off(p0, pju, q0, qiu) - off(pjd, p0, qjd, qjdiu);
+    const double dk = off(p0, pku, r0, riu) - off(pkd, p0, rkd, rkdiu);
+    sum = I == 2 ? (dj + dk) + di : (di + dj) + dk;
+  }
   return -0.25 * inv_h * sum;
 }
 
@@ -702,6 +717,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
     const unsigned mx = max(m[0], max(m[1], m[2]));
     const double S = 2.0 * visc * inv_h;
     E = fresh(mx, s_out);
+    weak = 0;
     slow = mx >= 0x7fe00000u || !(fabs(S) < 1e300) || E > FX_EMAX || E < FX_EMIN;
     if (!slow) {
       kexp = (FX_BITS - E) << 20;
@@ -751,8 +767,8 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
       for (int i = 0; i < NC; ++i) {
         const int r = NC * ty + 1 + i, gy = y0 + NC * ty + i;
         const Fx a = fxat(cur, 0, r, col), b = fxat(cur, 1, r, col), c = fxat(cur, 2, r, col);
-        double o1, o2, o3;
-        const int direct = slow || max(abs(a.h), max(abs(b.h), abs(c.h))) < tiny ? 7 : weak;
+        double o1 = 0, o2 = 0, o3 = 0;
+        const bool direct = slow || max(abs(a.h), max(abs(b.h), abs(c.h))) < tiny;
         if (!slow) {
           // u1: neighbours along x, y, z and (-x, +y), (-x, +z)
           const Fx axp = fxat(cur, 0, r, col + 1), axm = fxat(cur, 0, r, col - 1);
@@ -775,7 +791,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
           const Fx A12 = a + ayp - s2, B12 = b + bxp - s2;
           const Fx A13 = a + azp - s2, B13 = c + cxp - s2;
           const Fx A23 = b + bzp - s2, B23 = c + cyp - s2;
-          {
+          if (!S_OUT || !(weak & 1)) {
             FxSum s = s0;
             fx_mac(s, dz3 + (a - axm), s4);
             fx_mac(s, (a - aym) + (a - pw1[i]), s4);
@@ -789,7 +805,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
               o1 = fma(sm.by_s, linear((a - axm) + (b - bym), dz3 + (a - axm), (a - aym) + (a - pw1[i]), axp - axm,
                        (ayp - aym) + (b + bxp) - (bym + bxpym), (azp - pw1[i]) + (c + cxp) - (pb13[i] + s2)), o1);
           }
-          {
+          if (!S_OUT || !(weak & 2)) {
             FxSum s = s0;
             fx_mac(s, dz3 + (b - bxm), s4);
             fx_mac(s, (b - bym) + (b - pw2[i]), s4);
@@ -803,7 +819,7 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
               o2 = fma(sm.by_s, linear((a - axm) + (b - bym), dz3 + (b - bxm), (b - bym) + (b - pw2[i]), byp - bym,
                        (a + ayp) - (axm + axmyp) + (bxp - bxm), (bzp - pw2[i]) + (c + cyp) - (pb23[i] + s2)), o2);
           }
-          {
+          if (!S_OUT || !(weak & 4)) {
             FxSum s = s0;
             fx_mac(s, dz3 + (c - cxm), s4);
             fx_mac(s, (c - cym) + dz3, s4);
@@ -824,9 +840,14 @@ rhs_fixed_kernel(int n, double inv_h, double visc, const double* __restrict__ u,
           pb23[i] = B23;
         }
         if (gx < n && gy < n) {
-          if (direct & 1) o1 = rhs_cell_f64<0>(u, n, gx, gy, z, inv_h, visc);
-          if (direct & 2) o2 = rhs_cell_f64<1>(u, n, gx, gy, z, inv_h, visc);
-          if (direct & 4) o3 = rhs_cell_f64<2>(u, n, gx, gy, z, inv_h, visc);
+          if (weak & 1) o1 = rhs_cell_f64<0, true>(u, n, gx, gy, z, inv_h, visc);
+          if (weak & 2) o2 = rhs_cell_f64<1, true>(u, n, gx, gy, z, inv_h, visc);
+          if (weak & 4) o3 = rhs_cell_f64<2, true>(u, n, gx, gy, z, inv_h, visc);
+          if (direct) {
+            o1 = rhs_cell_f64<0, false>(u, n, gx, gy, z, inv_h, visc);
+            o2 = rhs_cell_f64<1, false>(u, n, gx, gy, z, inv_h, visc);
+            o3 = rhs_cell_f64<2, false>(u, n, gx, gy, z, inv_h, visc);
+          }
           double* const d = du + ((long long)z * n + gy) * n + gx;
           if (DOADD) {
             d[0] += o1;

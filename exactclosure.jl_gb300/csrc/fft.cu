@@ -3,6 +3,7 @@
 // and inverse z transforms, then C2R along x back into the work array.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "internal.cuh"
@@ -555,18 +556,31 @@ static std::vector<C> level_table(const std::vector<C>& tw, int part, int N1) {
   return t;
 }
 
+// The device tables of a solver in one allocation and one copy: W_n, with a register
+// plan its level twiddles for L = n and L = n / 2, sin^2.
 template <typename C>
-static int alloc_level_tables(exc_poisson* ps, const std::vector<C>& tw, int n1, int h1) {
-  const std::vector<C> tn = level_table(tw, 1, n1);
-  const std::vector<C> th = level_table(tw, 2, h1);
-  if (cudaMalloc(&ps->twl_n, tn.size() * sizeof(C)) != cudaSuccess ||
-      cudaMalloc(&ps->twl_h, th.size() * sizeof(C)) != cudaSuccess) {
-    set_last_error("out of device memory (poisson level twiddles)");
-    return EXC_ERR_OOM;
+static bool upload_tables(exc_poisson* ps, const std::vector<C>& tw, const std::vector<double>& sin2, bool plan) {
+  const int n = ps->n;
+  std::vector<C> all(tw);
+  if (plan) {
+    int n1 = reg_split_host(n), h1 = reg_split_host(n / 2);
+    if (ps->gen) gen_splits(n, ps->precision, &n1, &h1);
+    const std::vector<C> a = level_table(tw, 1, n1), b = level_table(tw, 2, h1);
+    all.insert(all.end(), a.begin(), a.end());
+    all.insert(all.end(), b.begin(), b.end());
   }
-  cudaMemcpy(ps->twl_n, tn.data(), tn.size() * sizeof(C), cudaMemcpyHostToDevice);
-  cudaMemcpy(ps->twl_h, th.data(), th.size() * sizeof(C), cudaMemcpyHostToDevice);
-  return EXC_OK;
+  const size_t bytes = all.size() * sizeof(C);
+  std::vector<char> host(bytes + n * sizeof(double));
+  std::memcpy(host.data(), all.data(), bytes);
+  std::memcpy(host.data() + bytes, sin2.data(), n * sizeof(double));
+  if (cudaMalloc(&ps->tw, host.size()) != cudaSuccess) return false;
+  cudaMemcpy(ps->tw, host.data(), host.size(), cudaMemcpyHostToDevice);
+  if (plan) {
+    ps->twl_n = reinterpret_cast<C*>(ps->tw) + n;
+    ps->twl_h = reinterpret_cast<C*>(ps->tw) + 2 * n;
+  }
+  ps->sin2 = reinterpret_cast<double*>(reinterpret_cast<char*>(ps->tw) + bytes);
+  return true;
 }
 
 // FP64 grids that solve by mixed-precision refinement: those with a compiled
@@ -598,14 +612,14 @@ static int init_with(exc_poisson* ps, const Tables& tables, int precision, int n
   size_t csz = precision == EXC_F64 ? sizeof(double2) : sizeof(float2);
   int crc = configure_device();
   if (crc) return crc;
-  if (cudaMalloc(&ps->tw, n * csz) != cudaSuccess || cudaMalloc(&ps->sin2, n * sizeof(double)) != cudaSuccess) {
+  const bool compiled = fftreg_supported(n, precision);
+  ps->gen = run_time_plans && !compiled && gen_supported(n, precision);
+  if (!(precision == EXC_F64 ? upload_tables(ps, tables.d, tables.sin2, ps->gen || compiled)
+                             : upload_tables(ps, tables.f, tables.sin2, ps->gen || compiled))) {
     set_last_error("out of device memory (poisson tables)");
     poisson_free(ps);
     return EXC_ERR_OOM;
   }
-  cudaMemcpy(ps->tw, precision == EXC_F64 ? (const void*)tables.d.data() : (const void*)tables.f.data(), n * csz,
-             cudaMemcpyHostToDevice);
-  cudaMemcpy(ps->sin2, tables.sin2.data(), n * sizeof(double), cudaMemcpyHostToDevice);
   {
     // 1/(lambda N) per mode with ky, kz folded to <= n/2 (lambda is even in
     // each wavenumber), from an exact float64 division
@@ -620,13 +634,6 @@ static int init_with(exc_poisson* ps, const Tables& tables, int precision, int n
     invlap_kernel<<<(int)std::min<long long>((tot + 255) / 256, 152LL * 32), 256>>>(n, ps->sin2, coef, ps->invlap);
     if (precision == EXC_F32)
       invlap_split_kernel<<<(int)std::min<long long>((tot + 255) / 256, 152LL * 32), 256>>>(tot, ps->invlap);
-  }
-  ps->gen = run_time_plans && !fftreg_supported(n, precision) && gen_supported(n, precision);
-  if (ps->gen || fftreg_supported(n, precision)) {
-    int n1 = reg_split_host(n), h1 = reg_split_host(n / 2);
-    if (ps->gen) gen_splits(n, precision, &n1, &h1);
-    const int rc = precision == EXC_F64 ? alloc_level_tables(ps, tables.d, n1, h1) : alloc_level_tables(ps, tables.f, n1, h1);
-    if (rc) { poisson_free(ps); return rc; }
   }
   if (precision == EXC_F64 && !work && mix_wanted(n) && (run_time_plans || fftmix_supported(n))) {
     // the mixed-precision solve's FP32 inner solver, with the factor 1/h of
@@ -684,12 +691,9 @@ void poisson_free(exc_poisson* ps) {
   if (ps->mix_d) cudaFree(ps->mix_d);
   ps->mix_d = ps->mix_part = nullptr;
   ps->mix_q = ps->mix_q2 = nullptr;
-  if (ps->tw) cudaFree(ps->tw);
-  if (ps->sin2) cudaFree(ps->sin2);
+  if (ps->tw) cudaFree(ps->tw);  // with sin2 and the level twiddles
   if (ps->invlap) cudaFree(ps->invlap);
   ps->invlap = nullptr;
-  if (ps->twl_n) cudaFree(ps->twl_n);
-  if (ps->twl_h) cudaFree(ps->twl_h);
   ps->twl_n = ps->twl_h = nullptr;
   if (ps->work && !ps->external_work) cudaFree(ps->work);
   ps->tw = nullptr;
